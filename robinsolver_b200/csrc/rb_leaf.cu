@@ -1,4 +1,4 @@
-// rb_leaf.cu -- structured leaf factor and leaf solve for sm_100a (one CTA per leaf).
+// rb_leaf.cu -- structured leaf factor and leaf solve for sm_100a.
 //
 // Leaf algebra.  The reference's leaf matrix A (FD_matrix_row, fd_module.f90:104-224) has its rows/
 // columns in lin2fgrid order: the nb = 2(a+b) cornerless boundary points first (faces
@@ -36,6 +36,7 @@
 //     f_r = 2 i kb / d_r.
 // The leaf solve applies A^-1 [g; f] (fd_leaf_solve + fd_leaf_update, fd_module.f90:390-566)
 // through the same block factors: t = f - A_ib A_bb^-1 g, S u_i = t, u_b = (g - A_bi u_i)/d.
+#include <algorithm>
 #include <cstdlib>
 #include <cstring>
 #include "rb_gemm_dmma.cuh"   // dmma884
@@ -289,493 +290,435 @@ __global__ void __launch_bounds__(256) leaf_block_factor_kernel(LeafGeom g, cons
     if (!ok && tid == 0) atomicOr(status, 1);
 }
 
-// ---------------------------------------------------------------------------------------------------
-// Warp-per-leaf factor for a = 16 (every leaf of a 16x16 grid): the same algebra as
-// leaf_block_factor_kernel with no block barriers.  A 16x16 block lives in registers, lane l
-// holding row l%16, columns 8*(l/16)..+7; Gauss-Jordan pivots by shuffles (|re|+|im|, first
-// maximum) and the column exchanges are undone through the warp's shared memory.  In the
-// S^T Z = C^T sweeps each lane carries one right-hand side (a 16-vector per block) at a time.
-__global__ void __launch_bounds__(128) leaf_warp_factor_kernel(LeafGeom g, int nleaves, const double* __restrict__ hh,
-                                                               const z* __restrict__ kv, z* __restrict__ sinv,
-                                                               z* __restrict__ Y, int* status) {
-    constexpr int A = 16, AA = 256;
-    __shared__ z wsm[4][AA];
-    __shared__ int wpiv[4][2 * A];
-    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    const int leaf = blockIdx.x * 4 + wib;
-    if (leaf >= nleaves) return;
-    z* sm = wsm[wib];
-    int* piv = wpiv[wib];
-    const int b = g.b, nb = g.nb, n = g.n, ab = A * b;
-    const LeafConst L = leaf_const(hh, leaf, g.kb);
-    const z* kl = kv + (size_t)leaf * ab;
-    z* Sl = sinv + (size_t)leaf * b * AA;
-    z* Yl = Y + (size_t)leaf * nb * n;
-    const int r = lane & 15, hf = lane >> 4;          // row, column half
-    z a[8], prev[8];
-    bool ok = true;
-
-    // ---- block LU ---------------------------------------------------------------------------------
-    for (int j = 0; j < b; ++j) {
-        const int jj = j + 1;
-        const z lm = jj > 1 ? zmul(block_lo(L, b, jj), block_up(L, b, jj - 1)) : zmk(0.0, 0.0);
-        const z kr = kl[j * A + r];
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-            z v = block_d(L, A, b, jj, r, hf * 8 + e, kr);
-            if (jj > 1) zfms(v, lm, prev[e]);
-            a[e] = v;
-        }
-#pragma unroll
-        for (int k = 0; k < A; ++k) {
-            const int hk = k >> 3, ek = k & 7;
-            double mag = (hf == hk && r >= k) ? zabs1(a[ek]) : -1.0;
-            int idx = r;
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                const double om = __shfl_xor_sync(0xffffffffu, mag, o);
-                const int oi = __shfl_xor_sync(0xffffffffu, idx, o);
-                if (om > mag || (om == mag && oi < idx)) { mag = om; idx = oi; }
-            }
-            const int p = idx;
-            if (lane == 0) piv[k] = p;
-            if (p != k) {                           // exchange rows k and p
-                const int src = (r == k ? p : (r == p ? k : r)) + 16 * hf;
-#pragma unroll
-                for (int e = 0; e < 8; ++e) {
-                    const double x = __shfl_sync(0xffffffffu, a[e].x, src);
-                    const double y = __shfl_sync(0xffffffffu, a[e].y, src);
-                    a[e] = zmk(x, y);
-                }
-            }
-            const z pv = zmk(__shfl_sync(0xffffffffu, a[ek].x, k + 16 * hk),
-                             __shfl_sync(0xffffffffu, a[ek].y, k + 16 * hk));
-            if (pv.x == 0.0 && pv.y == 0.0) ok = false;
-            const z pinv = zrcp(pv);
-            const z f = zmk(__shfl_sync(0xffffffffu, a[ek].x, r + 16 * hk),
-                            __shfl_sync(0xffffffffu, a[ek].y, r + 16 * hk));
-#pragma unroll
-            for (int e = 0; e < 8; ++e) {
-                const z pr = zmul(zmk(__shfl_sync(0xffffffffu, a[e].x, k + 16 * hf),
-                                      __shfl_sync(0xffffffffu, a[e].y, k + 16 * hf)), pinv);
-                const bool colk = (hf == hk) && (e == ek);
-                if (r == k) a[e] = colk ? pinv : pr;
-                else if (colk) a[e] = zneg(zmul(f, pinv));
-                else zfms(a[e], f, pr);
-            }
-        }
-        // undo the column exchanges: X = X_pre P, column c of X is column sig(c) of X_pre;
-        // piv[A + c'] receives the destination column of pre-column c'
-        __syncwarp();
-        if (lane == 0) {
-            int sg[A];
-            for (int c = 0; c < A; ++c) sg[c] = c;
-            for (int k = A - 1; k >= 0; --k) {
-                const int p = piv[k];
-                const int t = sg[k];
-                sg[k] = sg[p];
-                sg[p] = t;
-            }
-            for (int c = 0; c < A; ++c) piv[A + sg[c]] = c;
-        }
-        __syncwarp();
-#pragma unroll
-        for (int e = 0; e < 8; ++e) sm[r + piv[A + hf * 8 + e] * A] = a[e];
-        __syncwarp();
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-            prev[e] = sm[r + (hf * 8 + e) * A];
-            Sl[(size_t)j * AA + r + (hf * 8 + e) * A] = prev[e];
-        }
-        __syncwarp();
-    }
-    if (!ok && lane == 0) atomicOr(status, 1);
-
-    // ---- S^T Z = C^T, one right-hand side per lane at a time ---------------------------------------
-    for (int c = lane; c - lane < nb; c += 32) {
-        const bool live = c < nb;
-        int ax = 0, q1 = -1, q2 = -1;
-        if (live) leaf_bpoint2(A, b, c, ax, q1, q2);
-        const double hr = ax == 0 ? L.hx : L.hy;
-        const double c1 = -3.0 / hr, c2 = (1.0 / 3.0) / hr;
-        // Y(c, nb+s) = f_c Q(c, s): the backward sweep stores its final values already scaled
-        const z fc = zmul(zmk(0.0, 2.0 * g.kb), ax == 0 ? L.rdx : L.rdy);
-        z v[A];
-#pragma unroll
-        for (int i = 0; i < A; ++i) v[i] = zmk(0.0, 0.0);
-        // forward: v_j = Sig_j^-T (c_j - Up_{j-1} v_{j-1})
-        for (int j = 0; j < b; ++j) {
-            const int jj = j + 1;
-            const z mup = jj > 1 ? block_up(L, b, jj - 1) : zmk(0.0, 0.0);
-            __syncwarp();
-#pragma unroll
-            for (int e = 0; e < 8; ++e) sm[r + (hf * 8 + e) * A] = Sl[(size_t)j * AA + r + (hf * 8 + e) * A];
-            __syncwarp();
-            z rhs[A];
-#pragma unroll
-            for (int q = 0; q < A; ++q) {
-                const int eq = j * A + q;
-                rhs[q] = zmk((eq == q1 ? c1 : 0.0) + (eq == q2 ? c2 : 0.0), 0.0);
-                if (jj > 1) zfms(rhs[q], mup, v[q]);
-            }
-#pragma unroll
-            for (int i = 0; i < A; ++i) {
-                z acc = zmk(0.0, 0.0);
-#pragma unroll
-                for (int q = 0; q < A; ++q) zfma(acc, sm[q + i * A], rhs[q]);
-                v[i] = acc;
-                if (live) Yl[c + (size_t)(nb + j * A + i) * nb] = acc;
-            }
-        }
-        // backward: z_{j-1} = v_{j-1} - Sig_{j-1}^-T Lo_j z_j, z_{b-1} = v_{b-1}
-        if (live) {
-#pragma unroll
-            for (int i = 0; i < A; ++i) Yl[c + (size_t)(nb + (b - 1) * A + i) * nb] = zmul(fc, v[i]);
-        }
-        for (int j = b - 1; j >= 1; --j) {
-            const z lam = block_lo(L, b, j + 1);
-            __syncwarp();
-#pragma unroll
-            for (int e = 0; e < 8; ++e) sm[r + (hf * 8 + e) * A] = Sl[(size_t)(j - 1) * AA + r + (hf * 8 + e) * A];
-            __syncwarp();
-            z lz[A];
-#pragma unroll
-            for (int q = 0; q < A; ++q) lz[q] = zmul(lam, v[q]);
-#pragma unroll
-            for (int i = 0; i < A; ++i) {
-                z acc = live ? Yl[c + (size_t)(nb + (j - 1) * A + i) * nb] : zmk(0.0, 0.0);
-#pragma unroll
-                for (int q = 0; q < A; ++q) zfms(acc, sm[q + i * A], lz[q]);
-                v[i] = acc;
-                if (live) Yl[c + (size_t)(nb + (j - 1) * A + i) * nb] = zmul(fc, acc);
-            }
-        }
-    }
-    __syncwarp();
-    // ---- Y(:, 0:nb) from the scaled Y(r, nb+s) = f_r Q(r, s) ----------------------------------------
-    for (int e = lane; e < nb * nb; e += 32) {
-        const int rr = e % nb, c = e / nb;
-        int ax, p1, p2, axc, q1, q2;
-        leaf_bpoint2(A, b, rr, ax, p1, p2);
-        leaf_bpoint2(A, b, c, axc, q1, q2);
-        const z rd = ax == 0 ? L.rdx : L.rdy;
-        const z wd = axc == 0 ? zscale(L.wbx, L.rdx) : zscale(L.wby, L.rdy);
-        z val = zneg(zmul(wd, Yl[rr + (size_t)(nb + q1) * nb]));
-        if (c == rr) {
-            const double hr2 = ax == 0 ? L.hx : L.hy;
-            val = zadd(val, zmul(zmk((8.0 / 3.0) / hr2, -g.kb), rd));
-        }
-        Yl[e] = val;
-    }
-}
-
 size_t leaf_block_factor_smem(const LeafGeom& g) {
     return (2 * (size_t)g.a * g.a + 2 * (size_t)g.a * g.nb + g.a) * sizeof(z) + (g.a + 1) * sizeof(int) + 16;
 }
 
 // ---------------------------------------------------------------------------------------------------
-// Tensor-core leaf factor for 16 x b leaves with nb <= 64 boundary points: one warp per leaf, the
-// block LU of leaf_warp_factor_kernel, and the two sweeps of S^T Z = C^T as FP64 tensor-core
-// products (mma.sync m8n8k4 .f64, four real products per complex one) over chunks of 32
-// right-hand sides: block step j is V_j = Sig_j^-T R_j with R_j (16 x 32) in shared memory.
-// The forward step of block j runs as soon as the LU has Sig_j^-1 in the warp's shared memory,
-// so the forward sweep never reloads it; the backward sweep reloads one block per step.
+// Leaf factor for blocks of up to 32 x 32 in two kernels: the chain of block inverses, then the
+// sweeps of S^T Z = C^T, whose right-hand sides are independent of one another.
+//
+// leaf_chain: Sig_j^-1 for j = 0..b-1.  Each Sig_j needs Sig_{j-1}^-1, so a leaf is a chain of a*b
+// pivot steps, and the time of a step is what counts.  A thread holds one row and 8 columns of
+// the block in registers.  Rows are not exchanged: a lane remembers the step at which its row was
+// the pivot, and the row and column orders are restored once per block, on the way through shared
+// memory.  With row p the pivot of column k (largest |re|+|im| among the rows not yet used, first
+// on ties) and x = 1/A(p,k), one step is
+//     A(i,:) = A(i,:) - (A(i,k) x) A(p,:),  A(i,k) = -A(i,k) x     (i != p)
+//     A(p,:) = x A(p,:),                    A(p,k) = x,
+// and after the last step Sig^-1(k, p_q) = A(p_k, q).
+// Latency-bound: 0.31 us per pivot step for 16x16 blocks (81 us a leaf, 366 us for 4096 leaves),
+// 0.48 us for 32x32 (487 us a leaf).  The kernels this replaced formed Sig_j^-1 and the sweeps of a
+// leaf in one warp or CTA: 406 us for 16 leaves of 16x16 (now 128 with leaf_sweep), 2.25 ms for
+// 4096 (now 1.41), 6.6 ms for 64 leaves of 32x32 (now 0.80).
+constexpr int LC_CG = 8;         // columns a thread holds
+
+// row r of the diagonal block D_j in parts: diagonal, right and left neighbour
+struct ChainRow {
+    double wx0, wxp_h, wxm_h;    // x stencil of the row over hx^2
+    bool first, last;
+};
+__device__ __forceinline__ ChainRow chain_row(const LeafConst& L, int a, int r) {
+    ChainRow c;
+    double wm, w0, wp;
+    stencil1(r + 1, a, wm, w0, wp);
+    c.wx0 = w0 / L.hx2;
+    c.wxp_h = wp / L.hx2;
+    c.wxm_h = wm / L.hx2;
+    c.first = r == 0;
+    c.last = r == a - 1;
+    return c;
+}
+
+// the entries of row r at columns c0..c0+7 of D_j, minus lm * prev
+__device__ __forceinline__ void chain_form(const LeafConst& L, const ChainRow& cr, int a, int b, int j, int r, int c0,
+                                           z k, z lm, const z (&prev)[LC_CG], z (&v)[LC_CG]) {
+    double wym, wy0, wyp;
+    stencil1(j + 1, b, wym, wy0, wyp);
+    z d = zmk((k.x + cr.wx0) + wy0 / L.hy2, k.y);
+    if (cr.first || cr.last) d = zsub(d, zscale(L.wbx * L.c1x, L.rdx));
+    if (j == 0 || j == b - 1) d = zsub(d, zscale(L.wby * L.c1y, L.rdy));
+    z up = zmk(cr.wxp_h, 0.0), lo = zmk(cr.wxm_h, 0.0);
+    if (cr.first) up = zsub(up, zscale(L.wbx * L.c2x, L.rdx));
+    if (cr.last) lo = zsub(lo, zscale(L.wbx * L.c2x, L.rdx));
+#pragma unroll
+    for (int e = 0; e < LC_CG; ++e) {
+        const int c = c0 + e;
+        z x = zmk(0.0, 0.0);
+        if (r < a && c < a) {
+            if (c == r) x = d;
+            else if (c == r + 1) x = up;
+            else if (c == r - 1) x = lo;
+            if (j > 0) zfms(x, lm, prev[e]);
+        }
+        v[e] = x;
+    }
+}
+
+// One elimination step on a thread's 8 columns: q the pivot row's values there, mult = A(i,k) x
+// (-x for the pivot row itself); column `own` (if any) is the pivot column.
+__device__ __forceinline__ void chain_update(z& v, z q, z mult, bool is_p, bool is_k) {
+    z base = v;
+    if (is_p) base = zmk(0.0, 0.0);
+    zfms(base, mult, q);
+    v = is_k ? zneg(mult) : base;
+}
+
+// the pivot among the rows of one column: larger |re|+|im| wins (its bit pattern orders like the
+// value), then the smaller row; invalid rows take part as zeros with the largest index
+__device__ __forceinline__ int chain_pivot(z x, bool valid, int r) {
+    const double m = zabs1(x);
+    const unsigned hi = valid ? (unsigned)__double2hiint(m) : 0u;
+    const unsigned lo = valid ? (unsigned)__double2loint(m) : 0u;
+    const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
+    const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? lo : 0u);
+    return __reduce_min_sync(0xffffffffu, (valid && hi == mh && lo == ml) ? r : 0x7fff);
+}
+
+__device__ __forceinline__ z shfl_z(z v, int src) {
+    return zmk(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src));
+}
+
+// Blocks of up to 16 rows: one warp per leaf, lane = row + 16 * column group, no block barriers.
+__global__ void __launch_bounds__(128) leaf_chain16_kernel(LeafGeom g, int nleaves, const double* __restrict__ hh,
+                                                           const z* __restrict__ kv, z* __restrict__ sinv, int* status) {
+    __shared__ z blk[4][256];
+    __shared__ z prow[4][2][2 * LC_CG];
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    const int leaf = blockIdx.x * (blockDim.x >> 5) + wib;
+    if (leaf >= nleaves) return;
+    const int a = g.a, b = g.b, aa = a * a;
+    z* sm = blk[wib];
+    const LeafConst L = leaf_const(hh, leaf, g.kb);
+    const z* kl = kv + (size_t)leaf * a * b;
+    z* Sl = sinv + (size_t)leaf * b * aa;
+    const int r = lane & 15, hf = lane >> 4;
+    const ChainRow cr = chain_row(L, a, r);
+    z v[LC_CG], prev[LC_CG];
+#pragma unroll
+    for (int e = 0; e < LC_CG; ++e) prev[e] = zmk(0.0, 0.0);
+    bool ok = true;
+    z kn = r < a ? kl[r] : zmk(0.0, 0.0);
+    for (int j = 0; j < b; ++j) {
+        const z lm = j > 0 ? zmul(block_lo(L, b, j + 1), block_up(L, b, j)) : zmk(0.0, 0.0);
+        chain_form(L, cr, a, b, j, r, LC_CG * hf, kn, lm, prev, v);
+        if (j + 1 < b && r < a) kn = kl[(j + 1) * a + r];          // the next block's potential
+        bool used = r >= a;
+        int myk = 0, pk = 0;
+#pragma unroll
+        for (int grp = 0; grp < 2; ++grp) {
+#pragma unroll
+            for (int e = 0; e < LC_CG; ++e) {
+                const int k = grp * LC_CG + e;
+                if (k >= a) break;
+                const bool mine = hf == grp;
+                const int p = chain_pivot(v[e], mine && !used, r);
+                const z f = shfl_z(v[e], r + 16 * grp);
+                const z pv = shfl_z(v[e], p + 16 * grp);
+                z* pr = prow[wib][k & 1];
+                if (r == p) {
+#pragma unroll
+                    for (int c = 0; c < LC_CG; ++c) pr[hf * LC_CG + c] = v[c];
+                }
+                if (pv.x == 0.0 && pv.y == 0.0) ok = false;
+                const z x = zrcp(pv);
+                const bool is_p = r == p;
+                const z mult = is_p ? zneg(x) : zmul(f, x);
+                if (is_p) { used = true; myk = k; }
+                if (lane == k) pk = p;
+                __syncwarp();
+#pragma unroll
+                for (int c = 0; c < LC_CG; ++c) chain_update(v[c], pr[hf * LC_CG + c], mult, is_p, mine && c == e);
+            }
+        }
+#pragma unroll
+        for (int e = 0; e < LC_CG; ++e) {
+            const int q = hf * LC_CG + e;
+            const int pq = __shfl_sync(0xffffffffu, pk, q);
+            if (r < a && q < a) sm[myk + pq * a] = v[e];
+        }
+        __syncwarp();
+#pragma unroll
+        for (int e = 0; e < LC_CG; ++e) {
+            const int q = hf * LC_CG + e;
+            if (r < a && q < a) {
+                prev[e] = sm[r + q * a];
+                Sl[(size_t)j * aa + r + q * a] = prev[e];
+            }
+        }
+        __syncwarp();
+    }
+    if (!ok && lane == 0) atomicOr(status, RB_STATUS_ZERO_PIVOT);
+}
+
+// Blocks of 17 to 32 rows: one CTA of NG warps per leaf, lane = row, warp = column group.  The
+// warp that holds the next pivot column updates that column first, finds its pivot and publishes
+// it (its column, the pivot row and the reciprocal) before it updates its other columns, so one
+// block barrier per step is all the others wait for.
+template <int NG>
+__global__ void __launch_bounds__(32 * NG) leaf_chain32_kernel(LeafGeom g, const double* __restrict__ hh,
+                                                               const z* __restrict__ kv, z* __restrict__ sinv,
+                                                               int* status) {
+    __shared__ z sm[32 * 32];
+    __shared__ z prow[NG][2][LC_CG];
+    __shared__ z fcol[2][32];
+    __shared__ z pinv[2];
+    __shared__ int piv[2];
+    const int leaf = blockIdx.x;
+    const int r = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int a = g.a, b = g.b, aa = a * a;
+    const LeafConst L = leaf_const(hh, leaf, g.kb);
+    const z* kl = kv + (size_t)leaf * a * b;
+    z* Sl = sinv + (size_t)leaf * b * aa;
+    const ChainRow cr = chain_row(L, a, r);
+    z v[LC_CG], prev[LC_CG];
+#pragma unroll
+    for (int e = 0; e < LC_CG; ++e) prev[e] = zmk(0.0, 0.0);
+    bool ok = true;
+    z kn = r < a ? kl[r] : zmk(0.0, 0.0);
+    for (int j = 0; j < b; ++j) {
+        const z lm = j > 0 ? zmul(block_lo(L, b, j + 1), block_up(L, b, j)) : zmk(0.0, 0.0);
+        chain_form(L, cr, a, b, j, r, LC_CG * w, kn, lm, prev, v);
+        if (j + 1 < b && r < a) kn = kl[(j + 1) * a + r];
+        bool used = r >= a;
+        int myk = 0, pk = 0;
+        // finds and publishes the pivot of column k, held by this warp in x
+        auto publish = [&](z x, int k) {
+            const int p = chain_pivot(x, !used, r);
+            const int s = k & 1;
+            fcol[s][r] = x;
+            if (r == p) {
+                if (x.x == 0.0 && x.y == 0.0) ok = false;
+                pinv[s] = zrcp(x);
+                piv[s] = p;
+            }
+        };
+        if (w == 0) publish(v[0], 0);
+        for (int grp = 0; grp < NG; ++grp) {
+#pragma unroll
+            for (int e = 0; e < LC_CG; ++e) {
+                const int k = grp * LC_CG + e, s = k & 1;
+                if (k >= a) break;
+                __syncthreads();
+                const int p = piv[s];
+                const z x = pinv[s];
+                const z f = fcol[s][r];
+                const bool is_p = r == p;
+                z* pr = prow[w][s];
+                if (is_p) {
+#pragma unroll
+                    for (int c = 0; c < LC_CG; ++c) pr[c] = v[c];
+                }
+                const z mult = is_p ? zneg(x) : zmul(f, x);
+                if (is_p) { used = true; myk = k; }
+                if (r == k) pk = p;
+                __syncwarp();
+                const int en = (e + 1) % LC_CG;                    // the next pivot column
+                const bool next = k + 1 < a && w == (e + 1 == LC_CG ? grp + 1 : grp);
+                const bool mine = w == grp;
+                chain_update(v[en], pr[en], mult, is_p, false);
+                if (next) publish(v[en], k + 1);
+#pragma unroll
+                for (int c = 0; c < LC_CG; ++c)
+                    if (c != en) chain_update(v[c], pr[c], mult, is_p, mine && c == e);
+            }
+        }
+#pragma unroll
+        for (int e = 0; e < LC_CG; ++e) {
+            const int q = w * LC_CG + e;
+            const int pq = __shfl_sync(0xffffffffu, pk, q);
+            if (r < a && q < a) sm[myk + pq * a] = v[e];
+        }
+        __syncthreads();
+#pragma unroll
+        for (int e = 0; e < LC_CG; ++e) {
+            const int q = w * LC_CG + e;
+            if (r < a && q < a) {
+                prev[e] = sm[r + q * a];
+                Sl[(size_t)j * aa + r + q * a] = prev[e];
+            }
+        }
+        // sm is written again only after the next block's barriers
+    }
+    if (!ok) atomicOr(status, RB_STATUS_ZERO_PIVOT);
+}
+
+// leaf_sweep: Y = R A^-1 from the block inverses.  The sweeps of S^T Z = C^T treat every
+// right-hand side (a boundary point, a row of Y) alone, so a warp takes 8 of them through all
+// 2b - 1 block steps with the running block vector in registers:
 //   forward:  R_0 = C_0;  V_j = Sig_j^-T R_j;  R_{j+1} = C_{j+1} - Up_j V_j
 //   backward: Z_{b-1} = V_{b-1};  Z_{j-1} = V_{j-1} - Sig_{j-1}^-T (Lo_j Z_j)
-// C_j holds, per right-hand side c, c1 and c2 at the interior points next to boundary point c.
-constexpr int LTC_CH = 2;        // chunks of 32 right-hand sides (nb <= 64)
-constexpr int LTC_LDR = 18;      // padded leading dimension of the R buffers (bank spread)
+// A step is V^T (8 x a) = R^T (8 x a) Sig_j^-1 (a x a) on the FP64 tensor cores (m8n8k4, four real
+// products per complex one).  The k order of the MMAs is chosen so that the accumulator layout
+// (row lane/4, columns 2 (lane%4) + {0,1}) is the next step's A fragment as it stands: k-step
+// (t, h) sums the rows q = 8t + 2 (lane%4) + h of the block, so nothing moves between steps.  The
+// blocks stream through shared memory, double-buffered with cp.async, padded with zeros to
+// multiples of 8 and with an odd leading dimension (conflict-free 16-byte fragment loads).
+// C_j holds, per right-hand side, c1 and c2 at the interior points next to its boundary point.
+template <int NT>
+struct SweepCfg {
+    static constexpr int AP = 8 * NT;            // padded block size
+    static constexpr int LD = AP + 1;
+    static constexpr size_t SMEM = 2 * (size_t)AP * LD * sizeof(z);
+};
 
-// acc (2 x 4 tiles of 8x8, complex as re/im) += A B,  A(i,k) = As[k + 16 i],  B(k,c) = Bs[k + LTC_LDR c]
-__device__ __forceinline__ void ltc_mma(const z* As, const z* Bs, double (&cre)[2][4][2], double (&cim)[2][4][2],
-                                        int lane) {
+template <int NT>
+__global__ void __launch_bounds__(256) leaf_sweep_kernel(LeafGeom g, int nchunk, const double* __restrict__ hh,
+                                                         const z* __restrict__ sinv, z* __restrict__ Y) {
+    using Cfg = SweepCfg<NT>;
+    constexpr int LD = Cfg::LD;
+    extern __shared__ z sm[];
+    const int tid = threadIdx.x, nthr = blockDim.x, lane = tid & 31, warp = tid >> 5;
     const int lr = lane >> 2, lc = lane & 3;
-#pragma unroll
-    for (int ks = 0; ks < 4; ++ks) {
-        double ar[2], ai[2], nai[2], br[4], bi[4];
-#pragma unroll
-        for (int mi = 0; mi < 2; ++mi) {
-            const z a = As[(4 * ks + lc) + 16 * (8 * mi + lr)];
-            ar[mi] = a.x;
-            ai[mi] = a.y;
-            nai[mi] = -a.y;
-        }
-#pragma unroll
-        for (int ni = 0; ni < 4; ++ni) {
-            const z b = Bs[(4 * ks + lc) + LTC_LDR * (8 * ni + lr)];
-            br[ni] = b.x;
-            bi[ni] = b.y;
-        }
-#pragma unroll
-        for (int mi = 0; mi < 2; ++mi)
-#pragma unroll
-            for (int ni = 0; ni < 4; ++ni) dmma884(cre[mi][ni][0], cre[mi][ni][1], ar[mi], br[ni]);
-#pragma unroll
-        for (int mi = 0; mi < 2; ++mi)
-#pragma unroll
-            for (int ni = 0; ni < 4; ++ni) dmma884(cim[mi][ni][0], cim[mi][ni][1], ar[mi], bi[ni]);
-#pragma unroll
-        for (int mi = 0; mi < 2; ++mi)
-#pragma unroll
-            for (int ni = 0; ni < 4; ++ni) dmma884(cre[mi][ni][0], cre[mi][ni][1], nai[mi], bi[ni]);
-#pragma unroll
-        for (int mi = 0; mi < 2; ++mi)
-#pragma unroll
-            for (int ni = 0; ni < 4; ++ni) dmma884(cim[mi][ni][0], cim[mi][ni][1], ai[mi], br[ni]);
-    }
-}
-
-// R_j's sparse part: lane c (a right-hand side of chunk ch) adds c1, c2 where its two interior
-// points fall in block j (interior index q = 16 j + row)
-__device__ __forceinline__ void ltc_add_c(z* R, int ch, int j, int lane, int b, int nb, const LeafConst& L) {
-    const int c = 32 * ch + lane;
-    if (c >= nb) return;
-    int ax, q1, q2;
-    leaf_bpoint2(16, b, c, ax, q1, q2);
-    const double h = ax == 0 ? L.hx : L.hy;
-    const double c1 = -3.0 / h, c2 = (1.0 / 3.0) / h;
-    const int q0 = 16 * j;
-    if (q1 >= q0 && q1 < q0 + 16) R[(q1 - q0) + LTC_LDR * lane].x += c1;
-    if (q2 >= q0 && q2 < q0 + 16) R[(q2 - q0) + LTC_LDR * lane].x += c2;
-}
-
-__global__ void __launch_bounds__(128) leaf_tc_factor_kernel(LeafGeom g, int nleaves, const double* __restrict__ hh,
-                                                             const z* __restrict__ kv, z* __restrict__ sinv,
-                                                             z* __restrict__ Y, int* status) {
-    constexpr int A = 16, AA = 256;
-    extern __shared__ z ltc_smem[];
-    __shared__ int wpiv[4][2 * A];
-    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    const int leaf = blockIdx.x * 4 + wib;
-    if (leaf >= nleaves) return;
-    z* sm = ltc_smem + (size_t)wib * (AA + LTC_CH * LTC_LDR * 32);
-    z* R = sm + AA;                                  // LTC_CH buffers of LTC_LDR x 32
-    int* piv = wpiv[wib];
-    const int b = g.b, nb = g.nb, n = g.n, ab = A * b;
-    const int nch = (nb + 31) / 32;
+    const int leaf = blockIdx.x / nchunk, chunk = blockIdx.x % nchunk;
+    const int a = g.a, b = g.b, nb = g.nb, n = g.n, aa = a * a;
     const LeafConst L = leaf_const(hh, leaf, g.kb);
-    const z* kl = kv + (size_t)leaf * ab;
-    z* Sl = sinv + (size_t)leaf * b * AA;
+    const z* Sl = sinv + (size_t)leaf * b * aa;
     z* Yl = Y + (size_t)leaf * nb * n;
-    const int r = lane & 15, hf = lane >> 4;
-    const int lr = lane >> 2, lc = lane & 3;
-    z a[8], prev[8];
-    bool ok = true;
-
-    // R_0 = C_0
-    for (int ch = 0; ch < nch; ++ch) {
-        z* Rc = R + ch * LTC_LDR * 32;
-        for (int e = lane; e < LTC_LDR * 32; e += 32) Rc[e] = zmk(0.0, 0.0);
-        __syncwarp();
-        ltc_add_c(Rc, ch, 0, lane, b, nb, L);
+    const int nsteps = 2 * b - 1;
+    for (int e = tid; e < 2 * Cfg::AP * LD; e += nthr) sm[e] = zmk(0.0, 0.0);
+    __syncthreads();
+    auto issue = [&](int st) {
+        const int j = st < b ? st : 2 * b - 2 - st;
+        const z* src = Sl + (size_t)j * aa;
+        z* dst = sm + (st & 1) * Cfg::AP * LD;
+        for (int e = tid; e < aa; e += nthr) {
+            const int c = e / a;
+            cp_async16(dst + (e - c * a) + c * LD, src + e, 16);
+        }
+        cp_async_commit();
+    };
+    issue(0);
+    // this lane's right-hand side and its two interior points
+    const int row = (chunk * (nthr >> 5) + warp) * 8 + lr;
+    const bool live = row < nb;
+    int ax, q1, q2;
+    leaf_bpoint2(a, b, live ? row : 0, ax, q1, q2);
+    const double h = ax == 0 ? L.hx : L.hy;
+    const double c1 = live ? -3.0 / h : 0.0, c2 = live ? (1.0 / 3.0) / h : 0.0;
+    const z rd = ax == 0 ? L.rdx : L.rdy;
+    const z fc = zmul(zmk(0.0, 2.0 * g.kb), rd);                      // Y(r, nb+s) = f_r Q(r, s)
+    const z dg = zmul(zmk((8.0 / 3.0) / h, -g.kb), rd);               // (sigma'_r / d_r)
+    const z wdx = zscale(L.wbx, L.rdx), wdy = zscale(L.wby, L.rdy);
+    z* Yr = Yl + (live ? row : 0);
+    // the final value s = Y(row, nb + j a + i): it, and its multiples in the boundary columns
+    auto store = [&](int j, int i, z s) {
+        Yr[(size_t)(nb + j * a + i) * nb] = s;
+        auto bcol = [&](int c, z wd) {
+            z v = zneg(zmul(wd, s));
+            if (c == row) v = zadd(v, dg);
+            Yr[(size_t)c * nb] = v;
+        };
+        if (i == 0) bcol(j, wdx);
+        if (i == a - 1) bcol(b + j, wdx);
+        if (j == 0) bcol(2 * b + i, wdy);
+        if (j == b - 1) bcol(2 * b + a + i, wdy);
+    };
+    double rre[2 * NT], rim[2 * NT];                 // R^T, [2t + h]: column 8t + 2lc + h
+    z vn[2 * NT];                                    // the backward step's V, fetched a step ahead
+#pragma unroll
+    for (int e = 0; e < 2 * NT; ++e) {
+        const int q = 8 * (e >> 1) + 2 * lc + (e & 1);
+        rre[e] = q < a ? (q == q1 ? c1 : 0.0) + (q == q2 ? c2 : 0.0) : 0.0;
+        rim[e] = 0.0;
+        vn[e] = zmk(0.0, 0.0);
     }
-    __syncwarp();
-
-    for (int j = 0; j < b; ++j) {
-        // ---- block LU step: Sig_j^-1 (leaf_warp_factor_kernel's Gauss-Jordan) -----------------------
-        const int jj = j + 1;
-        const z lm = jj > 1 ? zmul(block_lo(L, b, jj), block_up(L, b, jj - 1)) : zmk(0.0, 0.0);
-        const z kr = kl[j * A + r];
+    for (int st = 0; st < nsteps; ++st) {
+        const bool fwd = st < b;
+        const int j = fwd ? st : 2 * b - 2 - st;
+        cp_async_wait<0>();
+        __syncthreads();               // block st landed; every warp is past step st-1's reads
+        if (st + 1 < nsteps) issue(st + 1);
+        double cre[NT][2], cim[NT][2];
 #pragma unroll
-        for (int e = 0; e < 8; ++e) {
-            z v = block_d(L, A, b, jj, r, hf * 8 + e, kr);
-            if (jj > 1) zfms(v, lm, prev[e]);
-            a[e] = v;
-        }
+        for (int t = 0; t < NT; ++t)
 #pragma unroll
-        for (int k = 0; k < A; ++k) {
-            const int hk = k >> 3, ek = k & 7;
-            double mag = (hf == hk && r >= k) ? zabs1(a[ek]) : -1.0;
-            int idx = r;
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                const double om = __shfl_xor_sync(0xffffffffu, mag, o);
-                const int oi = __shfl_xor_sync(0xffffffffu, idx, o);
-                if (om > mag || (om == mag && oi < idx)) { mag = om; idx = oi; }
+            for (int q = 0; q < 2; ++q) {
+                cre[t][q] = fwd ? 0.0 : vn[2 * t + q].x;
+                cim[t][q] = fwd ? 0.0 : vn[2 * t + q].y;
             }
-            const int p = idx;
-            if (lane == 0) piv[k] = p;
-            if (p != k) {
-                const int src = (r == k ? p : (r == p ? k : r)) + 16 * hf;
+        // the V of the next backward step: block b-2 first (written two steps before)
+        if (st + 1 >= b && st + 1 < nsteps) {
+            const int jn = 2 * b - 3 - st;
 #pragma unroll
-                for (int e = 0; e < 8; ++e) {
-                    const double x = __shfl_sync(0xffffffffu, a[e].x, src);
-                    const double y = __shfl_sync(0xffffffffu, a[e].y, src);
-                    a[e] = zmk(x, y);
-                }
-            }
-            const z pv = zmk(__shfl_sync(0xffffffffu, a[ek].x, k + 16 * hk),
-                             __shfl_sync(0xffffffffu, a[ek].y, k + 16 * hk));
-            if (pv.x == 0.0 && pv.y == 0.0) ok = false;
-            const z pinv = zrcp(pv);
-            const z f = zmk(__shfl_sync(0xffffffffu, a[ek].x, r + 16 * hk),
-                            __shfl_sync(0xffffffffu, a[ek].y, r + 16 * hk));
-#pragma unroll
-            for (int e = 0; e < 8; ++e) {
-                const z pr = zmul(zmk(__shfl_sync(0xffffffffu, a[e].x, k + 16 * hf),
-                                      __shfl_sync(0xffffffffu, a[e].y, k + 16 * hf)), pinv);
-                const bool colk = (hf == hk) && (e == ek);
-                if (r == k) a[e] = colk ? pinv : pr;
-                else if (colk) a[e] = zneg(zmul(f, pinv));
-                else zfms(a[e], f, pr);
+            for (int e = 0; e < 2 * NT; ++e) {
+                const int i = 8 * (e >> 1) + 2 * lc + (e & 1);
+                vn[e] = (live && i < a) ? Yr[(size_t)(nb + jn * a + i) * nb] : zmk(0.0, 0.0);
             }
         }
-        __syncwarp();
-        if (lane == 0) {
-            int sg[A];
-            for (int c = 0; c < A; ++c) sg[c] = c;
-            for (int k = A - 1; k >= 0; --k) {
-                const int p = piv[k];
-                const int t = sg[k];
-                sg[k] = sg[p];
-                sg[p] = t;
-            }
-            for (int c = 0; c < A; ++c) piv[A + sg[c]] = c;
+        const z* S = sm + (st & 1) * Cfg::AP * LD + 2 * lc + lr * LD;
+#pragma unroll
+        for (int e = 0; e < 2 * NT; ++e) {           // k-step (t, h): rows 8t + 2lc + h of the block
+            z bf[NT];
+#pragma unroll
+            for (int t = 0; t < NT; ++t) bf[t] = S[8 * (e >> 1) + (e & 1) + 8 * t * LD];
+#pragma unroll
+            for (int t = 0; t < NT; ++t) dmma884(cre[t][0], cre[t][1], rre[e], bf[t].x);
+#pragma unroll
+            for (int t = 0; t < NT; ++t) dmma884(cim[t][0], cim[t][1], rre[e], bf[t].y);
+#pragma unroll
+            for (int t = 0; t < NT; ++t) dmma884(cre[t][0], cre[t][1], -rim[e], bf[t].y);
+#pragma unroll
+            for (int t = 0; t < NT; ++t) dmma884(cim[t][0], cim[t][1], rim[e], bf[t].x);
         }
-        __syncwarp();
+        // next R: C_{j+1} - Up_j V_j forward, -Lo_j Z_j backward (Lo_j couples block j to j-1)
+        const bool up = fwd && j + 1 < b;
+        const z co = up ? block_up(L, b, j + 1) : block_lo(L, b, j + 1);
+        const bool fin = !up;
+        const int qn = (j + 1) * a;
 #pragma unroll
-        for (int e = 0; e < 8; ++e) sm[r + piv[A + hf * 8 + e] * A] = a[e];
-        __syncwarp();
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-            prev[e] = sm[r + (hf * 8 + e) * A];
-            Sl[(size_t)j * AA + r + (hf * 8 + e) * A] = prev[e];
-        }
-        __syncwarp();
-        // ---- forward step j for every chunk: V_j = Sig_j^-T R_j -----------------------------------
-        const z mup = block_up(L, b, jj);            // Up_j, for R_{j+1}
-        for (int ch = 0; ch < nch; ++ch) {
-            z* Rc = R + ch * LTC_LDR * 32;
-            double cre[2][4][2], cim[2][4][2];
-#pragma unroll
-            for (int mi = 0; mi < 2; ++mi)
-#pragma unroll
-                for (int ni = 0; ni < 4; ++ni) cre[mi][ni][0] = cre[mi][ni][1] = cim[mi][ni][0] = cim[mi][ni][1] = 0.0;
-            ltc_mma(sm, Rc, cre, cim, lane);
-            __syncwarp();                              // every lane has read R_j
-#pragma unroll
-            for (int mi = 0; mi < 2; ++mi)
-#pragma unroll
-                for (int ni = 0; ni < 4; ++ni)
-#pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        const int i = 8 * mi + lr, cl = 8 * ni + 2 * lc + h, c = 32 * ch + cl;
-                        const z v = zmk(cre[mi][ni][h], cim[mi][ni][h]);
-                        if (c < nb) Yl[c + (size_t)(nb + j * A + i) * nb] = v;
-                        // next: R_{j+1} = C_{j+1} - Up_j V_j  (backward start: -Lo_b Z_{b-1})
-                        Rc[i + LTC_LDR * cl] = zneg(zmul(jj < b ? mup : block_lo(L, b, b), v));
-                    }
-            __syncwarp();
-            if (jj < b) ltc_add_c(Rc, ch, j + 1, lane, b, nb, L);
-        }
-        __syncwarp();
-    }
-    if (!ok && lane == 0) atomicOr(status, 1);
-
-    // ---- backward sweep, Y(c, nb+s) = f_c Q(c, s) stored already scaled -------------------------------
-    z fcl[4][2];                                      // f_c of this lane's columns, per chunk below
-    for (int j = b - 1; j >= 0; --j) {
-        // j >= 1: Z_{j-1} = V_{j-1} + Sig_{j-1}^-T R  with R = -Lo_j Z_j;  the final step (j = 0) only
-        // rescales block... handled by storing Z_{b-1} first
-        if (j == b - 1) {
-            for (int ch = 0; ch < nch; ++ch) {
-                // Z_{b-1} = V_{b-1}, scaled
-#pragma unroll
-                for (int mi = 0; mi < 2; ++mi)
-#pragma unroll
-                    for (int ni = 0; ni < 4; ++ni)
-#pragma unroll
-                        for (int h = 0; h < 2; ++h) {
-                            const int i = 8 * mi + lr, c = 32 * ch + 8 * ni + 2 * lc + h;
-                            if (c >= nb) continue;
-                            int ax, q1, q2;
-                            leaf_bpoint2(A, b, c, ax, q1, q2);
-                            const z fc = zmul(zmk(0.0, 2.0 * g.kb), ax == 0 ? L.rdx : L.rdy);
-                            z* yp = Yl + c + (size_t)(nb + j * A + i) * nb;
-                            *yp = zmul(fc, *yp);
-                        }
+        for (int e = 0; e < 2 * NT; ++e) {
+            const int i = 8 * (e >> 1) + 2 * lc + (e & 1);
+            z s = zmk(cre[e >> 1][e & 1], cim[e >> 1][e & 1]);
+            z nx = zneg(zmul(co, s));
+            if (up && i < a) nx.x += (qn + i == q1 ? c1 : 0.0) + (qn + i == q2 ? c2 : 0.0);
+            rre[e] = nx.x;
+            rim[e] = nx.y;
+            if (live && i < a) {
+                if (fin) store(j, i, zmul(fc, s));
+                else Yr[(size_t)(nb + j * a + i) * nb] = s;
             }
         }
-        if (j == 0) break;
-#pragma unroll
-        for (int e = 0; e < 8; ++e) sm[r + (hf * 8 + e) * A] = Sl[(size_t)(j - 1) * AA + r + (hf * 8 + e) * A];
-        __syncwarp();
-        const z lamn = j >= 2 ? block_lo(L, b, j) : zmk(0.0, 0.0);   // Lo_{j-1}, for the next step
-        for (int ch = 0; ch < nch; ++ch) {
-            z* Rc = R + ch * LTC_LDR * 32;
-            double cre[2][4][2], cim[2][4][2];
-#pragma unroll
-            for (int mi = 0; mi < 2; ++mi)
-#pragma unroll
-                for (int ni = 0; ni < 4; ++ni)
-#pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        const int i = 8 * mi + lr, c = 32 * ch + 8 * ni + 2 * lc + h;
-                        const z v = c < nb ? Yl[c + (size_t)(nb + (j - 1) * A + i) * nb] : zmk(0.0, 0.0);
-                        cre[mi][ni][h] = v.x;
-                        cim[mi][ni][h] = v.y;
-                        int ax, q1, q2;
-                        leaf_bpoint2(A, b, c < nb ? c : 0, ax, q1, q2);
-                        fcl[ni][h] = zmul(zmk(0.0, 2.0 * g.kb), ax == 0 ? L.rdx : L.rdy);
-                    }
-            ltc_mma(sm, Rc, cre, cim, lane);
-            __syncwarp();
-#pragma unroll
-            for (int mi = 0; mi < 2; ++mi)
-#pragma unroll
-                for (int ni = 0; ni < 4; ++ni)
-#pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        const int i = 8 * mi + lr, cl = 8 * ni + 2 * lc + h, c = 32 * ch + cl;
-                        const z zv = zmk(cre[mi][ni][h], cim[mi][ni][h]);
-                        if (c < nb) Yl[c + (size_t)(nb + (j - 1) * A + i) * nb] = zmul(fcl[ni][h], zv);
-                        Rc[i + LTC_LDR * cl] = zneg(zmul(lamn, zv));
-                    }
-            __syncwarp();
-        }
-    }
-    __syncwarp();
-    // ---- Y(:, 0:nb) from the scaled Y(r, nb+s) = f_r Q(r, s) ----------------------------------------
-    for (int e = lane; e < nb * nb; e += 32) {
-        const int rr = e % nb, c = e / nb;
-        int ax, p1, p2, axc, q1, q2;
-        leaf_bpoint2(A, b, rr, ax, p1, p2);
-        leaf_bpoint2(A, b, c, axc, q1, q2);
-        const z rd = ax == 0 ? L.rdx : L.rdy;
-        const z wd = axc == 0 ? zscale(L.wbx, L.rdx) : zscale(L.wby, L.rdy);
-        z val = zneg(zmul(wd, Yl[rr + (size_t)(nb + q1) * nb]));
-        if (c == rr) {
-            const double hr2 = ax == 0 ? L.hx : L.hy;
-            val = zadd(val, zmul(zmk((8.0 / 3.0) / hr2, -g.kb), rd));
-        }
-        Yl[e] = val;
     }
 }
 
-static bool leaf_tc_enabled() {
-    const char* v = std::getenv("RB_LEAF_ENGINE");
-    return !(v && v[0] == 'd');       // RB_LEAF_ENGINE=dfma: the DFMA warp kernel (comparisons)
+template <int NT>
+static cudaError_t launch_sweep(const LeafGeom& g, int nleaves, const double* h, const z* sinv, z* Y, cudaStream_t s) {
+    const int units = (g.nb + 7) / 8;                // warps a leaf needs
+    // few leaves: two warps per CTA, to spread a leaf over several SMs; many: up to eight, which
+    // share each staged block
+    const int wpc = std::min(units, (long long)nleaves * units <= 8 * 148 ? 2 : 8);
+    const int nchunk = (units + wpc - 1) / wpc;
+    static DeviceAttrCache attr;
+    cudaError_t e = ensure_smem_attr(leaf_sweep_kernel<NT>, SweepCfg<NT>::SMEM, attr);
+    if (e != cudaSuccess) return e;
+    leaf_sweep_kernel<NT><<<(unsigned)nleaves * nchunk, 32 * wpc, SweepCfg<NT>::SMEM, s>>>(g, nchunk, h, sinv, Y);
+    note_launch();
+    return cudaGetLastError();
 }
 
 cudaError_t leaf_block_factor(const LeafGeom& g, int nleaves, const double* h, const z* k, z* sinv, z* Y,
                               int* status, cudaStream_t s) {
-    if (g.a == 16 && g.nb <= 32 * LTC_CH && leaf_tc_enabled()) {     // one warp per leaf, tensor cores
-        const size_t sh = 4 * (256 + (size_t)LTC_CH * LTC_LDR * 32) * sizeof(z);
-        static DeviceAttrCache attr;
-        {
-            cudaError_t e = ensure_smem_attr(leaf_tc_factor_kernel, sh, attr);
-            if (e != cudaSuccess) return e;
-        }
-        leaf_tc_factor_kernel<<<(nleaves + 3) / 4, 128, sh, s>>>(g, nleaves, h, k, sinv, Y, status);
-        note_launch();
-        return cudaGetLastError();
-    }
-    if (g.a == 16) {                        // one warp per leaf
-        leaf_warp_factor_kernel<<<(nleaves + 3) / 4, 128, 0, s>>>(g, nleaves, h, k, sinv, Y, status);
-        note_launch();
-        return cudaGetLastError();
-    }
     const size_t sh = leaf_block_factor_smem(g);
+    if (g.a <= 32) {
+        // leaf grids this library accepts: those of the one-CTA form below, and 16-cell blocks
+        if (g.a != 16 && sh > (size_t)227 * 1024) return cudaErrorInvalidValue;
+        if (g.a <= 16) {
+            const int wpc = nleaves >= 4 * 148 ? 4 : 1;
+            leaf_chain16_kernel<<<(nleaves + wpc - 1) / wpc, 32 * wpc, 0, s>>>(g, nleaves, h, k, sinv, status);
+        } else if (g.a <= 24) {
+            leaf_chain32_kernel<3><<<nleaves, 96, 0, s>>>(g, h, k, sinv, status);
+        } else {
+            leaf_chain32_kernel<4><<<nleaves, 128, 0, s>>>(g, h, k, sinv, status);
+        }
+        note_launch();
+        cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
+        if (g.a <= 8) return launch_sweep<1>(g, nleaves, h, sinv, Y, s);
+        if (g.a <= 16) return launch_sweep<2>(g, nleaves, h, sinv, Y, s);
+        if (g.a <= 24) return launch_sweep<3>(g, nleaves, h, sinv, Y, s);
+        return launch_sweep<4>(g, nleaves, h, sinv, Y, s);
+    }
     if (sh > 48 * 1024) {
         static DeviceAttrCache attr;
         cudaError_t e = ensure_smem_attr(leaf_block_factor_kernel, sh, attr);
