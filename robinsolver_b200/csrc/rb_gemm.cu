@@ -14,6 +14,7 @@
 #include <cstring>
 
 #include "rb_gemm_dmma.cuh"
+#include "rb_gemm_stream.cuh"
 #include "rb_gemm_tile.cuh"
 #include "rb_kernels.h"
 
@@ -63,8 +64,9 @@ __global__ void __launch_bounds__(256) zgemm_reduce_kernel(const GemmDesc* __res
     const z* p = work + (long long)blockIdx.y * ksplit * pstride + i + (long long)j * ldp;
     z acc = p[0];
     for (int r = 1; r < ksplit; ++r) acc = zadd(acc, p[r * pstride]);
-    z v = zmul(g.alpha, acc);
-    if (g.C.p && !(i >= g.nobeta_r0 && i < g.nobeta_r1)) zfma(v, g.beta, g.C.p[vrow(g.C, i) + (long long)vcol(g.C, j) * g.C.ld]);
+    z v = gemm_alpha(g.alpha, acc);
+    if (g.C.p && !(i >= g.nobeta_r0 && i < g.nobeta_r1))
+        v = gemm_beta(v, g.beta, g.C.p[vrow(g.C, i) + (long long)vcol(g.C, j) * g.C.ld]);
     g.D.p[vrow(g.D, i) + (long long)vcol(g.D, j) * g.D.ld] = v;
 }
 
@@ -259,13 +261,43 @@ static cudaError_t launch_split(const GemmBatch& b, cudaStream_t s) {
     return cudaGetLastError();
 }
 
+// up to 8 right-hand sides (rb_gemm_stream.cuh)
+template <int RT>
+static cudaError_t launch_stream(const GemmBatch& b, int ks, cudaStream_t s) {
+    const int groups = (b.max_m + 8 * RT - 1) / (8 * RT);
+    const int ngrp = std::max(1, std::min(groups, (ks > 1 ? STREAM_WARPS : 4) / ks));
+    for (int off = 0; off < b.count; off += 65535) {
+        const int cnt = std::min(b.count - off, 65535);
+        zgemm_stream_kernel<RT><<<dim3((groups + ngrp - 1) / ngrp, cnt), 32 * ngrp * ks, 0, s>>>(b.d_desc + off, ks,
+                                                                                                b.kchunk);
+        note_launch();
+    }
+    return cudaGetLastError();
+}
+
+// The solve's tensor-core kernels: one order of summation, so the kernel may follow the number
+// of right-hand sides.  Up to 8: rb_gemm_stream.cuh (512^2, one: 1065 -> 795 us a solve); up to 16:
+// 32x16 tiles, whose second half would be idle at 32 (512^2, 16: the leaves' product 131 -> 88 us,
+// the solve's GEMMs 1.15 -> 0.97 ms).
+static cudaError_t launch_solve_gemm(const GemmBatch& b, cudaStream_t s) {
+    const bool split = b.ksplit > 1;
+    if (b.max_n <= 8 && b.ksplit <= STREAM_WARPS) {
+        // two row tiles per warp once one per warp gives each scheduler more than four warps
+        const long long warps = (long long)b.count * ((b.max_m + 7) / 8) * b.ksplit;
+        return warps > 148 * 16 ? launch_stream<2>(b, b.ksplit, s) : launch_stream<1>(b, b.ksplit, s);
+    }
+    if (b.max_n <= 16)
+        return split ? launch_dmma_split<32, 16, 2, 2, 8>(b, s) : launch_dmma<32, 16, 2, 2, 8>(b, s);
+    return split ? launch_dmma_split<32, 32, 2, 2, 6>(b, s) : launch_dmma<32, 32, 2, 2, 6>(b, s);
+}
+
 // the kernel shape a batch runs on
 enum class GemmShape { Dfma16, Dfma32, Dmma32, Dmma64, DmmaKc64, DmmaFixed, Dfma128x64, Dfma64 };
 static GemmShape gemm_shape(const GemmBatch& b) {
     const int mm = b.max_m, nn = b.max_n;
     if (b.engine >= 0 && !b.fixed_order) return static_cast<GemmShape>(b.engine);
-    // fixed-order batches (the solve) on the tensor cores: one tile shape, split-K planned from
-    // count, m and k only; an element's sum runs over k in MMA steps of 4 in order whatever n is
+    // fixed-order batches (the solve) on the tensor cores: an element's sum runs over k in MMA
+    // steps of 4, in ranges planned from count, m and k only, whatever n and the kernel are
     if (use_dmma() && b.fixed_order) return GemmShape::DmmaFixed;
     if (mm <= 16 && nn <= 16) return GemmShape::Dfma16;
     // FP64 tensor cores, small problems (both sides <= 192: the merges below 128x256 boxes):
@@ -315,6 +347,8 @@ long long gemm_plan_split(GemmBatch& b) {
         return 0;
     }
     b.pstride = (long long)b.max_m * b.max_n;
+    // up to 8 right-hand sides the ranges of a problem meet in one CTA's shared memory
+    if (use_dmma() && b.max_n <= 8) return 0;
     return (long long)b.count * b.ksplit * b.pstride;
 }
 
@@ -368,8 +402,7 @@ cudaError_t launch_gemm_batch(const GemmBatch& b, cudaStream_t s) {
     static_assert(sizeof(GemmDesc) % 8 == 0, "descriptor copy assumes 8-byte words");
     if (b.count == 0 || b.max_m == 0 || b.max_n == 0) return cudaSuccess;
     const GemmShape shape = gemm_shape(b);
-    if (shape == GemmShape::DmmaFixed)
-        return (b.ksplit > 1 && b.work) ? launch_dmma_split<32, 32, 2, 2, 6>(b, s) : launch_dmma<32, 32, 2, 2, 6>(b, s);
+    if (shape == GemmShape::DmmaFixed) return launch_solve_gemm(b, s);
     if (b.ksplit > 1 && b.work) {
         if (shape == GemmShape::Dfma16) return launch_split<16, 16, 2, 2, 8, 6, 8>(b, s);
         if (shape == GemmShape::Dfma32) return launch_split<32, 32, 4, 2, 8, 4, 4>(b, s);
@@ -379,8 +412,8 @@ cudaError_t launch_gemm_batch(const GemmBatch& b, cudaStream_t s) {
     switch (shape) {
         case GemmShape::Dfma16: return launch_cfg<16, 16, 2, 2, 8, 6, 8>(b, s);
         case GemmShape::Dfma32: return launch_cfg<32, 32, 4, 2, 8, 4, 4>(b, s);
-        case GemmShape::Dmma32:
-        case GemmShape::DmmaFixed: return launch_dmma<32, 32, 2, 2, 6>(b, s);
+        case GemmShape::DmmaFixed:           // launched above
+        case GemmShape::Dmma32: return launch_dmma<32, 32, 2, 2, 6>(b, s);
         case GemmShape::Dmma64: return launch_dmma<64, 64, 2, 4, 2>(b, s);
         case GemmShape::DmmaKc64: return launch_dmma_kc<64, 64, 2, 2, 4, 8, 2>(b, s);
         case GemmShape::Dfma128x64: return launch_cfg<128, 64, 8, 4, 4, 4, 1>(b, s);

@@ -35,6 +35,15 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N)); }
 
+// alpha acc and alpha acc + beta c, every rounding spelled out: the solve's kernels must agree bit
+// for bit, and a compiler that fuses one product of a sum into it is free to choose which
+__device__ __forceinline__ z gemm_alpha(z alpha, z acc) {
+    return zmk(__fma_rn(alpha.x, acc.x, -__dmul_rn(alpha.y, acc.y)), __fma_rn(alpha.x, acc.y, __dmul_rn(alpha.y, acc.x)));
+}
+__device__ __forceinline__ z gemm_beta(z v, z beta, z c) {
+    return zmk(__fma_rn(-beta.y, c.y, __fma_rn(beta.x, c.x, v.x)), __fma_rn(beta.y, c.x, __fma_rn(beta.x, c.y, v.y)));
+}
+
 // D = alpha (P1 - P2 + i (P3 - P1 - P2)) + beta C for one warp's TMW x TNW MMA tiles, whose
 // top-left element is (r0, c0).  Column offsets are looked up once, and each row's C elements are
 // all loaded before any of its D elements is stored, so that the loads overlap: C aliases D, if
@@ -77,8 +86,8 @@ __device__ __forceinline__ void dmma_store(const GemmDesc& sd, const double (&p1
                 if (dcol[j][h] < 0) continue;
                 const double re = p1[i][j][h] - p2[i][j][h];
                 const double im = p3[i][j][h] - p1[i][j][h] - p2[i][j][h];
-                z v = zmul(alpha, zmk(re, im));
-                if (use_c) zfma(v, beta, c[j][h]);
+                z v = gemm_alpha(alpha, zmk(re, im));
+                if (use_c) v = gemm_beta(v, beta, c[j][h]);
                 D.p[drow + (long long)dcol[j][h] * D.ld] = v;
             }
     }

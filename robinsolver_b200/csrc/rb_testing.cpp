@@ -6,6 +6,7 @@
 //   engine 0: the FP64 launcher the FP64 path uses (tensor-core DMMA / DFMA tiles)
 //   engine 1: the tcgen05 kernel of the mixed-precision levels in split TF32
 //   engine 2: the tcgen05 kernel in int8 digit slices (the mixed-precision default)
+//   engine 3: the solve's fixed-order kernel
 // It allocates its descriptor array itself and synchronises; it returns 0, a negative RB_ERR_*
 // code for bad arguments or CUDA failures, or the device status word's bits (> 0) when a kernel
 // reported one.
@@ -47,6 +48,7 @@ static int test_zgemm(int engine, int m, int n, int k, const double* dA, long lo
     b.count = count;
     b.max_m = m; b.max_n = n; b.max_k = k;
     b.kcontig = true;
+    b.fixed_order = engine == 3;
     int* d_status = nullptr;
     if (cudaMalloc(&b.d_desc, sizeof(GemmDesc) * count) != cudaSuccess) return RB_ERR_CUDA;
     if (cudaMalloc(&d_status, sizeof(int)) != cudaSuccess) {
@@ -60,7 +62,11 @@ static int test_zgemm(int engine, int m, int n, int k, const double* dA, long lo
         if (pb) e = cudaMalloc(&b.t5_planes, pb);
         b.t5_plane_cap = pb;
     }
-    auto run = [&]() { return engine != 0 ? launch_gemm_tc5(b, d_status, 0) : launch_gemm_batch(b, 0); };
+    if (engine == 3) {
+        const long long w = gemm_plan_split(b);
+        if (w > 0 && e == cudaSuccess) e = cudaMalloc(&b.work, sizeof(z) * (size_t)w);
+    }
+    auto run = [&]() { return engine == 1 || engine == 2 ? launch_gemm_tc5(b, d_status, 0) : launch_gemm_batch(b, 0); };
     int rc = RB_OK;
     if (e == cudaSuccess) e = cudaMemcpy(b.d_desc, h.data(), sizeof(GemmDesc) * count, cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemset(d_status, 0, sizeof(int));
@@ -91,6 +97,7 @@ static int test_zgemm(int engine, int m, int n, int k, const double* dA, long lo
     cudaFree(b.d_desc);
     cudaFree(d_status);
     if (b.t5_planes) cudaFree(b.t5_planes);
+    if (b.work) cudaFree(b.work);
     return rc;
 }
 
