@@ -6,8 +6,8 @@
 // Gauss-Jordan elimination with partial pivoting, so that later applications are GEMMs.
 // Pivots are chosen as LAPACK's izamax does: largest |re|+|im| in the column, first on ties.
 //
-// m <= 32: one CTA per matrix holds the whole matrix in shared memory (gj_small).
-// m  > 32: blocked Gauss-Jordan by panels of nb = 8 columns.  Per panel:
+// m <= 64: the whole matrix in the registers of a warp (m <= 16) or a CTA (rb_pivot.cuh).
+// m  > 64: blocked Gauss-Jordan by panels of nb = 8 columns.  Per panel:
 //   1. elimination of the panel: the pivot search below the diagonal, row exchange, scaling and
 //      elimination of every other row, leaving the accumulated transform W in the panel columns;
 //   2. update of every other column: the panel's row exchanges, then
@@ -22,16 +22,17 @@
 #include <cstdlib>
 #include "rb_gemm_tile.cuh"
 #include "rb_kernels.h"
+#include "rb_pivot.cuh"
 
 namespace rb {
 
 int gj_panel_width(int m) {
-    if (m < GJ_BLOCKED_MIN) return 0;
+    if (m <= GJ_SMALL_MAX) return 0;
     return 8;
 }
 
 // one complex element per matrix: the resident path's two flag words
-long long gj_workspace_elems(int m) { return m < GJ_BLOCKED_MIN ? 0 : 1; }
+long long gj_workspace_elems(int m) { return m <= GJ_SMALL_MAX ? 0 : 1; }
 
 // warp argmax: larger value wins, equal values go to the smaller index
 __device__ __forceinline__ void argmax_warp(double& v, int& i) {
@@ -46,72 +47,57 @@ __device__ __forceinline__ void argmax_warp(double& v, int& i) {
 __device__ __forceinline__ bool zis0(z a) { return a.x == 0.0 && a.y == 0.0; }
 
 // ---------------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) gj_small_kernel(const GJDesc* __restrict__ descs, int m,
-                                                       int* status) {
-    extern __shared__ z S[];                  // m*m, column-major
-    __shared__ z fcol[GJ_SMALL_MAX];
-    __shared__ int ipiv[GJ_SMALL_MAX];
-    __shared__ int sp;
+// m <= 64: the whole matrix in registers (rb_pivot.cuh).  The result goes back in place with its
+// rows and columns in order; a column's permuted rows cover whole memory sectors between them.
+__global__ void __launch_bounds__(128) gj_warp_kernel(const GJDesc* __restrict__ descs, int count, int m, int* status) {
+    __shared__ z prow[4][32];
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    const int mat = blockIdx.x * (blockDim.x >> 5) + wib;
+    if (mat >= count) return;
+    const GJDesc g = descs[mat];
+    const int r = lane & 15, hf = lane >> 4;
+    z v[PV_CG];
+#pragma unroll
+    for (int e = 0; e < PV_CG; ++e) {
+        const int q = hf * PV_CG + e;
+        v[e] = r < m && q < m ? g.A[r + (long long)q * g.ld] : zmk(0.0, 0.0);
+    }
+    int myk, pk;
+    const bool ok = warp_invert16(v, m, prow[wib], myk, pk);
+    __syncwarp();
+#pragma unroll
+    for (int e = 0; e < PV_CG; ++e) {
+        const int q = hf * PV_CG + e;
+        const int pq = __shfl_sync(0xffffffffu, pk, q);
+        if (r < m && q < m) g.A[myk + (long long)pq * g.ld] = v[e];
+    }
+    if (!ok) atomicOr(status, RB_STATUS_ZERO_PIVOT);
+}
+
+template <int RPL, int NG>
+__global__ void __launch_bounds__(32 * NG) gj_cta_kernel(const GJDesc* __restrict__ descs, int m, int* status) {
+    __shared__ PivotShared<RPL, NG> sh;
     const GJDesc g = descs[blockIdx.x];
-    const int tid = threadIdx.x, nt = blockDim.x;
-    for (int e = tid; e < m * m; e += nt) {
-        const int r = e % m, c = e / m;
-        S[e] = g.A[r + (long long)c * g.ld];
-    }
-    __syncthreads();
-    bool bad = false;
-    for (int k = 0; k < m; ++k) {
-        if (tid < 32) {
-            double best = -1.0;
-            int bi = m;
-            for (int r = k + tid; r < m; r += 32) {
-                const double v = zabs1(S[r + k * m]);
-                if (v > best) { best = v; bi = r; }
-            }
-            argmax_warp(best, bi);
-            if (tid == 0) { sp = bi; ipiv[k] = bi; }
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    z v[RPL][PV_CG];
+#pragma unroll
+    for (int i = 0; i < RPL; ++i)
+#pragma unroll
+        for (int e = 0; e < PV_CG; ++e) {
+            const int r = lane + 32 * i, q = w * PV_CG + e;
+            v[i][e] = r < m && q < m ? g.A[r + (long long)q * g.ld] : zmk(0.0, 0.0);
         }
-        __syncthreads();
-        const int p = sp;
-        if (p != k)
-            for (int c = tid; c < m; c += nt) {
-                const z t = S[k + c * m];
-                S[k + c * m] = S[p + c * m];
-                S[p + c * m] = t;
-            }
-        __syncthreads();
-        const z piv = S[k + k * m];
-        const z pinv = zrcp(piv);
-        if (zis0(piv)) bad = true;
-        for (int i = tid; i < m; i += nt) fcol[i] = S[i + k * m];
-        __syncthreads();
-        for (int c = tid; c < m; c += nt) S[k + c * m] = (c == k) ? pinv : zmul(S[k + c * m], pinv);
-        __syncthreads();
-        for (int e = tid; e < m * m; e += nt) {
-            const int i = e % m, c = e / m;
-            if (i == k) continue;
-            const z f = fcol[i];
-            if (c == k) S[e] = zneg(zmul(f, pinv));
-            else zfms(S[e], f, S[k + c * m]);
+    int myk[RPL];
+    const bool ok = cta_invert<RPL, NG>(v, m, sh, myk);
+    __syncthreads();                              // sh.pk is complete
+#pragma unroll
+    for (int i = 0; i < RPL; ++i)
+#pragma unroll
+        for (int e = 0; e < PV_CG; ++e) {
+            const int r = lane + 32 * i, q = w * PV_CG + (RPL > 1 ? (e + m) % PV_CG : e);
+            if (r < m && q < m) g.A[myk[i] + (long long)sh.pk[q] * g.ld] = v[i][e];
         }
-        __syncthreads();
-    }
-    // undo the column exchanges, last first; each thread owns whole rows
-    for (int r = tid; r < m; r += nt)
-        for (int k = m - 1; k >= 0; --k) {
-            const int p = ipiv[k];
-            if (p != k) {
-                const z t = S[r + k * m];
-                S[r + k * m] = S[r + p * m];
-                S[r + p * m] = t;
-            }
-        }
-    __syncthreads();
-    for (int e = tid; e < m * m; e += nt) {
-        const int r = e % m, c = e / m;
-        g.A[r + (long long)c * g.ld] = S[e];
-    }
-    if (bad && tid == 0) atomicOr(status, 1);
+    if (!ok) atomicOr(status, RB_STATUS_ZERO_PIVOT);
 }
 
 // ---------------------------------------------------------------------------------------------------
@@ -681,28 +667,27 @@ static bool resident_enabled() {
 
 cudaError_t gj_invert_batch(const GJDesc* d_desc, int count, int m, void* work, int* d_status, cudaStream_t s) {
     if (count <= 0 || m <= 0) return cudaSuccess;
-    if (m < GJ_BLOCKED_MIN) {
-        const size_t sh = (size_t)m * m * sizeof(z);
-        static DeviceAttrCache attr;
-        {
-            cudaError_t e = ensure_smem_attr(gj_small_kernel, GJ_SMALL_MAX * GJ_SMALL_MAX * sizeof(z), attr);
-            if (e != cudaSuccess) return e;
+    if (m <= GJ_SMALL_MAX) {
+        if (m <= 16) {
+            const int wpc = count >= 4 * 148 ? 4 : 1;
+            gj_warp_kernel<<<(count + wpc - 1) / wpc, 32 * wpc, 0, s>>>(d_desc, count, m, d_status);
+        } else if (m <= 32) {
+            gj_cta_kernel<1, 4><<<count, (m + 7) / 8 * 32, 0, s>>>(d_desc, m, d_status);
+        } else {
+            gj_cta_kernel<2, 8><<<count, (m + 7) / 8 * 32, 0, s>>>(d_desc, m, d_status);
         }
-        gj_small_kernel<<<count, 256, sh, s>>>(d_desc, m, d_status);
         note_launch();
         return cudaGetLastError();
     }
     if (resident_enabled() && work) {
         bool done = false;
         cudaError_t e = cudaSuccess;
-        if (m <= 64) e = gj_resident<8, 64, 1>(d_desc, count, m, work, d_status, s, &done);
-        else if (m <= 128) e = gj_resident<8, 128, 1>(d_desc, count, m, work, d_status, s, &done);
+        if (m <= 128) e = gj_resident<8, 128, 1>(d_desc, count, m, work, d_status, s, &done);
         else if (m <= 256) e = gj_resident<8, 256, 1>(d_desc, count, m, work, d_status, s, &done);
         else if (m <= 512) e = gj_resident<8, 512, 1>(d_desc, count, m, work, d_status, s, &done);
         else if (m <= 1024) e = gj_resident<8, 512, 2>(d_desc, count, m, work, d_status, s, &done);
         if (e != cudaSuccess || done) return e;
     }
-    if (m <= 64) return gj_blocked<8, 64>(d_desc, count, m, d_status, s);
     if (m <= 256) return gj_blocked<8, 256>(d_desc, count, m, d_status, s);
     if (m <= 512) return gj_blocked<8, 512>(d_desc, count, m, d_status, s);
     if (m <= 1024) return gj_blocked<8, 1024>(d_desc, count, m, d_status, s);

@@ -41,6 +41,7 @@
 #include <cstring>
 #include "rb_gemm_dmma.cuh"   // dmma884
 #include "rb_kernels.h"
+#include "rb_pivot.cuh"
 
 namespace rb {
 
@@ -299,91 +300,67 @@ size_t leaf_block_factor_smem(const LeafGeom& g) {
 // sweeps of S^T Z = C^T, whose right-hand sides are independent of one another.
 //
 // leaf_chain: Sig_j^-1 for j = 0..b-1.  Each Sig_j needs Sig_{j-1}^-1, so a leaf is a chain of a*b
-// pivot steps, and the time of a step is what counts.  A thread holds one row and 8 columns of
-// the block in registers.  Rows are not exchanged: a lane remembers the step at which its row was
-// the pivot, and the row and column orders are restored once per block, on the way through shared
-// memory.  With row p the pivot of column k (largest |re|+|im| among the rows not yet used, first
-// on ties) and x = 1/A(p,k), one step is
-//     A(i,:) = A(i,:) - (A(i,k) x) A(p,:),  A(i,k) = -A(i,k) x     (i != p)
-//     A(p,:) = x A(p,:),                    A(p,k) = x,
-// and after the last step Sig^-1(k, p_q) = A(p_k, q).
-// Latency-bound: 0.31 us per pivot step for 16x16 blocks (81 us a leaf, 366 us for 4096 leaves),
-// 0.48 us for 32x32 (487 us a leaf).  The kernels this replaced formed Sig_j^-1 and the sweeps of a
-// leaf in one warp or CTA: 406 us for 16 leaves of 16x16 (now 128 with leaf_sweep), 2.25 ms for
-// 4096 (now 1.41), 6.6 ms for 64 leaves of 32x32 (now 0.80).
-constexpr int LC_CG = 8;         // columns a thread holds
+// pivot steps (rb_pivot.cuh), and the time of a step is what counts.  The row and column orders are
+// restored once per block, on the way through shared memory.
+// Latency-bound: 4.3 us a block of 16 rows (69 us a 16x16 leaf, 345 us for 4096 leaves), 13.9 us a
+// block of 32 (445 us a 32x32 leaf).  One warp or CTA forming Sig_j^-1 and both sweeps of a leaf took
+// 406 us for 16 leaves of 16x16 (now 116 with leaf_sweep), 2.25 ms for 4096 (now 1.39), and 6.6 ms
+// for 64 leaves of 32x32 (now 0.75).
 
-// row r of the diagonal block D_j in parts: diagonal, right and left neighbour
+// what one row of the diagonal blocks D_j is made of, formed once per leaf: the chain pays for
+// every division of a block
 struct ChainRow {
-    double wx0, wxp_h, wxm_h;    // x stencil of the row over hx^2
-    bool first, last;
+    double wx0, wy_in, wy_end;   // diagonal stencil weights over h^2: x; y of an inner and of an end block
+    z dx, dy;                    // what the condensed x (end rows) and y (end blocks) faces take off
+    z up, lo;                    // right and left neighbour
+    z lm_first, lm_in, lm_last;  // Lo_j Up_{j-1} of block 1, an inner block and block b-1
 };
-__device__ __forceinline__ ChainRow chain_row(const LeafConst& L, int a, int r) {
+__device__ __forceinline__ ChainRow chain_row(const LeafConst& L, int a, int b, int r) {
     ChainRow c;
     double wm, w0, wp;
     stencil1(r + 1, a, wm, w0, wp);
     c.wx0 = w0 / L.hx2;
-    c.wxp_h = wp / L.hx2;
-    c.wxm_h = wm / L.hx2;
-    c.first = r == 0;
-    c.last = r == a - 1;
+    c.up = zmk(wp / L.hx2, 0.0);
+    c.lo = zmk(wm / L.hx2, 0.0);
+    c.dx = zmk(0.0, 0.0);
+    if (r == 0 || r == a - 1) {
+        c.dx = zscale(L.wbx * L.c1x, L.rdx);
+        const z n = zscale(L.wbx * L.c2x, L.rdx);
+        if (r == 0) c.up = zsub(c.up, n);
+        if (r == a - 1) c.lo = zsub(c.lo, n);
+    }
+    stencil1(2, b, wm, w0, wp);
+    c.wy_in = w0 / L.hy2;
+    stencil1(1, b, wm, w0, wp);
+    c.wy_end = w0 / L.hy2;
+    c.dy = zscale(L.wby * L.c1y, L.rdy);
+    c.lm_first = zmul(block_lo(L, b, 2), block_up(L, b, 1));
+    c.lm_in = b > 3 ? zmul(block_lo(L, b, 3), block_up(L, b, 2)) : zmk(0.0, 0.0);
+    c.lm_last = zmul(block_lo(L, b, b), block_up(L, b, b - 1));
     return c;
 }
 
-// the entries of row r at columns c0..c0+7 of D_j, minus lm * prev
-__device__ __forceinline__ void chain_form(const LeafConst& L, const ChainRow& cr, int a, int b, int j, int r, int c0,
-                                           z k, z lm, const z (&prev)[LC_CG], z (&v)[LC_CG]) {
-    double wym, wy0, wyp;
-    stencil1(j + 1, b, wym, wy0, wyp);
-    z d = zmk((k.x + cr.wx0) + wy0 / L.hy2, k.y);
-    if (cr.first || cr.last) d = zsub(d, zscale(L.wbx * L.c1x, L.rdx));
-    if (j == 0 || j == b - 1) d = zsub(d, zscale(L.wby * L.c1y, L.rdy));
-    z up = zmk(cr.wxp_h, 0.0), lo = zmk(cr.wxm_h, 0.0);
-    if (cr.first) up = zsub(up, zscale(L.wbx * L.c2x, L.rdx));
-    if (cr.last) lo = zsub(lo, zscale(L.wbx * L.c2x, L.rdx));
+// the entries of row r at columns c0..c0+7 of D_j, minus Lo_j Up_{j-1} prev
+__device__ __forceinline__ void chain_form(const ChainRow& cr, int a, int b, int j, int r, int c0, z k,
+                                           const z (&prev)[PV_CG], z (&v)[PV_CG]) {
+    const bool end = j == 0 || j == b - 1;
+    z d = zsub(zmk((k.x + cr.wx0) + (end ? cr.wy_end : cr.wy_in), k.y), cr.dx);
+    if (end) d = zsub(d, cr.dy);
+    const z lm = j == 0 ? zmk(0.0, 0.0) : j == b - 1 ? cr.lm_last : j == 1 ? cr.lm_first : cr.lm_in;
 #pragma unroll
-    for (int e = 0; e < LC_CG; ++e) {
+    for (int e = 0; e < PV_CG; ++e) {
         const int c = c0 + e;
-        z x = zmk(0.0, 0.0);
-        if (r < a && c < a) {
-            if (c == r) x = d;
-            else if (c == r + 1) x = up;
-            else if (c == r - 1) x = lo;
-            if (j > 0) zfms(x, lm, prev[e]);
-        }
-        v[e] = x;
+        z x = c == r ? d : c == r + 1 ? cr.up : c == r - 1 ? cr.lo : zmk(0.0, 0.0);
+        zfms(x, lm, prev[e]);                        // prev is zero before block 1
+        v[e] = r < a && c < a ? x : zmk(0.0, 0.0);
     }
-}
-
-// One elimination step on a thread's 8 columns: q the pivot row's values there, mult = A(i,k) x
-// (-x for the pivot row itself); column `own` (if any) is the pivot column.
-__device__ __forceinline__ void chain_update(z& v, z q, z mult, bool is_p, bool is_k) {
-    z base = v;
-    if (is_p) base = zmk(0.0, 0.0);
-    zfms(base, mult, q);
-    v = is_k ? zneg(mult) : base;
-}
-
-// the pivot among the rows of one column: larger |re|+|im| wins (its bit pattern orders like the
-// value), then the smaller row; invalid rows take part as zeros with the largest index
-__device__ __forceinline__ int chain_pivot(z x, bool valid, int r) {
-    const double m = zabs1(x);
-    const unsigned hi = valid ? (unsigned)__double2hiint(m) : 0u;
-    const unsigned lo = valid ? (unsigned)__double2loint(m) : 0u;
-    const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
-    const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? lo : 0u);
-    return __reduce_min_sync(0xffffffffu, (valid && hi == mh && lo == ml) ? r : 0x7fff);
-}
-
-__device__ __forceinline__ z shfl_z(z v, int src) {
-    return zmk(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src));
 }
 
 // Blocks of up to 16 rows: one warp per leaf, lane = row + 16 * column group, no block barriers.
 __global__ void __launch_bounds__(128) leaf_chain16_kernel(LeafGeom g, int nleaves, const double* __restrict__ hh,
                                                            const z* __restrict__ kv, z* __restrict__ sinv, int* status) {
     __shared__ z blk[4][256];
-    __shared__ z prow[4][2][2 * LC_CG];
+    __shared__ z prow[4][32];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const int leaf = blockIdx.x * (blockDim.x >> 5) + wib;
     if (leaf >= nleaves) return;
@@ -393,54 +370,27 @@ __global__ void __launch_bounds__(128) leaf_chain16_kernel(LeafGeom g, int nleav
     const z* kl = kv + (size_t)leaf * a * b;
     z* Sl = sinv + (size_t)leaf * b * aa;
     const int r = lane & 15, hf = lane >> 4;
-    const ChainRow cr = chain_row(L, a, r);
-    z v[LC_CG], prev[LC_CG];
+    const ChainRow cr = chain_row(L, a, b, r);
+    z v[PV_CG], prev[PV_CG];
 #pragma unroll
-    for (int e = 0; e < LC_CG; ++e) prev[e] = zmk(0.0, 0.0);
+    for (int e = 0; e < PV_CG; ++e) prev[e] = zmk(0.0, 0.0);
     bool ok = true;
     z kn = r < a ? kl[r] : zmk(0.0, 0.0);
     for (int j = 0; j < b; ++j) {
-        const z lm = j > 0 ? zmul(block_lo(L, b, j + 1), block_up(L, b, j)) : zmk(0.0, 0.0);
-        chain_form(L, cr, a, b, j, r, LC_CG * hf, kn, lm, prev, v);
+        chain_form(cr, a, b, j, r, PV_CG * hf, kn, prev, v);
         if (j + 1 < b && r < a) kn = kl[(j + 1) * a + r];          // the next block's potential
-        bool used = r >= a;
-        int myk = 0, pk = 0;
+        int myk, pk;
+        if (!warp_invert16(v, a, prow[wib], myk, pk)) ok = false;
 #pragma unroll
-        for (int grp = 0; grp < 2; ++grp) {
-#pragma unroll
-            for (int e = 0; e < LC_CG; ++e) {
-                const int k = grp * LC_CG + e;
-                if (k >= a) break;
-                const bool mine = hf == grp;
-                const int p = chain_pivot(v[e], mine && !used, r);
-                const z f = shfl_z(v[e], r + 16 * grp);
-                const z pv = shfl_z(v[e], p + 16 * grp);
-                z* pr = prow[wib][k & 1];
-                if (r == p) {
-#pragma unroll
-                    for (int c = 0; c < LC_CG; ++c) pr[hf * LC_CG + c] = v[c];
-                }
-                if (pv.x == 0.0 && pv.y == 0.0) ok = false;
-                const z x = zrcp(pv);
-                const bool is_p = r == p;
-                const z mult = is_p ? zneg(x) : zmul(f, x);
-                if (is_p) { used = true; myk = k; }
-                if (lane == k) pk = p;
-                __syncwarp();
-#pragma unroll
-                for (int c = 0; c < LC_CG; ++c) chain_update(v[c], pr[hf * LC_CG + c], mult, is_p, mine && c == e);
-            }
-        }
-#pragma unroll
-        for (int e = 0; e < LC_CG; ++e) {
-            const int q = hf * LC_CG + e;
+        for (int e = 0; e < PV_CG; ++e) {
+            const int q = hf * PV_CG + e;
             const int pq = __shfl_sync(0xffffffffu, pk, q);
             if (r < a && q < a) sm[myk + pq * a] = v[e];
         }
         __syncwarp();
 #pragma unroll
-        for (int e = 0; e < LC_CG; ++e) {
-            const int q = hf * LC_CG + e;
+        for (int e = 0; e < PV_CG; ++e) {
+            const int q = hf * PV_CG + e;
             if (r < a && q < a) {
                 prev[e] = sm[r + q * a];
                 Sl[(size_t)j * aa + r + q * a] = prev[e];
@@ -448,91 +398,42 @@ __global__ void __launch_bounds__(128) leaf_chain16_kernel(LeafGeom g, int nleav
         }
         __syncwarp();
     }
-    if (!ok && lane == 0) atomicOr(status, RB_STATUS_ZERO_PIVOT);
+    if (!ok) atomicOr(status, RB_STATUS_ZERO_PIVOT);
 }
 
-// Blocks of 17 to 32 rows: one CTA of NG warps per leaf, lane = row, warp = column group.  The
-// warp that holds the next pivot column updates that column first, finds its pivot and publishes
-// it (its column, the pivot row and the reciprocal) before it updates its other columns, so one
-// block barrier per step is all the others wait for.
+// Blocks of 17 to 32 rows: one CTA of NG warps per leaf, lane = row, warp = column group.
 template <int NG>
 __global__ void __launch_bounds__(32 * NG) leaf_chain32_kernel(LeafGeom g, const double* __restrict__ hh,
                                                                const z* __restrict__ kv, z* __restrict__ sinv,
                                                                int* status) {
     __shared__ z sm[32 * 32];
-    __shared__ z prow[NG][2][LC_CG];
-    __shared__ z fcol[2][32];
-    __shared__ z pinv[2];
-    __shared__ int piv[2];
+    __shared__ PivotShared<1, NG> sh;
     const int leaf = blockIdx.x;
     const int r = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int a = g.a, b = g.b, aa = a * a;
     const LeafConst L = leaf_const(hh, leaf, g.kb);
     const z* kl = kv + (size_t)leaf * a * b;
     z* Sl = sinv + (size_t)leaf * b * aa;
-    const ChainRow cr = chain_row(L, a, r);
-    z v[LC_CG], prev[LC_CG];
+    const ChainRow cr = chain_row(L, a, b, r);
+    z v[1][PV_CG], prev[PV_CG];
 #pragma unroll
-    for (int e = 0; e < LC_CG; ++e) prev[e] = zmk(0.0, 0.0);
+    for (int e = 0; e < PV_CG; ++e) prev[e] = zmk(0.0, 0.0);
     bool ok = true;
     z kn = r < a ? kl[r] : zmk(0.0, 0.0);
     for (int j = 0; j < b; ++j) {
-        const z lm = j > 0 ? zmul(block_lo(L, b, j + 1), block_up(L, b, j)) : zmk(0.0, 0.0);
-        chain_form(L, cr, a, b, j, r, LC_CG * w, kn, lm, prev, v);
+        chain_form(cr, a, b, j, r, PV_CG * w, kn, prev, v[0]);
         if (j + 1 < b && r < a) kn = kl[(j + 1) * a + r];
-        bool used = r >= a;
-        int myk = 0, pk = 0;
-        // finds and publishes the pivot of column k, held by this warp in x
-        auto publish = [&](z x, int k) {
-            const int p = chain_pivot(x, !used, r);
-            const int s = k & 1;
-            fcol[s][r] = x;
-            if (r == p) {
-                if (x.x == 0.0 && x.y == 0.0) ok = false;
-                pinv[s] = zrcp(x);
-                piv[s] = p;
-            }
-        };
-        if (w == 0) publish(v[0], 0);
-        for (int grp = 0; grp < NG; ++grp) {
+        int myk[1];
+        if (!cta_invert<1, NG>(v, a, sh, myk)) ok = false;
 #pragma unroll
-            for (int e = 0; e < LC_CG; ++e) {
-                const int k = grp * LC_CG + e, s = k & 1;
-                if (k >= a) break;
-                __syncthreads();
-                const int p = piv[s];
-                const z x = pinv[s];
-                const z f = fcol[s][r];
-                const bool is_p = r == p;
-                z* pr = prow[w][s];
-                if (is_p) {
-#pragma unroll
-                    for (int c = 0; c < LC_CG; ++c) pr[c] = v[c];
-                }
-                const z mult = is_p ? zneg(x) : zmul(f, x);
-                if (is_p) { used = true; myk = k; }
-                if (r == k) pk = p;
-                __syncwarp();
-                const int en = (e + 1) % LC_CG;                    // the next pivot column
-                const bool next = k + 1 < a && w == (e + 1 == LC_CG ? grp + 1 : grp);
-                const bool mine = w == grp;
-                chain_update(v[en], pr[en], mult, is_p, false);
-                if (next) publish(v[en], k + 1);
-#pragma unroll
-                for (int c = 0; c < LC_CG; ++c)
-                    if (c != en) chain_update(v[c], pr[c], mult, is_p, mine && c == e);
-            }
-        }
-#pragma unroll
-        for (int e = 0; e < LC_CG; ++e) {
-            const int q = w * LC_CG + e;
-            const int pq = __shfl_sync(0xffffffffu, pk, q);
-            if (r < a && q < a) sm[myk + pq * a] = v[e];
+        for (int e = 0; e < PV_CG; ++e) {
+            const int q = w * PV_CG + e;
+            if (r < a && q < a) sm[myk[0] + sh.pk[q] * a] = v[0][e];
         }
         __syncthreads();
 #pragma unroll
-        for (int e = 0; e < LC_CG; ++e) {
-            const int q = w * LC_CG + e;
+        for (int e = 0; e < PV_CG; ++e) {
+            const int q = w * PV_CG + e;
             if (r < a && q < a) {
                 prev[e] = sm[r + q * a];
                 Sl[(size_t)j * aa + r + q * a] = prev[e];
