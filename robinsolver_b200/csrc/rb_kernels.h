@@ -135,8 +135,9 @@ cudaError_t merge_form_d(ChildStore c, int nnodes, int m, int o2, z zeta, z* dst
 // S = zeta*I - T1_ii - nu^2 * Dinv for every parent node (child1 = 2*node).
 cudaError_t merge_form_s(ChildStore c, int nnodes, int m, int o1, z zeta, z nu, const z* dinv, z* dst,
                          cudaStream_t s);
-// K = nu^2 I for every node, into dst + node*m*m.
-cudaError_t merge_form_k(int nnodes, int m, z nu, z* dst, cudaStream_t s);
+// K form: A2 = zeta*I - T2_ii, A1 = zeta*I - T1_ii, K = nu^2 I for every parent node.
+cudaError_t merge_form_kform_level(ChildStore c, int nnodes, int m, int o1, int o2, z zeta, z nu, z* a2, z* a1, z* k,
+                                   cudaStream_t s);
 // The three K-form merge inputs of one node of any tree and level (a forest's batched merge).
 struct MergeFormDesc {
     const z* t1;       // child1's Robin-to-Robin matrix
@@ -148,6 +149,20 @@ struct MergeFormDesc {
     z* a1;             // zeta I - T1_ii
     z* k;              // nu^2 I
 };
+// K-form merge of one level with a small interface (rb_merge.cu): A1, A2 and K^-1 of every node
+// (m <= MERGE_SMALL_MAX), and its Y1, Y2 and parent map (m <= MERGE_COLUMNS_MAX; par null: no map).
+constexpr int MERGE_SMALL_MAX = 32;
+constexpr int MERGE_COLUMNS_MAX = 16;
+struct MergeSmall {
+    ChildStore child;
+    int nnodes, m, o1, o2, n1, n2, nbp;
+    const int* pmap1;
+    const int* pmap2;
+    z zeta, nu;
+    z *a2, *a1, *kinv, *y1, *y2, *par;
+};
+cudaError_t merge_small_interface(const MergeSmall& g, int* status, cudaStream_t s);
+cudaError_t merge_small_columns(const MergeSmall& g, cudaStream_t s);
 cudaError_t merge_form_kform_batch(const MergeFormDesc* d_descs, int count, int max_m, cudaStream_t s);
 
 // ---- device-side sampling and check_solution (rb_sample.cu) -------------------------------------------

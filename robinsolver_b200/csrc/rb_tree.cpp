@@ -290,7 +290,7 @@ static int ensure_factor_storage(rb_tree* t) {
     for (int l = 0; l <= L; ++l) RB_CK(cudaEventCreateWithFlags(&t->ev_lvl[l], cudaEventDisableTiming));
     if (!t->ev_root_forms) RB_CK(cudaEventCreateWithFlags(&t->ev_root_forms, cudaEventDisableTiming));
     if (!t->ev_root_gj) RB_CK(cudaEventCreateWithFlags(&t->ev_root_gj, cudaEventDisableTiming));
-    for (auto* v : {&t->ev_face, &t->ev_rest, &t->ev_d, &t->ev_m1, &t->ev_m3}) {
+    for (auto* v : {&t->ev_face, &t->ev_rest, &t->ev_m1, &t->ev_m3}) {
         v->assign(L + 1, nullptr);
         for (auto& e : *v) RB_CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     }
@@ -446,8 +446,15 @@ static int ensure_factor_storage(rb_tree* t) {
                     g.C = zview(kv, m); g.beta = one;
                     mk.push_back(g);
                 }
-                // B1 = -A2 T1_iN, held in Y2's first n1 columns until Y2 is formed
-                m1.push_back(gdesc(m, n1, m, zview(dv, m), t1in, zout(y2, m), mone));
+                {   // B1 = -A2 T1_iN = T2_ii T1_iN - zeta T1_iN, held in Y2's first n1 columns until Y2 is
+                    // formed: it reads the children's maps only, not A2
+                    GemmDesc g = gdesc(m, n1, m, zview(r2 + o2 + (long long)o2 * ld, ld), t1in, zout(y2, m), one);
+                    if (t->zeta.x != 0.0 || t->zeta.y != 0.0) {
+                        g.C = t1in;
+                        g.beta = zneg(t->zeta);
+                    }
+                    m1.push_back(g);
+                }
                 // Y1 = [K^-1 B1, nu K^-1 T2_iN]
                 m2.push_back(gdesc(m, n1, m, zview(kv, m), zview(y2, m), zout(y1, m), one));
                 m2.push_back(gdesc(m, n2, m, zview(kv, m), t2in, zout(y1 + (long long)m * n1, m), t->nu));
@@ -688,6 +695,22 @@ static bool factor_pipelined(const rb_tree* t) {
     return !off && t->timing == 0 && t->kform && t->P.L >= 2;
 }
 
+// Levels whose interface has up to 32 points form and invert K in one launch, up to 16 points the
+// rest of the merge in another (rb_merge.cu), in either schedule.
+static bool small_merge(const rb_tree* t, int l) { return t->kform && t->P.lv[l].m <= MERGE_SMALL_MAX; }
+static bool small_columns(const rb_tree* t, int l) { return small_merge(t, l) && t->P.lv[l].m <= MERGE_COLUMNS_MAX; }
+static MergeSmall small_merge_args(const rb_tree* t, int l) {
+    const PlanLevel& p = t->P.lv[l];
+    return MergeSmall{child_store(t, l), p.nnodes, p.m, p.o1, p.o2, p.n1, p.n2, p.nb, t->d_pmap1[l], t->d_pmap2[l],
+                      t->zeta, t->nu, t->dinv[l], t->sinv[l], t->kinv[l], t->Y1[l], t->Y2[l], t->rtr[l]};
+}
+// algorithmic flops of the two launches: K and its inverse; B1, Y1, Y2 and the map
+static double small_interface_flops(const PlanLevel& p) { return 16.0 * p.m * p.m * p.m * p.nnodes; }
+static double small_columns_flops(const PlanLevel& p, bool map) {
+    const double n = p.n1 + p.n2;
+    return 8.0 * p.nnodes * p.m * (p.m * (p.n1 + 2.0 * n) + (map ? n * n : 0.0));
+}
+
 static int run_merges_pipelined(rb_tree* t, const std::vector<cudaEvent_t>* rec,
                                 const std::function<int()>* before_root_tail) {
     const Plan& P = t->P;
@@ -701,14 +724,42 @@ static int run_merges_pipelined(rb_tree* t, const std::vector<cudaEvent_t>* rec,
         const PlanLevel& p = P.lv[l];
         const ChildStore cs = child_store(t, l);
         RB_CK(cudaStreamWaitEvent(c, t->ev_face[l + 1], 0));
-        RB_LAUNCH(merge_form_d(cs, p.nnodes, p.m, p.o2, t->zeta, t->dinv[l], c));
+        if (!small_columns(t, l)) {
+            RB_CK(cudaStreamWaitEvent(s4, t->ev_face[l + 1], 0));
+            RB_LAUNCH(launch_gemm_level(t, t->fM1[l], l, s4));      // B1 = -A2 T1_iN
+            RB_CK(cudaEventRecord(t->ev_m1[l], s4));
+        }
+        if (small_merge(t, l)) {
+            // too little work to split the map: the whole level on the chain stream
+            const MergeSmall g = small_merge_args(t, l);
+            RB_LAUNCH(merge_small_interface(g, t->d_status, c));
+            if (rec && l == 0) RB_CK(cudaEventRecord(t->ev_root_forms, c));
+            if (rec) RB_CK(cudaEventRecord((*rec)[l], c));
+            if (!small_columns(t, l)) RB_CK(cudaStreamWaitEvent(c, t->ev_m1[l], 0));
+            RB_CK(cudaStreamWaitEvent(c, t->ev_rest[l + 1], 0));
+            cudaStream_t cs2 = c;
+            if (l == 0) {
+                RB_CK(cudaEventRecord(t->ev_root_gj, c));
+                RB_CK(cudaStreamWaitEvent(s, t->ev_root_gj, 0));   // joins both side streams
+                if (before_root_tail && (rc = (*before_root_tail)())) return rc;
+                cs2 = s;
+            }
+            if (small_columns(t, l)) {
+                RB_LAUNCH(merge_small_columns(g, cs2));
+            } else {
+                RB_LAUNCH(launch_gemm_level(t, t->fM2[l], l, cs2));
+                RB_LAUNCH(launch_gemm_level(t, t->fM3[l], l, cs2));
+                RB_LAUNCH(launch_gemm_level(t, t->fM4[l], l, cs2));
+            }
+            if (l > 0) {
+                RB_CK(cudaEventRecord(t->ev_face[l], c));
+                RB_CK(cudaEventRecord(t->ev_rest[l], c));
+            }
+            continue;
+        }
+        RB_LAUNCH(merge_form_kform_level(cs, p.nnodes, p.m, p.o1, p.o2, t->zeta, t->nu, t->dinv[l], t->sinv[l], t->kinv[l],
+                                         c));
         if (rec && l == 0) RB_CK(cudaEventRecord(t->ev_root_forms, c));
-        RB_CK(cudaEventRecord(t->ev_d[l], c));
-        RB_CK(cudaStreamWaitEvent(s4, t->ev_d[l], 0));
-        RB_LAUNCH(launch_gemm_level(t, t->fM1[l], l, s4));          // B1 = -A2 T1_iN
-        RB_CK(cudaEventRecord(t->ev_m1[l], s4));
-        RB_LAUNCH(merge_form_s(cs, p.nnodes, p.m, p.o1, t->zeta, zmk(0.0, 0.0), t->dinv[l], t->sinv[l], c));
-        RB_LAUNCH(merge_form_k(p.nnodes, p.m, t->nu, t->kinv[l], c));
         RB_LAUNCH(launch_gemm_level(t, t->fK[l], l, c));
         RB_LAUNCH(gj_invert_batch(t->gj_k[l].d_desc, p.nnodes, p.m, t->gj_work, t->d_status, c));
         // a solve's sweep at this level also waits for ev_rest[l + 1] (run_solve)
@@ -774,13 +825,29 @@ static int run_factor(rb_tree* t, const z* dk, const std::vector<cudaEvent_t>* r
         const PlanLevel& p = P.lv[l];
         const ChildStore cs = child_store(t, l);
         if ((rc = timer_begin(t, l < 17 ? lvl_names[l] : "merge_deep"))) return rc;
+        if (small_merge(t, l)) {
+            const MergeSmall g = small_merge_args(t, l);
+            RB_TIMED("merge_small_if", small_interface_flops(p), merge_small_interface(g, t->d_status, s));
+            if (rec && l == 0) RB_CK(cudaEventRecord(t->ev_root_forms, s));
+            if (rec) RB_CK(cudaEventRecord((*rec)[l], s));
+            if (l == 0 && before_root_tail && (rc = (*before_root_tail)())) return rc;
+            if (small_columns(t, l)) {
+                RB_TIMED("merge_small", small_columns_flops(p, g.par != nullptr), merge_small_columns(g, s));
+            } else {
+                RB_GEMM_L(t->fM1[l], l, s);
+                RB_GEMM_L(t->fM2[l], l, s);
+                RB_GEMM_L(t->fM3[l], l, s);
+                RB_GEMM_L(t->fM4[l], l, s);
+            }
+            if ((rc = timer_end(t))) return rc;
+            continue;
+        }
         if (t->kform) {
             // A2 = zeta I - T2_ii, A1 = zeta I - T1_ii; B1 = -A2 T1_iN on the second stream beside
             // K = nu^2 I - A2 A1 and its inversion
-            RB_TIMED("merge_form", 0.0, merge_form_d(cs, p.nnodes, p.m, p.o2, t->zeta, t->dinv[l], s));
+            RB_TIMED("merge_form", 0.0, merge_form_kform_level(cs, p.nnodes, p.m, p.o1, p.o2, t->zeta, t->nu, t->dinv[l],
+                                                               t->sinv[l], t->kinv[l], s));
             if (rec && l == 0) RB_CK(cudaEventRecord(t->ev_root_forms, s));
-            RB_TIMED("merge_form", 0.0, merge_form_s(cs, p.nnodes, p.m, p.o1, t->zeta, zmk(0.0, 0.0), t->dinv[l],
-                                                     t->sinv[l], s));
             const bool fork = t->timing == 0;
             if (fork) {
                 RB_CK(cudaEventRecord(t->ev_fork[l], s));
@@ -788,7 +855,6 @@ static int run_factor(rb_tree* t, const z* dk, const std::vector<cudaEvent_t>* r
                 RB_LAUNCH(launch_gemm_level(t, t->fM1[l], l, t->stream2));
                 RB_CK(cudaEventRecord(t->ev_join[l], t->stream2));
             }
-            RB_TIMED("merge_form", 0.0, merge_form_k(p.nnodes, p.m, t->nu, t->kinv[l], s));
             RB_GEMM_L(t->fK[l], l, s);
             RB_TIMED("gj_invert", gj_flops(p.m, p.nnodes),
                      gj_invert_batch(t->gj_k[l].d_desc, p.nnodes, p.m, t->gj_work, t->d_status, s));
@@ -1460,7 +1526,7 @@ int rb_tree_destroy(rb_tree* t) {
     for (auto& e : t->ev_fork) if (e) cudaEventDestroy(e);
     for (auto& e : t->ev_join) if (e) cudaEventDestroy(e);
     for (auto& e : t->ev_lvl) if (e) cudaEventDestroy(e);
-    for (auto* v : {&t->ev_face, &t->ev_rest, &t->ev_d, &t->ev_m1, &t->ev_m3})
+    for (auto* v : {&t->ev_face, &t->ev_rest, &t->ev_m1, &t->ev_m3})
         for (auto& e : *v) if (e) cudaEventDestroy(e);
     if (t->ev_root_gj) cudaEventDestroy(t->ev_root_gj);
     if (t->ev_root_forms) cudaEventDestroy(t->ev_root_forms);

@@ -120,7 +120,7 @@ struct rb_tree {
     // (fM4N), so that the parent level's forms, K and inversion run beside fM4N (levels 1..L-1)
     std::vector<GemmBatch> fM4F, fM4N;
     cudaStream_t stream4 = nullptr;      // the pipelined factor's B1 product beside the inversion
-    std::vector<cudaEvent_t> ev_face, ev_rest, ev_d, ev_m1, ev_m3;   // per level
+    std::vector<cudaEvent_t> ev_face, ev_rest, ev_m1, ev_m3;   // per level
     cudaEvent_t ev_root_gj = nullptr;
     bool factor_was_pipelined = false;   // the last factor ran the pipelined schedule
     bool factor_ready = false;
