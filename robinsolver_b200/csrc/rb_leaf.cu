@@ -117,6 +117,19 @@ __device__ __forceinline__ z block_up(const LeafConst& L, int b, int jj) {
     return v;
 }
 
+// Lo_j and Up_j of every block, formed once (block_lo and block_up divide)
+struct BlockCoupling {
+    z lo_in, lo_last, up_first, up_in;
+    int b;
+    __device__ __forceinline__ BlockCoupling(const LeafConst& L, int b_) : b(b_) {
+        lo_in = up_in = zmk(1.0 / L.hy2, 0.0);       // stencil1 inside
+        lo_last = block_lo(L, b, b);
+        up_first = block_up(L, b, 1);
+    }
+    __device__ __forceinline__ z lo(int jj) const { return jj == b ? lo_last : lo_in; }
+    __device__ __forceinline__ z up(int jj) const { return jj == 1 ? up_first : up_in; }
+};
+
 // In-place Gauss-Jordan inverse of an m x m column-major matrix in shared memory by the whole
 // CTA (partial pivoting by |re|+|im|, first maximum).  Returns false on an exactly zero pivot.
 __device__ bool cta_gj_invert(z* S, int m, z* fcol, int* ipiv, int* sp) {
@@ -304,8 +317,8 @@ size_t leaf_block_factor_smem(const LeafGeom& g) {
 // restored once per block, on the way through shared memory.
 // Latency-bound: 4.3 us a block of 16 rows (69 us a 16x16 leaf, 345 us for 4096 leaves), 13.9 us a
 // block of 32 (445 us a 32x32 leaf).  One warp or CTA forming Sig_j^-1 and both sweeps of a leaf took
-// 406 us for 16 leaves of 16x16 (now 116 with leaf_sweep), 2.25 ms for 4096 (now 1.39), and 6.6 ms
-// for 64 leaves of 32x32 (now 0.75).
+// 406 us for 16 leaves of 16x16 (now 105 with leaf_sweep), 2.25 ms for 4096 (now 1.28), and 6.6 ms
+// for 64 leaves of 32x32 (now 0.71).
 
 // what one row of the diagonal blocks D_j is made of, formed once per leaf: the chain pays for
 // every division of a block
@@ -453,23 +466,61 @@ __global__ void __launch_bounds__(32 * NG) leaf_chain32_kernel(LeafGeom g, const
 // products per complex one).  The k order of the MMAs is chosen so that the accumulator layout
 // (row lane/4, columns 2 (lane%4) + {0,1}) is the next step's A fragment as it stands: k-step
 // (t, h) sums the rows q = 8t + 2 (lane%4) + h of the block, so nothing moves between steps.  The
-// blocks stream through shared memory, double-buffered with cp.async, padded with zeros to
-// multiples of 8 and with an odd leading dimension (conflict-free 16-byte fragment loads).
+// blocks stream through shared memory in a ring of cp.async stages, padded with zeros to multiples of
+// 8 and with an odd leading dimension (conflict-free 16-byte fragment loads).
+// Measured: 16 leaves of 16x16 36 us, 4096 of them 0.93 ms (17.2 GFLOP, 18 TFLOP/s; two CTAs of 8 warps
+// per SM, three spill: 1.02); 64 leaves of 32x32 260 us.
 // C_j holds, per right-hand side, c1 and c2 at the interior points next to its boundary point.
 template <int NT>
 struct SweepCfg {
     static constexpr int AP = 8 * NT;            // padded block size
     static constexpr int LD = AP + 1;
-    static constexpr size_t SMEM = 2 * (size_t)AP * LD * sizeof(z);
+    static constexpr int STAGES = NT <= 2 ? 4 : 3;
+    static constexpr size_t SMEM = STAGES * (size_t)AP * LD * sizeof(z);
+};
+
+// The ring of a leaf's blocks in the order of a forward and a backward sweep: 0..b-1, b-2..0.
+template <int NT>
+struct BlockRing {
+    using Cfg = SweepCfg<NT>;
+    z* sm;
+    const z* Sl;
+    int a, aa, b, nsteps;
+    __device__ __forceinline__ void issue(int st) {
+        if (st < nsteps) {
+            const int j = st < b ? st : 2 * b - 2 - st;
+            const z* src = Sl + (size_t)j * aa;
+            z* dst = sm + (st % Cfg::STAGES) * Cfg::AP * Cfg::LD;
+            // a warp copies CPW columns at a time (no division by a: one warp may copy it all)
+            constexpr int CPW = NT == 1 ? 4 : NT == 2 ? 2 : 1;
+            const int i = threadIdx.x & (32 / CPW - 1);
+            if (i < a)
+                for (int c = threadIdx.x / (32 / CPW); c < a; c += blockDim.x / (32 / CPW))
+                    cp_async16(dst + i + c * Cfg::LD, src + i + c * a, 16);
+        }
+        cp_async_commit();
+    }
+    __device__ __forceinline__ void start() {
+        for (int e = threadIdx.x; e < Cfg::STAGES * Cfg::AP * Cfg::LD; e += blockDim.x) sm[e] = zmk(0.0, 0.0);
+        __syncthreads();
+        for (int st = 0; st < Cfg::STAGES - 1; ++st) issue(st);
+    }
+    // the block of step st, and the fetch of the block STAGES - 1 steps on
+    __device__ __forceinline__ const z* next(int st) {
+        cp_async_wait<Cfg::STAGES - 2>();
+        __syncthreads();               // block st landed; every warp is past step st-1's reads
+        issue(st + Cfg::STAGES - 1);
+        return sm + (st % Cfg::STAGES) * Cfg::AP * Cfg::LD;
+    }
 };
 
 template <int NT>
-__global__ void __launch_bounds__(256) leaf_sweep_kernel(LeafGeom g, int nchunk, const double* __restrict__ hh,
+__global__ void __launch_bounds__(256, NT <= 3 ? 2 : 1) leaf_sweep_kernel(LeafGeom g, int nchunk, const double* __restrict__ hh,
                                                          const z* __restrict__ sinv, z* __restrict__ Y) {
     using Cfg = SweepCfg<NT>;
     constexpr int LD = Cfg::LD;
     extern __shared__ z sm[];
-    const int tid = threadIdx.x, nthr = blockDim.x, lane = tid & 31, warp = tid >> 5;
+    const int nthr = blockDim.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int lr = lane >> 2, lc = lane & 3;
     const int leaf = blockIdx.x / nchunk, chunk = blockIdx.x % nchunk;
     const int a = g.a, b = g.b, nb = g.nb, n = g.n, aa = a * a;
@@ -477,19 +528,9 @@ __global__ void __launch_bounds__(256) leaf_sweep_kernel(LeafGeom g, int nchunk,
     const z* Sl = sinv + (size_t)leaf * b * aa;
     z* Yl = Y + (size_t)leaf * nb * n;
     const int nsteps = 2 * b - 1;
-    for (int e = tid; e < 2 * Cfg::AP * LD; e += nthr) sm[e] = zmk(0.0, 0.0);
-    __syncthreads();
-    auto issue = [&](int st) {
-        const int j = st < b ? st : 2 * b - 2 - st;
-        const z* src = Sl + (size_t)j * aa;
-        z* dst = sm + (st & 1) * Cfg::AP * LD;
-        for (int e = tid; e < aa; e += nthr) {
-            const int c = e / a;
-            cp_async16(dst + (e - c * a) + c * LD, src + e, 16);
-        }
-        cp_async_commit();
-    };
-    issue(0);
+    BlockRing<NT> ring{sm, Sl, a, aa, b, nsteps};
+    ring.start();
+    const BlockCoupling cpl(L, b);
     // this lane's right-hand side and its two interior points
     const int row = (chunk * (nthr >> 5) + warp) * 8 + lr;
     const bool live = row < nb;
@@ -527,9 +568,7 @@ __global__ void __launch_bounds__(256) leaf_sweep_kernel(LeafGeom g, int nchunk,
     for (int st = 0; st < nsteps; ++st) {
         const bool fwd = st < b;
         const int j = fwd ? st : 2 * b - 2 - st;
-        cp_async_wait<0>();
-        __syncthreads();               // block st landed; every warp is past step st-1's reads
-        if (st + 1 < nsteps) issue(st + 1);
+        const z* S = ring.next(st) + 2 * lc + lr * LD;
         double cre[NT][2], cim[NT][2];
 #pragma unroll
         for (int t = 0; t < NT; ++t)
@@ -547,7 +586,6 @@ __global__ void __launch_bounds__(256) leaf_sweep_kernel(LeafGeom g, int nchunk,
                 vn[e] = (live && i < a) ? Yr[(size_t)(nb + jn * a + i) * nb] : zmk(0.0, 0.0);
             }
         }
-        const z* S = sm + (st & 1) * Cfg::AP * LD + 2 * lc + lr * LD;
 #pragma unroll
         for (int e = 0; e < 2 * NT; ++e) {           // k-step (t, h): rows 8t + 2lc + h of the block
             z bf[NT];
@@ -564,7 +602,7 @@ __global__ void __launch_bounds__(256) leaf_sweep_kernel(LeafGeom g, int nchunk,
         }
         // next R: C_{j+1} - Up_j V_j forward, -Lo_j Z_j backward (Lo_j couples block j to j-1)
         const bool up = fwd && j + 1 < b;
-        const z co = up ? block_up(L, b, j + 1) : block_lo(L, b, j + 1);
+        const z co = up ? cpl.up(j + 1) : cpl.lo(j + 1);
         const bool fin = !up;
         const int qn = (j + 1) * a;
 #pragma unroll
@@ -634,17 +672,6 @@ cudaError_t leaf_block_factor(const LeafGeom& g, int nleaves, const double* h, c
 // Leaf solve: u = A^-1 [g; f] for every leaf and right-hand side into sol [rhs][leaf][n].
 // RHS are processed in chunks of KC columns; shared memory: sig (a^2), w0, w1 (a x KC each).
 constexpr int LEAF_KC = 32;
-
-// leaf solve engine: the half-warp kernel for 16-point leaves (default) or the block kernel
-// (RB_LEAF_SOLVE=block, read once; a comparison knob)
-static bool leaf_solve_engine_hw() {
-    static int v = -1;
-    if (v < 0) {
-        const char* e = std::getenv("RB_LEAF_SOLVE");
-        v = (e && std::strcmp(e, "block") == 0) ? 0 : 1;
-    }
-    return v == 1;
-}
 
 __global__ void __launch_bounds__(256) leaf_block_solve_kernel(LeafGeom g, int nleaves, int nrhs,
                                                                const double* __restrict__ hh,
@@ -726,154 +753,157 @@ __global__ void __launch_bounds__(256) leaf_block_solve_kernel(LeafGeom g, int n
     }
 }
 
-// The same solve for leaves 16 points wide (a == 16), one CTA of 8 warps per leaf and 32
-// right-hand sides at a time.  Each half-warp owns a right-hand side column, lane i its row i,
-// so a block step's recurrence stays in the lane's registers and its 16-term products exchange
-// values through shared memory within the warp.  The next step's Sig_j^-1 block and its right-hand
-// side block (f_j forward, the stored w_j backward) are fetched with cp.async while the current
-// step runs: one block barrier per step, which also releases the buffer the next fetch
-// overwrites.  Same operations in the same order as leaf_block_solve_kernel.
-constexpr int LHW_KC = 32;
-__global__ void __launch_bounds__(256, 3) leaf_hw_solve_kernel(LeafGeom g, int nleaves, int nrhs,
-                                                            const double* __restrict__ hh,
-                                                            const z* __restrict__ f, const z* __restrict__ gb,
-                                                            const z* __restrict__ sinv, z* __restrict__ sol) {
-    constexpr int A = 16, AA = A * A, KC = LHW_KC, CPH = KC / 16;   // columns per half-warp
+// The same solve for blocks of up to 32 x 32 on the FP64 tensor cores, with leaf_sweep's layout: a warp
+// takes 8 right-hand sides of a leaf through all block steps with the running block vector in
+// registers,
+//   forward:  w_j = Sig_j^-1 (t_j - Lo_j w_{j-1}),  t = f - A_ib A_bb^-1 g
+//   backward: x_{b-1} = w_{b-1};  x_j = w_j - Sig_j^-1 Up_j x_{j+1},
+// each step W^T (8 x a) = T^T (8 x a) Sig_j^-T (four real products per complex one).  The warps of a
+// CTA share a leaf's staged blocks.  The right-hand side (f forward, the stored w backward) is read
+// two steps ahead.  A right-hand side's operations do not depend on the others of its warp.
+// Measured: 4096 leaves of 16x16, 32 right-hand sides 0.69 ms (3 GB of loads and stores; half-warp
+// DFMA columns 0.76), 1024 leaves, 16: 102 us (205); 1024 leaves of 24x24, 64: 1.14 ms (one CTA per
+// leaf with scalar products 1.85); 64 leaves of 32x32, one: 205 us.  Two CTAs of 8 warps per SM: at
+// three (80 registers) the spills cost more (0.85 ms).
+template <int NT>
+__global__ void __launch_bounds__(256, NT <= 3 ? 2 : 1) leaf_solve_kernel(LeafGeom g, int nleaves, int nrhs, int nchunk,
+                                                         const double* __restrict__ hh, const z* __restrict__ f,
+                                                         const z* __restrict__ gb, const z* __restrict__ sinv,
+                                                         z* __restrict__ sol) {
+    using Cfg = SweepCfg<NT>;
+    constexpr int LD = Cfg::LD;
     extern __shared__ z sm[];
-    const int leaf = blockIdx.x;
-    const int b = g.b, nb = g.nb, n = g.n, ab = A * b;
-    z* sig = sm;                       // [2][AA]: Sig_j^-1 of the current and the next step
-    z* blk = sig + 2 * AA;             // [2][A*KC]: the steps' right-hand side blocks
-    z* gsm = blk + 2 * A * KC;         // [KC][nb]: boundary data of the chunk
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int i = lane & 15, half = lane >> 4;
+    const int nthr = blockDim.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int lr = lane >> 2, lc = lane & 3;
+    const int leaf = blockIdx.x / nchunk, chunk = blockIdx.x % nchunk;
+    const int a = g.a, b = g.b, nb = g.nb, n = g.n, ab = a * b, aa = a * a;
     const LeafConst L = leaf_const(hh, leaf, g.kb);
-    const z* Sl = sinv + (size_t)leaf * b * AA;
+    const int nsteps = 2 * b - 1;
+    BlockRing<NT> ring{sm, sinv + (size_t)leaf * b * aa, a, aa, b, nsteps};
+    ring.start();
+    const BlockCoupling cpl(L, b);
+    const int rh0 = (chunk * (nthr >> 5) + warp) * 8, rh = rh0 + lr;
+    const bool live = rh < nrhs;
+    const int rs = live ? rh : 0;
+    const z* fl = f ? f + ((size_t)rs * nleaves + leaf) * ab : nullptr;
+    const z* gl = gb + ((size_t)leaf * nrhs + rs) * nb;
+    z* ul = sol + ((size_t)rs * nleaves + leaf) * n;
     const z wdx = zscale(L.wbx, L.rdx), wdy = zscale(L.wby, L.rdy);
-    const int nsteps = 2 * b - 1;      // forward blocks 0..b-1, then backward blocks b-2..0
-    for (int r0 = 0; r0 < nrhs; r0 += KC) {
-        const int kc = min(KC, nrhs - r0);
-        auto issue = [&](int st) {
-            const int j = st < b ? st : 2 * b - 2 - st;
-            z* sd = sig + (st & 1) * AA;
-            for (int e = tid; e < AA; e += 256) cp_async16(sd + e, Sl + (size_t)j * AA + e, 16);
-            z* bd = blk + (st & 1) * A * KC;
-            for (int e = tid; e < A * KC; e += 256) {
-                const int q = e % A, rc = e / A, rh = r0 + rc;
-                const z* src = nullptr;
-                if (rc < kc) {
-                    if (st >= b) src = sol + ((size_t)rh * nleaves + leaf) * n + nb + j * A + q;
-                    else if (f) src = f + ((size_t)rh * nleaves + leaf) * ab + j * A + q;
-                }
-                cp_async16(bd + e, src ? src : Sl, src ? 16 : 0);
-            }
-        };
-        for (int e = tid; e < nb * KC; e += 256) {
-            const int r = e % nb, rc = e / nb;
-            const bool ok = rc < kc;
-            cp_async16(gsm + e, ok ? gb + ((size_t)leaf * nrhs + r0 + rc) * nb + r : gb, ok ? 16 : 0);
-        }
-        issue(0);
-        cp_async_commit();
-        z w[CPH];                      // this lane's entry of the running block vector per column
+    // this lane's part of step st's right-hand side
+    auto fetch = [&](int st, z (&v)[2 * NT]) {
+        const bool fwd = st < b;
+        const int j = fwd ? st : 2 * b - 2 - st;
 #pragma unroll
-        for (int c = 0; c < CPH; ++c) w[c] = zmk(0.0, 0.0);
-        for (int st = 0; st < nsteps; ++st) {
-            cp_async_wait<0>();
-            __syncthreads();           // step st's blocks landed; every thread is past step st-1
-            if (st + 1 < nsteps) issue(st + 1);
-            cp_async_commit();
-            const z* S = sig + (st & 1) * AA;
-            z* B = blk + (st & 1) * A * KC;
-            if (st < b) {
-                // forward: w_j = Sig_j^-1 (t_j - Lo_j w_{j-1}),  t = f - A_ib A_bb^-1 g
-                const int j = st, jj = j + 1;
-                const z lam = jj > 1 ? block_lo(L, b, jj) : zmk(0.0, 0.0);
-#pragma unroll
-                for (int c = 0; c < CPH; ++c) {
-                    const int rc = warp * (2 * CPH) + half + 2 * c;
-                    const z* gl = gsm + rc * nb;
-                    z t = B[i + rc * A];
-                    if (i == 0) zfms(t, wdx, gl[j]);
-                    if (i == A - 1) zfms(t, wdx, gl[b + j]);
-                    if (jj == 1) zfms(t, wdy, gl[2 * b + i]);
-                    if (jj == b) zfms(t, wdy, gl[2 * b + A + i]);
-                    if (jj > 1) zfms(t, lam, w[c]);
-                    B[i + rc * A] = t;
-                }
-                __syncwarp();
-                z acc[CPH];
-#pragma unroll
-                for (int c = 0; c < CPH; ++c) acc[c] = zmk(0.0, 0.0);
-#pragma unroll
-                for (int q = 0; q < A; ++q) {
-                    const z sq = S[i + q * A];
-#pragma unroll
-                    for (int c = 0; c < CPH; ++c) zfma(acc[c], sq, B[q + (warp * (2 * CPH) + half + 2 * c) * A]);
-                }
-#pragma unroll
-                for (int c = 0; c < CPH; ++c) {
-                    const int rc = warp * (2 * CPH) + half + 2 * c;
-                    w[c] = acc[c];
-                    if (rc < kc) sol[((size_t)(r0 + rc) * nleaves + leaf) * n + nb + j * A + i] = acc[c];
-                }
-            } else {
-                // backward: x_{b-1} = w_{b-1}; x_j = w_j - Sig_j^-1 Up_j x_{j+1}
-                const int j = 2 * b - 2 - st;
-                const z mu = block_up(L, b, j + 1);
-                z wj[CPH];
-#pragma unroll
-                for (int c = 0; c < CPH; ++c) {
-                    const int rc = warp * (2 * CPH) + half + 2 * c;
-                    wj[c] = B[i + rc * A];
-                    B[i + rc * A] = w[c];          // x_{j+1}, read by the other lanes of the half
-                }
-                __syncwarp();
-#pragma unroll
-                for (int q = 0; q < A; ++q) {
-                    const z sq = S[i + q * A];
-#pragma unroll
-                    for (int c = 0; c < CPH; ++c)
-                        zfms(wj[c], sq, zmul(mu, B[q + (warp * (2 * CPH) + half + 2 * c) * A]));
-                }
-#pragma unroll
-                for (int c = 0; c < CPH; ++c) {
-                    const int rc = warp * (2 * CPH) + half + 2 * c;
-                    w[c] = wj[c];
-                    if (rc < kc) sol[((size_t)(r0 + rc) * nleaves + leaf) * n + nb + j * A + i] = wj[c];
-                }
+        for (int e = 0; e < 2 * NT; ++e) {
+            const int i = 8 * (e >> 1) + 2 * lc + (e & 1);
+            v[e] = zmk(0.0, 0.0);
+            if (live && i < a && st < nsteps) {
+                if (!fwd) v[e] = ul[nb + j * a + i];
+                else if (fl) v[e] = fl[j * a + i];
             }
         }
-        cp_async_wait<0>();
-        __syncthreads();               // every interior value of the chunk is stored
-        // boundary values u_b = (g - c1 u(p1) - c2 u(p2)) / d
-        for (int e = tid; e < nb * kc; e += 256) {
-            const int r = e % nb, rc = e / nb, rh = r0 + rc;
-            int ax, p1, p2;
-            leaf_bpoint2(A, b, r, ax, p1, p2);
-            const double h = ax == 0 ? L.hx : L.hy;
-            z* u = sol + ((size_t)rh * nleaves + leaf) * n;
-            z v = gsm[rc * nb + r];
-            v = zsub(v, zadd(zscale(-3.0 / h, u[nb + p1]), zscale((1.0 / 3.0) / h, u[nb + p2])));
-            u[r] = zmul(v, ax == 0 ? L.rdx : L.rdy);
+    };
+    // and what the boundary data adds to it in a forward step
+    auto gfetch = [&](int j, z (&v)[2 * NT]) {
+#pragma unroll
+        for (int e = 0; e < 2 * NT; ++e) {
+            const int i = 8 * (e >> 1) + 2 * lc + (e & 1);
+            if (!live || i >= a || j >= b) continue;
+            if (i == 0) zfms(v[e], wdx, gl[j]);
+            if (i == a - 1) zfms(v[e], wdx, gl[b + j]);
+            if (j == 0) zfms(v[e], wdy, gl[2 * b + i]);
+            if (j == b - 1) zfms(v[e], wdy, gl[2 * b + a + i]);
         }
-        __syncthreads();               // the buffers are refilled for the next chunk
+    };
+    z t0[2 * NT], t1[2 * NT];              // right-hand sides of the current and the next step
+    fetch(0, t0);
+    gfetch(0, t0);
+    fetch(1, t1);
+    gfetch(1, t1);
+    double wre[2 * NT], wim[2 * NT];       // the running block vector
+#pragma unroll
+    for (int e = 0; e < 2 * NT; ++e) wre[e] = wim[e] = 0.0;
+    for (int st = 0; st < nsteps; ++st) {
+        const bool fwd = st < b;
+        const int j = fwd ? st : 2 * b - 2 - st;
+        const z* S = ring.next(st) + lr + 2 * lc * LD;
+        // forward: R = t - Lo_j w; backward: R = -Up_j x_{j+1}, added to w_j
+        const z co = fwd ? cpl.lo(j + 1) : cpl.up(j + 1);
+        double rre[2 * NT], rim[2 * NT], cre[NT][2], cim[NT][2];
+#pragma unroll
+        for (int e = 0; e < 2 * NT; ++e) {
+            z v = fwd ? t0[e] : zmk(0.0, 0.0);
+            if (st > 0) zfms(v, co, zmk(wre[e], wim[e]));
+            rre[e] = v.x;
+            rim[e] = v.y;
+            cre[e >> 1][e & 1] = fwd ? 0.0 : t0[e].x;
+            cim[e >> 1][e & 1] = fwd ? 0.0 : t0[e].y;
+            t0[e] = t1[e];
+        }
+        // two steps on: a forward block's f, or a w of this thread, stored at least two steps ago
+        if (st + 2 < b) {
+            fetch(st + 2, t1);
+            gfetch(st + 2, t1);
+        } else if (st + 2 > b) {
+            fetch(st + 2, t1);
+        }
+#pragma unroll
+        for (int e = 0; e < 2 * NT; ++e) {           // k-step: columns q = 8 (e/2) + 2 lc + e%2 of the block
+            z bf[NT];
+#pragma unroll
+            for (int t = 0; t < NT; ++t) bf[t] = S[8 * t + (8 * (e >> 1) + (e & 1)) * LD];
+#pragma unroll
+            for (int t = 0; t < NT; ++t) dmma884(cre[t][0], cre[t][1], rre[e], bf[t].x);
+#pragma unroll
+            for (int t = 0; t < NT; ++t) dmma884(cim[t][0], cim[t][1], rre[e], bf[t].y);
+#pragma unroll
+            for (int t = 0; t < NT; ++t) dmma884(cre[t][0], cre[t][1], -rim[e], bf[t].y);
+#pragma unroll
+            for (int t = 0; t < NT; ++t) dmma884(cim[t][0], cim[t][1], rim[e], bf[t].x);
+        }
+#pragma unroll
+        for (int e = 0; e < 2 * NT; ++e) {
+            const int i = 8 * (e >> 1) + 2 * lc + (e & 1);
+            wre[e] = cre[e >> 1][e & 1];
+            wim[e] = cim[e >> 1][e & 1];
+            if (live && i < a) ul[nb + j * a + i] = zmk(wre[e], wim[e]);
+            if (st + 2 == b) t1[e] = zmk(wre[e], wim[e]);          // w_{b-2}, the first backward step's
+        }
     }
+    __syncwarp();
+    // boundary values u_b = (g - c1 u(p1) - c2 u(p2)) / d of the warp's right-hand sides
+    const int live_rhs = min(8, nrhs - rh0);
+    for (int e = lane; e < nb * live_rhs; e += 32) {
+        const int r = e % nb, rr = rh0 + e / nb;
+        int ax, p1, p2;
+        leaf_bpoint2(a, b, r, ax, p1, p2);
+        const double h = ax == 0 ? L.hx : L.hy;
+        z* u = sol + ((size_t)rr * nleaves + leaf) * n;
+        z v = gb[((size_t)leaf * nrhs + rr) * nb + r];
+        v = zsub(v, zadd(zscale(-3.0 / h, u[nb + p1]), zscale((1.0 / 3.0) / h, u[nb + p2])));
+        u[r] = zmul(v, ax == 0 ? L.rdx : L.rdy);
+    }
+}
+
+template <int NT>
+static cudaError_t launch_solve(const LeafGeom& g, int nleaves, int nrhs, const double* h, const z* f, const z* gb,
+                                const z* sinv, z* sol, cudaStream_t s) {
+    const int units = (nrhs + 7) / 8, wpc = std::min(units, 8), nchunk = (units + wpc - 1) / wpc;
+    static DeviceAttrCache attr;
+    cudaError_t e = ensure_smem_attr(leaf_solve_kernel<NT>, SweepCfg<NT>::SMEM, attr);
+    if (e != cudaSuccess) return e;
+    leaf_solve_kernel<NT><<<(unsigned)nleaves * nchunk, 32 * wpc, SweepCfg<NT>::SMEM, s>>>(g, nleaves, nrhs, nchunk, h, f, gb,
+                                                                                        sinv, sol);
+    note_launch();
+    return cudaGetLastError();
 }
 
 cudaError_t leaf_block_solve(const LeafGeom& g, int nleaves, int nrhs, const double* h, const z* f, const z* gb,
                              const z* sinv, z* sol, cudaStream_t s) {
-    if (g.a == 16 && leaf_solve_engine_hw()) {
-        const size_t sh = ((size_t)2 * 256 + 2 * 16 * LHW_KC + (size_t)g.nb * LHW_KC) * sizeof(z);
-        static DeviceAttrCache attr;
-        {
-            cudaError_t e = ensure_smem_attr(leaf_hw_solve_kernel, sh, attr);
-            if (e != cudaSuccess) return e;
-        }
-        leaf_hw_solve_kernel<<<nleaves, 256, sh, s>>>(g, nleaves, nrhs, h, f, gb, sinv, sol);
-        note_launch();
-        return cudaGetLastError();
-    }
+    if (g.a <= 8) return launch_solve<1>(g, nleaves, nrhs, h, f, gb, sinv, sol, s);
+    if (g.a <= 16) return launch_solve<2>(g, nleaves, nrhs, h, f, gb, sinv, sol, s);
+    if (g.a <= 24) return launch_solve<3>(g, nleaves, nrhs, h, f, gb, sinv, sol, s);
+    if (g.a <= 32) return launch_solve<4>(g, nleaves, nrhs, h, f, gb, sinv, sol, s);
     const size_t sh = ((size_t)g.a * g.a + 2 * (size_t)g.a * LEAF_KC) * sizeof(z);
     if (sh > 48 * 1024) {
         static DeviceAttrCache attr;
