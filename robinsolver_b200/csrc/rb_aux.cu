@@ -116,6 +116,8 @@ __global__ void sweep_scatter_down_kernel(int nrhs, int nbp, int nbc, int m, int
     const int node = blockIdx.y;
     const int idx = blockIdx.x * blockDim.x + threadIdx.x;
     const int per = n1 + n2;
+    pdl_launch();
+    pdl_wait();
     if (idx >= per * nrhs) return;
     const int t = idx % per, rh = idx / per;
     const z* gp = gpar + ((long long)node * nrhs + rh) * nbp;
@@ -130,12 +132,13 @@ __global__ void sweep_scatter_down_kernel(int nrhs, int nbp, int nbc, int m, int
 }
 
 cudaError_t sweep_scatter_down(int nnodes, int nrhs, int nbp, int nbc, int m, int o1, int o2, int n1, int n2,
-                               const int* pmap1, const int* pmap2, const z* gpar, z* gchild, cudaStream_t s) {
+                               const int* pmap1, const int* pmap2, const z* gpar, z* gchild, cudaStream_t s,
+                               bool pdl) {
     const int tot = (n1 + n2) * nrhs;
     dim3 grid((tot + 255) / 256, nnodes);
-    sweep_scatter_down_kernel<<<grid, 256, 0, s>>>(nrhs, nbp, nbc, m, o1, o2, n1, n2, pmap1, pmap2, gpar, gchild);
     note_launch();
-    return cudaGetLastError();
+    return launch_kernel(sweep_scatter_down_kernel, grid, 256, 0, s, pdl, nrhs, nbp, nbc, m, o1, o2, n1, n2, pmap1, pmap2,
+                         gpar, gchild);
 }
 
 }  // namespace rb

@@ -41,6 +41,22 @@ __host__ __device__ __forceinline__ z zrcp(z a) {
 // |re| + |im|: the magnitude LAPACK's izamax ranks pivots by
 __host__ __device__ __forceinline__ double zabs1(z a) { return fabs(a.x) + fabs(a.y); }
 
+// Programmatic dependent launch.  A kernel of a chain launched with it may begin while the kernel
+// before it in the stream still runs: pdl_wait() returns once that kernel has ended and its stores are
+// visible (at once in a kernel launched the usual way), and comes before every access to anything a
+// kernel of the chain writes, in every CTA, early exits included -- so the chain's kernels still end
+// in order.  pdl_launch() lets the next kernel's CTAs be scheduled as this one's slots free up.
+__device__ __forceinline__ void pdl_wait() {
+#if defined(__CUDA_ARCH__)
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+#endif
+}
+__device__ __forceinline__ void pdl_launch() {
+#if defined(__CUDA_ARCH__)
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+#endif
+}
+
 // A matrix view: logical element (i, j) lives at p[row(i) + col(j) * ld], where row(i) is
 // rmap[i] when a map is given, else i shifted past a skipped band [rs, rs + rl) (same for
 // columns).  Maps and bands express the face gathers of the merge (non-interface faces of

@@ -56,6 +56,8 @@ zgemm_split_kernel(const GemmDesc* __restrict__ descs, int kchunk, z* work, long
 // split-K reduction: the ranges' sums added in range order, then the usual epilogue
 __global__ void __launch_bounds__(256) zgemm_reduce_kernel(const GemmDesc* __restrict__ descs, const z* __restrict__ work,
                                                           long long pstride, int ldp, int ksplit) {
+    pdl_launch();
+    pdl_wait();
     const GemmDesc& g = descs[blockIdx.y];
     const int m = g.m, n = g.n;
     const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -79,13 +81,15 @@ __global__ void __launch_bounds__(32 * WM * WN, MINB) zgemm_dmma_kernel(const Ge
         unsigned long long* dst = reinterpret_cast<unsigned long long*>(&sd);
         for (int w = threadIdx.x; w < (int)(sizeof(GemmDesc) / 8); w += 32 * WM * WN) dst[w] = src[w];
     }
+    pdl_launch();
+    pdl_wait();
     __syncthreads();
     zgemm_tile_dmma<BM, BN, WM, WN>(sd, blockIdx.x, dmma_smem);
 }
 
 // MINB CTAs per SM: the carveout is set to the largest shared-memory share so that they fit
 template <int BM, int BN, int WM, int WN, int MINB>
-static cudaError_t launch_dmma(const GemmBatch& b, cudaStream_t s) {
+static cudaError_t launch_dmma(const GemmBatch& b, cudaStream_t s, bool pdl = false) {
     using Cfg = DmmaCfg<BM, BN, WM, WN>;
     static DeviceAttrCache attr;
     {
@@ -96,10 +100,12 @@ static cudaError_t launch_dmma(const GemmBatch& b, cudaStream_t s) {
     for (int off = 0; off < b.count; off += 65535) {
         const int cnt = (b.count - off) < 65535 ? (b.count - off) : 65535;
         dim3 grid(tiles, cnt);
-        zgemm_dmma_kernel<BM, BN, WM, WN, MINB><<<grid, Cfg::NT, Cfg::SMEM_BYTES, s>>>(b.d_desc + off);
         note_launch();
+        const GemmDesc* d = b.d_desc + off;
+        cudaError_t e = launch_kernel(zgemm_dmma_kernel<BM, BN, WM, WN, MINB>, grid, Cfg::NT, Cfg::SMEM_BYTES, s, pdl, d);
+        if (e != cudaSuccess) return e;
     }
-    return cudaGetLastError();
+    return cudaSuccess;
 }
 
 // A view of the same matrix whose column j is column j + kb of v (B: row j is row j + kb)
@@ -144,6 +150,8 @@ zgemm_dmma_split_kernel(const GemmDesc* __restrict__ descs, int kchunk, z* work,
         unsigned long long* dst = reinterpret_cast<unsigned long long*>(&sd);
         for (int w = threadIdx.x; w < (int)(sizeof(GemmDesc) / 8); w += 32 * WM * WN) dst[w] = src[w];
     }
+    pdl_launch();
+    pdl_wait();
     __syncthreads();
     if (threadIdx.x == 0) {
         const int kb = blockIdx.z * kchunk;
@@ -159,7 +167,7 @@ zgemm_dmma_split_kernel(const GemmDesc* __restrict__ descs, int kchunk, z* work,
 }
 
 template <int BM, int BN, int WM, int WN, int MINB>
-static cudaError_t launch_dmma_split(const GemmBatch& b, cudaStream_t s) {
+static cudaError_t launch_dmma_split(const GemmBatch& b, cudaStream_t s, bool pdl) {
     using Cfg = DmmaCfg<BM, BN, WM, WN>;
     auto kern = zgemm_dmma_split_kernel<BM, BN, WM, WN, MINB>;
     static DeviceAttrCache attr;
@@ -169,14 +177,14 @@ static cudaError_t launch_dmma_split(const GemmBatch& b, cudaStream_t s) {
     }
     if (b.count > 65535 || b.ksplit > 65535) return cudaErrorInvalidValue;
     const int tiles = ((b.max_m + BM - 1) / BM) * ((b.max_n + BN - 1) / BN);
-    kern<<<dim3(tiles, b.count, b.ksplit), Cfg::NT, Cfg::SMEM_BYTES, s>>>(b.d_desc, b.kchunk, b.work, b.pstride,
-                                                                        b.max_m, b.ksplit);
     note_launch();
+    cudaError_t e = launch_kernel(kern, dim3(tiles, b.count, b.ksplit), Cfg::NT, Cfg::SMEM_BYTES, s, pdl, b.d_desc, b.kchunk,
+                                  b.work, b.pstride, b.max_m, b.ksplit);
+    if (e != cudaSuccess) return e;
     const long long elems = (long long)b.max_m * b.max_n;
-    zgemm_reduce_kernel<<<dim3((unsigned)((elems + 255) / 256), b.count), 256, 0, s>>>(b.d_desc, b.work, b.pstride,
-                                                                                     b.max_m, b.ksplit);
     note_launch();
-    return cudaGetLastError();
+    return launch_kernel(zgemm_reduce_kernel, dim3((unsigned)((elems + 255) / 256), b.count), 256, 0, s, pdl, b.d_desc, b.work,
+                         b.pstride, b.max_m, b.ksplit);
 }
 
 template <int BM, int BN, int WM, int WN, int BK, int STAGES, int MINB>
@@ -263,32 +271,33 @@ static cudaError_t launch_split(const GemmBatch& b, cudaStream_t s) {
 
 // up to 8 right-hand sides (rb_gemm_stream.cuh)
 template <int RT>
-static cudaError_t launch_stream(const GemmBatch& b, int ks, cudaStream_t s) {
+static cudaError_t launch_stream(const GemmBatch& b, int ks, cudaStream_t s, bool pdl) {
     const int groups = (b.max_m + 8 * RT - 1) / (8 * RT);
     const int ngrp = std::max(1, std::min(groups, (ks > 1 ? STREAM_WARPS : 4) / ks));
     for (int off = 0; off < b.count; off += 65535) {
         const int cnt = std::min(b.count - off, 65535);
-        zgemm_stream_kernel<RT><<<dim3((groups + ngrp - 1) / ngrp, cnt), 32 * ngrp * ks, 0, s>>>(b.d_desc + off, ks,
-                                                                                                b.kchunk);
         note_launch();
+        cudaError_t e = launch_kernel(zgemm_stream_kernel<RT>, dim3((groups + ngrp - 1) / ngrp, cnt), 32 * ngrp * ks, 0, s, pdl,
+                                      b.d_desc + off, ks, b.kchunk);
+        if (e != cudaSuccess) return e;
     }
-    return cudaGetLastError();
+    return cudaSuccess;
 }
 
 // The solve's tensor-core kernels: one order of summation, so the kernel may follow the number
 // of right-hand sides.  Up to 8: rb_gemm_stream.cuh (512^2, one: 1065 -> 795 us a solve); up to 16:
 // 32x16 tiles, whose second half would be idle at 32 (512^2, 16: the leaves' product 131 -> 88 us,
 // the solve's GEMMs 1.15 -> 0.97 ms).
-static cudaError_t launch_solve_gemm(const GemmBatch& b, cudaStream_t s) {
+static cudaError_t launch_solve_gemm(const GemmBatch& b, cudaStream_t s, bool pdl) {
     const bool split = b.ksplit > 1;
     if (b.max_n <= 8 && b.ksplit <= STREAM_WARPS) {
         // two row tiles per warp once one per warp gives each scheduler more than four warps
         const long long warps = (long long)b.count * ((b.max_m + 7) / 8) * b.ksplit;
-        return warps > 148 * 16 ? launch_stream<2>(b, b.ksplit, s) : launch_stream<1>(b, b.ksplit, s);
+        return warps > 148 * 16 ? launch_stream<2>(b, b.ksplit, s, pdl) : launch_stream<1>(b, b.ksplit, s, pdl);
     }
     if (b.max_n <= 16)
-        return split ? launch_dmma_split<32, 16, 2, 2, 8>(b, s) : launch_dmma<32, 16, 2, 2, 8>(b, s);
-    return split ? launch_dmma_split<32, 32, 2, 2, 6>(b, s) : launch_dmma<32, 32, 2, 2, 6>(b, s);
+        return split ? launch_dmma_split<32, 16, 2, 2, 8>(b, s, pdl) : launch_dmma<32, 16, 2, 2, 8>(b, s, pdl);
+    return split ? launch_dmma_split<32, 32, 2, 2, 6>(b, s, pdl) : launch_dmma<32, 32, 2, 2, 6>(b, s, pdl);
 }
 
 // the kernel shape a batch runs on
@@ -398,11 +407,11 @@ const char* gemm_stage_name(const GemmBatch& b) {
     return (sh == GemmShape::Dmma64 || sh == GemmShape::Dmma32) ? "zgemm_tc_small" : "zgemm_dfma";
 }
 
-cudaError_t launch_gemm_batch(const GemmBatch& b, cudaStream_t s) {
+cudaError_t launch_gemm_batch(const GemmBatch& b, cudaStream_t s, bool pdl) {
     static_assert(sizeof(GemmDesc) % 8 == 0, "descriptor copy assumes 8-byte words");
     if (b.count == 0 || b.max_m == 0 || b.max_n == 0) return cudaSuccess;
     const GemmShape shape = gemm_shape(b);
-    if (shape == GemmShape::DmmaFixed) return launch_solve_gemm(b, s);
+    if (shape == GemmShape::DmmaFixed) return launch_solve_gemm(b, s, pdl);
     if (b.ksplit > 1 && b.work) {
         if (shape == GemmShape::Dfma16) return launch_split<16, 16, 2, 2, 8, 6, 8>(b, s);
         if (shape == GemmShape::Dfma32) return launch_split<32, 32, 4, 2, 8, 4, 4>(b, s);

@@ -47,11 +47,15 @@ __global__ void __launch_bounds__(32 * STREAM_WARPS) zgemm_stream_kernel(const G
         for (int w = threadIdx.x; w < (int)(sizeof(GemmDesc) / 8); w += blockDim.x) dst[w] = src[w];
     }
     __syncthreads();
+    pdl_launch();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int lr = lane >> 2, lc = lane & 3;
     const int ngrp = (blockDim.x >> 5) / ks;
     const int slice = warp % ks, rg = warp / ks;
-    if (blockIdx.x * ngrp * 8 * RT >= g.m) return;   // the whole CTA
+    if (blockIdx.x * ngrp * 8 * RT >= g.m) {         // the whole CTA
+        pdl_wait();
+        return;
+    }
     const int r0 = (blockIdx.x * ngrp + rg) * 8 * RT;
     const bool work = r0 < g.m;
     const int kb = ks > 1 ? slice * kc : 0;
@@ -73,18 +77,30 @@ __global__ void __launch_bounds__(32 * STREAM_WARPS) zgemm_stream_kernel(const G
     const long long ald = g.A.ld;
 
     z a[2][U][RT], x[2][U];
-    auto fetch = [&](int k0, z (&fa)[U][RT], z (&fx)[U]) {
+    auto fetch_a = [&](int k0, z (&fa)[U][RT]) {
 #pragma unroll
         for (int s = 0; s < U; ++s) {
             const int k = k0 + 4 * s + lc;
             const bool ok = k < ke;
             const int kk = ok ? k : 0;
             const long long ac = (long long)(acm ? __ldg(acm + kk) : kk + (kk >= acs ? acl : 0)) * ald;
-            const int br = brm ? __ldg(brm + kk) : kk + (kk >= brs ? brl : 0);
 #pragma unroll
             for (int t = 0; t < RT; ++t) fa[s][t] = (ok && aok[t]) ? ap[t][ac] : zmk(0.0, 0.0);
+        }
+    };
+    auto fetch_x = [&](int k0, z (&fx)[U]) {
+#pragma unroll
+        for (int s = 0; s < U; ++s) {
+            const int k = k0 + 4 * s + lc;
+            const bool ok = k < ke;
+            const int kk = ok ? k : 0;
+            const int br = brm ? __ldg(brm + kk) : kk + (kk >= brs ? brl : 0);
             fx[s] = (ok && xok) ? xp[br] : zmk(0.0, 0.0);
         }
+    };
+    auto fetch = [&](int k0, z (&fa)[U][RT], z (&fx)[U]) {
+        fetch_a(k0, fa);
+        fetch_x(k0, fx);
     };
     double p1[RT][2], p2[RT][2], p3[RT][2];
 #pragma unroll
@@ -103,8 +119,10 @@ __global__ void __launch_bounds__(32 * STREAM_WARPS) zgemm_stream_kernel(const G
             for (int t = 0; t < RT; ++t) dmma884(p3[t][0], p3[t][1], xs, fa[s][t].x + fa[s][t].y);
         }
     };
+    if (kb < ke) fetch_a(kb, a[0]);                  // the factorization: complete before this chain
+    pdl_wait();
     if (kb < ke) {
-        fetch(kb, a[0], x[0]);
+        fetch_x(kb, x[0]);
         for (int k0 = kb; k0 < ke; k0 += 8 * U) {
             fetch(k0 + 4 * U, a[1], x[1]);           // beyond ke: zeros, no loads
             mac(a[0], x[0]);

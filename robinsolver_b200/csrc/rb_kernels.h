@@ -35,6 +35,23 @@ inline cudaError_t ensure_smem_attr(K kern, size_t bytes, DeviceAttrCache& c, bo
     return cudaSuccess;
 }
 
+// kernel launch, as a programmatic dependent of the kernel before it in the stream when pdl is set
+// (pdl_wait, rb_common.cuh)
+template <class... P, class... A>
+inline cudaError_t launch_kernel(void (*kern)(P...), dim3 grid, int threads, size_t smem, cudaStream_t s, bool pdl, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute la[1];
+    la[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    la[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = la;
+    cfg.numAttrs = pdl ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+}
+
 // ---- launch accounting --------------------------------------------------------------------------
 void note_launch();
 long long launch_count();
@@ -48,7 +65,9 @@ constexpr int RB_STATUS_GJ_TIMEOUT = 2;     // a resident Gauss-Jordan CTA gave 
 constexpr int RB_TC5_TIMEOUT = 4;           // a tensor-core GEMM CTA gave up waiting on an mbarrier
 
 // ---- batched GEMM ---------------------------------------------------------------------------------
-cudaError_t launch_gemm_batch(const GemmBatch& b, cudaStream_t s);
+// pdl: launch the batch's kernels as programmatic dependents (fixed-order batches only; others ignore
+// it).  The batch's A operands must be complete before the kernel that precedes it in the stream.
+cudaError_t launch_gemm_batch(const GemmBatch& b, cudaStream_t s, bool pdl = false);
 // The same batch on the tcgen05 tensor cores (rb_gemm_tc5.cu), for the mixed-precision levels, in
 // one of two arithmetics (b.t5_engine): split TF32 with FP32 accumulation (~1e-7 of
 // max|A| max|B| k), or the default, int8 digit slices of row- and column-scaled operands with
@@ -111,7 +130,7 @@ cudaError_t leaf_block_factor(const LeafGeom& g, int nleaves, const double* h, c
 // Structured leaf solve: u = A^-1 [g; f] into sol [rhs][leaf][n]; f is [rhs][leaf][a*b] (may be
 // null for zero sources), gb is [leaf][rhs][nb].
 cudaError_t leaf_block_solve(const LeafGeom& g, int nleaves, int nrhs, const double* h, const z* f, const z* gb,
-                             const z* sinv, z* sol, cudaStream_t s);
+                             const z* sinv, z* sol, cudaStream_t s, bool pdl = false);
 
 // Dense 3D leaf (rb_leaf3d.cu): A (n x n, column-major, at A + leaf*n*n) from the leaf's spacings
 // hh (3 per leaf) and potential kv (a*b*c per leaf, x fastest); Y = R A^-1 (nb x n, ld nb) from
@@ -200,6 +219,6 @@ cudaError_t refine_update(z* x, const z* dx, long long per, int nrhs, double* xn
 // g_child[phys(t)] = g_parent[pmap[t]] for both children, every node and RHS.
 cudaError_t sweep_scatter_down(int nnodes, int nrhs, int nbp, int nbc, int m, int o1, int o2, int n1,
                                int n2, const int* pmap1, const int* pmap2, const z* gpar, z* gchild,
-                               cudaStream_t s);
+                               cudaStream_t s, bool pdl = false);
 
 }  // namespace rb

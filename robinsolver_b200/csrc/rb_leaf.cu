@@ -780,8 +780,10 @@ __global__ void __launch_bounds__(256, NT <= 3 ? 2 : 1) leaf_solve_kernel(LeafGe
     const LeafConst L = leaf_const(hh, leaf, g.kb);
     const int nsteps = 2 * b - 1;
     BlockRing<NT> ring{sm, sinv + (size_t)leaf * b * aa, a, aa, b, nsteps};
+    pdl_launch();
     ring.start();
     const BlockCoupling cpl(L, b);
+    pdl_wait();                            // the factor's blocks are complete; f, g and sol are the chain's
     const int rh0 = (chunk * (nthr >> 5) + warp) * 8, rh = rh0 + lr;
     const bool live = rh < nrhs;
     const int rs = live ? rh : 0;
@@ -887,23 +889,22 @@ __global__ void __launch_bounds__(256, NT <= 3 ? 2 : 1) leaf_solve_kernel(LeafGe
 
 template <int NT>
 static cudaError_t launch_solve(const LeafGeom& g, int nleaves, int nrhs, const double* h, const z* f, const z* gb,
-                                const z* sinv, z* sol, cudaStream_t s) {
+                                const z* sinv, z* sol, cudaStream_t s, bool pdl) {
     const int units = (nrhs + 7) / 8, wpc = std::min(units, 8), nchunk = (units + wpc - 1) / wpc;
     static DeviceAttrCache attr;
     cudaError_t e = ensure_smem_attr(leaf_solve_kernel<NT>, SweepCfg<NT>::SMEM, attr);
     if (e != cudaSuccess) return e;
-    leaf_solve_kernel<NT><<<(unsigned)nleaves * nchunk, 32 * wpc, SweepCfg<NT>::SMEM, s>>>(g, nleaves, nrhs, nchunk, h, f, gb,
-                                                                                        sinv, sol);
     note_launch();
-    return cudaGetLastError();
+    return launch_kernel(leaf_solve_kernel<NT>, dim3((unsigned)nleaves * nchunk), 32 * wpc, SweepCfg<NT>::SMEM, s, pdl, g,
+                         nleaves, nrhs, nchunk, h, f, gb, sinv, sol);
 }
 
 cudaError_t leaf_block_solve(const LeafGeom& g, int nleaves, int nrhs, const double* h, const z* f, const z* gb,
-                             const z* sinv, z* sol, cudaStream_t s) {
-    if (g.a <= 8) return launch_solve<1>(g, nleaves, nrhs, h, f, gb, sinv, sol, s);
-    if (g.a <= 16) return launch_solve<2>(g, nleaves, nrhs, h, f, gb, sinv, sol, s);
-    if (g.a <= 24) return launch_solve<3>(g, nleaves, nrhs, h, f, gb, sinv, sol, s);
-    if (g.a <= 32) return launch_solve<4>(g, nleaves, nrhs, h, f, gb, sinv, sol, s);
+                             const z* sinv, z* sol, cudaStream_t s, bool pdl) {
+    if (g.a <= 8) return launch_solve<1>(g, nleaves, nrhs, h, f, gb, sinv, sol, s, pdl);
+    if (g.a <= 16) return launch_solve<2>(g, nleaves, nrhs, h, f, gb, sinv, sol, s, pdl);
+    if (g.a <= 24) return launch_solve<3>(g, nleaves, nrhs, h, f, gb, sinv, sol, s, pdl);
+    if (g.a <= 32) return launch_solve<4>(g, nleaves, nrhs, h, f, gb, sinv, sol, s, pdl);
     const size_t sh = ((size_t)g.a * g.a + 2 * (size_t)g.a * LEAF_KC) * sizeof(z);
     if (sh > 48 * 1024) {
         static DeviceAttrCache attr;
