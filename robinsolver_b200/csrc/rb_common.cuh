@@ -141,6 +141,9 @@ struct GemmBatch {
     // arithmetic of the tensor-core engine: 0 split TF32 ("TF32x3"), 1 int8 digit slices with
     // exact integer accumulation (Ozaki scheme); -1: the process default (tc5_engine)
     int t5_engine = -1;
+    // workspace of the residue engine (rb_gemm_crt.cu): set where the batch runs on it
+    void* crt_ws = nullptr;
+    size_t crt_cap = 0;
     // FP64 engine (tile shape) chosen by an autotuner; -1: the launcher's own rule
     int engine = -1;
 };

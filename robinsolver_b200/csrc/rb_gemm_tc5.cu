@@ -38,6 +38,7 @@
 #include <cstring>
 
 #include "rb_kernels.h"
+#include "rb_tc5.cuh"
 
 namespace rb {
 
@@ -47,7 +48,6 @@ constexpr int TC5_BM = 128;          // output rows per tile = UMMA M (one lane 
 constexpr int TC5_KB = 16;           // complex k per block / stage: 4 chunks of 4 TF32 = two UMMA k-steps
 constexpr int TC5_THREADS = 256;     // 8 warps
 constexpr int TC5_A_BLOCK = TC5_BM * TC5_KB * 16;          // bytes of one A plane block (32 KB)
-constexpr unsigned long long RB_TC5_WAIT_NS = 1000000000ull;   // 1 s per wait
 
 template <int BN>
 struct Tc5Cfg {
@@ -59,70 +59,6 @@ struct Tc5Cfg {
     static constexpr int SMEM = STAGES * STAGE + 1024;     // + 1024 for the alignment of the stages
     static constexpr int TMEM_COLS = 2 * BN;               // Cr, Ci
 };
-
-__device__ __forceinline__ uint32_t smem_u32(const void* p) {
-    return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
-
-__device__ __forceinline__ unsigned long long global_ns() {
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
-
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
-}
-
-// one arrival that also announces `bytes` of bulk-copy data the phase must wait for
-__device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-
-__device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.acquire.cta.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-
-// waits for the phase with the given parity to complete; false after RB_TC5_WAIT_NS or when
-// another warp has already given up (*abort, if given)
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort) {
-    if (mbar_try(bar, parity)) return true;
-    const unsigned long long t0 = global_ns();
-    for (unsigned it = 0;; ++it) {
-        if (mbar_try(bar, parity)) return true;
-        if ((it & 63) == 63) {
-            if (abort && *abort) return false;
-            if (global_ns() - t0 > RB_TC5_WAIT_NS) return false;
-        }
-    }
-}
-
-// 1-D bulk copy global -> this CTA's shared memory, completion counted on an mbarrier
-__device__ __forceinline__ void bulk_g2s(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
-                 "l"(src), "r"(bytes), "r"(bar)
-                 : "memory");
-}
-
-// UMMA shared-memory descriptor, K-major, no swizzle: core matrices of 8 rows x 16 bytes, rows
-// 16 bytes apart; sbo = bytes between 8-row groups, lbo = bytes between the two 16-byte K chunks
-// of one k-step.  Version 1 (sm_100), base offset 0, layout type 0 (SWIZZLE_NONE).
-__device__ __forceinline__ uint64_t umma_desc(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
-    uint64_t d = 0;
-    d |= (uint64_t)((saddr >> 4) & 0x3FFFu);
-    d |= (uint64_t)((lbo >> 4) & 0x3FFFu) << 16;
-    d |= (uint64_t)((sbo >> 4) & 0x3FFFu) << 32;
-    d |= (uint64_t)1 << 46;
-    return d;
-}
 
 // instruction descriptor of kind::tf32: D FP32, A and B TF32, both K-major, M = 128, N = n
 __host__ __device__ constexpr uint32_t tc5_idesc(int n, bool neg_a) {
@@ -136,10 +72,6 @@ __device__ __forceinline__ void umma_tf32(uint32_t tmem_d, uint64_t da, uint64_t
         "setp.ne.b32 p, %4, 0;\n\t"
         "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
         "l"(da), "l"(db), "r"(idesc), "r"(acc));
-}
-
-__device__ __forceinline__ void umma_commit(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
 
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
@@ -559,16 +491,6 @@ static_assert(OZ_BN % 8 == 0, "the column-scale kernel runs whole warps of 8 col
 
 namespace {
 
-// frexp exponent of |x| (x = m 2^ex, m in [0.5, 1)); -1022 for zero and subnormals
-__device__ __forceinline__ int oz_exponent(double x) {
-    return (int)(((uint32_t)__double2hiint(x) >> 20) & 0x7FFu) - 1022;
-}
-
-// exact 2^p for -1022 <= p <= 1023
-__device__ __forceinline__ double oz_pow2(int p) {
-    return __hiloint2double((p + 1023) << 20, 0);
-}
-
 // OZ_S balanced base-128 digits of v, |v| < 1/2: round(128 v) by the 1.5 * 2^52 rounding constant
 // (its low word holds the integer), the exact remainder carried to the next digit
 __device__ __forceinline__ void oz_digits(double v, int (&d)[OZ_S]) {
@@ -602,23 +524,9 @@ OzGeom oz_geom(const GemmBatch& b) {
     return g;
 }
 
-__device__ __forceinline__ void tmem_ld8(uint32_t taddr, int (&v)[8]) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
-                 : "r"(taddr));
-}
-
 // instruction descriptor of kind::i8: D S32, A and B signed 8-bit, both K-major, M = 128, N = 96
 __host__ __device__ constexpr uint32_t oz_idesc() {
     return (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(OZ_MMA_N >> 3) << 17) | ((uint32_t)(TC5_BM >> 4) << 24);
-}
-
-__device__ __forceinline__ void umma_i8(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t acc) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
-        "l"(da), "l"(db), "r"(idesc), "r"(acc));
 }
 
 }  // namespace
@@ -629,9 +537,9 @@ __device__ __forceinline__ void umma_i8(uint32_t tmem_d, uint64_t da, uint64_t d
 // max on ea, which the launcher fills with INT_MIN-like bytes first (a whole row per block left
 // most SMs idle, waiting on one long chain of loads each).
 constexpr int OZ_SCALE_KC = 64;
-__global__ void __launch_bounds__(256) oz_scale_a_kernel(const GemmDesc* __restrict__ descs, int MT, int* ea) {
+__global__ void __launch_bounds__(256) oz_scale_a_kernel(const GemmDesc* __restrict__ descs, int rows, int* ea) {
     __shared__ int red[8][32];
-    const int groups = MT * TC5_BM / 32;
+    const int groups = rows / 32;
     const int prob = blockIdx.x / groups, grp = blockIdx.x % groups;
     const int lane = threadIdx.x & 31, ph = threadIdx.x >> 5;
     const GemmDesc& g = descs[prob];
@@ -653,13 +561,12 @@ __global__ void __launch_bounds__(256) oz_scale_a_kernel(const GemmDesc* __restr
     if (ph == 0) {
 #pragma unroll
         for (int q = 1; q < 8; ++q) ex = max(ex, red[q][lane]);
-        atomicMax(ea + (long long)prob * MT * TC5_BM + i, ex + 1);
+        atomicMax(ea + (long long)prob * rows + i, ex + 1);
     }
 }
 
 // Column exponents of B, one warp per column (k runs contiguously down a column of B's view).
-__global__ void __launch_bounds__(256) oz_scale_b_kernel(const GemmDesc* __restrict__ descs, int NT, int* fb) {
-    const int cols = NT * OZ_BN;
+__global__ void __launch_bounds__(256) oz_scale_b_kernel(const GemmDesc* __restrict__ descs, int cols, int* fb) {
     const long long w = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
     const int prob = (int)(w / cols), j = (int)(w % cols);
@@ -676,6 +583,21 @@ __global__ void __launch_bounds__(256) oz_scale_b_kernel(const GemmDesc* __restr
 #pragma unroll
     for (int o = 16; o; o >>= 1) ex = max(ex, __shfl_xor_sync(0xffffffffu, ex, o));
     if (lane == 0) fb[(long long)prob * cols + j] = ex + 1;
+}
+
+// ea: count * rows (a multiple of 32), fb: count * cols (a multiple of 8); ea is filled here with
+// INT_MIN-like bytes for the atomic maxima
+cudaError_t launch_operand_scales(const GemmBatch& b, int rows, int cols, int* ea, int* fb, cudaStream_t s) {
+    const long long ga = (long long)b.count * (rows / 32), gb = ((long long)b.count * cols + 7) / 8;
+    const unsigned gk = (unsigned)((b.max_k + OZ_SCALE_KC - 1) / OZ_SCALE_KC);
+    if (rows % 32 || cols % 8 || ga > 0x7FFFFFFFLL || gb > 0x7FFFFFFFLL || gk > 65535u) return cudaErrorInvalidValue;
+    cudaError_t e = cudaMemsetAsync(ea, 0x80, sizeof(int) * (size_t)b.count * rows, s);     // far below -1022
+    if (e != cudaSuccess) return e;
+    oz_scale_a_kernel<<<dim3((unsigned)ga, gk), 256, 0, s>>>(b.d_desc, rows, ea);
+    note_launch();
+    oz_scale_b_kernel<<<(unsigned)gb, 256, 0, s>>>(b.d_desc, cols, fb);
+    note_launch();
+    return cudaGetLastError();
 }
 
 // Digit planes of one slab: s < nA an A block (problem, mt, kb: 128 rows x 32 k, in two 16-k
@@ -992,19 +914,11 @@ static cudaError_t launch_oz(const GemmBatch& b, int* status, cudaStream_t s) {
     int* fb = reinterpret_cast<int*>(planes + og.fb_off);
     // 1. row and column scales, 2. digit planes
     {
-        const long long ga = (long long)b.count * (og.MT * TC5_BM / 32);
-        const long long gb = ((long long)b.count * og.NT * OZ_BN + 7) / 8;
         const long long nA = (long long)b.count * og.MT * og.KBN;
         const long long nB = (long long)b.count * og.NT * og.KBN;
-        if (ga > 0x7FFFFFFFLL || gb > 0x7FFFFFFFLL || nA + nB > 0x7FFFFFFFLL) return cudaErrorInvalidValue;
-        e = cudaMemsetAsync(ea, 0x80, (size_t)(og.fb_off - og.ea_off), s);     // every int far below -1022
+        if (nA + nB > 0x7FFFFFFFLL) return cudaErrorInvalidValue;
+        e = launch_operand_scales(b, og.MT * TC5_BM, og.NT * OZ_BN, ea, fb, s);
         if (e != cudaSuccess) return e;
-        const unsigned gk = (unsigned)((b.max_k + OZ_SCALE_KC - 1) / OZ_SCALE_KC);
-        if (gk > 65535u) return cudaErrorInvalidValue;
-        oz_scale_a_kernel<<<dim3((unsigned)ga, gk), 256, 0, s>>>(b.d_desc, og.MT, ea);
-        note_launch();
-        oz_scale_b_kernel<<<(unsigned)gb, 256, 0, s>>>(b.d_desc, og.NT, fb);
-        note_launch();
         oz_split_kernel<<<(unsigned)(nA + nB), 256, 0, s>>>(b.d_desc, og.MT, og.NT, og.KBN, nA, planes, og.a_bytes,
                                                             ea, fb);
         note_launch();

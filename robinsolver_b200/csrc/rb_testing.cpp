@@ -7,6 +7,7 @@
 //   engine 1: the tcgen05 kernel of the mixed-precision levels in split TF32
 //   engine 2: the tcgen05 kernel in int8 digit slices (the mixed-precision default)
 //   engine 3: the solve's fixed-order kernel
+//   engine 4: the residue (int8) engine of the FP64 factor's large products
 // It allocates its descriptor array itself and synchronises; it returns 0, a negative RB_ERR_*
 // code for bad arguments or CUDA failures, or the device status word's bits (> 0) when a kernel
 // reported one.
@@ -66,7 +67,11 @@ static int test_zgemm(int engine, int m, int n, int k, const double* dA, long lo
         const long long w = gemm_plan_split(b);
         if (w > 0 && e == cudaSuccess) e = cudaMalloc(&b.work, sizeof(z) * (size_t)w);
     }
-    auto run = [&]() { return engine == 1 || engine == 2 ? launch_gemm_tc5(b, d_status, 0) : launch_gemm_batch(b, 0); };
+    if (engine == 4) {
+        b.crt_cap = crt_bytes(b);
+        if (e == cudaSuccess) e = b.crt_cap ? cudaMalloc(&b.crt_ws, b.crt_cap) : cudaErrorInvalidValue;
+    }
+    auto run = [&]() { return engine == 4 ? launch_gemm_crt(b, d_status, 0) : engine == 1 || engine == 2 ? launch_gemm_tc5(b, d_status, 0) : launch_gemm_batch(b, 0); };
     int rc = RB_OK;
     if (e == cudaSuccess) e = cudaMemcpy(b.d_desc, h.data(), sizeof(GemmDesc) * count, cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemset(d_status, 0, sizeof(int));
@@ -98,6 +103,7 @@ static int test_zgemm(int engine, int m, int n, int k, const double* dA, long lo
     cudaFree(d_status);
     if (b.t5_planes) cudaFree(b.t5_planes);
     if (b.work) cudaFree(b.work);
+    if (b.crt_ws) cudaFree(b.crt_ws);
     return rc;
 }
 
