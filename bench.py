@@ -520,10 +520,14 @@ def roofline_block(arm, torch, dev, steps, zpeak, bf16_peak):
     # multiply-add is 4 real ones x 3 split products (3 per flop).
     int8 = os.environ.get("RB_MIXED_ENGINE", "int8") != "tf32x3"
     tc5_peak = (bf16_peak * 2.0 / 15.0 if int8 else bf16_peak / 2.0 / 3.0) if bf16_peak else None
+    # the FP64 factor's residue products: 8 int8 operations per complex multiply-add (8 flops) in each of 16
+    # moduli
+    crt_peak = bf16_peak * 2.0 / 16.0 if bf16_peak else None
+    peaks = {"zgemm_tc5": tc5_peak, "zgemm_crt": crt_peak}
     fams = {}
     for k, v in per.items():
         if v[2] > 0:
-            pk = tc5_peak if k == "zgemm_tc5" else zpeak
+            pk = peaks.get(k, zpeak)
             fams[k] = {"launches": v[0], "ms": round(v[1], 3), "tflops": round(v[2] / (v[1] * 1e-3) / 1e12, 2),
                        "frac": round(v[2] / (v[1] * 1e-3) / 1e12 / pk, 3) if pk else None}
     if dname == "zgemm_tc5":
@@ -532,6 +536,9 @@ def roofline_block(arm, torch, dev, steps, zpeak, bf16_peak):
                            "flop)") if int8 else \
             (tc5_peak, "tf32 (tcgen05, split x3)",
              "MEASURED_PEAKS.json bf16_tflops / 2 (dense TF32) / 3 (split products per complex term)")
+    elif dname == "zgemm_crt":
+        peak, pipe, src = crt_peak, "int8 (tcgen05, 16 moduli)", \
+            "MEASURED_PEAKS.json bf16_tflops x 2 (dense int8) / 16 (int8 operations per algorithmic flop)"
     else:
         peak, pipe, src = zpeak, "fp64", "complex128 cuBLAS GEMM 4096^3 measured in this run (no FP64 entry in " \
                                          "MEASURED_PEAKS.json)"

@@ -47,7 +47,10 @@ extern "C" {
 #define RB_ERR_NO_SOLUTION   -11  /* get_solution before any solve, or irhs out of range              */
 
 /* ---- precision modes for rb_tree_factor ----------------------------------------------------- */
-#define RB_PREC_FP64  0           /* every operation in complex128                                    */
+#define RB_PREC_FP64  0           /* complex128 in, out and in every result; products of interfaces of
+                                     512 points and more are summed exactly on the int8 tensor cores
+                                     (operands as 57-bit integers of their row's or column's scale),
+                                     where device_budget and memory leave room for their workspaces  */
 #define RB_PREC_MIXED 1           /* merge levels l >= 2 with interfaces of >= 128 points: GEMMs on the
                                      tcgen05 tensor cores in split TF32 (FP32 accumulation, ~1e-6
                                      relative); the top two levels, the interface inverses, the leaves

@@ -11,19 +11,23 @@
 // passes:
 //  1. launch_operand_scales: the row and column exponents;
 //  2. crt_split_kernel: 16 residues of the real and imaginary parts, one byte each, laid out block by
-//     block as the product kernel's shared-memory stages hold them (K-major, no swizzle);
-//  3. zgemm_crt_kernel: one CTA per 128 x 80 output tile and group of moduli.  Per modulus it streams
-//     the residues of A (Ar, Ai) and B ([Br | Bi], 160 rows) through a ring of bulk-copied stages;
-//     two MMAs of 128 x 160 x 32 per k-step accumulate Ar Br, the sum Ar Bi + Ai Br and Ai Bi in 240
-//     tensor-memory columns (the second MMA's columns overlap the first's by half, so the sum forms by
-//     itself).  The next modulus' MMAs run on the other half of tensor memory while eight warps read
-//     the accumulators, reduce them and write one byte per real output;
+//     block as the product kernel's shared memory holds them (K-major, 128-byte swizzle);
+//  3. zgemm_crt_kernel: per modulus, the residues of B's column tile ([Br | Bi], 160 rows) stay in shared
+//     memory while those of A (Ar, Ai) stream past through a ring of bulk-copied stages.  MMAs of
+//     128 x 160 x 32 accumulate Ar Br, the sum Ar Bi + Ai Br and Ai Bi in 240 tensor-memory columns
+//     (Ai's columns overlap Ar's by half, so the sum forms by itself).  The next tile's MMAs run on the
+//     other half of tensor memory while eight warps read the accumulators, reduce them and write one
+//     byte per real output;
 //  4. crt_combine_kernel: the 16 residues of an output to its value, sum_s r_s w_s mod M with the
 //     weights in two parts of 41 bits (every sum exact in FP64), the scales, and the usual epilogue.
 // Why N = 160: an MMA reads its operands from shared memory, and below N of about 128 that, not the
 // tensor pipe, is its time; two accumulator sets of 3 x 80 columns fill tensor memory.
 // A row or column that holds an infinity or a NaN gives NaN.
-// @@FIG@@
+// Measured against the FP64 tensor-core tiles (complex m x n x k, count; us): 2048 x 2048 x 1024, 4: 3196 to
+// 1376; 1536 x 1536 x 512, 8: 1874 to 1016; 512 x 1536 x 512, 4: 357 to 261; 1024 x 2048 x 1024, 1: 462 to 230;
+// 768 x 768 x 256, 32: 988 to 826; 256 x 768 x 256, 16: 190 to 236; 384 x 384 x 128, 128: 548 to 808.  The first spends
+// 29 + 26 us on scales, 294 on the split (its 16 residues per entry are issue bound), 829 on products
+// (the tensor pipe alone would take 520) and 205 on the outputs (5.2 TB/s).
 #include <algorithm>
 #include <climits>
 #include <cstdint>
@@ -39,13 +43,14 @@ namespace {
 constexpr int CRT_S = 16;                    // moduli
 constexpr int CRT_P = 57;                    // bits of the scaled integers, sign included
 constexpr int CRT_BM = 128, CRT_BN = 80;     // output tile
-constexpr int CRT_KB = 32;                   // k of one MMA and of one plane block
-constexpr int CRT_A_BLOCK = 2 * CRT_BM * CRT_KB;           // bytes per block: Ar, Ai
+constexpr int CRT_KB = 128;                  // k of one plane block: a row is 128 bytes
+constexpr int CRT_A_BLOCK = CRT_BM * CRT_KB;               // bytes per block of one part (Ar or Ai)
 constexpr int CRT_B_ROWS = 2 * CRT_BN;                     // Br, Bi
 constexpr int CRT_B_BLOCK = CRT_B_ROWS * CRT_KB;
-constexpr int CRT_STAGE = 2 * (CRT_A_BLOCK + CRT_B_BLOCK); // two blocks (64 k)
-constexpr int CRT_STAGES = 8;
-constexpr int CRT_SMEM = CRT_STAGES * CRT_STAGE + 1024;
+constexpr int CRT_CHUNKS = 4;                              // blocks of a B tile that stay resident (k <= 512)
+constexpr int CRT_STAGES = 4;                              // stages of Ar and Ai (and B's block, above) of 128 k
+constexpr int CRT_SMEM = CRT_STAGES * (2 * CRT_A_BLOCK + CRT_B_BLOCK) + 1024;
+static_assert(CRT_SMEM <= 227 * 1024 - 1024, "shared memory");
 constexpr int CRT_THREADS = 384;             // producer, issuer, two idle, eight epilogue warps
 constexpr int CRT_EPI = 8;
 constexpr int CRT_OUT = CRT_BM * CRT_BN;     // residues of one part of a tile
@@ -76,16 +81,16 @@ constexpr double CRT_MHI = 0x1.146fdb6e6a000p+81, CRT_MLO = 0x1.f2fddf2940000p+3
 constexpr int CRT_LO = 44;
 
 struct CrtGeom {
-    int MT, NT, KB2;                         // row tiles, column tiles, 64-deep k-steps
+    int MT, NT, KB;                          // row tiles, column tiles, 128-deep blocks
     long long a_bytes, b_bytes, c_off, ea_off, fb_off, total;
 };
 CrtGeom crt_geom(const GemmBatch& b) {
     CrtGeom g;
     g.MT = (b.max_m + CRT_BM - 1) / CRT_BM;
     g.NT = (b.max_n + CRT_BN - 1) / CRT_BN;
-    g.KB2 = (b.max_k + 2 * CRT_KB - 1) / (2 * CRT_KB);
-    g.a_bytes = (long long)b.count * g.MT * CRT_S * g.KB2 * 2 * CRT_A_BLOCK;
-    g.b_bytes = (long long)b.count * g.NT * CRT_S * g.KB2 * 2 * CRT_B_BLOCK;
+    g.KB = (b.max_k + CRT_KB - 1) / CRT_KB;
+    g.a_bytes = (long long)b.count * g.MT * CRT_S * g.KB * 2 * CRT_A_BLOCK;
+    g.b_bytes = (long long)b.count * g.NT * CRT_S * g.KB * CRT_B_BLOCK;
     g.c_off = g.a_bytes + g.b_bytes;
     g.ea_off = g.c_off + (long long)b.count * g.MT * g.NT * CRT_S * 2 * CRT_OUT;
     g.fb_off = g.ea_off + 4LL * b.count * g.MT * CRT_BM;
@@ -97,37 +102,85 @@ __host__ __device__ constexpr uint32_t crt_idesc(int n) {
     return (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(CRT_BM >> 4) << 24);
 }
 
+// UMMA shared-memory descriptor, K-major, 128-byte swizzle: rows of 128 bytes, 16-byte chunk c of row r
+// at c ^ (r % 8), 8-row groups 1024 bytes apart and aligned; a k-step of 32 is 32 bytes further on.
+// Version 1 (sm_100), base offset 0, layout type 2 (SWIZZLE_128B).
+__device__ __forceinline__ uint64_t crt_desc(uint32_t saddr) {
+    return (uint64_t)((saddr >> 4) & 0x3FFFu) | ((uint64_t)1 << 16) | ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)1 << 46) |
+           ((uint64_t)2 << 61);
+}
+
+// 1 on one lane of a converged warp
+__device__ __forceinline__ uint32_t elect_one() {
+    uint32_t p;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "elect.sync _|p, 0xffffffff;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(p));
+    return p;
+}
+
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 
-// residues of x (an integer below 2^56 in magnitude) as signed bytes, byte kk & 3 of word[s]
-__device__ __forceinline__ void crt_residues(double x, int sh, uint32_t (&word)[CRT_S]) {
+// a pair of moduli: their product, and each, with reciprocals
+struct CrtPair {
+    double mp, ip;
+    float m0, i0, m1, i1;
+};
+constexpr CrtPair crt_pair(int p) {
+    const double mp = (double)(crt_mod(2 * p) * crt_mod(2 * p + 1));
+    const float m0 = (float)crt_mod(2 * p), m1 = (float)crt_mod(2 * p + 1);
+    return CrtPair{mp, 1.0 / mp, m0, 1.0f / m0, m1, 1.0f / m1};
+}
+__constant__ CrtPair c_pair[CRT_S / 2] = {crt_pair(0), crt_pair(1), crt_pair(2), crt_pair(3),
+                                          crt_pair(4), crt_pair(5), crt_pair(6), crt_pair(7)};
+
+// residues of x (an integer below 2^56 in magnitude) modulo a pair of moduli, as signed bytes
+__device__ __forceinline__ void crt_residues(double x, const CrtPair& c, uint32_t& r0, uint32_t& r1) {
     constexpr double magic = 6755399441055744.0;         // 1.5 * 2^52: rounds to an integer in the low word
     constexpr float fmagic = 12582912.0f;                // 1.5 * 2^23
-#pragma unroll
-    for (int p = 0; p < CRT_S / 2; ++p) {
-        // modulo the product of two moduli first: |y| <= (1/2 + 2^-12) 2^16
-        const double mp = (double)(crt_mod(2 * p) * crt_mod(2 * p + 1)), ip = 1.0 / mp;
-        const double q = rint(x * ip);
-        const double y = __fma_rn(-q, mp, x);
-        const float f = __int_as_float(0x4B400000 + __double2loint(__dadd_rn(y, magic))) - fmagic;
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const float m = (float)crt_mod(2 * p + h);
-            const float t = __fadd_rn(__fmaf_rn(f, 1.0f / m, fmagic), -fmagic);
-            const float r = __fmaf_rn(-t, m, f);         // |r| <= m / 2
-            word[2 * p + h] |= ((uint32_t)__float_as_int(__fadd_rn(r, fmagic)) & 0xFFu) << sh;
-        }
-    }
+    // modulo the product of the two first: |y| <= (1/2 + 2^-12) 2^16
+    const double q = __dadd_rn(__fma_rn(x, c.ip, magic), -magic);
+    const double y = __fma_rn(-q, c.mp, x);
+    const float f = __fadd_rn(__int_as_float(0x4B400000 + __double2loint(__dadd_rn(y, magic))), -fmagic);
+    const float t0 = __fadd_rn(__fmaf_rn(f, c.i0, fmagic), -fmagic), t1 = __fadd_rn(__fmaf_rn(f, c.i1, fmagic), -fmagic);
+    // |f - t m| <= m / 2, in the low byte
+    r0 = (uint32_t)__float_as_int(__fadd_rn(__fmaf_rn(-t0, c.m0, f), fmagic));
+    r1 = (uint32_t)__float_as_int(__fadd_rn(__fmaf_rn(-t1, c.m1, f), fmagic));
+}
+// the low bytes of four words
+__device__ __forceinline__ uint32_t crt_pack(uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+    return __byte_perm(__byte_perm(a, b, 0x0040), __byte_perm(c, d, 0x0040), 0x5410);
 }
 
-// v 2^(CRT_P - e) rounded to an integer; the power in two factors, since neither end of the exponent
-// range has it as one double.  Zero for a marked row.
-__device__ __forceinline__ double crt_round(double v, int e) {
-    if (e >= CRT_NONFINITE) return 0.0;
-    const int p = CRT_P - e, p1 = p / 2, p2 = p - p1;
-    return rint(v * oz_pow2(p1) * oz_pow2(p2));
+// v 2^p in two factors: neither end of the exponent range has 2^p as one double
+__device__ __forceinline__ double crt_scale(double v, int p) {
+    const int p1 = p / 2;
+    return v * oz_pow2(p1) * oz_pow2(p - p1);
+}
+
+// v 2^p for the outputs' wider range of p (both exponents): three factors
+__device__ __forceinline__ double crt_ldexp(double v, int p) {
+    const int p1 = p / 3, p2 = (p - p1) / 2;
+    return v * oz_pow2(p1) * oz_pow2(p2) * oz_pow2(p - p1 - p2);
+}
+
+// The problem whose A planes problem p uses: the first of the run of neighbours with the same A as its
+// own (the two column halves of Y1, Y2 and of a map's rows read one A: split once, 6 units of 8 of a map).
+__device__ __forceinline__ int crt_a_owner(const GemmDesc* descs, int p) {
+    const ZView a = descs[p].A;
+    const int m = descs[p].m, k = descs[p].k;
+    while (p > 0) {
+        const GemmDesc& o = descs[p - 1];
+        if (o.A.p != a.p || o.A.ld != a.ld || o.A.rmap != a.rmap || o.A.cmap != a.cmap || o.A.rs != a.rs || o.A.rl != a.rl ||
+            o.A.cs != a.cs || o.A.cl != a.cl || o.m != m || o.k != k)
+            break;
+        --p;
+    }
+    return p;
 }
 
 // exponents of rows or columns with an infinity or a NaN (frexp exponent 1025) become the mark
@@ -135,104 +188,114 @@ __device__ __forceinline__ int crt_exp(int e) { return e > 1025 ? CRT_NONFINITE 
 
 }  // namespace
 
-// Residue planes of one slab: s < nA an A block (problem, mt, kb: 128 rows x 32 k), else a B block
-// (problem, nt, kb: 80 columns x 32 k).  Block (tile, modulus, kb) holds 16-byte chunk c (16 k) of
-// row r of part p at ((p * 2 + c) * 128 + r) * 16 (A) or of row p * 80 + r at (c * 160 + row) * 16 (B).
-__global__ void __launch_bounds__(256, 2) crt_split_kernel(const GemmDesc* __restrict__ descs, int MT, int NT, int KBN,
+// Residue planes of one slab of 16 rows x 128 k: s < nA of A (problem, mt, kb, 16-row group), else of B
+// (problem, nt, kb, 16-column group).  Blocks: A [problem][mt][modulus][kb][part], B
+// [problem][nt][modulus][kb] with Br's 80 rows, then Bi's; chunk c (16 k) of row r of a block at
+// r * 128 + (c ^ (r % 8)) * 16.  A thread takes one chunk of one part of one row, so that a warp's store
+// of one modulus is 512 bytes in a row.
+__global__ void __launch_bounds__(256, 3) crt_split_kernel(const GemmDesc* __restrict__ descs, int MT, int NT, int KB,
                                                            long long nA, unsigned char* __restrict__ planes,
                                                            long long a_bytes, const int* __restrict__ ea,
                                                            const int* __restrict__ fb) {
-    __shared__ z S[CRT_BM * 17];             // also 80 x 17: half a block at a time
+    __shared__ z S[16 * 8 * 17];             // [row][chunk][16 of 17]
     const int tid = threadIdx.x;
     long long s = blockIdx.x;
     const bool isA = s < nA;
     if (!isA) s -= nA;
-    const int kb = (int)(s % KBN);
-    s /= KBN;
+    const int rows = isA ? CRT_BM : CRT_BN, groups = rows / 16;
+    const int grp = (int)(s % groups);
+    s /= groups;
+    const int kb = (int)(s % KB);
+    s /= KB;
     const int tiles = isA ? MT : NT;
     const int tile = (int)(s % tiles);
     const int prob = (int)(s / tiles);
+    if (isA && crt_a_owner(descs, prob) != prob) return;
     const GemmDesc& g = descs[prob];
-    const int rows = isA ? CRT_BM : CRT_BN;
-    const long long mstride = (long long)KBN * (isA ? CRT_A_BLOCK : CRT_B_BLOCK);      // between moduli
-    unsigned char* blk = planes + (isA ? 0 : a_bytes) +
-                         ((long long)prob * tiles + tile) * CRT_S * mstride + (long long)kb * (isA ? CRT_A_BLOCK : CRT_B_BLOCK);
-    const int* ex = (isA ? ea : fb) + ((long long)prob * tiles + tile) * rows;
-    for (int half = 0; half < 2; ++half) {
-        const int k0 = kb * CRT_KB + half * 16;
-        for (int e = tid; e < rows * 16; e += 256) {
-            // rows of A run contiguously, k runs contiguously down a column of B
-            const int r = isA ? e % CRT_BM : e / 16, kk = isA ? e / CRT_BM : e % 16;
-            const int i = tile * rows + r, k = k0 + kk;
-            z val = zmk(0.0, 0.0);
-            if (k < g.k) {
-                if (isA && i < g.m) val = g.A.p[vrow(g.A, i) + (long long)vcol(g.A, k) * g.A.ld];
-                if (!isA && i < g.n) val = g.B.p[vrow(g.B, k) + (long long)vcol(g.B, i) * g.B.ld];
-            }
-            S[r * 17 + kk] = val;
+    const int i0 = tile * rows + grp * 16, k0 = kb * CRT_KB;
+    for (int e = tid; e < 16 * CRT_KB; e += 256) {
+        // rows of A run contiguously, k runs contiguously down a column of B
+        const int r = isA ? e % 16 : e / CRT_KB, kk = isA ? e / 16 : e % CRT_KB;
+        const int i = i0 + r, k = k0 + kk;
+        z val = zmk(0.0, 0.0);
+        if (k < g.k) {
+            if (isA && i < g.m) val = g.A.p[vrow(g.A, i) + (long long)vcol(g.A, k) * g.A.ld];
+            if (!isA && i < g.n) val = g.B.p[vrow(g.B, k) + (long long)vcol(g.B, i) * g.B.ld];
         }
-        __syncthreads();
-        for (int u = tid; u < 2 * rows; u += 256) {
-            // unit: row r, part (0 re, 1 im): 16 values -> one 16-byte chunk per modulus
-            const int r = u % rows, part = u / rows;
-            const int e = crt_exp(ex[r]);
-            unsigned char* dst = blk + (isA ? ((part * 2 + half) * CRT_BM + r) * 16
-                                            : (half * CRT_B_ROWS + part * CRT_BN + r) * 16);
+        S[(r * 8 + (kk >> 4)) * 17 + (kk & 15)] = val;
+    }
+    __syncthreads();
+    const int c = tid & 7, r = (tid >> 3) & 15, part = tid >> 7;
+    const long long block = isA ? 2 * CRT_A_BLOCK : CRT_B_BLOCK, mstride = KB * block;      // per kb; between moduli
+    const int e = crt_exp((isA ? ea : fb)[(long long)prob * tiles * rows + i0 + r]);
+    const int rr = (isA ? 0 : part * CRT_BN) + grp * 16 + r;
+    unsigned char* dst = planes + (isA ? part * CRT_A_BLOCK : a_bytes) + ((long long)prob * tiles + tile) * CRT_S * mstride +
+                         kb * block + rr * CRT_KB + ((c ^ (rr & 7)) << 4);
+    double x[16];
+#pragma unroll
+    for (int kk = 0; kk < 16; ++kk) {
+        const z v = S[(r * 8 + c) * 17 + kk];
+        // 2^56 > |x|; zero for a marked row
+        x[kk] = e >= CRT_NONFINITE ? 0.0 : rint(crt_scale(part ? v.y : v.x, CRT_P - e));
+    }
+    // rolled: eight unrolled pairs of 16 values hold too many registers for three CTAs per SM
 #pragma unroll 1
-            for (int w = 0; w < 4; ++w) {
-                uint32_t word[CRT_S];
+    for (int p = 0; p < CRT_S / 2; ++p, dst += 2 * mstride) {
+        const CrtPair pr = c_pair[p];
+        uint32_t w0[4], w1[4];
 #pragma unroll
-                for (int j = 0; j < CRT_S; ++j) word[j] = 0u;
+        for (int w = 0; w < 4; ++w) {
+            uint32_t a[4], b[4];
 #pragma unroll
-                for (int kk = 0; kk < 4; ++kk) {
-                    const z x = S[r * 17 + 4 * w + kk];
-                    crt_residues(crt_round(part ? x.y : x.x, e), 8 * kk, word);
-                }
-#pragma unroll
-                for (int j = 0; j < CRT_S; ++j) *reinterpret_cast<uint32_t*>(dst + j * mstride + 4 * w) = word[j];
-            }
+            for (int kk = 0; kk < 4; ++kk) crt_residues(x[4 * w + kk], pr, a[kk], b[kk]);
+            w0[w] = crt_pack(a[0], a[1], a[2], a[3]);
+            w1[w] = crt_pack(b[0], b[1], b[2], b[3]);
         }
-        __syncthreads();
+        *reinterpret_cast<uint4*>(dst) = make_uint4(w0[0], w0[1], w0[2], w0[3]);
+        *reinterpret_cast<uint4*>(dst + mstride) = make_uint4(w1[0], w1[1], w1[2], w1[3]);
     }
 }
 
-// One CTA per output tile (blockIdx.x), problem (y) and group of moduli (z).  Every mbarrier wait is
-// bounded; a CTA that gives up sets RB_TC5_TIMEOUT, waits (bounded) for the copies and MMAs it
-// issued, frees its tensor memory and returns.
+// One CTA per column tile and run of up to R row tiles (blockIdx.x), problem (y) and group of moduli (z).
+// Up to k = 512 B's column tile (160 rows x k) stays in shared memory for a modulus while the row tiles
+// of A stream past it; its blocks are refilled for the next modulus as the last row tile lets go of
+// them.  Above, B's blocks stream beside A's: a resident tile would leave room for two stages only
+// (k = 1024: 1014 us of products for 4 x 2048 x 2048, 829 streaming).  Every mbarrier wait is bounded; a CTA that gives up sets RB_TC5_TIMEOUT, waits (bounded) for
+// the copies and MMAs it issued, frees its tensor memory and returns.
 __global__ void __launch_bounds__(CRT_THREADS, 1) zgemm_crt_kernel(const GemmDesc* __restrict__ descs, int prob0, int* status,
                                                                   const unsigned char* __restrict__ planes, int MT, int NT,
-                                                                  int KB2, long long a_bytes, unsigned char* __restrict__ out,
-                                                                  int per_group) {
+                                                                  int KB, long long a_bytes, unsigned char* __restrict__ out,
+                                                                  int R, int per_group) {
     extern __shared__ __align__(1024) unsigned char crt_smem[];
-    __shared__ __align__(8) unsigned long long bars[2 * CRT_STAGES + 5];
+    __shared__ __align__(8) unsigned long long bars[2 * CRT_STAGES + 2 * CRT_CHUNKS + 5];
     __shared__ uint32_t tmem_slot;
     __shared__ volatile int abort_flag;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const GemmDesc& g = descs[blockIdx.y];
     const int tiles_m = (g.m + CRT_BM - 1) / CRT_BM, tiles_n = (g.n + CRT_BN - 1) / CRT_BN;
-    if ((int)blockIdx.x >= tiles_m * tiles_n) return;            // the whole CTA
-    const int tm = blockIdx.x % tiles_m, tn = blockIdx.x / tiles_m;
+    const int runs = (MT + R - 1) / R;
+    const int tn = blockIdx.x / runs, t0 = (blockIdx.x % runs) * R, t1 = min(tiles_m, t0 + R);
+    if (tn >= tiles_n || t0 >= tiles_m) return;                  // the whole CTA
     const long long prob = prob0 + (long long)blockIdx.y;
     const int s0 = blockIdx.z * per_group, s1 = min(CRT_S, s0 + per_group);
-    const int nk = (g.k + 2 * CRT_KB - 1) / (2 * CRT_KB);        // 64-deep steps of this problem
-    const unsigned char* gA = planes + ((prob * MT + tm) * CRT_S) * (long long)KB2 * 2 * CRT_A_BLOCK;
-    const unsigned char* gB = planes + a_bytes + ((prob * NT + tn) * CRT_S) * (long long)KB2 * 2 * CRT_B_BLOCK;
+    const int nk = (g.k + CRT_KB - 1) / CRT_KB;                  // blocks of this problem
+    const long long a_mod = (long long)KB * 2 * CRT_A_BLOCK, b_mod = (long long)KB * CRT_B_BLOCK;
+    const unsigned char* gB = planes + a_bytes + (prob * NT + tn) * CRT_S * b_mod;
 
-    unsigned char* stage_base =
-        reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(crt_smem) + 1023) & ~uintptr_t(1023));
-    const uint32_t full0 = smem_u32(&bars[0]), empty0 = smem_u32(&bars[CRT_STAGES]);
-    const uint32_t accfull0 = smem_u32(&bars[2 * CRT_STAGES]), accempty0 = smem_u32(&bars[2 * CRT_STAGES + 2]);
-    const uint32_t done_bar = smem_u32(&bars[2 * CRT_STAGES + 4]);
+    unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(crt_smem) + 1023) & ~uintptr_t(1023));
+    // resident: four blocks of B, then the stages of A; streaming: stages of A and a block of B each
+    const bool resident = nk <= CRT_CHUNKS;
+    const uint32_t sB = smem_u32(base) + (resident ? 0u : (uint32_t)(2 * CRT_A_BLOCK));
+    const uint32_t sA = smem_u32(base) + (resident ? (uint32_t)(CRT_CHUNKS * CRT_B_BLOCK) : 0u);
+    const uint32_t stage_bytes = 2 * CRT_A_BLOCK + (resident ? 0 : CRT_B_BLOCK);
+    const uint32_t afull0 = smem_u32(&bars[0]), aempty0 = afull0 + 8 * CRT_STAGES;
+    const uint32_t bfull0 = aempty0 + 8 * CRT_STAGES, bempty0 = bfull0 + 8 * CRT_CHUNKS;
+    const uint32_t accfull0 = bempty0 + 8 * CRT_CHUNKS, accempty0 = accfull0 + 16, done_bar = accempty0 + 16;
     if (tid == 0) {
         abort_flag = 0;
-        for (int q = 0; q < CRT_STAGES; ++q) {
-            mbar_init(full0 + 8 * q, 1);
-            mbar_init(empty0 + 8 * q, 1);
-        }
-        for (int q = 0; q < 2; ++q) {
-            mbar_init(accfull0 + 8 * q, 1);
-            mbar_init(accempty0 + 8 * q, CRT_EPI);
-        }
+        for (int q = 0; q < 2 * CRT_STAGES + 2 * CRT_CHUNKS + 2; ++q) mbar_init(afull0 + 8 * q, 1);
+        mbar_init(accempty0, CRT_EPI);
+        mbar_init(accempty0 + 8, CRT_EPI);
         mbar_init(done_bar, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -247,122 +310,145 @@ __global__ void __launch_bounds__(CRT_THREADS, 1) zgemm_crt_kernel(const GemmDes
     const uint32_t tmem = tmem_slot;
 
     if (warp == 0) {
-        // ---------------- producer: both blocks of a step, then the next, through the moduli -----------------
-        bool ok = true;
-        int it = 0;
-        for (int s = s0; s < s1 && ok; ++s) {
-            const unsigned char* a = gA + (long long)s * KB2 * 2 * CRT_A_BLOCK;
-            const unsigned char* b = gB + (long long)s * KB2 * 2 * CRT_B_BLOCK;
-            for (int kb = 0; kb < nk; ++kb) {
-                const int q = it % CRT_STAGES, u = it / CRT_STAGES;
-                if (u > 0) {
-                    ok = __all_sync(0xffffffffu, mbar_wait(empty0 + 8 * q, (uint32_t)((u - 1) & 1), &abort_flag));
-                    if (!ok) break;
+        // ---------------- producer, in the issuer's order ------------------------------------------------
+        if (lane == 0) {
+            bool ok = true;
+            const unsigned char* gA = planes + (long long)crt_a_owner(descs - prob0, (int)prob) * MT * CRT_S * a_mod;
+            uint32_t q = 0;                          // stage
+            int it = 0, nb = 0;                      // stages and resident B blocks issued
+            uint32_t par = 1u;                       // parity of the A stage's previous release
+            for (int s = s0; s < s1 && ok; ++s) {
+                const unsigned char* a = gA + ((long long)t0 * CRT_S + s) * a_mod;
+                const unsigned char* bsrc = gB + s * b_mod;
+                for (int tm = t0; tm < t1 && ok; ++tm, a += CRT_S * a_mod) {
+                    for (int kb = 0; kb < nk && ok; ++kb) {
+                        if (resident && tm == t0) {
+                            if (s > s0) ok = mbar_wait(bempty0 + 8 * kb, (uint32_t)((s - s0 - 1) & 1), &abort_flag);
+                            if (!ok) break;
+                            mbar_arrive_expect_tx(bfull0 + 8 * kb, CRT_B_BLOCK);
+                            bulk_g2s(sB + (uint32_t)(kb * CRT_B_BLOCK), bsrc + kb * CRT_B_BLOCK, CRT_B_BLOCK, bfull0 + 8 * kb);
+                            ++nb;
+                        }
+                        if (it >= CRT_STAGES) ok = mbar_wait(aempty0 + 8 * q, par, &abort_flag);
+                        if (!ok) break;
+                        mbar_arrive_expect_tx(afull0 + 8 * q, stage_bytes);
+                        bulk_g2s(sA + q * stage_bytes, a + kb * 2 * CRT_A_BLOCK, 2 * CRT_A_BLOCK, afull0 + 8 * q);
+                        if (!resident) bulk_g2s(sB + q * stage_bytes, bsrc + kb * CRT_B_BLOCK, CRT_B_BLOCK, afull0 + 8 * q);
+                        ++it;
+                        if (++q == CRT_STAGES) {
+                            q = 0;
+                            par ^= 1u;
+                        }
+                    }
                 }
-                if (lane == 0) {
-                    const uint32_t st = smem_u32(stage_base + (size_t)q * CRT_STAGE);
-                    mbar_arrive_expect_tx(full0 + 8 * q, (uint32_t)CRT_STAGE);
-                    bulk_g2s(st, a + (long long)kb * 2 * CRT_A_BLOCK, 2 * CRT_A_BLOCK, full0 + 8 * q);
-                    bulk_g2s(st + 2 * CRT_A_BLOCK, b + (long long)kb * 2 * CRT_B_BLOCK, 2 * CRT_B_BLOCK, full0 + 8 * q);
-                }
-                __syncwarp();
-                ++it;
             }
-        }
-        if (!ok) {
-            abort_flag = 1;
-            if (lane == 0) atomicOr(status, RB_TC5_TIMEOUT);
-            for (int i = max(0, it - CRT_STAGES); i < it; ++i)
-                mbar_wait(full0 + 8 * (i % CRT_STAGES), (uint32_t)((i / CRT_STAGES) & 1), nullptr);
+            if (!ok) {
+                abort_flag = 1;
+                atomicOr(status, RB_TC5_TIMEOUT);
+                for (int i = max(0, it - CRT_STAGES); i < it; ++i)
+                    mbar_wait(afull0 + 8 * (i % CRT_STAGES), (uint32_t)((i / CRT_STAGES) & 1), nullptr);
+                for (int i = max(0, nb - nk); i < nb; ++i) mbar_wait(bfull0 + 8 * (i % nk), (uint32_t)((i / nk) & 1), nullptr);
+            }
         }
         __syncwarp();
     } else if (warp == 1) {
         // ---------------- MMA issuer ------------------------------------------------------------------------
-        constexpr uint32_t LBO_A = CRT_BM * 16, LBO_B = CRT_B_ROWS * 16, SBO = 128;
+        // the whole warp runs the loop (the descriptors then live in uniform registers); one elected lane
+        // issues.  Both parts of a k block are one wait and one commit: 640 cycles of MMAs.
         constexpr uint32_t id2 = crt_idesc(2 * CRT_BN), id1 = crt_idesc(CRT_BN);
+        const uint32_t elected = elect_one();
+        const uint64_t da0 = crt_desc(sA), db0 = crt_desc(sB);
         bool ok = true;
-        int it = 0;
+        uint32_t q = 0;                              // stage
+        int ai = 0;                                  // accumulator sets begun
+        uint32_t par = 0u;                           // parity of the A stage's fill
         for (int s = s0; s < s1 && ok; ++s) {
-            const int si = s - s0, buf = si & 1, ua = si >> 1;
-            if (ua > 0) {
-                ok = __all_sync(0xffffffffu, mbar_wait(accempty0 + 8 * buf, (uint32_t)((ua - 1) & 1), &abort_flag));
+            for (int tm = t0; tm < t1 && ok; ++tm, ++ai) {
+                const int buf = ai & 1, ua = ai >> 1;
+                if (ua > 0) ok = mbar_wait(accempty0 + 8 * buf, (uint32_t)((ua - 1) & 1), &abort_flag);
                 if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            }
-            const uint32_t acc = tmem + (uint32_t)(buf * 256);
-            for (int kb = 0; kb < nk; ++kb, ++it) {
-                const int q = it % CRT_STAGES;
-                ok = __all_sync(0xffffffffu, mbar_wait(full0 + 8 * q, (uint32_t)((it / CRT_STAGES) & 1), &abort_flag));
-                if (!ok) break;
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                if (lane == 0) {
-                    const uint32_t st = smem_u32(stage_base + (size_t)q * CRT_STAGE);
+                const uint32_t acc = tmem + (uint32_t)(buf * 256);
+                for (int kb = 0; kb < nk; ++kb) {
+                    if (resident && tm == t0) ok = mbar_wait(bfull0 + 8 * kb, (uint32_t)((s - s0) & 1), &abort_flag);
+                    ok = ok && mbar_wait(afull0 + 8 * q, par, &abort_flag);
+                    if (!ok) break;
+                    if (elected) {
+                        // Ar: columns Ar Br | Ar Bi; Ai: columns Ai Br (onto Ar Bi) | Ai Bi
+                        const uint64_t da = da0 + q * (stage_bytes >> 4), dai = da + (CRT_A_BLOCK >> 4);
+                        const uint64_t db = db0 + (resident ? (uint32_t)kb * (CRT_B_BLOCK >> 4) : q * (stage_bytes >> 4));
+                        umma_i8(acc, da, db, id2, kb > 0 ? 1u : 0u);
 #pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        const uint32_t sa = st + (uint32_t)(h * CRT_A_BLOCK);
-                        const uint32_t sb = st + (uint32_t)(2 * CRT_A_BLOCK + h * CRT_B_BLOCK);
-                        const uint64_t ar = umma_desc(sa, LBO_A, SBO), ai = umma_desc(sa + CRT_A_BLOCK / 2, LBO_A, SBO);
-                        const uint64_t bb = umma_desc(sb, LBO_B, SBO);
-                        // columns: Ar Br | Ar Bi + Ai Br | Ai Bi
-                        umma_i8(acc, ar, bb, id2, (kb > 0 || h > 0) ? 1u : 0u);
-                        if (kb > 0 || h > 0) {
-                            umma_i8(acc + CRT_BN, ai, bb, id2, 1u);
+                        for (int j = 1; j < CRT_KB / 32; ++j) umma_i8(acc, da + 2 * j, db + 2 * j, id2, 1u);
+                        if (kb > 0) {
+                            umma_i8(acc + CRT_BN, dai, db, id2, 1u);
                         } else {
-                            umma_i8(acc + CRT_BN, ai, bb, id1, 1u);
-                            umma_i8(acc + 2 * CRT_BN, ai, umma_desc(sb + CRT_BN * 16, LBO_B, SBO), id1, 0u);
+                            umma_i8(acc + CRT_BN, dai, db, id1, 1u);
+                            umma_i8(acc + 2 * CRT_BN, dai, db + (CRT_BN * CRT_KB >> 4), id1, 0u);
                         }
+#pragma unroll
+                        for (int j = 1; j < CRT_KB / 32; ++j) umma_i8(acc + CRT_BN, dai + 2 * j, db + 2 * j, id2, 1u);
+                        umma_commit(aempty0 + 8 * q);
+                        if (resident && tm + 1 == t1) umma_commit(bempty0 + 8 * kb);
+                        if (kb + 1 == nk) umma_commit(accfull0 + 8 * buf);
                     }
-                    umma_commit(empty0 + 8 * q);
-                    if (kb + 1 == nk) umma_commit(accfull0 + 8 * buf);
+                    __syncwarp();
+                    if (++q == CRT_STAGES) {
+                        q = 0;
+                        par ^= 1u;
+                    }
                 }
-                __syncwarp();
             }
         }
         if (!ok) {
             abort_flag = 1;
-            if (lane == 0) atomicOr(status, RB_TC5_TIMEOUT);
+            if (elected) atomicOr(status, RB_TC5_TIMEOUT);
         }
-        if (lane == 0) umma_commit(done_bar);
+        if (elected) umma_commit(done_bar);
         __syncwarp();
         mbar_wait(done_bar, 0u, nullptr);            // every MMA has ended before tensor memory is freed
     } else if (warp >= 4) {
         // ---------------- epilogue: residues of the accumulators -------------------------------------------
         const int quarter = warp & 3, half = (warp - 4) >> 2;
         const int row = quarter * 32 + lane;
-        unsigned char* tile_out = out + ((prob * MT + tm) * NT + tn) * (long long)CRT_S * 2 * CRT_OUT;
-        for (int s = s0; s < s1; ++s) {
-            const int si = s - s0, buf = si & 1, ua = si >> 1;
-            if (!__all_sync(0xffffffffu, mbar_wait(accfull0 + 8 * buf, (uint32_t)(ua & 1), &abort_flag))) {
-                abort_flag = 1;
-                if (lane == 0) atomicOr(status, RB_TC5_TIMEOUT);
-                break;
-            }
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        int ai = 0;
+        bool ok = true;
+        for (int s = s0; s < s1 && ok; ++s) {
             const int m = c_mod[s], mg = c_magic[s];
-            const uint32_t acc = tmem + (uint32_t)(buf * 256) + ((uint32_t)(quarter * 32) << 16);
-            unsigned char* o = tile_out + (long long)s * 2 * CRT_OUT + row * 8;
-#pragma unroll
-            for (int c = 0; c < CRT_BN / 16; ++c) {
-                const int c8 = half * (CRT_BN / 16) + c;         // columns 8 c8 .. 8 c8 + 7
-                int p1[8], p3[8], p2[8];
-                tmem_ld8(acc + (uint32_t)(c8 * 8), p1);
-                tmem_ld8(acc + (uint32_t)(CRT_BN + c8 * 8), p3);
-                tmem_ld8(acc + (uint32_t)(2 * CRT_BN + c8 * 8), p2);
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                uint32_t re[2] = {0u, 0u}, im[2] = {0u, 0u};
-#pragma unroll
-                for (int e = 0; e < 8; ++e) {
-                    const int x = p1[e] - p2[e], y = p3[e];
-                    const int rx = x - m * (__mulhi(x, mg) >> 6), ry = y - m * (__mulhi(y, mg) >> 6);
-                    re[e >> 2] |= (uint32_t)rx << (8 * (e & 3));
-                    im[e >> 2] |= (uint32_t)ry << (8 * (e & 3));
+            for (int tm = t0; tm < t1; ++tm, ++ai) {
+                const int buf = ai & 1, ua = ai >> 1;
+                ok = __all_sync(0xffffffffu, mbar_wait(accfull0 + 8 * buf, (uint32_t)(ua & 1), &abort_flag));
+                if (!ok) {
+                    abort_flag = 1;
+                    if (lane == 0) atomicOr(status, RB_TC5_TIMEOUT);
+                    break;
                 }
-                *reinterpret_cast<uint2*>(o + c8 * (CRT_BM * 8)) = make_uint2(re[0], re[1]);
-                *reinterpret_cast<uint2*>(o + CRT_OUT + c8 * (CRT_BM * 8)) = make_uint2(im[0], im[1]);
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint32_t acc = tmem + (uint32_t)(buf * 256) + ((uint32_t)(quarter * 32) << 16);
+                unsigned char* o = out + (((prob * MT + tm) * NT + tn) * CRT_S + s) * 2LL * CRT_OUT + row * 8;
+#pragma unroll
+                for (int c = 0; c < CRT_BN / 16; ++c) {
+                    const int c8 = half * (CRT_BN / 16) + c;         // columns 8 c8 .. 8 c8 + 7
+                    int p1[8], p3[8], p2[8];
+                    tmem_ld8(acc + (uint32_t)(c8 * 8), p1);
+                    tmem_ld8(acc + (uint32_t)(CRT_BN + c8 * 8), p3);
+                    tmem_ld8(acc + (uint32_t)(2 * CRT_BN + c8 * 8), p2);
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                    uint32_t re[2] = {0u, 0u}, im[2] = {0u, 0u};
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) {
+                        const int x = p1[e] - p2[e], y = p3[e];
+                        const int rx = x - m * (__mulhi(x, mg) >> 6), ry = y - m * (__mulhi(y, mg) >> 6);
+                        re[e >> 2] |= (uint32_t)rx << (8 * (e & 3));
+                        im[e >> 2] |= (uint32_t)ry << (8 * (e & 3));
+                    }
+                    *reinterpret_cast<uint2*>(o + c8 * (CRT_BM * 8)) = make_uint2(re[0], re[1]);
+                    *reinterpret_cast<uint2*>(o + CRT_OUT + c8 * (CRT_BM * 8)) = make_uint2(im[0], im[1]);
+                }
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) mbar_arrive(accempty0 + 8 * buf);
             }
-            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            __syncwarp();
-            if (lane == 0) mbar_arrive(accempty0 + 8 * buf);
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -373,33 +459,35 @@ __global__ void __launch_bounds__(CRT_THREADS, 1) zgemm_crt_kernel(const GemmDes
     }
 }
 
-// Outputs from their residues: a thread takes 8 columns of one row of a tile.
-__global__ void __launch_bounds__(256) crt_combine_kernel(const GemmDesc* __restrict__ descs, int prob0, int MT, int NT,
+// Outputs from their residues: a thread takes 4 columns of one row of a tile; two neighbours share the
+// 8 residues a row has in a column group.
+__global__ void __launch_bounds__(256, 4) crt_combine_kernel(const GemmDesc* __restrict__ descs, int prob0, int MT, int NT,
                                                           const unsigned char* __restrict__ out, const int* __restrict__ ea,
                                                           const int* __restrict__ fb) {
     const GemmDesc& g = descs[blockIdx.y];
     const long long prob = prob0 + (long long)blockIdx.y;
     const int tiles_m = (g.m + CRT_BM - 1) / CRT_BM;
-    // blockIdx.x: pairs of column groups of a tile (tm fastest)
-    const int per = CRT_BN / 16, t = blockIdx.x / per;
+    // blockIdx.x: column groups of a tile (tm fastest)
+    const int c8 = blockIdx.x % (CRT_BN / 8), t = blockIdx.x / (CRT_BN / 8);
     const int tm = t % tiles_m, tn = t / tiles_m;
-    const int row = threadIdx.x & 127, c8 = 2 * (blockIdx.x % per) + (threadIdx.x >> 7);
-    const int i = tm * CRT_BM + row, j0 = tn * CRT_BN + 8 * c8;
-    if (tn * CRT_BN >= g.n || i >= g.m || j0 >= g.n) return;
-    const unsigned char* p = out + ((prob * MT + tm) * NT + tn) * (long long)CRT_S * 2 * CRT_OUT + c8 * (CRT_BM * 8) + row * 8;
+    const int row = threadIdx.x >> 1, c4 = 2 * c8 + (threadIdx.x & 1);
+    const int i = tm * CRT_BM + row, j0 = tn * CRT_BN + 4 * c4;
+    if (i >= g.m || j0 >= g.n) return;
+    const unsigned char* p = out + ((prob * MT + tm) * NT + tn) * (long long)CRT_S * 2 * CRT_OUT + c8 * (CRT_BM * 8) +
+                             threadIdx.x * 4;
     constexpr double magic = 4503599627370496.0;         // 2^52
-    double hr[8], lr[8], hi[8], li[8];
+    double hr[4], lr[4], hi[4], li[4];
 #pragma unroll
-    for (int e = 0; e < 8; ++e) hr[e] = lr[e] = hi[e] = li[e] = 0.0;
-#pragma unroll 4
+    for (int e = 0; e < 4; ++e) hr[e] = lr[e] = hi[e] = li[e] = 0.0;
+#pragma unroll 8
     for (int s = 0; s < CRT_S; ++s) {
-        const uint2 a = *reinterpret_cast<const uint2*>(p + (long long)s * 2 * CRT_OUT);
-        const uint2 b = *reinterpret_cast<const uint2*>(p + (long long)s * 2 * CRT_OUT + CRT_OUT);
+        const uint32_t a = *reinterpret_cast<const uint32_t*>(p + (long long)s * 2 * CRT_OUT);
+        const uint32_t b = *reinterpret_cast<const uint32_t*>(p + (long long)s * 2 * CRT_OUT + CRT_OUT);
         const double wh = c_whi[s], wl = c_wlo[s];
 #pragma unroll
-        for (int e = 0; e < 8; ++e) {
-            const double x = __hiloint2double(0x43300000, (int)(((e < 4 ? a.x : a.y) >> (8 * (e & 3))) & 0xFFu)) - magic;
-            const double y = __hiloint2double(0x43300000, (int)(((e < 4 ? b.x : b.y) >> (8 * (e & 3))) & 0xFFu)) - magic;
+        for (int e = 0; e < 4; ++e) {
+            const double x = __hiloint2double(0x43300000, (int)((a >> (8 * e)) & 0xFFu)) - magic;
+            const double y = __hiloint2double(0x43300000, (int)((b >> (8 * e)) & 0xFFu)) - magic;
             hr[e] = __fma_rn(x, wh, hr[e]);
             lr[e] = __fma_rn(x, wl, lr[e]);
             hi[e] = __fma_rn(y, wh, hi[e]);
@@ -407,14 +495,14 @@ __global__ void __launch_bounds__(256) crt_combine_kernel(const GemmDesc* __rest
         }
     }
     const int er = crt_exp(ea[(prob * MT + tm) * CRT_BM + row]);
-    const int* fc = fb + (prob * NT + tn) * CRT_BN + 8 * c8;
+    const int* fc = fb + (prob * NT + tn) * CRT_BN + 4 * c4;
     const z alpha = g.alpha, beta = g.beta;
     const long long dro = vrow(g.D, i);
     const bool use_c = g.C.p && !(i >= g.nobeta_r0 && i < g.nobeta_r1);
     const long long cro = use_c ? (long long)vrow(g.C, i) : 0;
     constexpr double rm = 1.0 / CRT_MHI;
 #pragma unroll
-    for (int e = 0; e < 8; ++e) {
+    for (int e = 0; e < 4; ++e) {
         const int j = j0 + e;
         if (j >= g.n) break;
         // the symmetric representative: minus the nearest multiple of M, exact in both parts
@@ -423,9 +511,12 @@ __global__ void __launch_bounds__(256) crt_combine_kernel(const GemmDesc* __rest
         double im = __fma_rn(-qi, CRT_MHI, hi[e]) + __fma_rn(-qi, CRT_MLO, li[e]);
         const int fj = crt_exp(fc[e]);
         const int p2 = er + fj - 2 * CRT_P + CRT_LO;
-        re = ldexp(re, p2);
-        im = ldexp(im, p2);
-        if (er >= CRT_NONFINITE || fj >= CRT_NONFINITE) re = im = __longlong_as_double(0x7ff8000000000000LL);
+        if (er >= CRT_NONFINITE || fj >= CRT_NONFINITE) {
+            re = im = __longlong_as_double(0x7ff8000000000000LL);
+        } else {
+            re = crt_ldexp(re, p2);
+            im = crt_ldexp(im, p2);
+        }
         z v = gemm_alpha(alpha, zmk(re, im));
         if (use_c) v = gemm_beta(v, beta, g.C.p[cro + (long long)vcol(g.C, j) * g.C.ld]);
         g.D.p[dro + (long long)vcol(g.D, j) * g.D.ld] = v;
@@ -434,7 +525,11 @@ __global__ void __launch_bounds__(256) crt_combine_kernel(const GemmDesc* __rest
 
 size_t crt_bytes(const GemmBatch& b) {
     if (b.count == 0 || b.max_m == 0 || b.max_n == 0 || b.max_k == 0 || b.max_k > CRT_MAX_K) return 0;
-    return (size_t)crt_geom(b).total;
+    // the split and combine grids take one block per slab and per column group
+    const CrtGeom g = crt_geom(b);
+    const long long slabs = (long long)b.count * g.KB * (g.MT * (CRT_BM / 16) + g.NT * (CRT_BN / 16));
+    if (slabs > INT_MAX || (long long)g.MT * g.NT * (CRT_BN / 8) > INT_MAX) return 0;
+    return (size_t)g.total;
 }
 
 cudaError_t launch_gemm_crt(const GemmBatch& b, int* status, cudaStream_t s) {
@@ -449,21 +544,22 @@ cudaError_t launch_gemm_crt(const GemmBatch& b, int* status, cudaStream_t s) {
     unsigned char* ws = static_cast<unsigned char*>(b.crt_ws);
     int* ea = reinterpret_cast<int*>(ws + cg.ea_off);
     int* fb = reinterpret_cast<int*>(ws + cg.fb_off);
-    const long long nA = (long long)b.count * cg.MT * cg.KB2 * 2, nB = (long long)b.count * cg.NT * cg.KB2 * 2;
+    const long long nA = (long long)b.count * cg.MT * cg.KB * (CRT_BM / 16), nB = (long long)b.count * cg.NT * cg.KB * (CRT_BN / 16);
     const long long tiles = (long long)cg.MT * cg.NT;
-    if (nA + nB > 0x7FFFFFFFLL || tiles * (CRT_BN / 16) > 0x7FFFFFFFLL) return cudaErrorInvalidValue;
     if ((e = launch_operand_scales(b, cg.MT * CRT_BM, cg.NT * CRT_BN, ea, fb, s)) != cudaSuccess) return e;
-    crt_split_kernel<<<(unsigned)(nA + nB), 256, 0, s>>>(b.d_desc, cg.MT, cg.NT, cg.KB2 * 2, nA, ws, cg.a_bytes, ea, fb);
+    crt_split_kernel<<<(unsigned)(nA + nB), 256, 0, s>>>(b.d_desc, cg.MT, cg.NT, cg.KB, nA, ws, cg.a_bytes, ea, fb);
     note_launch();
-    // groups of moduli until there are about four CTAs per SM to even the last wave out
+    // runs of up to 8 row tiles per CTA (a resident B tile serves them all), and groups of moduli until there
+    // are about six CTAs per SM to even the last wave out
+    const int R = std::min(cg.MT, 8), runs = (cg.MT + R - 1) / R;
     int groups = 1;
-    while (groups < 8 && tiles * b.count * groups < 4 * 148) groups *= 2;
+    while (groups < CRT_S && (long long)runs * cg.NT * b.count * groups < 6 * 148) groups *= 2;
     for (int off = 0; off < b.count; off += 65535) {
         const int cnt = std::min(b.count - off, 65535);
-        zgemm_crt_kernel<<<dim3((unsigned)tiles, cnt, groups), CRT_THREADS, CRT_SMEM, s>>>(
-            b.d_desc + off, off, status, ws, cg.MT, cg.NT, cg.KB2, cg.a_bytes, ws + cg.c_off, CRT_S / groups);
+        zgemm_crt_kernel<<<dim3((unsigned)(runs * cg.NT), cnt, groups), CRT_THREADS, CRT_SMEM, s>>>(
+            b.d_desc + off, off, status, ws, cg.MT, cg.NT, cg.KB, cg.a_bytes, ws + cg.c_off, R, CRT_S / groups);
         note_launch();
-        crt_combine_kernel<<<dim3((unsigned)(tiles * (CRT_BN / 16)), cnt), 256, 0, s>>>(b.d_desc + off, off, cg.MT, cg.NT,
+        crt_combine_kernel<<<dim3((unsigned)(tiles * (CRT_BN / 8)), cnt), 256, 0, s>>>(b.d_desc + off, off, cg.MT, cg.NT,
                                                                                        ws + cg.c_off, ea, fb);
         note_launch();
     }

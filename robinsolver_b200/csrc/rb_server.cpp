@@ -40,6 +40,8 @@
 namespace rb {
 const z* tree_solutions(const rb_tree* t);
 double tree_bytes_estimate(const rb_tree* t, int nrhs, int precision);
+double tree_crt_bytes(const rb_tree* t);
+void tree_crt_off(rb_tree* t);
 }  // namespace rb
 
 using namespace rb;
@@ -134,7 +136,11 @@ static int admit(rb_server* s, TreeSlot& slot, std::unique_lock<std::mutex>& lk,
     if (slot.reserved > 0.0) return RB_OK;
     const int B = s->opts.max_batch_rhs;
     const double stage = ((double)B * slot.info.n_interior + (double)B * slot.info.root_nb + slot.info.n_interior) * 16.0;
-    const double need = tree_bytes_estimate(slot.t, B, s->opts.precision) + stage;
+    double need = tree_bytes_estimate(slot.t, B, s->opts.precision) + stage;
+    // the residue engine's workspaces count too; a tree that fits the budget without them only does
+    // without them
+    if (need + tree_crt_bytes(slot.t) <= s->budget) need += tree_crt_bytes(slot.t);
+    else tree_crt_off(slot.t);
     if (need > s->budget) {
         msg = "tree needs about " + std::to_string((long long)need) + " bytes of device memory, the server's budget is " +
               std::to_string((long long)s->budget);

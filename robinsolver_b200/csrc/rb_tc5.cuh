@@ -44,13 +44,14 @@ __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
 // waits for the phase with the given parity to complete; false after RB_TC5_WAIT_NS or when
 // another warp has already given up (*abort, if given)
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort) {
-    if (mbar_try(bar, parity)) return true;
-    const unsigned long long t0 = global_ns();
-    for (unsigned it = 0;; ++it) {
+    unsigned long long t0 = 0;
+    for (unsigned it = 1;; ++it) {
         if (mbar_try(bar, parity)) return true;
-        if ((it & 63) == 63) {
-            if (abort && *abort) return false;
-            if (global_ns() - t0 > RB_TC5_WAIT_NS) return false;
+        if ((it & 63) == 0 && abort && *abort) return false;
+        if ((it & 1023) == 0) {
+            const unsigned long long t = global_ns();
+            if (t0 == 0) t0 = t;
+            else if (t - t0 > RB_TC5_WAIT_NS) return false;
         }
     }
 }

@@ -76,15 +76,24 @@ static int fail(rb_tree* t, int code, const std::string& msg) {
     return code;
 }
 
+static void drop_crt_plan(rb_tree* t);
+
 static int dev_alloc(rb_tree* t, std::vector<DevBuf>& list, size_t bytes, void** out) {
     *out = nullptr;
     if (bytes == 0) return RB_OK;
     bytes = (bytes + 255) & ~size_t(255);
+    // the residue engine's workspaces give way to anything the handle cannot do without
+    if (t->budget > 0 && t->held + (int64_t)bytes > t->budget) drop_crt_plan(t);
     if (t->budget > 0 && t->held + (int64_t)bytes > t->budget)
         return fail(t, RB_ERR_OUT_OF_MEMORY, "device budget exceeded: need " + std::to_string(t->held + bytes) +
                                                  " bytes, budget " + std::to_string(t->budget));
     void* p = nullptr;
     cudaError_t e = cudaMalloc(&p, bytes);
+    if (e == cudaErrorMemoryAllocation && t->crt_state == rb_tree::CRT_HELD) {
+        cudaGetLastError();
+        drop_crt_plan(t);
+        e = cudaMalloc(&p, bytes);
+    }
     if (e != cudaSuccess) {
         cudaGetLastError();
         return fail(t, e == cudaErrorMemoryAllocation ? RB_ERR_OUT_OF_MEMORY : RB_ERR_CUDA,
@@ -602,7 +611,96 @@ static bool mixed_batch(const rb_tree* t, const GemmBatch& b, int l) {
     return bit == 0 || (mixed_stage_mask() & bit) != 0;
 }
 static cudaError_t launch_gemm_level(rb_tree* t, const GemmBatch& b, int l, cudaStream_t s) {
-    return mixed_batch(t, b, l) ? launch_gemm_tc5(b, t->d_status, s) : launch_gemm_batch(b, s);
+    if (mixed_batch(t, b, l)) return launch_gemm_tc5(b, t->d_status, s);
+    return b.crt_ws ? launch_gemm_crt(b, t->d_status, s) : launch_gemm_batch(b, s);
+}
+
+// The FP64 products of levels whose interface has CRT_MIN_M points or more (k of every product of a
+// level) run on the residue engine.
+// Whole steps, FP64 tiles everywhere against this rule: 1024^2 27.3 to 22.2 ms, 512^2 (the root alone)
+// 6.0 to 5.7, 32^3 28.7 to 19.9.  At 256 points the passes over the operands and outputs cost what the
+// products save (768 x 768 x 256 in 32 problems 988 to 826 us, 256 x 768 in 16 190 to 236).
+// The rule is one per level, so that the row sets of the pipelined factor and the whole map of the
+// serial one take the same engine: its sums are exact, and the two agree bit for bit.
+constexpr int CRT_MIN_M = 512;
+static bool crt_level(const rb_tree* t, int l) {
+    const int m = t->P.lv[l].m;
+    return m >= CRT_MIN_M && m <= CRT_MAX_K;
+}
+// the batches of a level on the main stream (lane 0), the chain stream (1) and B1's (2); the serial
+// factor runs the first two on the main stream, one after another
+static std::vector<GemmBatch*> crt_stages(rb_tree* t, int l, int lane) {
+    const bool tail = l == 0 || !t->kform;
+    if (lane == 2) return {&t->fM1[l]};
+    if (lane == 1) return tail ? std::vector<GemmBatch*>{&t->fK[l]}
+                               : std::vector<GemmBatch*>{&t->fK[l], &t->fM2[l], &t->fM3[l], &t->fM4F[l]};
+    return tail ? std::vector<GemmBatch*>{&t->fM2[l], &t->fM3[l], &t->fM4[l]}
+                : std::vector<GemmBatch*>{&t->fM4[l], &t->fM4N[l]};
+}
+// bytes of the lanes' workspaces, from the plan alone
+static size_t crt_lane_bytes(const rb_tree* t, size_t need[3]) {
+    auto bytes = [](int count, int m, int n, int k) {
+        GemmBatch b;
+        b.count = count;
+        b.max_m = m;
+        b.max_n = n;
+        b.max_k = k;
+        return crt_bytes(b);
+    };
+    need[0] = need[1] = need[2] = 0;
+    for (int l = 0; l < t->P.L; ++l) {
+        if (!crt_level(t, l)) continue;
+        const PlanLevel& p = t->P.lv[l];
+        const int n = std::max(p.n1, p.n2), m = p.m, nn = p.nnodes;
+        const bool tail = l == 0 || !t->kform;
+        if (!(l == 0 && t->skip_root)) need[0] = std::max(need[0], bytes(4 * nn, n, n, m));
+        need[tail ? 0 : 1] = std::max(need[tail ? 0 : 1], bytes(2 * nn, m, n, m));
+        if (t->kform) need[1] = std::max(need[1], bytes(nn, m, m, m));
+        // the rows on the face the parent merges across: at most its interface's points
+        if (!tail) need[1] = std::max(need[1], bytes(4 * nn, std::min(n, t->P.lv[l - 1].m), n, m));
+        need[2] = std::max(need[2], bytes(nn, m, n, m));
+    }
+    return need[0] + need[1] + need[2];
+}
+// One workspace per stream that runs such products (the streams of a factor run side by side, a
+// stream's products one after another).  They are a convenience: taken where they fit the handle's
+// budget and a sixteenth of the device's free memory, given back when a later allocation of the
+// handle would fail (dev_alloc), and without them the FP64 tiles do the work.
+static int ensure_crt_plan(rb_tree* t) {
+    if (t->crt_state != rb_tree::CRT_NONE) return RB_OK;
+    t->crt_state = rb_tree::CRT_OFF;
+    size_t need[3], fr = 0, all = 0;
+    const size_t total = crt_lane_bytes(t, need);
+    if (total == 0) return RB_OK;
+    RB_CK(cudaMemGetInfo(&fr, &all));
+    if (total > fr / 16 || (t->budget > 0 && t->held + (int64_t)total > t->budget)) return RB_OK;
+    void* ws[3];
+    for (int lane = 0; lane < 3; ++lane)
+        if (dev_alloc(t, t->crt_bufs, need[lane], &ws[lane]) != RB_OK) {
+            free_list(t, t->crt_bufs);
+            return RB_OK;
+        }
+    for (int l = 0; l < t->P.L; ++l)
+        for (int lane = 0; lane < 3 && crt_level(t, l); ++lane)
+            for (GemmBatch* b : crt_stages(t, l, lane)) {
+                const size_t bytes = crt_bytes(*b);
+                if (bytes == 0 || bytes > need[lane]) continue;
+                b->crt_ws = ws[lane];
+                b->crt_cap = need[lane];
+            }
+    t->crt_state = rb_tree::CRT_HELD;
+    return RB_OK;
+}
+static void drop_crt_plan(rb_tree* t) {
+    if (t->crt_state != rb_tree::CRT_HELD) return;
+    t->crt_state = rb_tree::CRT_OFF;
+    cudaStreamSynchronize(t->stream);                 // every stream of a factor joins it
+    drop_graph(t->gx_factor);
+    t->factor_runs = 0;
+    for (int l = 0; l < t->P.L; ++l)
+        for (int lane = 0; lane < 3; ++lane)
+            for (GemmBatch* b : crt_stages(t, l, lane)) b->crt_ws = nullptr;
+    free_list(t, t->crt_bufs);
 }
 // The mixed solve applies its factor with the FP64 GEMMs: the sweeps' products are narrow (n =
 // the right-hand sides), where the tcgen05 tile is slower than the FP64 one (1024^2, L=12, 32
@@ -667,8 +765,8 @@ static int ensure_mixed_factor_plan(rb_tree* t) {
 }
 
 #define RB_GEMM_L(batch, level, stream)                                                          \
-    RB_TIMED(mixed_batch(t, batch, level) ? "zgemm_tc5" : gemm_stage_name(batch), (batch).flops,  \
-             launch_gemm_level(t, batch, level, stream))
+    RB_TIMED(mixed_batch(t, batch, level) ? "zgemm_tc5" : (batch).crt_ws ? "zgemm_crt" : gemm_stage_name(batch),  \
+             (batch).flops, launch_gemm_level(t, batch, level, stream))
 
 static double gj_flops(int m, int count) { return 8.0 * (double)m * m * m * count; }
 // arithmetic of one structured leaf factor: b block inverses (8 a^3 each) and two block sweeps
@@ -1534,6 +1632,7 @@ int rb_tree_destroy(rb_tree* t) {
     free_list(t, t->solve_bufs);
     free_list(t, t->refine_bufs);
     free_list(t, t->mixed_bufs);
+    free_list(t, t->crt_bufs);
     free_list(t, t->bufs);
     if (t->h_norms) cudaFreeHost(t->h_norms);
     for (auto& e : t->ev)
@@ -1753,6 +1852,8 @@ static int settle_solution(rb_tree* t) {
     if (t->h_status[1]) {
         t->factored = false;
         t->nrhs = 0;
+        if (t->h_status[1] & (RB_STATUS_GJ_TIMEOUT | RB_TC5_TIMEOUT))
+            return fail(t, RB_ERR_CUDA, "a device wait timed out during the factorization");
         return fail(t, RB_ERR_NUMERIC, "zero pivot met while inverting a leaf or interface matrix");
     }
     return RB_OK;
@@ -1783,6 +1884,7 @@ static int factor_common(rb_tree* t, const double* k, int precision, bool host, 
         t->factor_runs = 0;
     }
     if (precision == RB_PREC_MIXED && (rc = ensure_mixed_factor_plan(t))) return rc;
+    if ((rc = ensure_crt_plan(t))) return rc;
     if (t->timing == 1) {
         timers_collect(t);
         t->stage_ms.clear();
@@ -2172,6 +2274,15 @@ double tree_bytes_estimate(const rb_tree* t, int nrhs, int precision) {
     per_rhs *= 1.5;                                   // split-K workspace and the root's x1, x2
     if (precision == RB_PREC_MIXED) per_rhs += (double)Q.nleaves() * (Q.leaf_n() + Q.leaf_nb()) * 16.0;
     return need * 1.02 + per_rhs * nrhs + (64 << 20);
+}
+// device bytes of the residue engine's workspaces, and a tree that is to do without them (before its
+// first factorization)
+double tree_crt_bytes(const rb_tree* t) {
+    size_t need[3];
+    return (double)crt_lane_bytes(t, need);
+}
+void tree_crt_off(rb_tree* t) {
+    if (t->crt_state == rb_tree::CRT_NONE) t->crt_state = rb_tree::CRT_OFF;
 }
 }  // namespace rb
 

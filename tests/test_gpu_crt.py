@@ -62,3 +62,54 @@ def test_crt_gemm_scales_zero_rows_and_nonfinite():
     mask[20, :] = mask[:, 30] = False
     assert np.isnan(bad[0, 20]).all() and np.isnan(bad[0, :, 30]).all()
     assert np.array_equal(bad[0][mask], got[0][mask])
+
+
+@pytest.mark.parametrize("m,n,k", [(130, 85, 70), (257, 80, 1024)])
+def test_crt_gemm_problems_that_share_an_operand(m, n, k):
+    """Neighbours with one A use one set of its planes: the same bits as with an A each."""
+    import torch
+
+    from robinsolver_b200 import _lib
+    rng = np.random.default_rng(m)
+    cx = lambda *s: rng.standard_normal(s) + 1j * rng.standard_normal(s)  # noqa: E731
+    A, B, C0 = np.repeat(cx(1, m, k), 3, axis=0), cx(3, k, n), cx(3, m, n)
+    ref = _run(4, A, B, C0, ALPHA, BETA)
+    dA, dB, dC = (torch.from_numpy(np.ascontiguousarray(x.transpose(0, 2, 1))).cuda() for x in (A[:1], B, C0))
+    rc = _lib.lib.rb_test_zgemm(4, m, n, k, dA.data_ptr(), m, 0, dB.data_ptr(), k, k * n, dC.data_ptr(), m, m * n, ALPHA.real,
+                                ALPHA.imag, BETA.real, BETA.imag, 3)
+    assert rc == 0, _lib.last_error(None)
+    assert np.array_equal(dC.cpu().numpy().transpose(0, 2, 1), ref)
+
+
+def test_factor_without_room_for_the_residue_workspaces():
+    """A budget that the workspaces do not fit leaves the products to the FP64 tiles, and one that
+    they fit only until the solve's buffers come gives them back; nothing is refused.  Tolerance: both
+    engines are FP64-accurate, and this system loses about 4 digits of 16 (1e-10 with room to spare)."""
+    from helpers import gpu_rhs, gpu_tree
+    from robinsolver_b200 import _lib
+    from robinsolver_b200 import workloads as W
+    wl = W.make_workload(2, nrhs=2)
+
+    def run(budget):
+        T, op, opts = gpu_tree(wl, device_budget=budget)
+        T.plan(wl.L, op, opts)
+        k = op.k(T.sample_points(_lib.RB_POINTS_POTENTIAL))
+        T.factor_samples(k)
+        held = T.info().device_bytes
+        T.solve(gpu_rhs(wl.rhs))
+        out = np.stack([T.solution_array(r) for r in range(2)])
+        after = T.info().device_bytes
+        T.factor_samples(k)                          # and again in the state that the solve left
+        T.solve(gpu_rhs(wl.rhs))
+        again = np.stack([T.solution_array(r) for r in range(2)])
+        T.close()
+        return held, after, out, again
+
+    free = run(0)
+    tight = run(free[0] - 1)
+    assert tight[0] < free[0]
+    late = run(free[0])
+    assert late[0] == free[0] and late[1] == tight[1] < free[1]
+    assert np.array_equal(late[2], free[2]) and np.array_equal(late[3], tight[3])
+    for u in (tight[2], tight[3], late[3]):
+        assert np.abs(u - free[2]).max() < 1e-10 * np.abs(free[2]).max()
