@@ -16,9 +16,12 @@
 //      instead cancels catastrophically: W_P's diagonal holds the reciprocal pivots, ~h^2 for
 //      the FD matrices here.)
 //   The resident kernel (gj_resident) runs the whole batch in one cooperative launch with the
-//   columns held in shared memory; gj_panel + gj_apply, two launches per panel, are the same
-//   arithmetic in the same order, used when the batch does not fit on the device at once.
-// After the last panel the column exchanges are undone in reverse order (gj_unscramble).
+//   columns held in shared memory (in several, when they do not fit at once); gj_panel + gj_apply, two
+//   launches per panel, are the same arithmetic in the same order, used when a device cannot hold one
+//   matrix and to compare.
+// After the last panel the column exchanges are undone in reverse order (by the resident kernel as it
+// writes, by gj_unscramble after the blocked path).
+#include <algorithm>
 #include <cstdlib>
 #include "rb_gemm_tile.cuh"
 #include "rb_kernels.h"
@@ -31,8 +34,8 @@ int gj_panel_width(int m) {
     return 8;
 }
 
-// one complex element per matrix: the resident path's two flag words
-long long gj_workspace_elems(int m) { return m <= GJ_SMALL_MAX ? 0 : 1; }
+// the resident path's two words per panel of 8 columns and its counter, in complex elements per matrix
+long long gj_workspace_elems(int m) { return m <= GJ_SMALL_MAX ? 0 : (m + 7) / 8 + 1; }
 
 // warp argmax: larger value wins, equal values go to the smaller index
 __device__ __forceinline__ void argmax_warp(double& v, int& i) {
@@ -42,6 +45,16 @@ __device__ __forceinline__ void argmax_warp(double& v, int& i) {
         const int oi = __shfl_down_sync(0xffffffffu, i, o);
         if (ov > v || (ov == v && oi < i)) { v = ov; i = oi; }
     }
+}
+
+// a b and 1/a with the roundings spelled out: the two paths above m = 64 agree bit for bit whichever
+// product of a sum the compiler would have fused
+__device__ __forceinline__ z gj_mul(z a, z b) {
+    return zmk(__fma_rn(-a.y, b.y, __dmul_rn(a.x, b.x)), __fma_rn(a.y, b.x, __dmul_rn(a.x, b.y)));
+}
+__device__ __forceinline__ z gj_rcp(z a) {
+    const double r = 1.0 / __fma_rn(a.y, a.y, __dmul_rn(a.x, a.x));
+    return zmk(__dmul_rn(a.x, r), __dmul_rn(-a.y, r));
 }
 
 __device__ __forceinline__ bool zis0(z a) { return a.x == 0.0 && a.y == 0.0; }
@@ -140,9 +153,9 @@ __global__ void __launch_bounds__(MAXT) gj_panel_kernel(const GJDesc* __restrict
         const int p = __shfl_sync(0xffffffffu, idx, 0);
         if (r == p) {
             if (zis0(row[kk])) bad = true;
-            const z pinv = zrcp(row[kk]);
+            const z pinv = gj_rcp(row[kk]);
 #pragma unroll
-            for (int j = 0; j < NB; ++j) prow[sb][j] = (j == kk) ? pinv : zmul(row[j], pinv);
+            for (int j = 0; j < NB; ++j) prow[sb][j] = (j == kk) ? pinv : gj_mul(row[j], pinv);
             g.ipiv[c] = p;
         }
         if (r == c && p != c) {
@@ -162,7 +175,7 @@ __global__ void __launch_bounds__(MAXT) gj_panel_kernel(const GJDesc* __restrict
 #pragma unroll
             for (int j = 0; j < NB; ++j)
                 if (j != kk) zfms(row[j], f, prow[sb][j]);
-            row[kk] = zneg(zmul(f, prow[sb][kk]));
+            row[kk] = zneg(gj_mul(f, prow[sb][kk]));
         }
     }
     if (own) {
@@ -227,18 +240,20 @@ __global__ void __launch_bounds__(256) gj_apply_kernel(const GJDesc* __restrict_
 // ---------------------------------------------------------------------------------------------------
 // Resident Gauss-Jordan: the whole batch in one launch.  Matrix i is split over P CTAs by whole
 // panels of NB columns; CTA j keeps its ppc panels (m x cw complex, cw <= ppc*NB) in shared
-// memory for the whole inversion.  The owner of panel p eliminates it (one row per thread in
-// registers, as gj_panel_kernel), writes the accumulated transform W_p to the matrix's own
-// global storage at panel p's columns (unused while the columns live in shared memory) and its
-// pivots to ipiv, and publishes p+1 in the matrix's flag word.  Every CTA then applies step p
-// (the exchanges, then A += W_p Z outside the panel rows and W_p Z on them) to its resident
-// columns.  The owner of panel p+1 applies step p to that panel first, eliminates and publishes
-// it, and only then updates its other columns, so the dependent chain per step is one flag
-// hand-off, one panel update and one panel elimination.  After the last step a per-matrix
-// counter holds every CTA until all have stopped reading W slots; then the columns go back.
+// memory for the whole inversion.  No row is exchanged: a pivot's row stays where it is and is passed
+// over by later searches, and the permutation goes into the final write.  The owner of panel p
+// eliminates it (one or two rows per thread in registers), writes the accumulated transform W_p to the
+// matrix's own global storage at panel p's columns (unused while the columns live in shared memory), and
+// publishes the panel's pivot rows in its two words.  Every CTA then applies step p (A += W_p Z outside
+// the pivots' rows and W_p Z on them, Z the pivots' rows) to its resident columns.  The owner of panel
+// p+1 applies step p to that panel first, eliminates and publishes it, and only then updates its other
+// columns, so the dependent chain per step is one hand-off, one panel update and one panel elimination.
+// After the last step a per-matrix counter holds every CTA until all have stopped reading W slots; then
+// the columns go back.  The arithmetic is the blocked path's, in its order (rows of equal magnitude are
+// ranked by where they stand, so exactly tied pivots may fall differently).
 //
 // The launch is cooperative (all CTAs co-resident), and every wait is bounded in time: a CTA
-// that waits longer than GJ_WAIT_NS sets bit 2 of the status word and returns.
+// that waits longer than GJ_WAIT_NS sets RB_STATUS_GJ_TIMEOUT in the status word and returns.
 constexpr unsigned long long GJ_WAIT_NS = 1000000000ull;
 
 __device__ __forceinline__ unsigned long long global_ns() {
@@ -251,144 +266,172 @@ __device__ __forceinline__ int ld_acquire_gpu(const int* p) {
     asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
     return v;
 }
-__device__ __forceinline__ void st_release_gpu(int* p, int v) {
-    asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+
+__device__ __forceinline__ unsigned long long ld_acquire_gpu(const unsigned long long* p) {
+    unsigned long long v;
+    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void st_release_gpu(unsigned long long* p, unsigned long long v) {
+    asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
 
-// thread 0 waits until *flag >= target; the outcome is returned to every thread of the CTA
-__device__ bool cta_wait_geq(const int* flag, int target, int* status, int* s_ok) {
-    if (threadIdx.x == 0) {
-        int ok = 1;
-        if (ld_acquire_gpu(flag) < target) {
+// Shared state of a CTA.  Everything is double-buffered by the parity of its column or step: it is
+// written again two later, after a block barrier that follows its last read.
+template <int NB>
+struct ResShared {
+    z prow[2][NB];                       // a column's scaled pivot row
+    uint4 cand[2][32];                   // per warp: its candidate's key (high, low word) and row
+    int spv[2][NB];                      // a step's pivot rows
+    int ok[2], done_ok;
+};
+
+// A panel's two words: four pivot rows each, 12 bits a row, under the top bit
+static_assert(8 == 2 * 4, "pivots of a panel in two words");
+constexpr unsigned long long GJ_READY = 1ull << 63;
+
+// The words of step p, awaited by two lanes (bounded); the pivots go to shared memory, the outcome to
+// every thread of the CTA.
+template <int NB>
+__device__ __forceinline__ bool res_wait_step(const unsigned long long* words, int p, int* status, ResShared<NB>& sh) {
+    if (threadIdx.x < 2) {
+        unsigned long long w = ld_acquire_gpu(words + 2 * p + threadIdx.x);
+        if (!(w & GJ_READY)) {
             const unsigned long long t0 = global_ns();
             int spins = 0;
-            while (ld_acquire_gpu(flag) < target) {
+            while (!((w = ld_acquire_gpu(words + 2 * p + threadIdx.x)) & GJ_READY)) {
                 if (++spins > 32) __nanosleep(40);
                 if (global_ns() - t0 > GJ_WAIT_NS) {
-                    ok = 0;
-                    atomicOr(status, 2);
+                    sh.ok[p & 1] = 0;
+                    atomicOr(status, RB_STATUS_GJ_TIMEOUT);
                     break;
                 }
             }
         }
-        *s_ok = ok;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) sh.spv[p & 1][4 * threadIdx.x + i] = (int)((w >> (12 * i)) & 0xFFF);
     }
     __syncthreads();
-    const bool ok = *s_ok != 0;
-    __syncthreads();                     // s_ok may be rewritten by the next wait
-    return ok;
+    return sh.ok[p & 1] != 0;
 }
 
-// Slots of one elimination column, double-buffered by column parity: column kk writes set kk & 1,
-// so a column's slots are rewritten two columns later, after every thread has passed the block
-// barrier that follows its last read of them -- one barrier per column fewer than single slots.
-template <int NB>
-struct ResShared {
-    z xb[2][NB], prow[2][NB];
-    unsigned kh[2][32], kl[2][32];
-    int ki[2][32];
-    int spv[NB];                         // pivots of the step being applied
-    int ok;
-};
-
-// warp argmax over (hi, lo) = the bit pattern of a non-negative double (which orders like the
-// value), ties to the smaller row: three warp reductions instead of a shuffle tree
-__device__ __forceinline__ void warp_key_max(unsigned& hi, unsigned& lo, int& id) {
+// The largest key (hi, lo) -- the bit pattern of a non-negative double, which orders like the value -- of a
+// warp, ties to the smaller row: true on the lane that holds it.  One reduction and a vote unless two
+// high words tie.
+__device__ __forceinline__ bool warp_key_best(unsigned hi, unsigned lo, int id, unsigned& best) {
     const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
-    const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? lo : 0u);
-    id = __reduce_min_sync(0xffffffffu, (hi == mh && lo == ml) ? id : 0x7fffffff);
-    hi = mh;
-    lo = ml;
-}
-
-// CTA-wide argmax of v over the valid rows (largest first, then smallest row), in slot set b:
-// one block barrier; every thread gets the row
-template <int NB>
-__device__ __forceinline__ int block_argmax(double v, bool valid, int r, ResShared<NB>& sh, int b) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = (blockDim.x + 31) >> 5;
-    unsigned hi = valid ? (unsigned)__double2hiint(v) : 0u;
-    unsigned lo = valid ? (unsigned)__double2loint(v) : 0u;
-    int id = valid ? r : 0x7fffffff;
-    warp_key_max(hi, lo, id);
-    if (lane == 0) {
-        sh.kh[b][warp] = hi;
-        sh.kl[b][warp] = lo;
-        sh.ki[b][warp] = id;
+    best = __ballot_sync(0xffffffffu, hi == mh);
+    if (best & (best - 1)) {
+        const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? lo : 0u);
+        const bool tie = hi == mh && lo == ml;
+        const int mi = __reduce_min_sync(0xffffffffu, tie ? id : 0x7fffffff);
+        best = __ballot_sync(0xffffffffu, tie && id == mi);
     }
-    __syncthreads();
-    hi = lane < nwarps ? sh.kh[b][lane] : 0u;
-    lo = lane < nwarps ? sh.kl[b][lane] : 0u;
-    id = lane < nwarps ? sh.ki[b][lane] : 0x7fffffff;
-    warp_key_max(hi, lo, id);
-    return id;
+    return (best >> (threadIdx.x & 31)) & 1u;
 }
 
-// Eliminates a panel of nbk columns (matrix columns k0..) whose current values are in row[][]:
-// RPT rows per thread (rows tid + i*blockDim.x), two block barriers per column (pivot candidates;
-// scaled pivot row and displaced row).  On return row[][] holds the panel's transform W and the
-// pivots are in ipiv.
+// this thread's candidate for column kk (its largest entry in rows no pivot has taken) reduced over the
+// warp into the column's slots
 template <int NB, int RPT>
-__device__ __forceinline__ void res_eliminate_regs(z (&row)[RPT][NB], int m, int k0, int nbk, int* ipiv, int* status,
-                                                   ResShared<NB>& sh) {
+__device__ __forceinline__ void res_candidate(const z (&row)[RPT][NB], int kk, int m, unsigned used, ResShared<NB>& sh) {
     const int tid = threadIdx.x, nt = blockDim.x;
+    double v = 0.0;
+    int vr = -1;
+#pragma unroll
+    for (int i = 0; i < RPT; ++i) {
+        const int r = tid + i * nt;
+        const double a = zabs1(row[i][kk]);
+        if (r < m && !((used >> i) & 1u) && (vr < 0 || a > v)) { v = a; vr = r; }
+    }
+    const unsigned hi = vr >= 0 ? (unsigned)__double2hiint(v) : 0u, lo = vr >= 0 ? (unsigned)__double2loint(v) : 0u;
+    const int id = vr >= 0 ? vr : 0x7fffffff;
+    unsigned best;
+    if (warp_key_best(hi, lo, id, best)) sh.cand[kk & 1][tid >> 5] = make_uint4(hi, lo, (unsigned)id, 0u);
+}
+
+// Eliminates a panel of nbk columns whose current values are in row[][]: RPT rows per thread (rows
+// tid + i*blockDim.x), two block barriers per column (pivot candidates; scaled pivot row).  Rows stay where
+// they are: a pivot's row is marked in `used` (bit i: row i of this thread).  On return row[][] holds the
+// panel's transform W and pv its pivot rows.  The chain of a column is its latency: of a column's update
+// only the next column is brought up to date before that one's pivot search; the rest runs beside the
+// pivot's reciprocal.
+template <int NB, int RPT>
+__device__ __forceinline__ void res_eliminate_regs(z (&row)[RPT][NB], int m, int nbk, unsigned& used, int (&pv)[NB], int* status,
+                                                   ResShared<NB>& sh) {
+    const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, nwarps = (nt + 31) >> 5;
     bool bad = false;
+    z f[RPT];                                     // the multipliers of the column before
+    unsigned upd = 0;                             // rows it updates: all but its own
+    res_candidate<NB, RPT>(row, 0, m, used, sh);
+#pragma unroll
+    for (int kk = 0; kk < NB; ++kk) pv[kk] = 0xFFF;
 #pragma unroll
     for (int kk = 0; kk < NB; ++kk) {
         if (kk >= nbk) break;
-        const int c = k0 + kk, b = kk & 1;
-        // this thread's candidate: its largest entry on or below row c, first on ties
-        double v = 0.0;
-        int vr = -1;
-#pragma unroll
-        for (int i = 0; i < RPT; ++i) {
-            const int r = tid + i * nt;
-            const double a = zabs1(row[i][kk]);
-            if (r < m && r >= c && (vr < 0 || a > v)) { v = a; vr = r; }
-        }
-        const int p = block_argmax<NB>(v, vr >= 0, vr, sh, b);
-#pragma unroll
-        for (int i = 0; i < RPT; ++i) {
-            const int r = tid + i * nt;
-            if (r == p) {
-                if (zis0(row[i][kk])) bad = true;
-                const z pinv = zrcp(row[i][kk]);
-#pragma unroll
-                for (int j = 0; j < NB; ++j) sh.prow[b][j] = (j == kk) ? pinv : zmul(row[i][j], pinv);
-                ipiv[c] = p;
-            }
-            if (r == c && p != c) {
-#pragma unroll
-                for (int j = 0; j < NB; ++j) sh.xb[b][j] = row[i][j];
-            }
-        }
+        const int b = kk & 1;
         __syncthreads();
+        const uint4 q = lane < nwarps ? sh.cand[b][lane] : make_uint4(0u, 0u, 0x7fffffffu, 0u);
+        unsigned best;
+        warp_key_best(q.x, q.y, (int)q.z, best);
+        const int p = __shfl_sync(0xffffffffu, (int)q.z, __ffs(best) - 1);
+        pv[kk] = p;
+        z pinv[RPT];
+#pragma unroll
+        for (int i = 0; i < RPT; ++i)
+            if (tid + i * nt == p) {
+                if (zis0(row[i][kk])) bad = true;
+                pinv[i] = gj_rcp(row[i][kk]);
+            }
+        if (kk > 0) {
+#pragma unroll
+            for (int i = 0; i < RPT; ++i)
+                if ((upd >> i) & 1u) {
+#pragma unroll
+                    for (int j = 0; j < NB; ++j)
+                        if (j != kk - 1 && j != kk) zfms(row[i][j], f[i], sh.prow[b ^ 1][j]);
+                    row[i][kk - 1] = zneg(gj_mul(f[i], sh.prow[b ^ 1][kk - 1]));
+                }
+        }
+        upd = (1u << RPT) - 1u;
+#pragma unroll
+        for (int i = 0; i < RPT; ++i)
+            if (tid + i * nt == p) {
+#pragma unroll
+                for (int j = 0; j < NB; ++j) {
+                    row[i][j] = (j == kk) ? pinv[i] : gj_mul(row[i][j], pinv[i]);
+                    sh.prow[b][j] = row[i][j];
+                }
+                used |= 1u << i;
+                upd &= ~(1u << i);
+            }
+        __syncthreads();
+        const bool more = kk + 1 < NB && kk + 1 < nbk;
 #pragma unroll
         for (int i = 0; i < RPT; ++i) {
-            const int r = tid + i * nt;
-            if (r == c) {
+            f[i] = row[i][kk];
+            if (((upd >> i) & 1u) && more) zfms(row[i][(kk + 1) % NB], f[i], sh.prow[b][(kk + 1) % NB]);
+        }
+        if (more) {
+            res_candidate<NB, RPT>(row, (kk + 1) % NB, m, used, sh);
+        } else {
 #pragma unroll
-                for (int j = 0; j < NB; ++j) row[i][j] = sh.prow[b][j];
-            } else if (r < m) {
-                if (r == p) {
+            for (int i = 0; i < RPT; ++i)
+                if ((upd >> i) & 1u) {
 #pragma unroll
-                    for (int j = 0; j < NB; ++j) row[i][j] = sh.xb[b][j];
+                    for (int j = 0; j < NB; ++j)
+                        if (j != kk) zfms(row[i][j], f[i], sh.prow[b][j]);
+                    row[i][kk] = zneg(gj_mul(f[i], sh.prow[b][kk]));
                 }
-                const z f = row[i][kk];
-#pragma unroll
-                for (int j = 0; j < NB; ++j)
-                    if (j != kk) zfms(row[i][j], f, sh.prow[b][j]);
-                row[i][kk] = zneg(zmul(f, sh.prow[b][kk]));
-            }
         }
     }
-    if (bad) atomicOr(status, 1);
+    if (bad) atomicOr(status, RB_STATUS_ZERO_PIVOT);
 }
 
-// Stores an eliminated panel: W to the local columns [q0, q0+nbk) and to Wg (ld wld), then a
-// block barrier.
+// Stores an eliminated panel, W to the local columns at c and to Wg (ld wld), then publishes it with its
+// pivots: the releases order the stores of the whole CTA, ahead of them by the block barrier.
 template <int NB, int RPT>
-__device__ __forceinline__ void res_store_panel(const z (&row)[RPT][NB], z* cols, int m, int q0, int nbk, z* Wg,
-                                                long long wld) {
+__device__ __forceinline__ void res_publish(const z (&row)[RPT][NB], const int (&pv)[NB], z* c, int m, int nbk, z* Wg, long long wld,
+                                            unsigned long long* words, int p, ResShared<NB>& sh) {
     const int tid = threadIdx.x, nt = blockDim.x;
 #pragma unroll
     for (int i = 0; i < RPT; ++i) {
@@ -397,111 +440,64 @@ __device__ __forceinline__ void res_store_panel(const z (&row)[RPT][NB], z* cols
 #pragma unroll
         for (int kk = 0; kk < NB; ++kk) {
             if (kk >= nbk) break;
-            cols[r + (q0 + kk) * m] = row[i][kk];
             Wg[r + (long long)kk * wld] = row[i][kk];
+            c[r + kk * m] = row[i][kk];
         }
     }
+    if (tid == 0) {
+#pragma unroll
+        for (int kk = 0; kk < NB; ++kk) sh.spv[p & 1][kk] = pv[kk];
+    }
     __syncthreads();
+    if (tid < 2) {
+        unsigned long long w = GJ_READY;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) w |= (unsigned long long)(tid == 0 ? pv[i] : pv[4 + i]) << (12 * i);
+        st_release_gpu(words + 2 * p + tid, w);
+    }
 }
 
-// Eliminates the panel held at local columns [q0, q0+nbk) (matrix columns k0..) and stores it.
+// The values that a step (nbk pivots, W at W with ld wld, read through L2 when w_global) gives the rows
+// of this thread in the nq <= NB columns at c: A + W Z outside the pivots' rows, W_P Z on them (bit i of
+// `mine`), Z = the pivots' rows.  The columns in shared memory are read only; w holds W already when `held`.
 template <int NB, int RPT>
-__device__ __noinline__ void res_eliminate(z* cols, int m, int q0, int k0, int nbk, z* Wg, long long wld, int* ipiv,
-                                           int* status, ResShared<NB>& sh) {
+__device__ __forceinline__ void res_updated(z (&row)[RPT][NB], const z (&w)[RPT][NB], bool held, unsigned mine, const z* c, int nq,
+                                            int m, int nbk, const z* W, long long wld, bool w_global, const int* spv) {
     const int tid = threadIdx.x, nt = blockDim.x;
-    z row[RPT][NB];
 #pragma unroll
     for (int i = 0; i < RPT; ++i) {
         const int r = tid + i * nt;
+        const bool keep = r < m && !((mine >> i) & 1u);
 #pragma unroll
-        for (int kk = 0; kk < NB; ++kk) row[i][kk] = (r < m && kk < nbk) ? cols[r + (q0 + kk) * m] : zmk(0.0, 0.0);
+        for (int q = 0; q < NB; ++q) row[i][q] = keep && q < nq ? c[r + q * m] : zmk(0.0, 0.0);
     }
-    res_eliminate_regs<NB, RPT>(row, m, k0, nbk, ipiv, status, sh);
-    res_store_panel<NB, RPT>(row, cols, m, q0, nbk, Wg, wld);
+#pragma unroll
+    for (int kk = 0; kk < NB; ++kk) {
+        if (kk >= nbk) break;
+        z wk[RPT];
+#pragma unroll
+        for (int i = 0; i < RPT; ++i) {
+            const int r = tid + i * nt;
+            if (held) wk[i] = w[i][kk];
+            else wk[i] = r < m ? (w_global ? __ldcg(W + r + kk * wld) : W[r + kk * wld]) : zmk(0.0, 0.0);
+        }
+        const z* zk = c + spv[kk];
+#pragma unroll
+        for (int q = 0; q < NB; ++q) {
+            const z zv = q < nq ? zk[q * m] : zmk(0.0, 0.0);
+#pragma unroll
+            for (int i = 0; i < RPT; ++i) zfma(row[i][q], wk[i], zv);
+        }
+    }
 }
 
-// Applies step (panel at matrix columns k0.., nbk wide, pivots at piv (shared memory), W at W with
-// ld wld, read through L2 when w_global) to the local columns [qa, qb) except [xa, xb).  The panel's row
-// exchanges move only the panel rows and the pivot rows below the panel; their exchanged values
-// (row a takes stored row src(a), src = the transpositions traced backwards) are gathered in
-// parallel into zs (2*NB slots per column: slot t < NB panel row k0+t, slot NB+t pivot row t
-// unless it repeats), the displaced pivot rows are written back, and then every thread updates
-// its rows: A + W Z outside the panel rows, W_P Z on them, Z = the gathered panel rows.  Same
-// operations, in the same order, as exchanging row by row and then updating.
-template <int NB, int RPT>
-__device__ __noinline__ void res_apply(z* cols, z* zs, int m, int k0, int nbk, const z* W, long long wld,
-                                       bool w_global, const int* piv, int qa, int qb, int xa, int xb) {
-    if (qb <= qa) return;
-    const int tid = threadIdx.x, nt = blockDim.x;
-    const int nq = qb - qa;
-    {
-        int pv[NB];
-#pragma unroll
-        for (int kk = 0; kk < NB; ++kk) pv[kk] = kk < nbk ? piv[kk] : -1;
-        for (int e = tid; e < 2 * NB * nq; e += nt) {
-            const int t = e % (2 * NB), q = qa + e / (2 * NB);
-            if (q >= xa && q < xb) continue;
-            int a = -1;
-            if (t < nbk) {
-                a = k0 + t;
-            } else if (t >= NB && t - NB < nbk) {
-                int pt = -1;
-#pragma unroll
-                for (int u = 0; u < NB; ++u)
-                    if (u == t - NB) pt = pv[u];
-                bool dup = pt < k0 + nbk;
-#pragma unroll
-                for (int u = 0; u < NB; ++u)
-                    if (u < t - NB && pv[u] == pt) dup = true;
-                if (!dup) a = pt;
-            }
-            if (a < 0) continue;
-            int jr = a;
-#pragma unroll
-            for (int kk = NB - 1; kk >= 0; --kk) {
-                const int c = k0 + kk;
-                if (kk < nbk) jr = (jr == c) ? pv[kk] : (jr == pv[kk] ? c : jr);
-            }
-            zs[t + (q - qa) * 2 * NB] = cols[jr + q * m];
-        }
-        __syncthreads();
-        for (int e = tid; e < NB * nq; e += nt) {
-            const int t = e % NB, q = qa + e / NB;
-            if ((q >= xa && q < xb) || t >= nbk) continue;
-            int pt = -1;
-#pragma unroll
-            for (int u = 0; u < NB; ++u)
-                if (u == t) pt = pv[u];
-            bool dup = pt < k0 + nbk;
-#pragma unroll
-            for (int u = 0; u < NB; ++u)
-                if (u < t && pv[u] == pt) dup = true;
-            if (!dup) cols[pt + q * m] = zs[NB + t + (q - qa) * 2 * NB];
-        }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int i = 0; i < RPT; ++i) {
-        const int r = tid + i * nt;
-        if (r >= m) continue;
-        z w[NB];
-#pragma unroll
-        for (int kk = 0; kk < NB; ++kk)
-            w[kk] = kk < nbk ? (w_global ? __ldcg(W + r + kk * wld) : W[r + kk * wld]) : zmk(0.0, 0.0);
-        const bool in_panel = r >= k0 && r < k0 + nbk;
-        for (int q = qa; q < qb; ++q) {
-            if (q >= xa && q < xb) continue;
-            z v = in_panel ? zmk(0.0, 0.0) : cols[r + q * m];
-            const z* zq = zs + (q - qa) * 2 * NB;
-#pragma unroll
-            for (int kk = 0; kk < NB; ++kk)
-                if (kk < nbk) zfma(v, w[kk], zq[kk]);
-            cols[r + q * m] = v;
-        }
-    }
-    __syncthreads();
-}
-
+// A step takes the CTA that owns the next panel through wait, W, update and elimination of that panel and
+// the hand-over; that chain, latencies and one SM's FP64 rate, is the time.  A column waits for two
+// barriers, two warp reductions and a reciprocal; the update goes from shared memory through registers
+// into the elimination.
+// Against exchanging rows in registers and shared memory and a gather, an update and an elimination in
+// separate passes, with the columns' exchanges undone by a kernel of their own: one matrix of 128 135 to 112
+// us, 256 297 to 248, 512 786 to 656, 1024 2490 to 2113.
 template <int NB, int MAXT, int RPT>
 __global__ void __launch_bounds__(MAXT, MAXT <= 256 ? 512 / MAXT : 1) gj_resident_kernel(
     const GJDesc* __restrict__ descs, int m, int npanels, int ppc, int P, int* status) {
@@ -512,59 +508,104 @@ __global__ void __launch_bounds__(MAXT, MAXT <= 256 ? 512 / MAXT : 1) gj_residen
     const int pa = j * ppc, pb = min(npanels, pa + ppc);
     const int c0 = pa * NB, cw = min(m, pb * NB) - c0;
     z* cols = sm;                                   // m x cw, column-major (ld m)
-    z* zs = sm + (size_t)m * ppc * NB;              // 2NB x cw: exchanged panel and pivot rows
-    int* pub = reinterpret_cast<int*>(g.Zb);        // panels published
-    int* done = pub + 1;                            // CTAs past their last step
+    int* perm = reinterpret_cast<int*>(sm + (size_t)m * ppc * NB);    // the pivot row of every column
+    unsigned long long* words = reinterpret_cast<unsigned long long*>(g.Zb);      // two per panel
+    int* done = reinterpret_cast<int*>(words + 2 * npanels);          // CTAs past their last step
     const int tid = threadIdx.x, nt = blockDim.x;
+    if (tid == 0) sh.ok[0] = sh.ok[1] = sh.done_ok = 1;
     for (int e = tid; e < m * cw; e += nt) {
         const int r = e % m, q = e / m;
         cols[r + q * m] = __ldcg(g.A + r + (long long)(c0 + q) * g.ld);
     }
     __syncthreads();
-    auto publish = [&](int p) {          // res_eliminate ended with a block barrier
-        if (tid == 0) {
-            __threadfence();
-            st_release_gpu(pub, p + 1);
-        }
-    };
+    z row[RPT][NB];
+    int pv[NB];
+    unsigned used = 0;                              // rows of this thread that a pivot has taken
     if (pa == 0) {
-        res_eliminate<NB, RPT>(cols, m, 0, 0, min(NB, m), g.A, g.ld, g.ipiv, status, sh);
-        publish(0);
+        const int nb0 = min(NB, m);
+#pragma unroll
+        for (int i = 0; i < RPT; ++i) {
+            const int r = tid + i * nt;
+#pragma unroll
+            for (int q = 0; q < NB; ++q) row[i][q] = r < m && q < nb0 ? cols[r + q * m] : zmk(0.0, 0.0);
+        }
+        res_eliminate_regs<NB, RPT>(row, m, nb0, used, pv, status, sh);
+        res_publish<NB, RPT>(row, pv, cols, m, nb0, g.A, g.ld, words, 0, sh);
     }
     for (int p = 0; p < npanels; ++p) {
         const int k0 = p * NB, nbk = min(NB, m - k0);
         const bool own = p >= pa && p < pb;
-        if (!own && !cta_wait_geq(pub, p + 1, status, &sh.ok)) return;
-        // the step's pivots, read once by the CTA: read by every thread, the same 32 bytes made an
-        // L2 hot spot of thousands of requests per step that cost the chain ~2.5 us a panel
-        if (tid < NB) sh.spv[tid] = tid < nbk ? __ldcg(g.ipiv + k0 + tid) : -1;
-        __syncthreads();
+        // the step's pivots are here, and every column that the step before wrote
+        if (own) __syncthreads();
+        else if (!res_wait_step<NB>(words, p, status, sh)) return;
+        const int* spv = sh.spv[p & 1];
         const z* W = own ? cols + (size_t)(k0 - c0) * m : g.A + (long long)k0 * g.ld;
         const long long wld = own ? m : g.ld;
-        const int* piv = sh.spv;
-        const int xa = own ? k0 - c0 : 0, xb = own ? k0 - c0 + nbk : 0;
+        constexpr bool HELD = RPT == 1;             // with one row a thread there are registers for W
+        z w[RPT][NB];
+        if (HELD) {
+#pragma unroll
+            for (int i = 0; i < RPT; ++i)
+#pragma unroll
+                for (int kk = 0; kk < NB; ++kk) {
+                    const int r = tid + i * nt;
+                    w[i][kk] = r < m && kk < nbk ? (own ? W[r + kk * wld] : __ldcg(W + r + kk * wld)) : zmk(0.0, 0.0);
+                }
+        }
+        unsigned mine = 0;                          // this step's pivots among this thread's rows
+#pragma unroll
+        for (int i = 0; i < RPT; ++i)
+#pragma unroll
+            for (int kk = 0; kk < NB; ++kk)
+                if (kk < nbk && spv[kk] == tid + i * nt) mine |= 1u << i;
+        used |= mine;
+        if (tid < nbk) perm[k0 + tid] = spv[tid];
         const int nx = p + 1;
-        if (nx < npanels && nx >= pa && nx < pb) {
+        const bool next = nx < npanels && nx >= pa && nx < pb;
+        if (next) {
             const int qn = nx * NB - c0, nbn = min(NB, m - nx * NB);
-            res_apply<NB, RPT>(cols, zs, m, k0, nbk, W, wld, !own, piv, qn, qn + nbn, xa, xb);
-            res_eliminate<NB, RPT>(cols, m, qn, nx * NB, nbn, g.A + (long long)nx * NB * g.ld, g.ld, g.ipiv, status,
-                                   sh);
-            publish(nx);
-            res_apply<NB, RPT>(cols, zs, m, k0, nbk, W, wld, !own, piv, 0, qn, xa, xb);
-            res_apply<NB, RPT>(cols, zs, m, k0, nbk, W, wld, !own, piv, qn + nbn, cw, xa, xb);
-        } else {
-            res_apply<NB, RPT>(cols, zs, m, k0, nbk, W, wld, !own, piv, 0, cw, xa, xb);
+            res_updated<NB, RPT>(row, w, HELD, mine, cols + (size_t)qn * m, nbn, m, nbk, W, wld, !own, spv);
+            // its barriers end every read of the panel's columns before they are stored
+            res_eliminate_regs<NB, RPT>(row, m, nbn, used, pv, status, sh);
+            res_publish<NB, RPT>(row, pv, cols + (size_t)qn * m, m, nbn, g.A + (long long)nx * NB * g.ld, g.ld, words, nx, sh);
+        }
+        for (int lp = pa; lp < pb; ++lp) {
+            if (lp == p || (next && lp == nx)) continue;
+            const int nq = min(NB, m - lp * NB);
+            z* c = cols + (size_t)(lp - pa) * NB * m;
+            res_updated<NB, RPT>(row, w, HELD, mine, c, nq, m, nbk, W, wld, !own, spv);
+            __syncthreads();
+#pragma unroll
+            for (int i = 0; i < RPT; ++i) {
+                const int r = tid + i * nt;
+#pragma unroll
+                for (int q = 0; q < NB; ++q)
+                    if (r < m && q < nq) c[r + q * m] = row[i][q];
+            }
         }
     }
     // no CTA of this matrix reads a W slot any more once all have arrived here
+    __syncthreads();
     if (tid == 0) {
         __threadfence();
         atomicAdd(done, 1);
+        const unsigned long long t0 = global_ns();
+        while (ld_acquire_gpu(done) < P) {
+            __nanosleep(40);
+            if (global_ns() - t0 > GJ_WAIT_NS) {
+                sh.done_ok = 0;
+                atomicOr(status, RB_STATUS_GJ_TIMEOUT);
+                break;
+            }
+        }
     }
-    if (!cta_wait_geq(done, P, status, &sh.ok)) return;
+    __syncthreads();
+    if (!sh.done_ok) return;
+    // column q was eliminated by row perm[q]: the inverse has its rows in the columns' order and its
+    // columns in the pivots'
     for (int e = tid; e < m * cw; e += nt) {
         const int r = e % m, q = e / m;
-        g.A[r + (long long)(c0 + q) * g.ld] = cols[r + q * m];
+        g.A[r + (long long)perm[c0 + q] * g.ld] = cols[perm[r] + q * m];
     }
 }
 
@@ -608,8 +649,8 @@ static cudaError_t gj_blocked(const GJDesc* d, int count, int m, int* st, cudaSt
     return cudaGetLastError();
 }
 
-// Resident path: the smallest number of panels per CTA whose grid is co-resident; false when
-// even one CTA per panel group cannot hold the batch (the caller then runs the blocked path).
+// Resident path: the fewest launches, then the fewest panels per CTA, whose grids are co-resident; false
+// when not even one matrix is (the caller then runs the blocked path).
 template <int NB, int MAXT, int RPT>
 static cudaError_t gj_resident(const GJDesc* d, int count, int m, void* flags, int* st, cudaStream_t s, bool* done) {
     *done = false;
@@ -626,37 +667,43 @@ static cudaError_t gj_resident(const GJDesc* d, int count, int m, void* flags, i
     static DeviceAttrCache attr;
     e = ensure_smem_attr(gj_resident_kernel<NB, MAXT, RPT>, SMEM_MAX - sizeof(ResShared<NB>), attr);
     if (e != cudaSuccess) return e;
-    // fewest panels per CTA: a CTA that owns more panels updates its others before it can
+    // A batch that is not co-resident as a whole goes in as few equal launches as make it so: 512 matrices
+    // of 160 2604 to 1923 us, 8 of 512 2086 to 1429 against the blocked path, whose two launches per panel pass over
+    // every matrix in memory.  (65 to 512 points: faster at every count up to 4096, by 6 to 60%.  Above 512 a launch
+    // holds one or two matrices, and four of 600 take 2438 against 2195 us: two launches for up to three only.)
+    // Fewest panels per CTA: a CTA that owns more panels updates its others before it can
     // eliminate its next one, which lengthens the chain (1024^2, L=12: 25.5 ms factor with one
     // panel per CTA, 26.9 with at least two, 29.3 with at least six)
-    for (int ppc = 1; ppc <= npanels; ++ppc) {
-        const int P = (npanels + ppc - 1) / ppc;
-        const size_t sh = ((size_t)m + 2 * NB) * ppc * NB * sizeof(z);
-        if (sh + sizeof(ResShared<NB>) > (size_t)SMEM_MAX) break;
-        int per_sm = 0;
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gj_resident_kernel<NB, MAXT, RPT>, threads, sh);
-        if (e != cudaSuccess) return e;
-        if ((long long)count * P > (long long)per_sm * nsm) continue;
-        if ((e = cudaMemsetAsync(flags, 0, (size_t)count * sizeof(z), s)) != cudaSuccess) return e;
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3((unsigned)(count * P));
-        cfg.blockDim = dim3((unsigned)threads);
-        cfg.dynamicSmemBytes = sh;
-        cfg.stream = s;
-        cudaLaunchAttribute la[1];
-        la[0].id = cudaLaunchAttributeCooperative;
-        la[0].val.cooperative = 1;
-        cfg.attrs = la;
-        cfg.numAttrs = 1;
-        e = cudaLaunchKernelEx(&cfg, gj_resident_kernel<NB, MAXT, RPT>, d, m, npanels, ppc, P, st);
-        if (e != cudaSuccess) return e;
-        note_launch();
-        gj_unscramble_kernel<<<dim3((m + 127) / 128, count), 128, 0, s>>>(d, m);
-        note_launch();
-        *done = true;
-        return cudaGetLastError();
+    for (int parts = 1, chunk = count;; chunk = (count + ++parts - 1) / parts) {
+        for (int ppc = 1; ppc <= npanels; ++ppc) {
+            const int P = (npanels + ppc - 1) / ppc;
+            const size_t sh = (size_t)m * ppc * NB * sizeof(z) + (size_t)m * sizeof(int);
+            if (sh + sizeof(ResShared<NB>) > (size_t)SMEM_MAX) break;
+            int per_sm = 0;
+            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gj_resident_kernel<NB, MAXT, RPT>, threads, sh);
+            if (e != cudaSuccess) return e;
+            if ((long long)chunk * P > (long long)per_sm * nsm) continue;
+            if ((e = cudaMemsetAsync(flags, 0, (size_t)(count * gj_workspace_elems(m)) * sizeof(z), s)) != cudaSuccess) return e;
+            cudaLaunchConfig_t cfg = {};
+            cfg.blockDim = dim3((unsigned)threads);
+            cfg.dynamicSmemBytes = sh;
+            cfg.stream = s;
+            cudaLaunchAttribute la[1];
+            la[0].id = cudaLaunchAttributeCooperative;
+            la[0].val.cooperative = 1;
+            cfg.attrs = la;
+            cfg.numAttrs = 1;
+            for (int off = 0; off < count; off += chunk) {
+                cfg.gridDim = dim3((unsigned)(std::min(chunk, count - off) * P));
+                e = cudaLaunchKernelEx(&cfg, gj_resident_kernel<NB, MAXT, RPT>, d + off, m, npanels, ppc, P, st);
+                if (e != cudaSuccess) return e;
+                note_launch();
+            }
+            *done = true;
+            return cudaGetLastError();
+        }
+        if (chunk == 1 || (m > 512 && count > 3)) return cudaSuccess;
     }
-    return cudaSuccess;
 }
 
 // RB_GJ_RESIDENT=0 selects the blocked path (read at every launch, so that a process can compare)

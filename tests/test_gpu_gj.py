@@ -51,3 +51,14 @@ def test_gj_leading_dimension_and_repeat():
     X, ms = _invert(A, ld=320, reps=2)       # inverting twice returns the input
     assert ms > 0.0
     assert np.abs(X - A).max() / np.abs(A).max() < 1e-12
+
+
+@pytest.mark.parametrize("m,cnt", [(65, 700), (160, 76), (257, 31), (512, 5)])
+def test_gj_batches_that_take_several_launches(m, cnt):
+    """Batches that are not co-resident as a whole (uneven last launch included)."""
+    A = _matrices(m, cnt, 3 * m + cnt, True)
+    X, _ = _invert(A)
+    for i in (0, cnt // 2, cnt - 1):
+        ref = np.linalg.inv(A[i])
+        assert np.abs(X[i] - ref).max() / np.abs(ref).max() < 1e-12, i
+    assert np.abs(X @ A - np.eye(m)).max() < 1e-9
