@@ -128,6 +128,8 @@ struct GemmBatch {
     // every problem's k runs contiguously through both operands (gemm_k_contiguous), so operand
     // copies may advance by a fixed stride per k-tile
     bool kcontig = false;
+    // ... and through A at least, whatever B's rows are
+    bool acontig = false;
     // split-K of the same batch on the tcgen05 kernel (128-row tiles): t5_ksplit ranges of
     // t5_kchunk, raw sums in `work` (t5_pstride elements per range and problem, ld max_m)
     int t5_ksplit = 1;
@@ -150,8 +152,9 @@ struct GemmBatch {
 
 // A(i, k) sits at A.p[row(i) + k * A.ld] and B(k, j) at B.p[k + col(j) * B.ld] for every k < K:
 // no map on A's columns or B's rows, and no skipped band that starts below K
+__host__ __device__ inline bool gemm_a_contiguous(const GemmDesc& g) { return !g.A.cmap && (g.A.cl == 0 || g.A.cs >= g.k); }
 __host__ __device__ inline bool gemm_k_contiguous(const GemmDesc& g) {
-    return !g.A.cmap && (g.A.cl == 0 || g.A.cs >= g.k) && !g.B.rmap && (g.B.rl == 0 || g.B.rs >= g.k);
+    return gemm_a_contiguous(g) && !g.B.rmap && (g.B.rl == 0 || g.B.rs >= g.k);
 }
 
 }  // namespace rb

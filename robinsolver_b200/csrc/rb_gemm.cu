@@ -72,7 +72,16 @@ __global__ void __launch_bounds__(256) zgemm_reduce_kernel(const GemmDesc* __res
     g.D.p[vrow(g.D, i) + (long long)vcol(g.D, j) * g.D.ld] = v;
 }
 
-template <int BM, int BN, int WM, int WN, int MINB>
+// the tile of a kernel: the general one, or one for batches whose k runs contiguously through both
+// operands, or through A
+enum DmmaKind { DMMA_GENERAL = 0, DMMA_KCONTIG = 1, DMMA_ACONTIG = 2 };
+template <int BM, int BN, int WM, int WN, int ST, int KIND>
+__device__ __forceinline__ void dmma_tile(const GemmDesc& sd, int tile, z* smem) {
+    if constexpr (KIND == DMMA_GENERAL) zgemm_tile_dmma<BM, BN, WM, WN, ST>(sd, tile, smem);
+    else zgemm_tile_dmma_kc<BM, BN, WM, WN, 8, ST, KIND == DMMA_ACONTIG>(sd, tile, smem);
+}
+
+template <int BM, int BN, int WM, int WN, int MINB, int ST, int KIND>
 __global__ void __launch_bounds__(32 * WM * WN, MINB) zgemm_dmma_kernel(const GemmDesc* __restrict__ descs) {
     extern __shared__ z dmma_smem[];
     __shared__ GemmDesc sd;
@@ -84,16 +93,16 @@ __global__ void __launch_bounds__(32 * WM * WN, MINB) zgemm_dmma_kernel(const Ge
     pdl_launch();
     pdl_wait();
     __syncthreads();
-    zgemm_tile_dmma<BM, BN, WM, WN>(sd, blockIdx.x, dmma_smem);
+    dmma_tile<BM, BN, WM, WN, ST, KIND>(sd, blockIdx.x, dmma_smem);
 }
 
 // MINB CTAs per SM: the carveout is set to the largest shared-memory share so that they fit
-template <int BM, int BN, int WM, int WN, int MINB>
+template <int BM, int BN, int WM, int WN, int MINB, int ST = 4, int KIND = DMMA_GENERAL>
 static cudaError_t launch_dmma(const GemmBatch& b, cudaStream_t s, bool pdl = false) {
-    using Cfg = DmmaCfg<BM, BN, WM, WN>;
+    using Cfg = DmmaCfg<BM, BN, WM, WN, ST>;
     static DeviceAttrCache attr;
     {
-        cudaError_t e = ensure_smem_attr(zgemm_dmma_kernel<BM, BN, WM, WN, MINB>, Cfg::SMEM_BYTES, attr, true);
+        cudaError_t e = ensure_smem_attr(zgemm_dmma_kernel<BM, BN, WM, WN, MINB, ST, KIND>, Cfg::SMEM_BYTES, attr, true);
         if (e != cudaSuccess) return e;
     }
     const int tiles = ((b.max_m + BM - 1) / BM) * ((b.max_n + BN - 1) / BN);
@@ -102,7 +111,7 @@ static cudaError_t launch_dmma(const GemmBatch& b, cudaStream_t s, bool pdl = fa
         dim3 grid(tiles, cnt);
         note_launch();
         const GemmDesc* d = b.d_desc + off;
-        cudaError_t e = launch_kernel(zgemm_dmma_kernel<BM, BN, WM, WN, MINB>, grid, Cfg::NT, Cfg::SMEM_BYTES, s, pdl, d);
+        cudaError_t e = launch_kernel(zgemm_dmma_kernel<BM, BN, WM, WN, MINB, ST, KIND>, grid, Cfg::NT, Cfg::SMEM_BYTES, s, pdl, d);
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
@@ -140,7 +149,7 @@ __device__ __forceinline__ ZView view_from_row(ZView v, int kb) {
 // raw product (3M-combined, alpha = 1, no C) goes to the batch's workspace, laid out as the DFMA
 // split pass writes it, for zgemm_reduce_kernel.  Every output element still sums its k range in
 // MMA k-steps of 4 in order, so the result does not depend on n or on the tile shape.
-template <int BM, int BN, int WM, int WN, int MINB>
+template <int BM, int BN, int WM, int WN, int MINB, int ST, int KIND>
 __global__ void __launch_bounds__(32 * WM * WN, MINB)
 zgemm_dmma_split_kernel(const GemmDesc* __restrict__ descs, int kchunk, z* work, long long pstride, int ldp, int ksplit) {
     extern __shared__ z dmma_smem[];
@@ -163,13 +172,13 @@ zgemm_dmma_split_kernel(const GemmDesc* __restrict__ descs, int kchunk, z* work,
         sd.D = zout(work + ((long long)blockIdx.y * ksplit + blockIdx.z) * pstride, ldp);
     }
     __syncthreads();
-    zgemm_tile_dmma<BM, BN, WM, WN>(sd, blockIdx.x, dmma_smem);
+    dmma_tile<BM, BN, WM, WN, ST, KIND>(sd, blockIdx.x, dmma_smem);
 }
 
-template <int BM, int BN, int WM, int WN, int MINB>
+template <int BM, int BN, int WM, int WN, int MINB, int ST = 4, int KIND = DMMA_GENERAL>
 static cudaError_t launch_dmma_split(const GemmBatch& b, cudaStream_t s, bool pdl) {
-    using Cfg = DmmaCfg<BM, BN, WM, WN>;
-    auto kern = zgemm_dmma_split_kernel<BM, BN, WM, WN, MINB>;
+    using Cfg = DmmaCfg<BM, BN, WM, WN, ST>;
+    auto kern = zgemm_dmma_split_kernel<BM, BN, WM, WN, MINB, ST, KIND>;
     static DeviceAttrCache attr;
     {
         cudaError_t e = ensure_smem_attr(kern, Cfg::SMEM_BYTES, attr, true);
@@ -284,20 +293,35 @@ static cudaError_t launch_stream(const GemmBatch& b, int ks, cudaStream_t s, boo
     return cudaSuccess;
 }
 
+template <int BM, int BN, int WM, int WN, int MINB, int ST, int KIND>
+static cudaError_t launch_solve_tile(const GemmBatch& b, cudaStream_t s, bool pdl) {
+    return b.ksplit > 1 ? launch_dmma_split<BM, BN, WM, WN, MINB, ST, KIND>(b, s, pdl)
+                        : launch_dmma<BM, BN, WM, WN, MINB, ST, KIND>(b, s, pdl);
+}
+template <int BM, int BN, int WM, int WN, int MINB, int ST>
+static cudaError_t launch_solve_kind(const GemmBatch& b, cudaStream_t s, bool pdl) {
+    if (b.kcontig) return launch_solve_tile<BM, BN, WM, WN, MINB, ST, DMMA_KCONTIG>(b, s, pdl);
+    if (b.acontig) return launch_solve_tile<BM, BN, WM, WN, MINB, ST, DMMA_ACONTIG>(b, s, pdl);
+    return launch_solve_tile<BM, BN, WM, WN, MINB, ST, DMMA_GENERAL>(b, s, pdl);
+}
 // The solve's tensor-core kernels: one order of summation, so the kernel may follow the number
 // of right-hand sides.  Up to 8: rb_gemm_stream.cuh (512^2, one: 1065 -> 795 us a solve); up to 16:
 // 32x16 tiles, whose second half would be idle at 32 (512^2, 16: the leaves' product 131 -> 88 us,
-// the solve's GEMMs 1.15 -> 0.97 ms).
+// the solve's GEMMs 1.15 -> 0.97 ms).  Above, problems of up to 16 rows take 16x32 tiles (16 x 32 x 96,
+// 4096 of them: 112 -> 88 us) and the rest 32x32.  What bounds them is the latency of the operands,
+// read once: five stages at five CTAs per SM against four at six, and copies that advance by strides
+// wherever A's k is contiguous, take 128 x 32 x 512 in 128 problems from 86 to 78 us, 64 x 32 x 256 in 512 from
+// 84 to 72, 1024^2 with 32 right-hand sides from 4.03 to 3.72 ms a solve, 768^2 with 64 from 4.38 to 4.25
+// (64-column tiles: 4.49 and more).
 static cudaError_t launch_solve_gemm(const GemmBatch& b, cudaStream_t s, bool pdl) {
-    const bool split = b.ksplit > 1;
     if (b.max_n <= 8 && b.ksplit <= STREAM_WARPS) {
         // two row tiles per warp once one per warp gives each scheduler more than four warps
         const long long warps = (long long)b.count * ((b.max_m + 7) / 8) * b.ksplit;
         return warps > 148 * 16 ? launch_stream<2>(b, b.ksplit, s, pdl) : launch_stream<1>(b, b.ksplit, s, pdl);
     }
-    if (b.max_n <= 16)
-        return split ? launch_dmma_split<32, 16, 2, 2, 8>(b, s, pdl) : launch_dmma<32, 16, 2, 2, 8>(b, s, pdl);
-    return split ? launch_dmma_split<32, 32, 2, 2, 6>(b, s, pdl) : launch_dmma<32, 32, 2, 2, 6>(b, s, pdl);
+    if (b.max_n <= 16) return launch_solve_kind<32, 16, 2, 2, 6, 6>(b, s, pdl);
+    if (b.max_m <= 16) return launch_solve_kind<16, 32, 1, 4, 8, 4>(b, s, pdl);
+    return launch_solve_kind<32, 32, 2, 2, 5, 5>(b, s, pdl);
 }
 
 // the kernel shape a batch runs on

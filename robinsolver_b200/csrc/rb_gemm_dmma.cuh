@@ -128,11 +128,11 @@ __device__ __forceinline__ void dmma_k4(const z* __restrict__ As, const z* __res
         for (int j = 0; j < TNW; ++j) dmma884(p3[i][j][0], p3[i][j][1], fas[i], fbs[j]);
 }
 
-template <int BM, int BN, int WM, int WN>
+template <int BM, int BN, int WM, int WN, int ST = 4>
 struct DmmaCfg {
     static constexpr int NT = 32 * WM * WN;     // threads
     static constexpr int BK = 8;                // complex k per stage (2 MMA k-steps)
-    static constexpr int STAGES = 4;
+    static constexpr int STAGES = ST;
     static constexpr int LDA = BM + 2;          // complex elements per k-row of an A stage
     static constexpr int LDB = BN + 2;
     static constexpr int TMW = BM / WM / 8;     // MMA tiles per warp along M
@@ -141,9 +141,9 @@ struct DmmaCfg {
     static constexpr size_t SMEM_BYTES = (size_t)STAGES * STAGE_Z * sizeof(z);
 };
 
-template <int BM, int BN, int WM, int WN>
+template <int BM, int BN, int WM, int WN, int ST = 4>
 __device__ __forceinline__ void zgemm_tile_dmma(const GemmDesc& sd, int tile, z* smem) {
-    using Cfg = DmmaCfg<BM, BN, WM, WN>;
+    using Cfg = DmmaCfg<BM, BN, WM, WN, ST>;
     constexpr int NT = Cfg::NT, BK = Cfg::BK, LDA = Cfg::LDA, LDB = Cfg::LDB, STAGES = Cfg::STAGES;
     constexpr int TMW = Cfg::TMW, TNW = Cfg::TNW;
     constexpr int A_PER = BM * BK / NT;
@@ -239,7 +239,7 @@ __device__ __forceinline__ void zgemm_tile_dmma(const GemmDesc& sd, int tile, z*
 // halves the instructions issued per MMA against the general tile, whose per-element map and
 // band look-ups dominate its issue slots; with 32x32 warp tiles (4 warps, 96 accumulators a
 // thread, two CTAs per SM) the MMA pipe stays busy 87% of the time on the large merges, where
-// the general tile reaches 74%.
+// the general tile reaches 74%.  With BMAP only A's k has to: B's rows are looked up (row map or band).
 template <int BM, int BN, int WM, int WN, int BK, int STAGES>
 struct DmmaKcCfg {
     static constexpr int NT = 32 * WM * WN;
@@ -249,7 +249,7 @@ struct DmmaKcCfg {
     static constexpr size_t SMEM_BYTES = (size_t)STAGES * STAGE_Z * sizeof(z);
 };
 
-template <int BM, int BN, int WM, int WN, int BK, int STAGES>
+template <int BM, int BN, int WM, int WN, int BK, int STAGES, bool BMAP = false>
 __device__ __forceinline__ void zgemm_tile_dmma_kc(const GemmDesc& sd, int tile, z* smem) {
     using Cfg = DmmaKcCfg<BM, BN, WM, WN, BK, STAGES>;
     constexpr int NT = Cfg::NT, LDA = Cfg::LDA, LDB = Cfg::LDB, TMW = Cfg::TMW, TNW = Cfg::TNW;
@@ -277,7 +277,7 @@ __device__ __forceinline__ void zgemm_tile_dmma_kc(const GemmDesc& sd, int tile,
     for (int e = 0; e < B_PER; ++e) {
         const int j = n0 + bj0 + e * (NT / BK);
         bcol_ok[e] = j < n;
-        b_src[e] = B.p + (bcol_ok[e] ? (long long)vcol(B, j) * B.ld : 0) + bkk;
+        b_src[e] = B.p + (bcol_ok[e] ? (long long)vcol(B, j) * B.ld : 0) + (BMAP ? 0 : bkk);
     }
     const int ktiles = (K + BK - 1) / BK, kfull = K / BK;
     const int a_dst = akk0 * LDA + ai;
@@ -286,11 +286,12 @@ __device__ __forceinline__ void zgemm_tile_dmma_kc(const GemmDesc& sd, int tile,
         z* S = smem + stage * STAGE_Z;
         const long long ka = (long long)kt * a_ks;
         const int kb = kt * BK;
+        const int br = !BMAP ? kb : kb + bkk < K ? vrow(B, kb + bkk) : 0;
         if (kt < kfull) {
 #pragma unroll
             for (int e = 0; e < A_PER; ++e) cp_async16(S + a_dst + e * (NT / BM) * LDA, a_src + ka + e * a_es, a_bytes);
 #pragma unroll
-            for (int e = 0; e < B_PER; ++e) cp_async16(S + b_dst + e * (NT / BK), b_src[e] + kb, bcol_ok[e] ? 16 : 0);
+            for (int e = 0; e < B_PER; ++e) cp_async16(S + b_dst + e * (NT / BK), b_src[e] + br, bcol_ok[e] ? 16 : 0);
         } else {
 #pragma unroll
             for (int e = 0; e < A_PER; ++e) {
@@ -301,7 +302,7 @@ __device__ __forceinline__ void zgemm_tile_dmma_kc(const GemmDesc& sd, int tile,
 #pragma unroll
             for (int e = 0; e < B_PER; ++e) {
                 const bool ok = kok && bcol_ok[e];
-                cp_async16(S + b_dst + e * (NT / BK), ok ? b_src[e] + kb : B.p, ok ? 16 : 0);
+                cp_async16(S + b_dst + e * (NT / BK), ok ? b_src[e] + br : B.p, ok ? 16 : 0);
             }
         }
     };

@@ -48,7 +48,7 @@ static int test_zgemm(int engine, int m, int n, int k, const double* dA, long lo
     GemmBatch b;
     b.count = count;
     b.max_m = m; b.max_n = n; b.max_k = k;
-    b.kcontig = true;
+    b.kcontig = b.acontig = true;
     b.fixed_order = engine == 3;
     int* d_status = nullptr;
     if (cudaMalloc(&b.d_desc, sizeof(GemmDesc) * count) != cudaSuccess) return RB_ERR_CUDA;

@@ -26,3 +26,21 @@ def test_solve_gemm_columns_do_not_depend_on_their_number(m, k, cnt):
     assert np.abs(full - ref).max() / scale < 1e-13          # the FP64 engines' bar (test_gpu_tc5)
     for n in (1, 3, 8, 9, 16, 17, 32):
         assert np.array_equal(_run(3, A, B[:, :, :n], C0[:, :, :n], alpha, beta), full[:, :, :n]), n
+
+
+@pytest.mark.parametrize("cells,L", [(112, 6), (96, 5)])
+def test_a_column_does_not_depend_on_the_batch_it_is_solved_in(cells, L):
+    """Whole solves, whose products gather their right-hand sides through maps: one column (the streaming
+    kernel), 17 (32- and 16-row tiles of 32 columns) and 33 (two of them), bit for bit."""
+    from helpers import gpu_rhs, gpu_tree
+    from robinsolver_b200 import workloads as W
+    wl = W.make_workload(1, N=cells, L=L, nrhs=33)
+    T, op, opts = gpu_tree(wl)
+    T.factor(wl.L, op, opts)
+    out = {}
+    for n in (33, 17, 1):
+        T.solve(gpu_rhs(wl.rhs[:n]))
+        out[n] = np.stack([T.solution_array(r) for r in range(n)])
+    T.close()
+    assert np.array_equal(out[33][:17], out[17])
+    assert np.array_equal(out[33][:1], out[1])
