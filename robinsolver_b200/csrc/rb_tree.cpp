@@ -620,18 +620,30 @@ static cudaError_t launch_gemm_level(rb_tree* t, const GemmBatch& b, int l, cuda
 // level) run on the residue engine.
 // Whole steps, FP64 tiles everywhere against this rule: 1024^2 27.3 to 22.2 ms, 512^2 (the root alone)
 // 6.0 to 5.7, 32^3 28.7 to 19.9.  At 256 points the passes over the operands and outputs cost what the
-// products save (768 x 768 x 256 in 32 problems 988 to 826 us, 256 x 768 in 16 190 to 236).
+// products save (768 x 768 x 256 in 32 problems 988 to 826 us, 256 x 768 in 16 190 to 236); a level's map,
+// whose products are the largest and share their operands, gains from m n = CRT_MIN_MN on (n: the outer
+// points of a child): 32^3 18.5 to 18.1 ms, a 768^2 step 12.6 to 12.3 (from m = 256 at any n: 1024^2 21.87 to 21.98).
 // The rule is one per level, so that the row sets of the pipelined factor and the whole map of the
 // serial one take the same engine: its sums are exact, and the two agree bit for bit.
-constexpr int CRT_MIN_M = 512;
-static bool crt_level(const rb_tree* t, int l) {
-    const int m = t->P.lv[l].m;
-    return m >= CRT_MIN_M && m <= CRT_MAX_K;
+constexpr int CRT_MIN_M = 512, CRT_MIN_MAP_M = 256;
+constexpr long long CRT_MIN_MN = 1 << 18;
+enum { CRT_NO, CRT_MAP, CRT_ALL };
+static int crt_level(const rb_tree* t, int l) {
+    const PlanLevel& p = t->P.lv[l];
+    if (p.m > CRT_MAX_K) return CRT_NO;
+    if (p.m >= CRT_MIN_M) return CRT_ALL;
+    return p.m >= CRT_MIN_MAP_M && (long long)p.m * std::min(p.n1, p.n2) >= CRT_MIN_MN ? CRT_MAP : CRT_NO;
 }
 // the batches of a level on the main stream (lane 0), the chain stream (1) and B1's (2); the serial
 // factor runs the first two on the main stream, one after another
 static std::vector<GemmBatch*> crt_stages(rb_tree* t, int l, int lane) {
     const bool tail = l == 0 || !t->kform;
+    const int which = crt_level(t, l);
+    if (which == CRT_NO) return {};
+    if (which == CRT_MAP) {
+        if (lane == 0) return tail ? std::vector<GemmBatch*>{&t->fM4[l]} : std::vector<GemmBatch*>{&t->fM4[l], &t->fM4N[l]};
+        return lane == 1 && !tail ? std::vector<GemmBatch*>{&t->fM4F[l]} : std::vector<GemmBatch*>{};
+    }
     if (lane == 2) return {&t->fM1[l]};
     if (lane == 1) return tail ? std::vector<GemmBatch*>{&t->fK[l]}
                                : std::vector<GemmBatch*>{&t->fK[l], &t->fM2[l], &t->fM3[l], &t->fM4F[l]};
@@ -650,15 +662,17 @@ static size_t crt_lane_bytes(const rb_tree* t, size_t need[3]) {
     };
     need[0] = need[1] = need[2] = 0;
     for (int l = 0; l < t->P.L; ++l) {
-        if (!crt_level(t, l)) continue;
+        const int which = crt_level(t, l);
+        if (which == CRT_NO) continue;
         const PlanLevel& p = t->P.lv[l];
         const int n = std::max(p.n1, p.n2), m = p.m, nn = p.nnodes;
         const bool tail = l == 0 || !t->kform;
         if (!(l == 0 && t->skip_root)) need[0] = std::max(need[0], bytes(4 * nn, n, n, m));
-        need[tail ? 0 : 1] = std::max(need[tail ? 0 : 1], bytes(2 * nn, m, n, m));
-        if (t->kform) need[1] = std::max(need[1], bytes(nn, m, m, m));
         // the rows on the face the parent merges across: at most its interface's points
         if (!tail) need[1] = std::max(need[1], bytes(4 * nn, std::min(n, t->P.lv[l - 1].m), n, m));
+        if (which == CRT_MAP) continue;
+        need[tail ? 0 : 1] = std::max(need[tail ? 0 : 1], bytes(2 * nn, m, n, m));
+        if (t->kform) need[1] = std::max(need[1], bytes(nn, m, m, m));
         need[2] = std::max(need[2], bytes(nn, m, n, m));
     }
     return need[0] + need[1] + need[2];
@@ -682,7 +696,7 @@ static int ensure_crt_plan(rb_tree* t) {
             return RB_OK;
         }
     for (int l = 0; l < t->P.L; ++l)
-        for (int lane = 0; lane < 3 && crt_level(t, l); ++lane)
+        for (int lane = 0; lane < 3; ++lane)
             for (GemmBatch* b : crt_stages(t, l, lane)) {
                 const size_t bytes = crt_bytes(*b);
                 if (bytes == 0 || bytes > need[lane]) continue;
