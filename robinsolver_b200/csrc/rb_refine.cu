@@ -20,6 +20,7 @@
 // (zeta - T_ii) g_i + nu g_i' = h_particular - r.
 #include <cstdint>
 
+#include "rb_gemm_dmma.cuh"      // cp_async16
 #include "rb_kernels.h"
 
 namespace rb {
@@ -47,11 +48,11 @@ __device__ __forceinline__ void leaf_bnd(int r, int a, int b, int& e1, int& e2, 
     e2 = leaf_lin(i + 2 * si, j + 2 * sj, a, b);
 }
 
-__device__ __forceinline__ z dn_u(const z* u, int r, int e1, int e2, double hn) {
-    // (8/3 u_b - 3 u_1 + 1/3 u_2) / h, in the order fd_module.f90:207-215 adds the terms
-    z v = zscale((8.0 / 3.0) / hn, u[r]);
-    v = zadd(v, zscale(-3.0 / hn, u[e1]));
-    v = zadd(v, zscale((1.0 / 3.0) / hn, u[e2]));
+__device__ __forceinline__ z dn_u(const z* u, int r, int e1, int e2, const double* w) {
+    // (8/3 u_b - 3 u_1 + 1/3 u_2) / h, in the order fd_module.f90:207-215 adds the terms; w: the weights / h
+    z v = zscale(w[0], u[r]);
+    v = zadd(v, zscale(w[1], u[e1]));
+    v = zadd(v, zscale(w[2], u[e2]));
     return v;
 }
 
@@ -69,44 +70,66 @@ __device__ __forceinline__ void atomic_max_nonneg(double* p, double v) {
 // domain-boundary point, < 0 -1 - (leaf'*nb + r') of the neighbour's row for the same point.
 // rnorm[rhs]: max |r| over every row, accumulated with one atomic per CTA (one per warp and leaf
 // serialised half a million atomics on the L2 slices holding rnorm).
+// Memory bounds it (u read, f read and written, the neighbours' rows), once the stencil's weights are
+// divided by h^2 per leaf and not per point: 1024^2 with 32 right-hand sides 989 to 728 us, and
+// the next leaf's u is copied while this one's is used: 604.
 constexpr int RES_LEAVES = 16;
 constexpr int RES_THREADS = 128;
 __global__ void __launch_bounds__(RES_THREADS) fd_residual_kernel(RefineGeom g, const z* __restrict__ d, z* f,
                                                                  z* groot, z* ri, const z* __restrict__ kv,
                                                                  const double* __restrict__ hh,
                                                                  const int* __restrict__ bclass, int first,
-                                                                 double* rnorm) {
-    extern __shared__ z ush[];
+                                                                 int bufs, double* rnorm) {
+    extern __shared__ z usm[];                   // bufs = 2 leaves' u, one used, one on its way, or 1
     __shared__ double wmax[RES_THREADS / 32];
+    __shared__ double wst[2][3][3], wdn[2][3];   // the leaf's weights: [dim][first, last, between][w0, w1, w2]; D_n
+    const float inv_a = 1.0f / (float)g.a;
     const int rhs = blockIdx.y;
     const int a = g.a, b = g.b, nb = 2 * (a + b), ab = a * b, n = nb + ab;
     const z ikb = zmk(0.0, g.kb), mikb = zmk(0.0, -g.kb);
     double mx = 0.0;
     const int l0 = blockIdx.x * RES_LEAVES;
     const int l1 = min(g.nleaves, l0 + RES_LEAVES);
-    for (int leaf = l0; leaf < l1; ++leaf) {
+    auto load = [&](int leaf) {
         const z* u = d + ((long long)rhs * g.nleaves + leaf) * n;
-        __syncthreads();                       // the previous leaf's reads of ush are done
-        for (int e = threadIdx.x; e < n; e += blockDim.x) ush[e] = u[e];
-        __syncthreads();
+        z* dst = usm + ((leaf - l0) & (bufs - 1)) * n;
+        for (int e = threadIdx.x; e < n; e += blockDim.x) cp_async16(dst + e, u + e, 16);
+    };
+    load(l0);
+    cp_async_commit();
+    for (int leaf = l0; leaf < l1; ++leaf) {
+        z* ush = usm + ((leaf - l0) & (bufs - 1)) * n;
+        // into the buffer whose reads ended with the last barrier
+        if (bufs == 2 ? leaf + 1 < l1 : leaf > l0) load(bufs == 2 ? leaf + 1 : leaf);
+        cp_async_commit();
         const double hx = hh[2 * leaf], hy = hh[2 * leaf + 1];
+        if (threadIdx.x < 18) {
+            const int dim = threadIdx.x / 9, at = threadIdx.x / 3 % 3, w = threadIdx.x % 3;
+            const double wv = w == 1 ? (at == 2 ? -2.0 : -4.0) : at == 2 ? 1.0 : (w == 0) == (at == 0) ? 8.0 / 3.0 : 4.0 / 3.0;
+            wst[dim][at][w] = wv / (dim == 0 ? hx * hx : hy * hy);
+        } else if (threadIdx.x >= 32 && threadIdx.x < 38) {
+            const int dim = (threadIdx.x - 32) / 3, w = (threadIdx.x - 32) % 3;
+            wdn[dim][w] = (w == 0 ? 8.0 / 3.0 : w == 1 ? -3.0 : 1.0 / 3.0) / (dim == 0 ? hx : hy);
+        }
+        if (bufs == 2) cp_async_wait<1>();     // this leaf's u
+        else cp_async_wait<0>();
+        __syncthreads();
         for (int e = threadIdx.x; e < n; e += blockDim.x) {
             if (e >= nb) {
                 const int q = e - nb;
-                const int gi = q % a + 1, gj = q / a + 1;
+                // q / a: (q + 1/2) / a is at least 1/(2a) from a whole number
+                const int row = __float2int_rz(((float)q + 0.5f) * inv_a);
+                const int gi = q - row * a + 1, gj = row + 1;
                 z acc = zmul(kv[(long long)leaf * ab + q], ush[e]);
                 // x then y, each the [w0, w1, w2] stencil of FD_matrix_row (fd_module.f90:150-181)
                 for (int dim = 0; dim < 2; ++dim) {
                     const int gg = dim == 0 ? gi : gj, len = dim == 0 ? a : b;
-                    double w0 = 1.0, w1 = -2.0, w2 = 1.0;
-                    if (gg == 1) { w0 = 8.0 / 3.0; w1 = -4.0; w2 = 4.0 / 3.0; }
-                    else if (gg == len) { w0 = 4.0 / 3.0; w1 = -4.0; w2 = 8.0 / 3.0; }
-                    const double h2 = dim == 0 ? hx * hx : hy * hy;
+                    const double* w = wst[dim][gg == 1 ? 0 : gg == len ? 1 : 2];
                     const int eu = dim == 0 ? leaf_lin(gi + 1, gj, a, b) : leaf_lin(gi, gj + 1, a, b);
                     const int ed = dim == 0 ? leaf_lin(gi - 1, gj, a, b) : leaf_lin(gi, gj - 1, a, b);
-                    acc = zadd(acc, zscale(w1 / h2, ush[e]));
-                    acc = zadd(acc, zscale(w2 / h2, ush[eu]));
-                    acc = zadd(acc, zscale(w0 / h2, ush[ed]));
+                    acc = zadd(acc, zscale(w[1], ush[e]));
+                    acc = zadd(acc, zscale(w[2], ush[eu]));
+                    acc = zadd(acc, zscale(w[0], ush[ed]));
                 }
                 z* fp = f + ((long long)rhs * g.nleaves + leaf) * ab + q;
                 const z r = zsub(*fp, acc);
@@ -115,8 +138,7 @@ __global__ void __launch_bounds__(RES_THREADS) fd_residual_kernel(RefineGeom g, 
             } else {
                 int e1, e2, axis;
                 leaf_bnd(e, a, b, e1, e2, axis);
-                const double hn = axis == 0 ? hx : hy;
-                const z dn = dn_u(ush, e, e1, e2, hn);
+                const z dn = dn_u(ush, e, e1, e2, wdn[axis]);
                 const z gin = zadd(zmul(ikb, ush[e]), dn);
                 const int cls = bclass[(long long)leaf * nb + e];
                 z r;
@@ -131,9 +153,13 @@ __global__ void __launch_bounds__(RES_THREADS) fd_residual_kernel(RefineGeom g, 
                     int f1, f2, ax2;
                     leaf_bnd(rj, a, b, f1, f2, ax2);
                     const double hn2 = ax2 == 0 ? hh[2 * lj] : hh[2 * lj + 1];
-                    z dn2 = zscale((8.0 / 3.0) / hn2, un[rj]);
-                    dn2 = zadd(dn2, zscale(-3.0 / hn2, un[f1]));
-                    dn2 = zadd(dn2, zscale((1.0 / 3.0) / hn2, un[f2]));
+                    z dn2;
+                    if (hn2 == (ax2 == 0 ? hx : hy)) {
+                        dn2 = dn_u(un, rj, f1, f2, wdn[ax2]);
+                    } else {
+                        const double w2[3] = {(8.0 / 3.0) / hn2, -3.0 / hn2, (1.0 / 3.0) / hn2};
+                        dn2 = dn_u(un, rj, f1, f2, w2);
+                    }
                     const z gin2 = zadd(zmul(ikb, un[rj]), dn2);
                     const z hout = zadd(zmul(mikb, ush[e]), dn);
                     // transmission row: h_out - zeta g_in - nu g_in' = 0
@@ -145,6 +171,7 @@ __global__ void __launch_bounds__(RES_THREADS) fd_residual_kernel(RefineGeom g, 
                 mx = fmax(mx, fabs(r.x) + fabs(r.y));
             }
         }
+        __syncthreads();                       // this leaf's reads of ush, wst and wdn are done
     }
     // max over the CTA, then over CTAs
     for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
@@ -201,14 +228,16 @@ __global__ void refine_update_kernel(z* x, const z* __restrict__ dx, long long p
 cudaError_t fd_residual(const RefineGeom& g, int nrhs, const z* d, z* f, z* groot, z* ri, const z* kv,
                         const double* hh, const int* bclass, bool first, double* rnorm, cudaStream_t s) {
     const int n = 2 * (g.a + g.b) + g.a * g.b;
-    const size_t sh = (size_t)n * sizeof(z);
+    // both buffers while four CTAs still fit an SM
+    const int bufs = 2 * (size_t)n * sizeof(z) <= 56 * 1024 ? 2 : 1;
+    const size_t sh = bufs * (size_t)n * sizeof(z);
     if (sh > 48 * 1024) {
         static DeviceAttrCache attr;
         cudaError_t e = ensure_smem_attr(fd_residual_kernel, sh, attr);
         if (e != cudaSuccess) return e;
     }
     fd_residual_kernel<<<dim3((g.nleaves + RES_LEAVES - 1) / RES_LEAVES, nrhs), RES_THREADS, sh, s>>>(
-        g, d, f, groot, ri, kv, hh, bclass, first ? 1 : 0, rnorm);
+        g, d, f, groot, ri, kv, hh, bclass, first ? 1 : 0, bufs, rnorm);
     note_launch();
     return cudaGetLastError();
 }

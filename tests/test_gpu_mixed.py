@@ -118,3 +118,18 @@ def test_mixed_int8_top_levels():
         assert 1e-15 < d < 1e-8, (lvl, d)
     Tf.close()
     Tm.close()
+
+
+@pytest.mark.parametrize("N,L", [(64, 1), (100, 4)])
+def test_mixed_residual_on_large_and_ragged_leaves(N, L):
+    """The residual kernel on leaves that take one buffer (32 x 64 cells) and two, of a size that is no power of
+    two: the refined solution reaches the FP64 one, at the refinement's tolerance."""
+    wl = W.make_workload(1, N=N, L=L, nrhs=3)
+    sols = []
+    for precision in ("fp64", "mixed"):
+        T, op, opts = gpu_tree(wl)
+        T.factor(wl.L, op, opts, precision)
+        T.solve(gpu_rhs(wl.rhs))
+        sols.append(np.stack([T.solution_array(r) for r in range(3)]))
+        T.close()
+    assert np.abs(sols[1] - sols[0]).max() < 1e-9 * np.abs(sols[0]).max()
