@@ -325,7 +325,7 @@ static cudaError_t launch_solve_gemm(const GemmBatch& b, cudaStream_t s, bool pd
 }
 
 // the kernel shape a batch runs on
-enum class GemmShape { Dfma16, Dfma32, Dmma32, Dmma64, DmmaKc64, DmmaFixed, Dfma128x64, Dfma64 };
+enum class GemmShape { Dfma16, Dfma32, Dmma32, Dmma64, DmmaKc64, DmmaFixed, Dfma128x64, Dfma64, DmmaKc32 };
 static GemmShape gemm_shape(const GemmBatch& b) {
     const int mm = b.max_m, nn = b.max_n;
     if (b.engine >= 0 && !b.fixed_order) return static_cast<GemmShape>(b.engine);
@@ -349,7 +349,15 @@ static GemmShape gemm_shape(const GemmBatch& b) {
         // contiguous-k batches with k >= 128: 32x32 warp tiles on stride-advanced copies,
         // measured 1.06-1.22x the tile above on the merge shapes 256x256x128 x256 ..
         // 2048x4096x1024 x2 (0.95x on 256x768x256 x8 and 128x512x128 x64, under two waves)
-        if (b.kcontig && b.max_k >= 128) return GemmShape::DmmaKc64;
+        if (b.kcontig && b.max_k >= 128) {
+            // two 64x64 tiles fit an SM; where a batch leaves much of its last wave of them empty, 32x32
+            // tiles (the same sums) finish sooner: 256 x 256 x 256 alone 46 -> 19 us, 128 x 256 x 128 in 4
+            // problems 27 -> 12, 256 x 768 x 256 in 4 (0.65 of a wave) 66 -> 60, in 8 (1.3) 116 -> 102; but
+            // 512 x 512 x 256 in 4 (0.86) 66 -> 69, 384 x 384 x 128 in 16 (1.95) 73 -> 81
+            const long long tiles = (long long)b.count * ((mm + 63) / 64) * ((nn + 63) / 64), wave = 2 * 148;
+            const long long waves = (tiles + wave - 1) / wave;
+            return 10 * tiles < 7 * waves * wave ? GemmShape::DmmaKc32 : GemmShape::DmmaKc64;
+        }
         return GemmShape::Dmma64;
     }
     // large problems: 8x4 complex register tile per thread (1.5 B of shared memory per DFMA)
@@ -402,7 +410,10 @@ int gemm_engine_candidates(const GemmBatch& b, int* out) {
     if (use_dmma()) {
         out[n++] = (int)GemmShape::Dmma32;
         out[n++] = (int)GemmShape::Dmma64;
-        if (b.kcontig) out[n++] = (int)GemmShape::DmmaKc64;
+        if (b.kcontig) {
+            out[n++] = (int)GemmShape::DmmaKc64;
+            out[n++] = (int)GemmShape::DmmaKc32;
+        }
     }
     if (b.max_m >= 128) out[n++] = (int)GemmShape::Dfma128x64;
     return n;
@@ -415,6 +426,7 @@ const char* gemm_engine_name(int e) {
         case GemmShape::Dmma32: return "dmma32";
         case GemmShape::Dmma64: return "dmma64";
         case GemmShape::DmmaKc64: return "dmma_kc64";
+        case GemmShape::DmmaKc32: return "dmma_kc32";
         case GemmShape::DmmaFixed: return "dmma_fixed";
         case GemmShape::Dfma128x64: return "dfma128x64";
         case GemmShape::Dfma64: return "dfma64";
@@ -428,7 +440,7 @@ const char* gemm_stage_name(const GemmBatch& b) {
     // tensor-core factor tiles; zgemm_tc_fixed: the solve's
     if (sh == GemmShape::DmmaFixed) return "zgemm_tc_fixed";
     if (sh == GemmShape::DmmaKc64) return "zgemm_tc";
-    return (sh == GemmShape::Dmma64 || sh == GemmShape::Dmma32) ? "zgemm_tc_small" : "zgemm_dfma";
+    return (sh == GemmShape::Dmma64 || sh == GemmShape::Dmma32 || sh == GemmShape::DmmaKc32) ? "zgemm_tc_small" : "zgemm_dfma";
 }
 
 cudaError_t launch_gemm_batch(const GemmBatch& b, cudaStream_t s, bool pdl) {
@@ -448,6 +460,7 @@ cudaError_t launch_gemm_batch(const GemmBatch& b, cudaStream_t s, bool pdl) {
         case GemmShape::DmmaFixed:           // launched above
         case GemmShape::Dmma32: return launch_dmma<32, 32, 2, 2, 6>(b, s);
         case GemmShape::Dmma64: return launch_dmma<64, 64, 2, 4, 2>(b, s);
+        case GemmShape::DmmaKc32: return launch_dmma<32, 32, 2, 2, 5, 5, DMMA_KCONTIG>(b, s, pdl);
         case GemmShape::DmmaKc64: return launch_dmma_kc<64, 64, 2, 2, 4, 8, 2>(b, s);
         case GemmShape::Dfma128x64: return launch_cfg<128, 64, 8, 4, 4, 4, 1>(b, s);
         case GemmShape::Dfma64: break;
