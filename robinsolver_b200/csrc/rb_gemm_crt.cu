@@ -13,7 +13,8 @@
 //  2. crt_split_kernel: 16 residues of the real and imaginary parts, one byte each, laid out block by
 //     block as the product kernel's shared memory holds them (K-major, 128-byte swizzle);
 //  3. zgemm_crt_kernel: per modulus, the residues of B's column tile ([Br | Bi], 160 rows) stay in shared
-//     memory while those of A (Ar, Ai) stream past through a ring of bulk-copied stages.  MMAs of
+//     memory (k up to 512; above, they stream too) while those of A (Ar, Ai) stream past through a ring
+//     of bulk-copied stages.  MMAs of
 //     128 x 160 x 32 accumulate Ar Br, the sum Ar Bi + Ai Br and Ai Bi in 240 tensor-memory columns
 //     (Ai's columns overlap Ar's by half, so the sum forms by itself).  The next tile's MMAs run on the
 //     other half of tensor memory while eight warps read the accumulators, reduce them and write one
@@ -27,7 +28,8 @@
 // 1376; 1536 x 1536 x 512, 8: 1874 to 1016; 512 x 1536 x 512, 4: 357 to 261; 1024 x 2048 x 1024, 1: 462 to 230;
 // 768 x 768 x 256, 32: 988 to 826; 256 x 768 x 256, 16: 190 to 236; 384 x 384 x 128, 128: 548 to 808.  The first spends
 // 29 + 26 us on scales, 294 on the split (its 16 residues per entry are issue bound), 829 on products
-// (the tensor pipe alone would take 520) and 205 on the outputs (5.2 TB/s).
+// (the tensor pipe alone would take 520) and 205 on the outputs (FP64 sums, issue
+// bound too; DRAM 43% busy).
 #include <algorithm>
 #include <climits>
 #include <cstdint>

@@ -6,7 +6,7 @@
 //
 // Factor (robin_tree_factor -> compute_RTR, robin_tree_module.f90:96-185, 375-650):
 //   leaves:  block-tridiagonal factor of S = A_ii - A_ib A_bb^-1 A_bi from the potential
-//            samples and Y = R A^-1 (RtR in its first nb columns), one CTA per leaf (rb_leaf.cu)
+//            samples and Y = R A^-1 (RtR in its first nb columns; rb_leaf.cu)
 //   level l = L-1 .. 0, all nodes of the level in one launch per stage.  [Y1; Y2] =
 //   M^-1 blockdiag(T1_iN, T2_iN) solves the interface system M = [[A1, nu I], [nu I, A2]],
 //   A1 = zeta I - T1_ii, A2 = zeta I - T2_ii, then
