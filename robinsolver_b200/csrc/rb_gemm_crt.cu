@@ -262,8 +262,8 @@ __global__ void __launch_bounds__(256, 3) crt_split_kernel(const GemmDesc* __res
 // Up to k = 512 B's column tile (160 rows x k) stays in shared memory for a modulus while the row tiles
 // of A stream past it; its blocks are refilled for the next modulus as the last row tile lets go of
 // them.  Above, B's blocks stream beside A's: a resident tile would leave room for two stages only
-// (k = 1024: 1014 us of products for 4 x 2048 x 2048, 829 streaming).  Every mbarrier wait is bounded; a CTA that gives up sets RB_TC5_TIMEOUT, waits (bounded) for
-// the copies and MMAs it issued, frees its tensor memory and returns.
+// (k = 1024: 1014 us of products for 4 x 2048 x 2048, 829 streaming).  Every mbarrier wait is bounded; a CTA that gives up sets RB_TC5_TIMEOUT; in every
+// CTA the copies and MMAs it issued are waited for (bounded) before its tensor memory is freed and it returns.
 __global__ void __launch_bounds__(CRT_THREADS, 1) zgemm_crt_kernel(const GemmDesc* __restrict__ descs, int prob0, int* status,
                                                                   const unsigned char* __restrict__ planes, int MT, int NT,
                                                                   int KB, long long a_bytes, unsigned char* __restrict__ out,
@@ -347,10 +347,12 @@ __global__ void __launch_bounds__(CRT_THREADS, 1) zgemm_crt_kernel(const GemmDes
             if (!ok) {
                 abort_flag = 1;
                 atomicOr(status, RB_TC5_TIMEOUT);
-                for (int i = max(0, it - CRT_STAGES); i < it; ++i)
-                    mbar_wait(afull0 + 8 * (i % CRT_STAGES), (uint32_t)((i / CRT_STAGES) & 1), nullptr);
-                for (int i = max(0, nb - nk); i < nb; ++i) mbar_wait(bfull0 + 8 * (i % nk), (uint32_t)((i / nk) & 1), nullptr);
             }
+            // no copy may still target this CTA's memory when it exits, whichever warp gave up: wait
+            // (bounded) for the last fill of every stage and resident block
+            for (int i = max(0, it - CRT_STAGES); i < it; ++i)
+                mbar_wait(afull0 + 8 * (i % CRT_STAGES), (uint32_t)((i / CRT_STAGES) & 1), nullptr);
+            for (int i = max(0, nb - nk); i < nb; ++i) mbar_wait(bfull0 + 8 * (i % nk), (uint32_t)((i / nk) & 1), nullptr);
         }
         __syncwarp();
     } else if (warp == 1) {

@@ -298,11 +298,11 @@ __global__ void __launch_bounds__(TC5_THREADS, 1) zgemm_tc5_kernel(const GemmDes
         if (!ok) {
             abort_flag = 1;
             if (lane == 0) atomicOr(status, RB_TC5_TIMEOUT);
-            // no copy may still target this CTA's memory when it exits: wait (bounded) for the
-            // stages filled last, whatever the MMA warp did with them
-            for (int kb = max(0, issued - STAGES); kb < issued; ++kb)
-                mbar_wait(full0 + 8 * (kb % STAGES), (uint32_t)((kb / STAGES) & 1), nullptr);
         }
+        // no copy may still target this CTA's memory when it exits, whichever warp gave up: wait
+        // (bounded) for the stages filled last
+        for (int kb = max(0, issued - STAGES); kb < issued; ++kb)
+            mbar_wait(full0 + 8 * (kb % STAGES), (uint32_t)((kb / STAGES) & 1), nullptr);
         __syncwarp();
     } else if (warp == 1) {
         // ---------------- MMA issuer: one lane, the warp kept converged ----------------------------
@@ -791,9 +791,10 @@ __global__ void __launch_bounds__(TC5_THREADS, 1) zgemm_oz_kernel(const GemmDesc
         if (!ok) {
             abort_flag = 1;
             if (lane == 0) atomicOr(status, RB_TC5_TIMEOUT);
-            for (int kb = max(0, issued - STAGES); kb < issued; ++kb)
-                mbar_wait(full0 + 8 * (kb % STAGES), (uint32_t)((kb / STAGES) & 1), nullptr);
         }
+        // as above: no copy in flight at the exit
+        for (int kb = max(0, issued - STAGES); kb < issued; ++kb)
+            mbar_wait(full0 + 8 * (kb % STAGES), (uint32_t)((kb / STAGES) & 1), nullptr);
         __syncwarp();
     } else if (warp == 1) {
         // ---------------- MMA issuer --------------------------------------------------------------------
