@@ -280,7 +280,7 @@ __global__ void __launch_bounds__(CRT_THREADS, 1) zgemm_crt_kernel(const GemmDes
     if (tn >= tiles_n || t0 >= tiles_m) return;                  // the whole CTA
     const long long prob = prob0 + (long long)blockIdx.y;
     const int s0 = blockIdx.z * per_group, s1 = min(CRT_S, s0 + per_group);
-    const int nk = (g.k + CRT_KB - 1) / CRT_KB;                  // blocks of this problem
+    const int nk = max(1, (g.k + CRT_KB - 1) / CRT_KB);          // blocks of this problem (k = 0: one of zeros)
     const long long a_mod = (long long)KB * 2 * CRT_A_BLOCK, b_mod = (long long)KB * CRT_B_BLOCK;
     const unsigned char* gB = planes + a_bytes + (prob * NT + tn) * CRT_S * b_mod;
 
@@ -470,7 +470,7 @@ __global__ void __launch_bounds__(256, 4) crt_combine_kernel(const GemmDesc* __r
                                                           const int* __restrict__ fb) {
     const GemmDesc& g = descs[blockIdx.y];
     const long long prob = prob0 + (long long)blockIdx.y;
-    const int tiles_m = (g.m + CRT_BM - 1) / CRT_BM;
+    const int tiles_m = max(1, (g.m + CRT_BM - 1) / CRT_BM);
     // blockIdx.x: column groups of a tile (tm fastest)
     const int c8 = blockIdx.x % (CRT_BN / 8), t = blockIdx.x / (CRT_BN / 8);
     const int tm = t % tiles_m, tn = t / tiles_m;

@@ -11,6 +11,7 @@
 // It allocates its descriptor array itself and synchronises; it returns 0, a negative RB_ERR_*
 // code for bad arguments or CUDA failures, or the device status word's bits (> 0) when a kernel
 // reported one.
+#include <algorithm>
 #include <string>
 #include <vector>
 
@@ -19,36 +20,19 @@
 
 using namespace rb;
 
-// rb_test_zgemm_timed is the same call repeated `reps` times after one untimed run, and writes
-// the mean device time of one batched launch in milliseconds to *ms (CUDA events; the engine's
-// operand-split pass included).
-static int test_zgemm(int engine, int m, int n, int k, const double* dA, long long lda, long long strideA,
-                      const double* dB, long long ldb, long long strideB, double* dC, long long ldc,
-                      long long strideC, double ar, double ai, double br, double bi, int count, int reps,
-                      double* ms) {
-    if (m <= 0 || n <= 0 || k <= 0 || count <= 0 || !dA || !dB || !dC || lda < m || ldb < k || ldc < m || reps < 0)
-        return RB_ERR_INVALID;
-    std::vector<GemmDesc> h(count);
-    const z* A = reinterpret_cast<const z*>(dA);
-    const z* B = reinterpret_cast<const z*>(dB);
-    z* C = reinterpret_cast<z*>(dC);
-    const bool use_beta = br != 0.0 || bi != 0.0;
-    for (int i = 0; i < count; ++i) {
-        GemmDesc& g = h[i];
-        g = GemmDesc{};
-        g.A = zview(A + i * strideA, lda);
-        g.B = zview(B + i * strideB, ldb);
-        g.C = use_beta ? zview(C + i * strideC, ldc) : zview(nullptr, 1);
-        g.D = zout(C + i * strideC, ldc);
-        g.alpha = zmk(ar, ai);
-        g.beta = zmk(br, bi);
-        g.m = m; g.n = n; g.k = k;
-        g.nobeta_r0 = g.nobeta_r1 = 0;
-    }
+// `h` on one engine, with the sizes of its largest problem; reps and ms as below
+static int run_descs(int engine, const std::vector<GemmDesc>& h, int reps, double* ms) {
+    const int count = (int)h.size();
     GemmBatch b;
     b.count = count;
-    b.max_m = m; b.max_n = n; b.max_k = k;
     b.kcontig = b.acontig = true;
+    for (const GemmDesc& g : h) {
+        b.max_m = std::max(b.max_m, g.m);
+        b.max_n = std::max(b.max_n, g.n);
+        b.max_k = std::max(b.max_k, g.k);
+        b.kcontig = b.kcontig && gemm_k_contiguous(g);
+        b.acontig = b.acontig && gemm_a_contiguous(g);
+    }
     b.fixed_order = engine == 3;
     int* d_status = nullptr;
     if (cudaMalloc(&b.d_desc, sizeof(GemmDesc) * count) != cudaSuccess) return RB_ERR_CUDA;
@@ -107,6 +91,35 @@ static int test_zgemm(int engine, int m, int n, int k, const double* dA, long lo
     return rc;
 }
 
+// rb_test_zgemm_timed is the same call repeated `reps` times after one untimed run, and writes
+// the mean device time of one batched launch in milliseconds to *ms (CUDA events; the engine's
+// operand-split pass included).
+static int test_zgemm(int engine, int m, int n, int k, const double* dA, long long lda, long long strideA,
+                      const double* dB, long long ldb, long long strideB, double* dC, long long ldc,
+                      long long strideC, double ar, double ai, double br, double bi, int count, int reps,
+                      double* ms) {
+    if (m <= 0 || n <= 0 || k <= 0 || count <= 0 || !dA || !dB || !dC || lda < m || ldb < k || ldc < m || reps < 0)
+        return RB_ERR_INVALID;
+    std::vector<GemmDesc> h(count);
+    const z* A = reinterpret_cast<const z*>(dA);
+    const z* B = reinterpret_cast<const z*>(dB);
+    z* C = reinterpret_cast<z*>(dC);
+    const bool use_beta = br != 0.0 || bi != 0.0;
+    for (int i = 0; i < count; ++i) {
+        GemmDesc& g = h[i];
+        g = GemmDesc{};
+        g.A = zview(A + i * strideA, lda);
+        g.B = zview(B + i * strideB, ldb);
+        g.C = use_beta ? zview(C + i * strideC, ldc) : zview(nullptr, 1);
+        g.D = zout(C + i * strideC, ldc);
+        g.alpha = zmk(ar, ai);
+        g.beta = zmk(br, bi);
+        g.m = m; g.n = n; g.k = k;
+        g.nobeta_r0 = g.nobeta_r1 = 0;
+    }
+    return run_descs(engine, h, reps, ms);
+}
+
 extern "C" int rb_test_zgemm(int engine, int m, int n, int k, const double* dA, long long lda, long long strideA,
                              const double* dB, long long ldb, long long strideB, double* dC, long long ldc,
                              long long strideC, double ar, double ai, double br, double bi, int count) {
@@ -120,6 +133,14 @@ extern "C" int rb_test_zgemm_timed(int engine, int m, int n, int k, const double
                                    int count, int reps, double* ms) {
     return test_zgemm(engine, m, n, k, dA, lda, strideA, dB, ldb, strideB, dC, ldc, strideC, ar, ai, br, bi, count,
                       reps, ms);
+}
+
+// rb_test_zgemm_descs: any problems at all -- `descs` is a host array of GemmDesc (rb_common.cuh), each with
+// its own sizes, row and column maps and skipped bands, every pointer in it a device pointer.
+extern "C" int rb_test_zgemm_descs(int engine, int count, const void* descs) {
+    if (count <= 0 || !descs) return RB_ERR_INVALID;
+    const GemmDesc* d = static_cast<const GemmDesc*>(descs);
+    return run_descs(engine, std::vector<GemmDesc>(d, d + count), 0, nullptr);
 }
 
 // rb_test_zinvert inverts `count` complex m x m matrices in place (column-major, device pointers,
