@@ -48,11 +48,11 @@ __device__ __forceinline__ void leaf_bnd(int r, int a, int b, int& e1, int& e2, 
     e2 = leaf_lin(i + 2 * si, j + 2 * sj, a, b);
 }
 
-__device__ __forceinline__ z dn_u(const z* u, int r, int e1, int e2, const double* w) {
-    // (8/3 u_b - 3 u_1 + 1/3 u_2) / h, in the order fd_module.f90:207-215 adds the terms; w: the weights / h
-    z v = zscale(w[0], u[r]);
-    v = zadd(v, zscale(w[1], u[e1]));
-    v = zadd(v, zscale(w[2], u[e2]));
+__device__ __forceinline__ z dn_u(const z* u, int r, int e1, int e2, double third, double m3) {
+    // (8/3 u_b - 3 u_1 + 1/3 u_2) / h, in the order fd_module.f90:207-215 adds the terms; third: (1/3)/h, m3: -3/h
+    z v = zscale(8.0 * third, u[r]);
+    v = zadd(v, zscale(m3, u[e1]));
+    v = zadd(v, zscale(third, u[e2]));
     return v;
 }
 
@@ -81,8 +81,11 @@ __global__ void __launch_bounds__(RES_THREADS) fd_residual_kernel(RefineGeom g, 
                                                                  const int* __restrict__ bclass, int first,
                                                                  int bufs, double* rnorm) {
     extern __shared__ z usm[];                   // bufs = 2 leaves' u, one used, one on its way, or 1
-    __shared__ double wmax[RES_THREADS / 32];
-    __shared__ double wst[2][3][3], wdn[2][3];   // the leaf's weights: [dim][first, last, between][w0, w1, w2]; D_n
+    // the leaf's weights, [dim][1/h^2, (4/3)/h^2, (1/3)/h, -3/h]; the others are these times a power of two.  Few,
+    // because they come on top of u: the largest leaves leave 96 bytes of an SM's shared memory.
+    __shared__ double wt[2][4];
+    double* wmax = &wt[0][0];                    // the warps' maxima, after the last leaf
+    static_assert(RES_THREADS / 32 <= 8, "wmax");
     const float inv_a = 1.0f / (float)g.a;
     const int rhs = blockIdx.y;
     const int a = g.a, b = g.b, nb = 2 * (a + b), ab = a * b, n = nb + ab;
@@ -103,13 +106,10 @@ __global__ void __launch_bounds__(RES_THREADS) fd_residual_kernel(RefineGeom g, 
         if (bufs == 2 ? leaf + 1 < l1 : leaf > l0) load(bufs == 2 ? leaf + 1 : leaf);
         cp_async_commit();
         const double hx = hh[2 * leaf], hy = hh[2 * leaf + 1];
-        if (threadIdx.x < 18) {
-            const int dim = threadIdx.x / 9, at = threadIdx.x / 3 % 3, w = threadIdx.x % 3;
-            const double wv = w == 1 ? (at == 2 ? -2.0 : -4.0) : at == 2 ? 1.0 : (w == 0) == (at == 0) ? 8.0 / 3.0 : 4.0 / 3.0;
-            wst[dim][at][w] = wv / (dim == 0 ? hx * hx : hy * hy);
-        } else if (threadIdx.x >= 32 && threadIdx.x < 38) {
-            const int dim = (threadIdx.x - 32) / 3, w = (threadIdx.x - 32) % 3;
-            wdn[dim][w] = (w == 0 ? 8.0 / 3.0 : w == 1 ? -3.0 : 1.0 / 3.0) / (dim == 0 ? hx : hy);
+        if (threadIdx.x < 8) {
+            const int dim = threadIdx.x >> 2, w = threadIdx.x & 3;
+            const double h = dim == 0 ? hx : hy;
+            wt[dim][w] = (w == 0 ? 1.0 : w == 1 ? 4.0 / 3.0 : w == 2 ? 1.0 / 3.0 : -3.0) / (w < 2 ? h * h : h);
         }
         if (bufs == 2) cp_async_wait<1>();     // this leaf's u
         else cp_async_wait<0>();
@@ -124,12 +124,15 @@ __global__ void __launch_bounds__(RES_THREADS) fd_residual_kernel(RefineGeom g, 
                 // x then y, each the [w0, w1, w2] stencil of FD_matrix_row (fd_module.f90:150-181)
                 for (int dim = 0; dim < 2; ++dim) {
                     const int gg = dim == 0 ? gi : gj, len = dim == 0 ? a : b;
-                    const double* w = wst[dim][gg == 1 ? 0 : gg == len ? 1 : 2];
+                    const double* w = wt[dim];
+                    const double w0 = gg == 1 ? 2.0 * w[1] : gg == len ? w[1] : w[0];
+                    const double w1 = (gg == 1 || gg == len ? -4.0 : -2.0) * w[0];
+                    const double w2 = gg == 1 ? w[1] : gg == len ? 2.0 * w[1] : w[0];
                     const int eu = dim == 0 ? leaf_lin(gi + 1, gj, a, b) : leaf_lin(gi, gj + 1, a, b);
                     const int ed = dim == 0 ? leaf_lin(gi - 1, gj, a, b) : leaf_lin(gi, gj - 1, a, b);
-                    acc = zadd(acc, zscale(w[1], ush[e]));
-                    acc = zadd(acc, zscale(w[2], ush[eu]));
-                    acc = zadd(acc, zscale(w[0], ush[ed]));
+                    acc = zadd(acc, zscale(w1, ush[e]));
+                    acc = zadd(acc, zscale(w2, ush[eu]));
+                    acc = zadd(acc, zscale(w0, ush[ed]));
                 }
                 z* fp = f + ((long long)rhs * g.nleaves + leaf) * ab + q;
                 const z r = zsub(*fp, acc);
@@ -138,7 +141,7 @@ __global__ void __launch_bounds__(RES_THREADS) fd_residual_kernel(RefineGeom g, 
             } else {
                 int e1, e2, axis;
                 leaf_bnd(e, a, b, e1, e2, axis);
-                const z dn = dn_u(ush, e, e1, e2, wdn[axis]);
+                const z dn = dn_u(ush, e, e1, e2, wt[axis][2], wt[axis][3]);
                 const z gin = zadd(zmul(ikb, ush[e]), dn);
                 const int cls = bclass[(long long)leaf * nb + e];
                 z r;
@@ -155,10 +158,9 @@ __global__ void __launch_bounds__(RES_THREADS) fd_residual_kernel(RefineGeom g, 
                     const double hn2 = ax2 == 0 ? hh[2 * lj] : hh[2 * lj + 1];
                     z dn2;
                     if (hn2 == (ax2 == 0 ? hx : hy)) {
-                        dn2 = dn_u(un, rj, f1, f2, wdn[ax2]);
+                        dn2 = dn_u(un, rj, f1, f2, wt[ax2][2], wt[ax2][3]);
                     } else {
-                        const double w2[3] = {(8.0 / 3.0) / hn2, -3.0 / hn2, (1.0 / 3.0) / hn2};
-                        dn2 = dn_u(un, rj, f1, f2, w2);
+                        dn2 = dn_u(un, rj, f1, f2, (1.0 / 3.0) / hn2, -3.0 / hn2);
                     }
                     const z gin2 = zadd(zmul(ikb, un[rj]), dn2);
                     const z hout = zadd(zmul(mikb, ush[e]), dn);
@@ -171,7 +173,7 @@ __global__ void __launch_bounds__(RES_THREADS) fd_residual_kernel(RefineGeom g, 
                 mx = fmax(mx, fabs(r.x) + fabs(r.y));
             }
         }
-        __syncthreads();                       // this leaf's reads of ush, wst and wdn are done
+        __syncthreads();                       // this leaf's reads of ush and wt are done
     }
     // max over the CTA, then over CTAs
     for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
@@ -231,11 +233,10 @@ cudaError_t fd_residual(const RefineGeom& g, int nrhs, const z* d, z* f, z* groo
     // both buffers while four CTAs still fit an SM
     const int bufs = 2 * (size_t)n * sizeof(z) <= 56 * 1024 ? 2 : 1;
     const size_t sh = bufs * (size_t)n * sizeof(z);
-    if (sh > 48 * 1024) {
-        static DeviceAttrCache attr;
-        cudaError_t e = ensure_smem_attr(fd_residual_kernel, sh, attr);
-        if (e != cudaSuccess) return e;
-    }
+    // the 48 KB that need no opt-in hold the kernel's static shared memory too: always opt in
+    static DeviceAttrCache attr;
+    cudaError_t e = ensure_smem_attr(fd_residual_kernel, sh, attr);
+    if (e != cudaSuccess) return e;
     fd_residual_kernel<<<dim3((g.nleaves + RES_LEAVES - 1) / RES_LEAVES, nrhs), RES_THREADS, sh, s>>>(
         g, d, f, groot, ri, kv, hh, bclass, first ? 1 : 0, bufs, rnorm);
     note_launch();
