@@ -4,7 +4,9 @@
 // and applies D and S through their LU factors.  Here every dense inverse the factor/solve
 // needs (the leaf's interior Schur complement, D and S of each merge) is formed explicitly by
 // Gauss-Jordan elimination with partial pivoting, so that later applications are GEMMs.
-// Pivots are chosen as LAPACK's izamax does: largest |re|+|im| in the column, first on ties.
+// Pivots are ranked as LAPACK's izamax does, by |re|+|im| in all its bits.  Exactly equal ones go to the row
+// that stands first: in the matrix as given where rows stay in place, after the exchanges so far in the
+// blocked path.
 //
 // m <= 64: the whole matrix in the registers of a warp (m <= 16) or a CTA (rb_pivot.cuh).
 // m  > 64: blocked Gauss-Jordan by panels of nb = 8 columns.  Per panel:

@@ -9,9 +9,10 @@
 //     A(i,:) = A(i,:) - (A(i,k) x) A(p,:),  A(i,k) = -A(i,k) x     (i != p)
 //     A(p,:) = x A(p,:),                    A(p,k) = x,
 // and after the last step inv(A)(k, p_q) = A(p_k, q).
-// The pivot is the row not yet used with the largest |re|+|im|, compared in its leading 15 (m <= 32)
-// or 14 bits so that value and row travel in one 32-bit warp reduction; equal ones go to the smaller
-// row.  The growth of a step is bounded as with the exact maximum, up to that rounding.
+// The pivot is the row not yet used with the largest |re|+|im|; equal ones go to the smaller row.  The
+// leading 15 (m <= 32) or 14 bits of the value and the row travel in one 32-bit warp reduction, and only
+// where two rows share the largest such bits are their values compared whole (PivotPick; the step of
+// 64^2 461 us without that, 465 with).
 // Measured (launch included): m = 16: 6.8 us (21 with the matrix in shared memory and five block
 // barriers a step), m = 32: 17 (53), m = 64: 56 (74 over several CTAs).
 // With two rows per lane (m > 32) the columns rotate by one register with each step, so that the
@@ -24,12 +25,34 @@ namespace rb {
 
 constexpr int PV_CG = 8;         // columns a thread holds
 
-// BITS: width of the row index
+// The row of a warp's largest magnitude, ties to the smaller row, in two parts: what follows from the leading
+// bits, and, where those tie, from the whole values.  BITS: width of the row index.  The bits of a
+// non-negative double order like its value.
 template <int BITS>
-__device__ __forceinline__ unsigned pivot_key(z x, bool valid, int r) {
-    const unsigned hi = (unsigned)__double2hiint(zabs1(x)) >> BITS;
-    return valid ? ((hi + 1u) << BITS) | (unsigned)((1 << BITS) - 1 - r) : 0u;
-}
+struct PivotPick {
+    double mag;
+    int r;
+    unsigned key, best;
+    // mag, r: this lane's candidate, if it has one (valid)
+    __device__ __forceinline__ PivotPick(double mag_, bool valid, int r_) : mag(mag_), r(r_) {
+        key = valid ? ((((unsigned)__double2hiint(mag) >> BITS) + 1u) << BITS) | (unsigned)((1 << BITS) - 1 - r) : 0u;
+        best = __reduce_max_sync(0xffffffffu, key);
+    }
+    __device__ __forceinline__ int row() const { return (1 << BITS) - 1 - (int)(best & ((1u << BITS) - 1)); }
+    __device__ __forceinline__ bool leads() const { return (key >> BITS) == (best >> BITS); }
+    __device__ __forceinline__ bool tied() const {
+        const unsigned t = __ballot_sync(0xffffffffu, leads());
+        return (t & (t - 1)) != 0;
+    }
+    __device__ __forceinline__ int exact_row() const {
+        bool in = leads();
+        const unsigned hi = (unsigned)__double2hiint(mag), lo = (unsigned)__double2loint(mag);
+        const unsigned mh = __reduce_max_sync(0xffffffffu, in ? hi : 0u);
+        in = in && hi == mh;
+        const unsigned ml = __reduce_max_sync(0xffffffffu, in ? lo : 0u);
+        return (int)__reduce_min_sync(0xffffffffu, in && lo == ml ? (unsigned)r : 0xffffffffu);
+    }
+};
 
 __device__ __forceinline__ z shfl_z(z v, int src) {
     return zmk(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src));
@@ -59,18 +82,24 @@ __device__ __forceinline__ bool warp_invert16(z (&v)[PV_CG], int m, z* prow, int
             const int k = grp * PV_CG + e;
             if (k >= m) break;
             const bool mine = hf == grp;
-            const unsigned key = __reduce_max_sync(0xffffffffu, pivot_key<5>(v[e], mine && !used, r));
+            const PivotPick<5> pick(zabs1(v[e]), mine && !used, r);
             const z f = shfl_z(v[e], r + 16 * grp);
-            const int p = 31 - (int)(key & 31u);
+            int p = pick.row();
+            const bool tied = pick.tied();
+            z pv, x;
+            for (bool again = tied;; again = false) {  // looked at behind the reciprocal, where it is free
+                pv = shfl_z(v[e], p + 16 * grp);
+                x = zrcp(pv);
+                if (!again) break;
+                p = pick.exact_row();
+            }
             const bool is_p = r == p;
             z* pr = prow + (k & 1) * 16 + hf * PV_CG;
-            const z pv = shfl_z(v[e], p + 16 * grp);
             if (is_p) {
 #pragma unroll
                 for (int c = 0; c < PV_CG; ++c) pr[c] = v[c];
             }
             if (pv.x == 0.0 && pv.y == 0.0) ok = false;
-            const z x = zrcp(pv);
             const z mult = is_p ? zneg(x) : zmul(f, x);
             if (is_p) { used = true; myk = k; }
             if (lane == k) pk = p;
@@ -111,21 +140,38 @@ __device__ __forceinline__ bool cta_invert(z (&v)[RPL][PV_CG], int m, PivotShare
     // finds and publishes the pivot of column k, this warp's register column c
     auto publish = [&](int c, int k) {
         const int s = k & 1;
-        unsigned key = 0;
-#pragma unroll
-        for (int i = 0; i < RPL; ++i) key = max(key, pivot_key<BITS>(v[i][c], !used[i], lane + 32 * i));
-        key = __reduce_max_sync(0xffffffffu, key);
-        const int p = (1 << BITS) - 1 - (int)(key & ((1u << BITS) - 1));
+        double mag = 0.0;
+        int row = -1;
 #pragma unroll
         for (int i = 0; i < RPL; ++i) {
-            sh.fcol[s][lane + 32 * i] = v[i][c];
-            if (lane + 32 * i == p) {
-                sh.pinv[s] = zrcp(v[i][c]);
-                sh.piv[s] = p;
-                sh.pk[k] = p;
-                if (v[i][c].x == 0.0 && v[i][c].y == 0.0) ok = false;
+            const double a = zabs1(v[i][c]);
+            if (!used[i] && (row < 0 || a > mag)) {
+                mag = a;
+                row = lane + 32 * i;
             }
         }
+        const PivotPick<BITS> pick(mag, row >= 0, row);
+        const bool tied = pick.tied();
+        bool zero = false;
+        auto put = [&](int p) {
+            zero = false;
+#pragma unroll
+            for (int i = 0; i < RPL; ++i)
+                if (lane + 32 * i == p) {
+                    sh.pinv[s] = zrcp(v[i][c]);
+                    sh.piv[s] = p;
+                    sh.pk[k] = p;
+                    zero = v[i][c].x == 0.0 && v[i][c].y == 0.0;
+                }
+        };
+#pragma unroll
+        for (int i = 0; i < RPL; ++i) sh.fcol[s][lane + 32 * i] = v[i][c];
+        put(pick.row());
+        if (tied) {                                    // looked at behind the reciprocal, where it is free
+            __syncwarp();
+            put(pick.exact_row());
+        }
+        if (zero) ok = false;
     };
     if (w == 0) publish(0, 0);
     constexpr int STEPS = RPL == 1 ? PV_CG : 1;      // steps per loop body; with 1 the columns rotate
