@@ -166,6 +166,9 @@ static GemmDesc gdesc(int m, int n, int k, ZView A, ZView B, ZOut D, z alpha) {
     return g;
 }
 
+// whether B1 = -A2 T1_iN reads T2_ii in place of A2 = zeta I - T2_ii
+static bool b1_from_map(const rb_tree* t) { return t->zeta.x == 0.0 && t->zeta.y == 0.0; }
+
 static ChildStore child_store(const rb_tree* t, int l) {   // storage of level l+1's RtR
     const Plan& P = t->P;
     ChildStore c;
@@ -456,15 +459,11 @@ static int ensure_factor_storage(rb_tree* t) {
                     g.C = zview(kv, m); g.beta = one;
                     mk.push_back(g);
                 }
-                {   // B1 = -A2 T1_iN = T2_ii T1_iN - zeta T1_iN, held in Y2's first n1 columns until Y2 is
-                    // formed: it reads the children's maps only, not A2
-                    GemmDesc g = gdesc(m, n1, m, zview(r2 + o2 + (long long)o2 * ld, ld), t1in, zout(y2, m), one);
-                    if (t->zeta.x != 0.0 || t->zeta.y != 0.0) {
-                        g.C = t1in;
-                        g.beta = zneg(t->zeta);
-                    }
-                    m1.push_back(g);
-                }
+                // B1 = -A2 T1_iN, held in Y2's first n1 columns until Y2 is formed.  With zeta = 0, -A2 is T2_ii
+                // as it stands in the child's map, and B1 need not wait for A2 (b1_from_map); otherwise the
+                // difference is taken before the product, as in K.
+                m1.push_back(b1_from_map(t) ? gdesc(m, n1, m, zview(r2 + o2 + (long long)o2 * ld, ld), t1in, zout(y2, m), one)
+                                            : gdesc(m, n1, m, zview(dv, m), t1in, zout(y2, m), mone));
                 // Y1 = [K^-1 B1, nu K^-1 T2_iN]
                 m2.push_back(gdesc(m, n1, m, zview(kv, m), zview(y2, m), zout(y1, m), one));
                 m2.push_back(gdesc(m, n2, m, zview(kv, m), t2in, zout(y1 + (long long)m * n1, m), t->nu));
@@ -837,15 +836,23 @@ static int run_merges_pipelined(rb_tree* t, const std::vector<cudaEvent_t>* rec,
         const PlanLevel& p = P.lv[l];
         const ChildStore cs = child_store(t, l);
         RB_CK(cudaStreamWaitEvent(c, t->ev_face[l + 1], 0));
-        if (!small_columns(t, l)) {
-            RB_CK(cudaStreamWaitEvent(s4, t->ev_face[l + 1], 0));
-            RB_LAUNCH(launch_gemm_level(t, t->fM1[l], l, s4));      // B1 = -A2 T1_iN
+        // B1 = -A2 T1_iN beside the rest, from the event on after which its operands are there
+        auto launch_b1 = [&](cudaEvent_t after) -> int {
+            RB_CK(cudaStreamWaitEvent(s4, after, 0));
+            RB_LAUNCH(launch_gemm_level(t, t->fM1[l], l, s4));
             RB_CK(cudaEventRecord(t->ev_m1[l], s4));
-        }
+            return RB_OK;
+        };
+        const bool b1 = !small_columns(t, l), early = b1_from_map(t);
+        if (b1 && early && (rc = launch_b1(t->ev_face[l + 1]))) return rc;
         if (small_merge(t, l)) {
             // too little work to split the map: the whole level on the chain stream
             const MergeSmall g = small_merge_args(t, l);
             RB_LAUNCH(merge_small_interface(g, t->d_status, c));
+            if (b1 && !early) {
+                RB_CK(cudaEventRecord(t->ev_fork[l], c));
+                if ((rc = launch_b1(t->ev_fork[l]))) return rc;
+            }
             if (rec && l == 0) RB_CK(cudaEventRecord(t->ev_root_forms, c));
             if (rec) RB_CK(cudaEventRecord((*rec)[l], c));
             if (!small_columns(t, l)) RB_CK(cudaStreamWaitEvent(c, t->ev_m1[l], 0));
@@ -873,6 +880,10 @@ static int run_merges_pipelined(rb_tree* t, const std::vector<cudaEvent_t>* rec,
         RB_LAUNCH(merge_form_kform_level(cs, p.nnodes, p.m, p.o1, p.o2, t->zeta, t->nu, t->dinv[l], t->sinv[l], t->kinv[l],
                                          c));
         if (rec && l == 0) RB_CK(cudaEventRecord(t->ev_root_forms, c));
+        if (!early) {
+            RB_CK(cudaEventRecord(t->ev_fork[l], c));
+            if ((rc = launch_b1(t->ev_fork[l]))) return rc;
+        }
         RB_LAUNCH(launch_gemm_level(t, t->fK[l], l, c));
         RB_LAUNCH(gj_invert_batch(t->gj_k[l].d_desc, p.nnodes, p.m, t->gj_work, t->d_status, c));
         // a solve's sweep at this level also waits for ev_rest[l + 1] (run_solve)
