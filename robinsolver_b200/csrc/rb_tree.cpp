@@ -615,42 +615,36 @@ static cudaError_t launch_gemm_level(rb_tree* t, const GemmBatch& b, int l, cuda
     return b.crt_ws ? launch_gemm_crt(b, t->d_status, s) : launch_gemm_batch(b, s);
 }
 
-// The FP64 products of levels whose interface has CRT_MIN_M points or more (k of every product of a
-// level) run on the residue engine.
-// Whole steps, FP64 tiles everywhere against this rule: 1024^2 27.3 to 22.2 ms, 512^2 (the root alone)
-// 6.0 to 5.7, 32^3 28.7 to 19.9.  At 256 points the passes over the operands and outputs cost what the
-// products save (768 x 768 x 256 in 32 problems 988 to 826 us, 256 x 768 in 16 190 to 236); a level's map,
-// whose products are the largest and share their operands, gains from m n = CRT_MIN_MN on (n: the outer
-// points of a child): 32^3 18.5 to 18.1 ms, a 768^2 step 12.6 to 12.3 (from m = 256 at any n: 1024^2 21.87 to 21.98).
+// The parent maps of FP64 levels with interfaces of CRT_MIN_M points or more, and m n of CRT_MIN_MN (n: the
+// outer points of a child), run on the residue engine: the largest products of a level, whose problems
+// share their operands, and the ones it serves at least as exactly as the FP64 tiles do.  A bound by the
+// largest entry of a row and of a column is weaker than the tiles' by |A| |B| where both are graded, so
+// that was measured on the operands themselves, against extended precision (the largest error relative to
+// (|A| |B|)_ij, tiles and residues): maps 2e-15 to 6e-15 and 1e-16 to 1e-15 in every one of 22 merges of
+// 1024^2, 768^2, 512^2, 32^3 and boxes between, and ten times less in the mean; but K = nu^2 I - A2 A1,
+// whose operands peak at the diagonal, 2e-15 to 4e-15 and 5e-15 to 9e-13, B1 and Y1, Y2 up to 5e-13 and 2e-14.
+// Those stay on the tiles.
+// At 256 points: 32^3 18.5 to 18.1 ms, a 768^2 step 12.6 to 12.3 (at any n: 1024^2 21.87 to 21.98).
 // The rule is one per level, so that the row sets of the pipelined factor and the whole map of the
-// serial one take the same engine: its sums are exact, and the two agree bit for bit.
-constexpr int CRT_MIN_M = 512, CRT_MIN_MAP_M = 256;
+// serial one take the same engine, whose result for an element depends on its row and column only: the
+// two agree bit for bit.
+constexpr int CRT_MIN_M = 256;
 constexpr long long CRT_MIN_MN = 1 << 18;
-enum { CRT_NO, CRT_MAP, CRT_ALL };
-static int crt_level(const rb_tree* t, int l) {
+static bool crt_level(const rb_tree* t, int l) {
     const PlanLevel& p = t->P.lv[l];
-    if (p.m > CRT_MAX_K) return CRT_NO;
-    if (p.m >= CRT_MIN_M) return CRT_ALL;
-    return p.m >= CRT_MIN_MAP_M && (long long)p.m * std::min(p.n1, p.n2) >= CRT_MIN_MN ? CRT_MAP : CRT_NO;
+    return p.m >= CRT_MIN_M && p.m <= CRT_MAX_K && (long long)p.m * std::min(p.n1, p.n2) >= CRT_MIN_MN;
 }
-// the batches of a level on the main stream (lane 0), the chain stream (1) and B1's (2); the serial
-// factor runs the first two on the main stream, one after another
+// a level's map on the main stream (lane 0: whole, or without the face rows) and on the chain stream (lane 1:
+// the face rows); the serial factor runs the whole one
+constexpr int CRT_LANES = 2;
 static std::vector<GemmBatch*> crt_stages(rb_tree* t, int l, int lane) {
+    if (!crt_level(t, l)) return {};
     const bool tail = l == 0 || !t->kform;
-    const int which = crt_level(t, l);
-    if (which == CRT_NO) return {};
-    if (which == CRT_MAP) {
-        if (lane == 0) return tail ? std::vector<GemmBatch*>{&t->fM4[l]} : std::vector<GemmBatch*>{&t->fM4[l], &t->fM4N[l]};
-        return lane == 1 && !tail ? std::vector<GemmBatch*>{&t->fM4F[l]} : std::vector<GemmBatch*>{};
-    }
-    if (lane == 2) return {&t->fM1[l]};
-    if (lane == 1) return tail ? std::vector<GemmBatch*>{&t->fK[l]}
-                               : std::vector<GemmBatch*>{&t->fK[l], &t->fM2[l], &t->fM3[l], &t->fM4F[l]};
-    return tail ? std::vector<GemmBatch*>{&t->fM2[l], &t->fM3[l], &t->fM4[l]}
-                : std::vector<GemmBatch*>{&t->fM4[l], &t->fM4N[l]};
+    if (lane == 0) return tail ? std::vector<GemmBatch*>{&t->fM4[l]} : std::vector<GemmBatch*>{&t->fM4[l], &t->fM4N[l]};
+    return tail ? std::vector<GemmBatch*>{} : std::vector<GemmBatch*>{&t->fM4F[l]};
 }
 // bytes of the lanes' workspaces, from the plan alone
-static size_t crt_lane_bytes(const rb_tree* t, size_t need[3]) {
+static size_t crt_lane_bytes(const rb_tree* t, size_t need[CRT_LANES]) {
     auto bytes = [](int count, int m, int n, int k) {
         GemmBatch b;
         b.count = count;
@@ -659,22 +653,16 @@ static size_t crt_lane_bytes(const rb_tree* t, size_t need[3]) {
         b.max_k = k;
         return crt_bytes(b);
     };
-    need[0] = need[1] = need[2] = 0;
+    need[0] = need[1] = 0;
     for (int l = 0; l < t->P.L; ++l) {
-        const int which = crt_level(t, l);
-        if (which == CRT_NO) continue;
+        if (!crt_level(t, l)) continue;
         const PlanLevel& p = t->P.lv[l];
         const int n = std::max(p.n1, p.n2), m = p.m, nn = p.nnodes;
-        const bool tail = l == 0 || !t->kform;
         if (!(l == 0 && t->skip_root)) need[0] = std::max(need[0], bytes(4 * nn, n, n, m));
         // the rows on the face the parent merges across: at most its interface's points
-        if (!tail) need[1] = std::max(need[1], bytes(4 * nn, std::min(n, t->P.lv[l - 1].m), n, m));
-        if (which == CRT_MAP) continue;
-        need[tail ? 0 : 1] = std::max(need[tail ? 0 : 1], bytes(2 * nn, m, n, m));
-        if (t->kform) need[1] = std::max(need[1], bytes(nn, m, m, m));
-        need[2] = std::max(need[2], bytes(nn, m, n, m));
+        if (l > 0 && t->kform) need[1] = std::max(need[1], bytes(4 * nn, std::min(n, t->P.lv[l - 1].m), n, m));
     }
-    return need[0] + need[1] + need[2];
+    return need[0] + need[1];
 }
 // One workspace per stream that runs such products (the streams of a factor run side by side, a
 // stream's products one after another).  They are a convenience: taken where they fit the handle's
@@ -683,19 +671,19 @@ static size_t crt_lane_bytes(const rb_tree* t, size_t need[3]) {
 static int ensure_crt_plan(rb_tree* t) {
     if (t->crt_state != rb_tree::CRT_NONE) return RB_OK;
     t->crt_state = rb_tree::CRT_OFF;
-    size_t need[3], fr = 0, all = 0;
+    size_t need[CRT_LANES], fr = 0, all = 0;
     const size_t total = crt_lane_bytes(t, need);
     if (total == 0) return RB_OK;
     RB_CK(cudaMemGetInfo(&fr, &all));
     if (total > fr / 16 || (t->budget > 0 && t->held + (int64_t)total > t->budget)) return RB_OK;
-    void* ws[3];
-    for (int lane = 0; lane < 3; ++lane)
+    void* ws[CRT_LANES];
+    for (int lane = 0; lane < CRT_LANES; ++lane)
         if (dev_alloc(t, t->crt_bufs, need[lane], &ws[lane]) != RB_OK) {
             free_list(t, t->crt_bufs);
             return RB_OK;
         }
     for (int l = 0; l < t->P.L; ++l)
-        for (int lane = 0; lane < 3; ++lane)
+        for (int lane = 0; lane < CRT_LANES; ++lane)
             for (GemmBatch* b : crt_stages(t, l, lane)) {
                 const size_t bytes = crt_bytes(*b);
                 if (bytes == 0 || bytes > need[lane]) continue;
@@ -712,7 +700,7 @@ static void drop_crt_plan(rb_tree* t) {
     drop_graph(t->gx_factor);
     t->factor_runs = 0;
     for (int l = 0; l < t->P.L; ++l)
-        for (int lane = 0; lane < 3; ++lane)
+        for (int lane = 0; lane < CRT_LANES; ++lane)
             for (GemmBatch* b : crt_stages(t, l, lane)) b->crt_ws = nullptr;
     free_list(t, t->crt_bufs);
 }
@@ -2304,7 +2292,7 @@ double tree_bytes_estimate(const rb_tree* t, int nrhs, int precision) {
 // device bytes of the residue engine's workspaces, and a tree that is to do without them (before its
 // first factorization)
 double tree_crt_bytes(const rb_tree* t) {
-    size_t need[3];
+    size_t need[CRT_LANES];
     return (double)crt_lane_bytes(t, need);
 }
 void tree_crt_off(rb_tree* t) {

@@ -1,0 +1,75 @@
+"""Which products of the FP64 factor run on the residue engine (run on a GPU), and what they are worth: parent
+maps only, as exact as the FP64 tiles by every measure on the factor's own operands."""
+import numpy as np
+import pytest
+
+from robinsolver_b200 import workloads as W
+from helpers import gpu_tree
+from test_gpu_tc5 import _run
+
+pytestmark = pytest.mark.gpu
+
+
+def _map_operands(T, level):
+    """[(name, A, B)] of the two row blocks of a level's first map, and its interface points: T_Ni and [Y1; Y2]
+    (K form, zeta = 0, nu = -1) formed on the host from the children's maps."""
+    a, b, _ = T._level_grid(level + 1)
+    r1, r2 = np.array(T.get_rtr(level + 1, 0)), np.array(T.get_rtr(level + 1, 1))
+    pa, pb, _ = T._level_grid(level)
+    off = np.cumsum([0, b, b, a, a])                      # faces x1 x2 y1 y2
+    f1, f2 = (1, 0) if pa > a else (3, 2)
+    i1, i2 = np.arange(off[f1], off[f1 + 1]), np.arange(off[f2], off[f2 + 1])
+    N1, N2 = np.setdiff1d(np.arange(off[4]), i1), np.setdiff1d(np.arange(off[4]), i2)
+    A1, A2 = -r1[np.ix_(i1, i1)], -r2[np.ix_(i2, i2)]
+    T1iN, T2iN = r1[np.ix_(i1, N1)], r2[np.ix_(i2, N2)]
+    Ki = np.linalg.inv(np.eye(len(i1)) - A2 @ A1)
+    Y1 = Ki @ np.concatenate([-A2 @ T1iN, -T2iN], 1)
+    Y2 = A1 @ Y1
+    Y2[:, :len(N1)] -= T1iN
+    return [("map1", r1[np.ix_(N1, i1)], Y1), ("map2", r2[np.ix_(N2, i2)], Y2)], len(i1)
+
+
+@pytest.mark.parametrize("N,L", [(512, 10), (768, 10)])
+def test_only_the_maps_run_on_the_residue_engine(N, L):
+    wl = W.make_workload(2, N=N, L=L, nrhs=1)
+    T, op, opts = gpu_tree(wl)
+    T.plan(L, op, opts)
+    k = wl.potential(T.sample_points(0))
+    T.factor_samples(k)
+    T.set_timing(2)
+    T.clear_stage_times()
+    T.factor_samples(k)
+    flops = sum(f for name, _, f in T.stage_times(with_flops=True) if name == "zgemm_crt")
+    want = 0.0
+    for l in range(L):
+        pa, pb, _ = T._level_grid(l)
+        a, b, _ = T._level_grid(l + 1)
+        m = b if pa > a else a
+        n = 2 * (a + b) - m
+        if m >= 256 and m * n >= 1 << 18:
+            want += 2 ** l * 4 * 8.0 * n * n * m
+    assert want > 0 and abs(flops - want) < 1e-9 * want, (flops, want)
+    T.close()
+
+
+@pytest.mark.parametrize("N,L", [(512, 10), (768, 10)])
+def test_map_products_are_as_exact_as_the_fp64_tiles(N, L):
+    """On a root's own operands, every element's error relative to (|A| |B|)_ij, largest and mean square, no
+    larger than the tiles', whose own is at most 8 2^-53 (k + 4) (three real products and their sum)."""
+    wl = W.make_workload(2, N=N, L=L, nrhs=1)
+    T, op, opts = gpu_tree(wl)
+    T.factor(L, op, opts)
+    rng = np.random.default_rng(N)
+    prods, m = _map_operands(T, 0)
+    T.close()
+    for name, A, B in prods:
+        A, B = np.ascontiguousarray(A), np.ascontiguousarray(B)
+        rows = np.sort(rng.choice(A.shape[0], 24, replace=False))
+        cols = np.sort(rng.choice(B.shape[1], 60, replace=False))
+        ref = A[rows].astype(np.clongdouble) @ B[:, cols].astype(np.clongdouble)
+        sab = np.abs(A[rows]) @ np.abs(B[:, cols])
+        C0 = np.zeros((1, A.shape[0], B.shape[1]), dtype=np.complex128)
+        e = {eng: np.abs(_run(eng, A[None], B[None], C0, 1.0 + 0j, 0j)[0][np.ix_(rows, cols)] - ref).astype(float) / sab
+             for eng in (0, 4)}
+        assert e[0].max() < 8 * 2.0 ** -53 * (m + 4)
+        assert e[4].max() <= e[0].max() and np.sqrt((e[4] ** 2).mean()) <= np.sqrt((e[0] ** 2).mean()), name
