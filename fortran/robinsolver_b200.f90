@@ -111,7 +111,7 @@ module robinsolver_b200
         real(c_double) :: h_last(3)
         integer(c_int64_t) :: n_interior, device_bytes
         integer(c_int32_t) :: factored, nrhs
-        integer(c_int32_t) :: d, leaf_c, root_c, reserved
+        integer(c_int32_t) :: d, leaf_c, root_c, residue_maps
     end type
 
     integer(c_int), parameter :: RB_POINTS_POTENTIAL = 0, RB_POINTS_SOURCE = 1, RB_POINTS_BOUNDARY = 2

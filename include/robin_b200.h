@@ -129,7 +129,8 @@ typedef struct rb_info {
     int32_t leaf_c, root_c;    /* grid in z of a leaf and of the whole domain (1 in 2D); in 3D
                                   leaf_nb = 2(bc + ac + ab), leaf_n = leaf_nb + abc, root_nb likewise,
                                   n_interior = nleaves * abc                                         */
-    int32_t reserved;
+    int32_t residue_maps;      /* 1: the last factorization formed its large FP64 maps on the int8 tensor
+                                  cores (see RB_PREC_FP64), 0: on the FP64 units                      */
 } rb_info;
 
 /* Builds the tree (robin_tree_factor's setup and bin_tree, robin_tree_module.f90:114-159):

@@ -91,7 +91,7 @@ class rb_info(C.Structure):
         ("d", C.c_int32),
         ("leaf_c", C.c_int32),
         ("root_c", C.c_int32),
-        ("reserved", C.c_int32),
+        ("residue_maps", C.c_int32),
     ]
 
 

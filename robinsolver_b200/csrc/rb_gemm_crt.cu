@@ -264,7 +264,7 @@ __global__ void __launch_bounds__(256, 3) crt_split_kernel(const GemmDesc* __res
 // them.  Above, B's blocks stream beside A's: a resident tile would leave room for two stages only
 // (k = 1024: 1014 us of products for 4 x 2048 x 2048, 829 streaming).  Every mbarrier wait is bounded; a CTA that gives up sets RB_TC5_TIMEOUT; in every
 // CTA the copies and MMAs it issued are waited for (bounded) before its tensor memory is freed and it returns.
-__global__ void __launch_bounds__(CRT_THREADS, 1) zgemm_crt_kernel(const GemmDesc* __restrict__ descs, int prob0, int* status,
+__global__ void __launch_bounds__(CRT_THREADS, 1) zgemm_crt_kernel(const GemmDesc* __restrict__ descs, int* status,
                                                                   const unsigned char* __restrict__ planes, int MT, int NT,
                                                                   int KB, long long a_bytes, unsigned char* __restrict__ out,
                                                                   int R, int per_group) {
@@ -278,7 +278,7 @@ __global__ void __launch_bounds__(CRT_THREADS, 1) zgemm_crt_kernel(const GemmDes
     const int runs = (MT + R - 1) / R;
     const int tn = blockIdx.x / runs, t0 = (blockIdx.x % runs) * R, t1 = min(tiles_m, t0 + R);
     if (tn >= tiles_n || t0 >= tiles_m) return;                  // the whole CTA
-    const long long prob = prob0 + (long long)blockIdx.y;
+    const long long prob = blockIdx.y;
     const int s0 = blockIdx.z * per_group, s1 = min(CRT_S, s0 + per_group);
     const int nk = max(1, (g.k + CRT_KB - 1) / CRT_KB);          // blocks of this problem (k = 0: one of zeros)
     const long long a_mod = (long long)KB * 2 * CRT_A_BLOCK, b_mod = (long long)KB * CRT_B_BLOCK;
@@ -315,7 +315,7 @@ __global__ void __launch_bounds__(CRT_THREADS, 1) zgemm_crt_kernel(const GemmDes
         // ---------------- producer, in the issuer's order ------------------------------------------------
         if (lane == 0) {
             bool ok = true;
-            const unsigned char* gA = planes + (long long)crt_a_owner(descs - prob0, (int)prob) * MT * CRT_S * a_mod;
+            const unsigned char* gA = planes + (long long)crt_a_owner(descs, (int)prob) * MT * CRT_S * a_mod;
             uint32_t q = 0;                          // stage
             int it = 0, nb = 0;                      // stages and resident B blocks issued
             uint32_t par = 1u;                       // parity of the A stage's previous release
@@ -465,11 +465,11 @@ __global__ void __launch_bounds__(CRT_THREADS, 1) zgemm_crt_kernel(const GemmDes
 
 // Outputs from their residues: a thread takes 4 columns of one row of a tile; two neighbours share the
 // 8 residues a row has in a column group.
-__global__ void __launch_bounds__(256, 4) crt_combine_kernel(const GemmDesc* __restrict__ descs, int prob0, int MT, int NT,
+__global__ void __launch_bounds__(256, 4) crt_combine_kernel(const GemmDesc* __restrict__ descs, int MT, int NT,
                                                           const unsigned char* __restrict__ out, const int* __restrict__ ea,
                                                           const int* __restrict__ fb) {
     const GemmDesc& g = descs[blockIdx.y];
-    const long long prob = prob0 + (long long)blockIdx.y;
+    const long long prob = blockIdx.y;
     const int tiles_m = max(1, (g.m + CRT_BM - 1) / CRT_BM);
     // blockIdx.x: column groups of a tile (tm fastest)
     const int c8 = blockIdx.x % (CRT_BN / 8), t = blockIdx.x / (CRT_BN / 8);
@@ -527,30 +527,38 @@ __global__ void __launch_bounds__(256, 4) crt_combine_kernel(const GemmDesc* __r
     }
 }
 
-size_t crt_bytes(const GemmBatch& b) {
+// problems a workspace of cap bytes takes at a time, 0 for a batch the engine does not take: all of them, or
+// an even number, so that the neighbours that share an A stay together, or one
+static int crt_part(const GemmBatch& b, size_t cap) {
     if (b.count == 0 || b.max_m == 0 || b.max_n == 0 || b.max_k == 0 || b.max_k > CRT_MAX_K) return 0;
-    // the split and combine grids take one block per slab and per column group
-    const CrtGeom g = crt_geom(b);
-    const long long slabs = (long long)b.count * g.KB * (g.MT * (CRT_BM / 16) + g.NT * (CRT_BN / 16));
+    GemmBatch c = b;
+    c.count = 1;
+    const CrtGeom g = crt_geom(c);
+    // the split and combine grids take one block per slab and per column group, the product's y a problem
+    const long long slabs = (long long)g.KB * (g.MT * (CRT_BM / 16) + g.NT * (CRT_BN / 16));
     if (slabs > INT_MAX || (long long)g.MT * g.NT * (CRT_BN / 8) > INT_MAX) return 0;
-    return (size_t)g.total;
+    const long long fit = std::min<long long>((long long)cap / g.total, std::min<long long>(INT_MAX / slabs, 65535));
+    if (fit >= b.count) return b.count;
+    return fit >= 2 ? (int)(fit / 2 * 2) : (int)fit;
+}
+size_t crt_bytes(const GemmBatch& b, size_t cap) {
+    GemmBatch c = b;
+    c.count = 1;
+    if (crt_part(c, SIZE_MAX / 2) == 0) return 0;
+    c.count = std::max(1, crt_part(b, cap));
+    return (size_t)crt_geom(c).total;
 }
 
-cudaError_t launch_gemm_crt(const GemmBatch& b, int* status, cudaStream_t s) {
-    if (b.count == 0 || b.max_m == 0 || b.max_n == 0) return cudaSuccess;
-    const size_t need = crt_bytes(b);
-    if (need == 0 || !status || !b.crt_ws || (reinterpret_cast<uintptr_t>(b.crt_ws) & 255) || need > b.crt_cap)
-        return cudaErrorInvalidValue;
-    static DeviceAttrCache attr;
-    cudaError_t e = ensure_smem_attr(zgemm_crt_kernel, CRT_SMEM, attr, true);
-    if (e != cudaSuccess) return e;
+// a sub-batch whose planes and residues fit the workspace
+static cudaError_t launch_crt_part(const GemmBatch& b, int* status, cudaStream_t s) {
     const CrtGeom cg = crt_geom(b);
     unsigned char* ws = static_cast<unsigned char*>(b.crt_ws);
     int* ea = reinterpret_cast<int*>(ws + cg.ea_off);
     int* fb = reinterpret_cast<int*>(ws + cg.fb_off);
     const long long nA = (long long)b.count * cg.MT * cg.KB * (CRT_BM / 16), nB = (long long)b.count * cg.NT * cg.KB * (CRT_BN / 16);
     const long long tiles = (long long)cg.MT * cg.NT;
-    if ((e = launch_operand_scales(b, cg.MT * CRT_BM, cg.NT * CRT_BN, ea, fb, s)) != cudaSuccess) return e;
+    cudaError_t e = launch_operand_scales(b, cg.MT * CRT_BM, cg.NT * CRT_BN, ea, fb, s);
+    if (e != cudaSuccess) return e;
     crt_split_kernel<<<(unsigned)(nA + nB), 256, 0, s>>>(b.d_desc, cg.MT, cg.NT, cg.KB, nA, ws, cg.a_bytes, ea, fb);
     note_launch();
     // runs of up to 8 row tiles per CTA (a resident B tile serves them all), and groups of moduli until there
@@ -558,16 +566,30 @@ cudaError_t launch_gemm_crt(const GemmBatch& b, int* status, cudaStream_t s) {
     const int R = std::min(cg.MT, 8), runs = (cg.MT + R - 1) / R;
     int groups = 1;
     while (groups < CRT_S && (long long)runs * cg.NT * b.count * groups < 6 * 148) groups *= 2;
-    for (int off = 0; off < b.count; off += 65535) {
-        const int cnt = std::min(b.count - off, 65535);
-        zgemm_crt_kernel<<<dim3((unsigned)(runs * cg.NT), cnt, groups), CRT_THREADS, CRT_SMEM, s>>>(
-            b.d_desc + off, off, status, ws, cg.MT, cg.NT, cg.KB, cg.a_bytes, ws + cg.c_off, R, CRT_S / groups);
-        note_launch();
-        crt_combine_kernel<<<dim3((unsigned)(tiles * (CRT_BN / 8)), cnt), 256, 0, s>>>(b.d_desc + off, off, cg.MT, cg.NT,
-                                                                                       ws + cg.c_off, ea, fb);
-        note_launch();
-    }
+    zgemm_crt_kernel<<<dim3((unsigned)(runs * cg.NT), b.count, groups), CRT_THREADS, CRT_SMEM, s>>>(
+        b.d_desc, status, ws, cg.MT, cg.NT, cg.KB, cg.a_bytes, ws + cg.c_off, R, CRT_S / groups);
+    note_launch();
+    crt_combine_kernel<<<dim3((unsigned)(tiles * (CRT_BN / 8)), b.count), 256, 0, s>>>(b.d_desc, cg.MT, cg.NT, ws + cg.c_off, ea,
+                                                                                      fb);
+    note_launch();
     return cudaGetLastError();
+}
+
+cudaError_t launch_gemm_crt(const GemmBatch& b, int* status, cudaStream_t s) {
+    if (b.count == 0 || b.max_m == 0 || b.max_n == 0) return cudaSuccess;
+    // as many problems at a time as the workspace holds; an element's result does not depend on it
+    const int part = crt_part(b, b.crt_cap);
+    if (part == 0 || !status || !b.crt_ws || (reinterpret_cast<uintptr_t>(b.crt_ws) & 255)) return cudaErrorInvalidValue;
+    static DeviceAttrCache attr;
+    cudaError_t e = ensure_smem_attr(zgemm_crt_kernel, CRT_SMEM, attr, true);
+    if (e != cudaSuccess) return e;
+    GemmBatch c = b;
+    for (int off = 0; off < b.count; off += part) {
+        c.count = std::min(part, b.count - off);
+        c.d_desc = b.d_desc + off;
+        if ((e = launch_crt_part(c, status, s)) != cudaSuccess) return e;
+    }
+    return cudaSuccess;
 }
 
 }  // namespace rb

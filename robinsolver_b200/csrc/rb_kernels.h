@@ -83,10 +83,11 @@ int tc5_tile_n(const GemmBatch& b);
 // largest real or imaginary part of the row or column below 1/2.
 cudaError_t launch_operand_scales(const GemmBatch& b, int rows, int cols, int* ea, int* fb, cudaStream_t s);
 // The same batch to FP64 accuracy on the int8 tensor cores (rb_gemm_crt.cu), for the FP64 factor's large
-// products; crt_bytes is the workspace it needs (b.crt_ws, 256-byte aligned), 0 for a batch it does
-// not take (k above CRT_MAX_K).
+// products, as many problems at a time as its workspace holds (b.crt_ws of b.crt_cap bytes, 256-byte
+// aligned).  crt_bytes: the workspace it makes use of within cap, or the one problem's that is its least;
+// 0 for a batch it does not take (k above CRT_MAX_K).
 constexpr int CRT_MAX_K = 1024;
-size_t crt_bytes(const GemmBatch& b);
+size_t crt_bytes(const GemmBatch& b, size_t cap);
 cudaError_t launch_gemm_crt(const GemmBatch& b, int* status, cudaStream_t s);
 // Bytes of operand planes launch_gemm_tc5 needs for this batch (b.t5_planes).
 size_t tc5_plane_bytes(const GemmBatch& b);

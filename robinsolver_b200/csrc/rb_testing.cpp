@@ -7,11 +7,13 @@
 //   engine 1: the tcgen05 kernel of the mixed-precision levels in split TF32
 //   engine 2: the tcgen05 kernel in int8 digit slices (the mixed-precision default)
 //   engine 3: the solve's fixed-order kernel
-//   engine 4: the residue (int8) engine of the FP64 factor's large products
+//   engine 4: the residue (int8) engine of the FP64 factor's maps
+//   engine 5: the same with a workspace for two problems, whatever their number
 // It allocates its descriptor array itself and synchronises; it returns 0, a negative RB_ERR_*
 // code for bad arguments or CUDA failures, or the device status word's bits (> 0) when a kernel
 // reported one.
 #include <algorithm>
+#include <cstdint>
 #include <string>
 #include <vector>
 
@@ -51,11 +53,17 @@ static int run_descs(int engine, const std::vector<GemmDesc>& h, int reps, doubl
         const long long w = gemm_plan_split(b);
         if (w > 0 && e == cudaSuccess) e = cudaMalloc(&b.work, sizeof(z) * (size_t)w);
     }
-    if (engine == 4) {
-        b.crt_cap = crt_bytes(b);
+    const bool crt = engine == 4 || engine == 5;
+    if (crt) {
+        GemmBatch two = b;
+        two.count = std::min(count, 2);
+        b.crt_cap = crt_bytes(engine == 5 ? two : b, SIZE_MAX / 2);
         if (e == cudaSuccess) e = b.crt_cap ? cudaMalloc(&b.crt_ws, b.crt_cap) : cudaErrorInvalidValue;
     }
-    auto run = [&]() { return engine == 4 ? launch_gemm_crt(b, d_status, 0) : engine == 1 || engine == 2 ? launch_gemm_tc5(b, d_status, 0) : launch_gemm_batch(b, 0); };
+    auto run = [&]() {
+        return crt ? launch_gemm_crt(b, d_status, 0)
+                   : engine == 1 || engine == 2 ? launch_gemm_tc5(b, d_status, 0) : launch_gemm_batch(b, 0);
+    };
     int rc = RB_OK;
     if (e == cudaSuccess) e = cudaMemcpy(b.d_desc, h.data(), sizeof(GemmDesc) * count, cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemset(d_status, 0, sizeof(int));

@@ -630,9 +630,14 @@ static cudaError_t launch_gemm_level(rb_tree* t, const GemmBatch& b, int l, cuda
 // two agree bit for bit.
 constexpr int CRT_MIN_M = 256;
 constexpr long long CRT_MIN_MN = 1 << 18;
+// The engine runs a batch in parts that fit its workspace: a lane's holds up to 1 GiB, or one problem's.  (All
+// of a batch at once took 1.6 GB at 1024^2 and 3 at 32^3 for the same step, 23.48 ms against 23.55 and 20.66
+// against 20.56; 512 MiB gives 23.89 and 20.58, 256 MiB 23.98 and 20.96.)
+constexpr size_t CRT_WS = size_t(1) << 30;
 static bool crt_level(const rb_tree* t, int l) {
     const PlanLevel& p = t->P.lv[l];
-    return p.m >= CRT_MIN_M && p.m <= CRT_MAX_K && (long long)p.m * std::min(p.n1, p.n2) >= CRT_MIN_MN;
+    return p.m >= CRT_MIN_M && p.m <= CRT_MAX_K && (long long)p.m * std::min(p.n1, p.n2) >= CRT_MIN_MN &&
+           !mixed_batch(t, t->fM4[l], l);
 }
 // a level's map on the main stream (lane 0: whole, or without the face rows) and on the chain stream (lane 1:
 // the face rows); the serial factor runs the whole one
@@ -643,7 +648,7 @@ static std::vector<GemmBatch*> crt_stages(rb_tree* t, int l, int lane) {
     if (lane == 0) return tail ? std::vector<GemmBatch*>{&t->fM4[l]} : std::vector<GemmBatch*>{&t->fM4[l], &t->fM4N[l]};
     return tail ? std::vector<GemmBatch*>{} : std::vector<GemmBatch*>{&t->fM4F[l]};
 }
-// bytes of the lanes' workspaces, from the plan alone
+// bytes of the lanes' workspaces, from the plan and the precision alone
 static size_t crt_lane_bytes(const rb_tree* t, size_t need[CRT_LANES]) {
     auto bytes = [](int count, int m, int n, int k) {
         GemmBatch b;
@@ -651,7 +656,7 @@ static size_t crt_lane_bytes(const rb_tree* t, size_t need[CRT_LANES]) {
         b.max_m = m;
         b.max_n = n;
         b.max_k = k;
-        return crt_bytes(b);
+        return crt_bytes(b, CRT_WS);
     };
     need[0] = need[1] = 0;
     for (int l = 0; l < t->P.L; ++l) {
@@ -664,45 +669,62 @@ static size_t crt_lane_bytes(const rb_tree* t, size_t need[CRT_LANES]) {
     }
     return need[0] + need[1];
 }
-// One workspace per stream that runs such products (the streams of a factor run side by side, a
-// stream's products one after another).  They are a convenience: taken where they fit the handle's
-// budget and a sixteenth of the device's free memory, given back when a later allocation of the
-// handle would fail (dev_alloc), and without them the FP64 tiles do the work.
-static int ensure_crt_plan(rb_tree* t) {
-    if (t->crt_state != rb_tree::CRT_NONE) return RB_OK;
-    t->crt_state = rb_tree::CRT_OFF;
-    size_t need[CRT_LANES], fr = 0, all = 0;
-    const size_t total = crt_lane_bytes(t, need);
-    if (total == 0) return RB_OK;
-    RB_CK(cudaMemGetInfo(&fr, &all));
-    if (total > fr / 16 || (t->budget > 0 && t->held + (int64_t)total > t->budget)) return RB_OK;
-    void* ws[CRT_LANES];
-    for (int lane = 0; lane < CRT_LANES; ++lane)
-        if (dev_alloc(t, t->crt_bufs, need[lane], &ws[lane]) != RB_OK) {
-            free_list(t, t->crt_bufs);
-            return RB_OK;
-        }
-    for (int l = 0; l < t->P.L; ++l)
-        for (int lane = 0; lane < CRT_LANES; ++lane)
-            for (GemmBatch* b : crt_stages(t, l, lane)) {
-                const size_t bytes = crt_bytes(*b);
-                if (bytes == 0 || bytes > need[lane]) continue;
-                b->crt_ws = ws[lane];
-                b->crt_cap = need[lane];
-            }
-    t->crt_state = rb_tree::CRT_HELD;
-    return RB_OK;
-}
 static void drop_crt_plan(rb_tree* t) {
     if (t->crt_state != rb_tree::CRT_HELD) return;
-    t->crt_state = rb_tree::CRT_OFF;
+    t->crt_state = rb_tree::CRT_NONE;
     cudaStreamSynchronize(t->stream);                 // every stream of a factor joins it
     drop_graph(t->gx_factor);
     t->factor_runs = 0;
     for (int l = 0; l < t->P.L; ++l)
-        for (int lane = 0; lane < CRT_LANES; ++lane)
-            for (GemmBatch* b : crt_stages(t, l, lane)) b->crt_ws = nullptr;
+        for (GemmBatch* b : {&t->fM4[l], &t->fM4F[l], &t->fM4N[l]}) b->crt_ws = nullptr;
     free_list(t, t->crt_bufs);
+}
+// One workspace per stream that runs such products (the streams of a factor run side by side, a
+// stream's products one after another), looked at by every factorization.  They are a convenience: taken
+// where they fit the handle's budget and half of the device's free memory (2 GiB of 180 GB at most: only a
+// full device decides otherwise), given back when a later allocation of the handle would fail (dev_alloc);
+// without them the FP64 tiles do the work, and the next factorization tries again.
+static int ensure_crt_plan(rb_tree* t) {
+    if (t->crt_state == rb_tree::CRT_OFF) return RB_OK;
+    size_t need[CRT_LANES], fr = 0, all = 0;
+    const size_t total = crt_lane_bytes(t, need);
+    if (t->crt_state == rb_tree::CRT_HELD) {
+        if (need[0] <= t->crt_held[0] && need[1] <= t->crt_held[1]) return RB_OK;
+        drop_crt_plan(t);                             // another precision's, smaller
+    }
+    if (total == 0 || (t->budget > 0 && t->held + (int64_t)total > t->budget)) return RB_OK;
+    RB_CK(cudaMemGetInfo(&fr, &all));
+    if (total > fr / 2) return RB_OK;
+    void* ws[CRT_LANES];
+    const std::string err = t->err;
+    for (int lane = 0; lane < CRT_LANES; ++lane)
+        if (dev_alloc(t, t->crt_bufs, need[lane], &ws[lane]) != RB_OK) {
+            free_list(t, t->crt_bufs);
+            t->err = err;                             // not a failure of the call
+            return RB_OK;
+        }
+    if (t->gx_factor) cudaStreamSynchronize(t->stream);
+    drop_graph(t->gx_factor);
+    t->factor_runs = 0;
+    for (int l = 0; l < t->P.L; ++l)
+        for (int lane = 0; lane < CRT_LANES; ++lane)
+            for (GemmBatch* b : crt_stages(t, l, lane)) {
+                const size_t bytes = crt_bytes(*b, need[lane]);
+                if (bytes == 0 || bytes > need[lane]) continue;
+                b->crt_ws = ws[lane];
+                b->crt_cap = need[lane];
+            }
+    t->crt_held[0] = need[0];
+    t->crt_held[1] = need[1];
+    t->crt_state = rb_tree::CRT_HELD;
+    return RB_OK;
+}
+// whether a factorization's maps run on the engine (all of them or none)
+static bool crt_in_use(const rb_tree* t) {
+    if (t->crt_state != rb_tree::CRT_HELD) return false;
+    for (int l = 0; l < t->P.L; ++l)
+        if (crt_level(t, l)) return true;
+    return false;
 }
 // The mixed solve applies its factor with the FP64 GEMMs: the sweeps' products are narrow (n =
 // the right-hand sides), where the tcgen05 tile is slower than the FP64 one (1024^2, L=12, 32
@@ -1693,7 +1715,7 @@ int rb_tree_info(const rb_tree* t, rb_info* info) {
     info->d = P.d;
     info->leaf_c = P.leaf_c();
     info->root_c = P.lv[0].c;
-    info->reserved = 0;
+    info->residue_maps = t->factored && t->residue_maps ? 1 : 0;
     info->device_bytes = t->held;
     info->factored = t->factored ? 1 : 0;
     info->nrhs = t->nrhs;
@@ -1899,6 +1921,7 @@ static int factor_common(rb_tree* t, const double* k, int precision, bool host, 
     }
     if (precision == RB_PREC_MIXED && (rc = ensure_mixed_factor_plan(t))) return rc;
     if ((rc = ensure_crt_plan(t))) return rc;
+    t->residue_maps = crt_in_use(t);
     if (t->timing == 1) {
         timers_collect(t);
         t->stage_ms.clear();
@@ -2260,6 +2283,7 @@ void tree_mark_factored(rb_tree* t, double f_time) {
     t->factored = true;
     t->factor_pending = false;
     t->factor_deferred = false;
+    t->residue_maps = false;
     t->nrhs = 0;
     if (t->prec != RB_PREC_FP64) {
         t->prec = RB_PREC_FP64;
@@ -2289,8 +2313,8 @@ double tree_bytes_estimate(const rb_tree* t, int nrhs, int precision) {
     if (precision == RB_PREC_MIXED) per_rhs += (double)Q.nleaves() * (Q.leaf_n() + Q.leaf_nb()) * 16.0;
     return need * 1.02 + per_rhs * nrhs + (64 << 20);
 }
-// device bytes of the residue engine's workspaces, and a tree that is to do without them (before its
-// first factorization)
+// device bytes of the residue engine's workspaces at their largest, and a tree that is to do without them
+// (before its first factorization)
 double tree_crt_bytes(const rb_tree* t) {
     size_t need[CRT_LANES];
     return (double)crt_lane_bytes(t, need);

@@ -174,9 +174,11 @@ struct rb_tree {
     int refine_cap = 0;
     bool mixed_plan = false;          // split-K plans and workspaces of the tcgen05 factor stages
     std::vector<DevBuf> mixed_bufs;
-    // workspaces of the residue GEMM engine (ensure_crt_plan): not tried yet, held, or done without
+    // workspaces of the residue GEMM engine (ensure_crt_plan): none now, held, or never to be held
     enum { CRT_NONE, CRT_HELD, CRT_OFF } crt_state = CRT_NONE;
     std::vector<DevBuf> crt_bufs;
+    size_t crt_held[2] = {0, 0};
+    bool residue_maps = false;        // the last factorization's maps ran on it
     z* dsol = nullptr;                // the correction of the current refinement step
     z* d_ri = nullptr;                // interface rows of the residual [rhs][leaf][nb]
     double* d_norms = nullptr;        // [0, k) max|r|, [k, 2k) max|x|, [2k, 3k) max|dx|
