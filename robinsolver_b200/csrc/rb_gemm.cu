@@ -243,10 +243,9 @@ static cudaError_t launch_cfg(const GemmBatch& b, cudaStream_t s) {
     constexpr int NT = (BM / TM) * (BN / TN);
     constexpr size_t SMEM = DfmaCfg<BM, BN, BK, STAGES>::SMEM_BYTES;
     static DeviceAttrCache attr;
-    if (SMEM > 48 * 1024) {
-        cudaError_t e = ensure_smem_attr(zgemm_desc_kernel<BM, BN, TM, TN, BK, STAGES, MINB>, SMEM, attr);
-        if (e != cudaSuccess) return e;
-    }
+    // the 48 KB that need no opt-in hold the descriptor's static shared memory too
+    cudaError_t e = ensure_smem_attr(zgemm_desc_kernel<BM, BN, TM, TN, BK, STAGES, MINB>, SMEM, attr);
+    if (e != cudaSuccess) return e;
     const int tiles = ((b.max_m + BM - 1) / BM) * ((b.max_n + BN - 1) / BN);
     for (int off = 0; off < b.count; off += 65535) {
         const int cnt = (b.count - off) < 65535 ? (b.count - off) : 65535;
@@ -262,10 +261,9 @@ static cudaError_t launch_split(const GemmBatch& b, cudaStream_t s) {
     constexpr int NT = (BM / TM) * (BN / TN);
     constexpr size_t SMEM = DfmaCfg<BM, BN, BK, STAGES>::SMEM_BYTES;
     static DeviceAttrCache attr;
-    if (SMEM > 48 * 1024) {
-        cudaError_t e = ensure_smem_attr(zgemm_split_kernel<BM, BN, TM, TN, BK, STAGES, MINB>, SMEM, attr);
-        if (e != cudaSuccess) return e;
-    }
+    // the 48 KB that need no opt-in hold the descriptor's static shared memory too
+    cudaError_t e = ensure_smem_attr(zgemm_split_kernel<BM, BN, TM, TN, BK, STAGES, MINB>, SMEM, attr);
+    if (e != cudaSuccess) return e;
     if (b.count > 65535 || b.ksplit > 65535) return cudaErrorInvalidValue;
     const int tiles = ((b.max_m + BM - 1) / BM) * ((b.max_n + BN - 1) / BN);
     zgemm_split_kernel<BM, BN, TM, TN, BK, STAGES, MINB><<<dim3(tiles, b.count, b.ksplit), NT, SMEM, s>>>(
