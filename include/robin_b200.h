@@ -47,16 +47,24 @@ extern "C" {
 #define RB_ERR_NO_SOLUTION   -11  /* get_solution before any solve, or irhs out of range              */
 
 /* ---- precision modes for rb_tree_factor ----------------------------------------------------- */
-#define RB_PREC_FP64  0           /* complex128 in, out and in every result; products of interfaces of
-                                     512 points and more are summed exactly on the int8 tensor cores
-                                     (operands as 57-bit integers of their row's or column's scale),
-                                     where device_budget and memory leave room for their workspaces  */
-#define RB_PREC_MIXED 1           /* merge levels l >= 2 with interfaces of >= 128 points: GEMMs on the
-                                     tcgen05 tensor cores in split TF32 (FP32 accumulation, ~1e-6
-                                     relative); the top two levels, the interface inverses, the leaves
-                                     and the FD residual in FP64; every solve refined against the FP64
+#define RB_PREC_FP64  0           /* complex128 in, out and in every result.  All operations in FP64 but
+                                     one kind of product, unless RB_FLAG_FP64_PRODUCTS is set: parent
+                                     maps T_NN + T_Ni Y of interfaces of m >= 256 points with n >= 2^18/m
+                                     outer points a child run on the int8 tensor cores, with operands
+                                     rounded to 2^-57 of the largest entry of their row (T_Ni) or column
+                                     (Y).  Their error is then bounded by these entries, at about 2^-56
+                                     per term, and not by |T_Ni| |Y| elementwise; on the maps of this
+                                     library's workloads it is a tenth of the FP64 products'.  They need
+                                     up to 2 GiB of workspaces; where device_budget or the device has no
+                                     room for them, FP64 products are used (rb_info.residue_maps)      */
+#define RB_PREC_MIXED 1           /* merge levels l >= 2 with interfaces of >= 256 points: B1, Y1, Y2 and
+                                     the maps on the int8 tensor cores in digit slices (~1e-11 relative;
+                                     RB_MIXED_ENGINE=tf32x3: split TF32 from 128 points, ~1e-6); the top
+                                     two levels (as RB_PREC_FP64), the interface inverses, the leaves and
+                                     the FD residual in FP64; every solve refined against the FP64
                                      residual of the global FD system to the tree's tolerance
-                                     (rb_tree_set_refinement, default 1e-10 relative)                  */
+                                     (rb_tree_set_refinement, default 1e-10 relative).  At 1024^2 a step
+                                     takes longer than RB_PREC_FP64's                                  */
 
 /* ---- sample-point kinds for rb_tree_sample_points ------------------------------------------- */
 #define RB_POINTS_POTENTIAL 0     /* interior cell centres where elliptic_operator%k is sampled       */
@@ -87,6 +95,8 @@ extern "C" {
                                      int8 tensor-core engine (~1e-11 of max|A| max|B| k); their
                                      interface inversions stay FP64.  Without it those levels are FP64,
                                      as the mixed-precision configuration prescribes.               */
+#define RB_FLAG_FP64_PRODUCTS 64  /* every FP64 product of the factorization on the FP64 units: an error bound
+                                     of |A| |B| elementwise, and the same bits whatever memory is free     */
 #define RB_FLAG_MERGE_DS      8   /* interface solve as the reference writes it, inv(D) and inv(S)
                                      (compute_RTR, robin_tree_module.f90:449-470), instead of the
                                      default single inversion of K = nu^2 I - (zeta I - T2_ii)(zeta I -

@@ -238,6 +238,8 @@ static bool use_dmma() {
     return v == 1;
 }
 
+bool gemm_on_tensor_cores() { return use_dmma(); }
+
 template <int BM, int BN, int TM, int TN, int BK, int STAGES, int MINB>
 static cudaError_t launch_cfg(const GemmBatch& b, cudaStream_t s) {
     constexpr int NT = (BM / TM) * (BN / TN);

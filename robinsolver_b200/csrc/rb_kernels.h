@@ -89,6 +89,8 @@ cudaError_t launch_operand_scales(const GemmBatch& b, int rows, int cols, int* e
 constexpr int CRT_MAX_K = 1024;
 size_t crt_bytes(const GemmBatch& b, size_t cap);
 cudaError_t launch_gemm_crt(const GemmBatch& b, int* status, cudaStream_t s);
+// false with RB_GEMM_ENGINE=dfma: every batched FP64 GEMM on the DFMA tiles, none on any tensor core
+bool gemm_on_tensor_cores();
 // Bytes of operand planes launch_gemm_tc5 needs for this batch (b.t5_planes).
 size_t tc5_plane_bytes(const GemmBatch& b);
 // Engines (tile shapes) of the FP64 launcher that can run a non-fixed-order batch, for the

@@ -637,7 +637,7 @@ constexpr size_t CRT_WS = size_t(1) << 30;
 static bool crt_level(const rb_tree* t, int l) {
     const PlanLevel& p = t->P.lv[l];
     return p.m >= CRT_MIN_M && p.m <= CRT_MAX_K && (long long)p.m * std::min(p.n1, p.n2) >= CRT_MIN_MN &&
-           !mixed_batch(t, t->fM4[l], l);
+           !mixed_batch(t, t->fM4[l], l) && !t->fp64_products && gemm_on_tensor_cores();
 }
 // a level's map on the main stream (lane 0: whole, or without the face rows) and on the chain stream (lane 1:
 // the face rows); the serial factor runs the whole one
@@ -648,7 +648,7 @@ static std::vector<GemmBatch*> crt_stages(rb_tree* t, int l, int lane) {
     if (lane == 0) return tail ? std::vector<GemmBatch*>{&t->fM4[l]} : std::vector<GemmBatch*>{&t->fM4[l], &t->fM4N[l]};
     return tail ? std::vector<GemmBatch*>{} : std::vector<GemmBatch*>{&t->fM4F[l]};
 }
-// bytes of the lanes' workspaces, from the plan and the precision alone
+// bytes of the lanes' workspaces, from the plan, the flags and the precision alone
 static size_t crt_lane_bytes(const rb_tree* t, size_t need[CRT_LANES]) {
     auto bytes = [](int count, int m, int n, int k) {
         GemmBatch b;
@@ -1637,6 +1637,7 @@ int rb_tree_create(const rb_geom* geom, rb_tree** out) {
     t->graphs = (geom->flags & RB_FLAG_NO_GRAPHS) == 0;
     t->async_factor = (geom->flags & RB_FLAG_ASYNC_FACTOR) != 0;
     t->mixed_int8_top = (geom->flags & RB_FLAG_MIXED_INT8_TOP) != 0;
+    t->fp64_products = (geom->flags & RB_FLAG_FP64_PRODUCTS) != 0;
     // refuse up front a problem the budget cannot hold (persistent factor storage only)
     if (t->budget > 0) {
         const Plan& Q = t->P;

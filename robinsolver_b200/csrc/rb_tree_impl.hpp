@@ -178,6 +178,7 @@ struct rb_tree {
     enum { CRT_NONE, CRT_HELD, CRT_OFF } crt_state = CRT_NONE;
     std::vector<DevBuf> crt_bufs;
     size_t crt_held[2] = {0, 0};
+    bool fp64_products = false;       // RB_FLAG_FP64_PRODUCTS: never
     bool residue_maps = false;        // the last factorization's maps ran on it
     z* dsol = nullptr;                // the correction of the current refinement step
     z* d_ri = nullptr;                // interface rows of the residual [rhs][leaf][nb]

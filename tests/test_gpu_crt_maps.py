@@ -73,3 +73,44 @@ def test_map_products_are_as_exact_as_the_fp64_tiles(N, L):
              for eng in (0, 4)}
         assert e[0].max() < 8 * 2.0 ** -53 * (m + 4)
         assert e[4].max() <= e[0].max() and np.sqrt((e[4] ** 2).mean()) <= np.sqrt((e[0] ** 2).mean()), name
+
+
+def _map_with(wl, factors=1, **kw):
+    T, op, opts = gpu_tree(wl, **kw)
+    T.plan(wl.L, op, opts)
+    k = wl.potential(T.sample_points(0))
+    for _ in range(factors):
+        T.factor_samples(k)
+    out = np.array(T.get_rtr(0, 0)), T.info().residue_maps, T.info().device_bytes
+    T.close()
+    return out
+
+
+def test_a_caller_can_keep_the_fp64_products():
+    """RB_FLAG_FP64_PRODUCTS: the bits of a tree whose budget has no room for the workspaces, and no workspaces
+    held; the default differs from them by rounding only."""
+    wl = W.make_workload(2, nrhs=1)
+    ref, on, held = _map_with(wl)
+    fp64, off, less = _map_with(wl, factors=3, fp64_products=True)
+    assert (on, off) == (1, 0) and less < held
+    tight, off2, _ = _map_with(wl, device_budget=less)
+    assert off2 == 0 and np.array_equal(fp64, tight)
+    assert not np.array_equal(ref, fp64) and np.abs(ref - fp64).max() < 1e-11 * np.abs(fp64).max()
+
+
+def test_the_dfma_engine_reaches_every_product():
+    """RB_GEMM_ENGINE=dfma (read once a process): no batched GEMM on any tensor core."""
+    import os
+    import subprocess
+    import sys
+    from pathlib import Path
+    root = Path(__file__).resolve().parents[1]
+    prog = ("import sys; sys.path[:0] = [r'%s', r'%s/tests']\n"
+            "from robinsolver_b200 import workloads as W\nfrom helpers import gpu_tree\n"
+            "wl = W.make_workload(2, nrhs=1)\nT, op, opts = gpu_tree(wl)\nT.plan(wl.L, op, opts)\n"
+            "k = wl.potential(T.sample_points(0))\nT.factor_samples(k)\nT.set_timing(2)\nT.clear_stage_times()\nT.factor_samples(k)\n"
+            "assert T.info().residue_maps == 0\n"
+            "names = {e[0] for e in T.stage_times()}\nassert not {n for n in names if 'crt' in n or 'tc' in n}, names\n" % (root, root))
+    r = subprocess.run([sys.executable, "-c", prog], env=dict(os.environ, RB_GEMM_ENGINE="dfma"), capture_output=True, text=True,
+                       timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
