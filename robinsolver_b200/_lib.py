@@ -179,6 +179,7 @@ def _load():
                                           C.c_double, C.c_double, C.c_double, C.c_int, C.c_int, D]),
         "rb_test_zgemm_descs": (C.c_int, [C.c_int, C.c_int, P]),
         # test hook of the batched Gauss-Jordan inversion (rb_testing.cpp)
+        "rb_test_gj_split": (C.c_int, [C.c_int, C.POINTER(C.c_int), C.c_int, C.POINTER(C.c_int)]),
         "rb_test_zinvert": (C.c_int, [C.c_int, C.c_int, P, C.c_longlong, C.c_longlong, C.c_int, D]),
     }
     for name, (res, args) in sig.items():

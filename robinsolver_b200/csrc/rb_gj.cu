@@ -651,6 +651,19 @@ static cudaError_t gj_blocked(const GJDesc* d, int count, int m, int* st, cudaSt
     return cudaGetLastError();
 }
 
+// slots[i]: matrices that are co-resident with i + 1 panels per CTA.  The fewest launches that take `count`
+// matrices, in equal parts of *chunk, and the fewest panels per CTA that hold one; 0 where not one does.
+int gj_resident_split(int count, const int* slots, int n, int* chunk) {
+    int most = 0;
+    for (int i = 0; i < n; ++i) most = std::max(most, slots[i]);
+    if (most == 0) return 0;
+    const int parts = (count + most - 1) / most;
+    *chunk = (count + parts - 1) / parts;
+    int i = 0;
+    while (slots[i] < *chunk) ++i;
+    return i + 1;
+}
+
 // Resident path: the fewest launches, then the fewest panels per CTA, whose grids are co-resident; false
 // when not even one matrix is (the caller then runs the blocked path).
 template <int NB, int MAXT, int RPT>
@@ -676,36 +689,38 @@ static cudaError_t gj_resident(const GJDesc* d, int count, int m, void* flags, i
     // Fewest panels per CTA: a CTA that owns more panels updates its others before it can
     // eliminate its next one, which lengthens the chain (1024^2, L=12: 25.5 ms factor with one
     // panel per CTA, 26.9 with at least two, 29.3 with at least six)
-    for (int parts = 1, chunk = count;; chunk = (count + ++parts - 1) / parts) {
-        for (int ppc = 1; ppc <= npanels; ++ppc) {
-            const int P = (npanels + ppc - 1) / ppc;
-            const size_t sh = (size_t)m * ppc * NB * sizeof(z) + (size_t)m * sizeof(int);
-            if (sh + sizeof(ResShared<NB>) > (size_t)SMEM_MAX) break;
-            int per_sm = 0;
-            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gj_resident_kernel<NB, MAXT, RPT>, threads, sh);
-            if (e != cudaSuccess) return e;
-            if ((long long)chunk * P > (long long)per_sm * nsm) continue;
-            if ((e = cudaMemsetAsync(flags, 0, (size_t)(count * gj_workspace_elems(m)) * sizeof(z), s)) != cudaSuccess) return e;
-            cudaLaunchConfig_t cfg = {};
-            cfg.blockDim = dim3((unsigned)threads);
-            cfg.dynamicSmemBytes = sh;
-            cfg.stream = s;
-            cudaLaunchAttribute la[1];
-            la[0].id = cudaLaunchAttributeCooperative;
-            la[0].val.cooperative = 1;
-            cfg.attrs = la;
-            cfg.numAttrs = 1;
-            for (int off = 0; off < count; off += chunk) {
-                cfg.gridDim = dim3((unsigned)(std::min(chunk, count - off) * P));
-                e = cudaLaunchKernelEx(&cfg, gj_resident_kernel<NB, MAXT, RPT>, d + off, m, npanels, ppc, P, st);
-                if (e != cudaSuccess) return e;
-                note_launch();
-            }
-            *done = true;
-            return cudaGetLastError();
-        }
-        if (chunk == 1 || (m > 512 && count > 3)) return cudaSuccess;
+    auto smem = [&](int ppc) { return (size_t)m * ppc * NB * sizeof(z) + (size_t)m * sizeof(int); };
+    int slots[GJ_MAX_PPC];                           // matrices co-resident with 1, 2, .. panels per CTA
+    int n = 0;
+    while (n < npanels && n < GJ_MAX_PPC && smem(n + 1) + sizeof(ResShared<NB>) <= (size_t)SMEM_MAX) {
+        int per_sm = 0;
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gj_resident_kernel<NB, MAXT, RPT>, threads, smem(n + 1));
+        if (e != cudaSuccess) return e;
+        slots[n] = (int)((long long)per_sm * nsm / ((npanels + n) / (n + 1)));
+        if (slots[n++] >= count) break;              // the whole batch: no need to look further
     }
+    int chunk = 0;
+    const int ppc = gj_resident_split(count, slots, n, &chunk);
+    if (ppc == 0 || (chunk < count && m > 512 && count > 3)) return cudaSuccess;
+    const int P = (npanels + ppc - 1) / ppc;
+    if ((e = cudaMemsetAsync(flags, 0, (size_t)(count * gj_workspace_elems(m)) * sizeof(z), s)) != cudaSuccess) return e;
+    cudaLaunchConfig_t cfg = {};
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = smem(ppc);
+    cfg.stream = s;
+    cudaLaunchAttribute la[1];
+    la[0].id = cudaLaunchAttributeCooperative;
+    la[0].val.cooperative = 1;
+    cfg.attrs = la;
+    cfg.numAttrs = 1;
+    for (int off = 0; off < count; off += chunk) {
+        cfg.gridDim = dim3((unsigned)(std::min(chunk, count - off) * P));
+        e = cudaLaunchKernelEx(&cfg, gj_resident_kernel<NB, MAXT, RPT>, d + off, m, npanels, ppc, P, st);
+        if (e != cudaSuccess) return e;
+        note_launch();
+    }
+    *done = true;
+    return cudaGetLastError();
 }
 
 // RB_GJ_RESIDENT=0 selects the blocked path (read at every launch, so that a process can compare)

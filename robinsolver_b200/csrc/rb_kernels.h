@@ -124,6 +124,8 @@ struct GJDesc {
 constexpr int GJ_SMALL_MAX = 64;       // largest matrix held whole in registers; above: resident (else blocked) path
 int gj_panel_width(int m);                         // nb of the blocked path (0 for the small path)
 long long gj_workspace_elems(int m);               // complex elements of Zb per matrix
+constexpr int GJ_MAX_PPC = 32;                     // panels of 8 columns a resident CTA can hold, and more
+int gj_resident_split(int count, const int* slots, int n, int* chunk);
 // work: the count descriptors' Zb areas, contiguous (count * gj_workspace_elems(m) elements)
 cudaError_t gj_invert_batch(const GJDesc* d_desc, int count, int m, void* work, int* d_status, cudaStream_t s);
 

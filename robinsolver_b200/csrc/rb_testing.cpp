@@ -151,6 +151,11 @@ extern "C" int rb_test_zgemm_descs(int engine, int count, const void* descs) {
     return run_descs(engine, std::vector<GemmDesc>(d, d + count), 0, nullptr);
 }
 
+// rb_test_gj_split: the resident inversion's choice of launches (host only): panels per CTA, 0 for none
+extern "C" int rb_test_gj_split(int count, const int* slots, int n, int* chunk) {
+    return gj_resident_split(count, slots, n, chunk);
+}
+
 // rb_test_zinvert inverts `count` complex m x m matrices in place (column-major, device pointers,
 // A_i = dA + i * stride, leading dimension ld) with the batched Gauss-Jordan kernels of the
 // factorization, `reps` times in a row (each call inverts the previous result), and writes the
