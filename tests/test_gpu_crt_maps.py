@@ -114,3 +114,36 @@ def test_the_dfma_engine_reaches_every_product():
     r = subprocess.run([sys.executable, "-c", prog], env=dict(os.environ, RB_GEMM_ENGINE="dfma"), capture_output=True, text=True,
                        timeout=300)
     assert r.returncode == 0, r.stderr[-2000:]
+
+
+# one split level (768^2) and two (1024^2), and the largest cube: the parts of a workspace, the rule of 256 points
+@pytest.mark.parametrize("case", ["768", "1024", "cube"])
+def test_pipelined_and_serial_maps_agree_bit_for_bit(case):
+    """The pipelined factor's face rows and other rows against the serial one's whole maps, on every level that
+    uses the engine, direct and from a graph."""
+    import robinsolver_b200 as rb
+    if case == "cube":
+        T = rb.robin_tree(skip_root_rtr=False)
+        T.bndry_params = np.array([[1j, 1.0], [-1j, 1.0]], dtype=np.complex128)
+        L = 9
+        T.plan(L, rb.elliptic_operator(d=3, domain=np.array([[0.0, 0.0, 0.0], [1.0, 1.0, 1.0]])), rb.solve_opts(h_tgt=1.0 / 32, kb=1.0))
+        X = T.sample_points(0)
+        k = 1.0 + 0.3 * np.exp(-((X - 0.4) ** 2).sum(1) / 0.02) + 0.01j
+    else:
+        wl = W.make_workload(2 if case == "768" else 4, N=int(case), L={"768": 10, "1024": 12}[case], nrhs=1)
+        T, op, opts = gpu_tree(wl)
+        T.plan(wl.L, op, opts)
+        k = wl.potential(T.sample_points(0))
+    nodes = [(0, 0), (1, 0), (1, 1), (2, 1), (2, 2)]
+    T.factor_samples(k)
+    assert T.info().residue_maps == 1
+    maps = [np.array(T.get_rtr(*v)) for v in nodes]
+    for _ in range(2):                                    # captured, replayed
+        T.factor_samples(k)
+    for v, a in zip(nodes, maps):
+        assert np.array_equal(np.array(T.get_rtr(*v)), a), v
+    T.set_timing(2)                                       # the serial schedule
+    T.factor_samples(k)
+    for v, a in zip(nodes, maps):
+        assert np.array_equal(np.array(T.get_rtr(*v)), a), v
+    T.close()

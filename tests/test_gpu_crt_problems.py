@@ -87,3 +87,94 @@ def test_a_problem_without_terms_beside_others():
         probs.append((A, B, D, D, 1.0 + 0j, 2.0 + 0j, m, n, k))
     for got, ref in zip(run(4, probs), refs):
         assert same(got, ref)
+
+
+@pytest.mark.parametrize("engine", [0, 4, 5])
+def test_maps_bands_and_uneven_problems(engine):
+    """What the parent maps are made of: rows by a map or around a skipped band, columns around a band, D
+    through row and column maps, C from a band of the same matrix, problems of different rows beside each
+    other, neighbours with one A -- all on one engine, on the FP64 tiles (0) and in parts (5) alike."""
+    rng = np.random.default_rng(7)
+    T = whole(rng, 420, 420)                                  # a child's map: interface rows and columns 100 .. 229
+    m, o = 130, 100
+    N = np.setdiff1d(np.arange(420), np.arange(o, o + m))
+    Y = whole(rng, m, 2 * len(N))
+    face, rest = N[::3], np.setdiff1d(N, N[::3])
+    probs, refs, n = [], [], len(N)
+    for rows in (face, rest):
+        for half in range(2):
+            A = Operand(T[:, o:o + m], rows=rows)
+            B = Operand(Y[:, half * n:(half + 1) * n])
+            D = Operand(np.zeros((900, 900), dtype=np.complex128), rows=rng.permutation(900)[:len(rows)], cols=rng.permutation(900)[:n])
+            Cm = Operand(T, rows=rows, cband=(o, m)) if half == 0 else None
+            ref = T[np.ix_(rows, np.arange(o, o + m))] @ B.M + (Cm.host(len(rows), n) if Cm else 0.0)
+            out = np.zeros((900, 900), dtype=np.complex128)
+            out[np.ix_(D.ix[0], D.ix[1])] = ref
+            refs.append(out)
+            probs.append((A, B, Cm, D, 1.0 + 0j, 1.0 + 0j, len(rows), n, m))
+    # and the whole map of the serial schedule: A and C around the band's rows
+    A = Operand(T[:, o:o + m], rband=(o, m))
+    D = Operand(np.zeros((n, n), dtype=np.complex128))
+    Cm = Operand(T, rband=(o, m), cband=(o, m))
+    refs.append(A.host(n, m) @ Y[:, :n] + Cm.host(n, n))
+    probs.append((A, Operand(Y[:, :n]), Cm, D, 1.0 + 0j, 1.0 + 0j, n, n, m))
+    for i, (got, ref) in enumerate(zip(run(engine, probs), refs)):
+        assert same(got, ref), i
+
+
+def test_a_map_in_row_sets_has_the_bits_of_the_whole():
+    """An element depends on its row and column only: the face rows and the others, of other problem sizes,
+    against the whole map, on operands of no special values."""
+    rng = np.random.default_rng(8)
+    cx = lambda *s: rng.standard_normal(s) + 1j * rng.standard_normal(s)  # noqa: E731
+    M, n, k = 700, 333, 576
+    T, Y, C0 = cx(M, k), cx(k, n), cx(M, n)
+    rows = [np.sort(rng.permutation(M)[:257])]
+    rows.append(np.setdiff1d(np.arange(M), rows[0]))
+
+    def problem(sel):
+        out = Operand(np.zeros((M, n), dtype=np.complex128), rows=sel)
+        return (Operand(T, rows=sel), Operand(Y), Operand(C0, rows=sel), out, 0.7 - 0.2j, -0.5 + 0.25j, len(sel), n, k)
+
+    full, = run(4, [problem(np.arange(M))])
+    a, b = run(4, [problem(r) for r in rows])
+    assert np.array_equal(a[rows[0]], full[rows[0]]) and np.array_equal(b[rows[1]], full[rows[1]])
+
+
+def _units(X, axis):
+    """The spacing that X's entries are rounded to: 2^-57 times a power of two above twice their row's or
+    column's largest part."""
+    big = np.maximum(np.abs(X.real), np.abs(X.imag)).max(axis=axis)
+    return 2.0 ** (np.frexp(big)[1] + 1 - 57)
+
+
+# k around the blocks of 128, up to and past the four of a resident B (512), blocks that do not fill the four stages
+@pytest.mark.parametrize("k", [1, 2, 31, 127, 128, 129, 513, 576, 640, 1000, 1024])
+@pytest.mark.parametrize("graded", [False, True])
+def test_error_is_the_rounding_of_the_operands(k, graded):
+    """Against extended precision, with one rounding of every entry to its row's or column's units ua, ub:
+    per part at most  sum_k ua/2 (|br| + |bi|) + ub/2 (|ar| + |ai|) + ua ub/2, the weights' cut, 2^53.4 ua ub, and a
+    rounding of the result at 2^-53; and in the mean square twice what uniform roundings give,
+    sum_k ua^2/12 |b|^2 + ub^2/12 |a|^2.  Neither has a factor of k for what does not grow with it.  Graded: entries
+    spread over 2^-40 .. 1 inside every row and column."""
+    from test_gpu_tc5 import _run
+    rng = np.random.default_rng(1000 * graded + k)
+    m, n = 173, 91
+    cx = lambda *s: rng.standard_normal(s) + 1j * rng.standard_normal(s)  # noqa: E731
+    A, B = cx(m, k), cx(k, n)
+    if graded:
+        A *= 2.0 ** -rng.uniform(0.0, 40.0, (m, k))
+        B *= 2.0 ** -rng.uniform(0.0, 40.0, (k, n))
+    got = _run(4, A[None], B[None], np.zeros((1, m, n), dtype=np.complex128), 1.0 + 0j, 0j)[0]
+    ref = A.astype(np.clongdouble) @ B.astype(np.clongdouble)
+    ua, ub = _units(A, 1)[:, None], _units(B, 0)[None, :]
+    sa, sb = (np.abs(A.real) + np.abs(A.imag)).sum(1)[:, None], (np.abs(B.real) + np.abs(B.imag)).sum(0)[None, :]
+    cut = 2.0 ** 53.4 * ua * ub
+    e = got - ref
+    for part, r in ((e.real, ref.real), (e.imag, ref.imag)):
+        bound = ua / 2 * sb + ub / 2 * sa + k * ua * ub / 2 + cut + 2.0 ** -53 * (np.abs(r) + cut)
+        assert np.all(np.abs(part) <= bound.astype(float)), float(np.max(np.abs(part) / bound))
+    sa2, sb2 = (np.abs(A) ** 2).sum(1)[:, None], (np.abs(B) ** 2).sum(0)[None, :]
+    mean = ua ** 2 / 12 * sb2 + ub ** 2 / 12 * sa2 + cut ** 2 + (2.0 ** -53 * np.abs(ref)).astype(float) ** 2 / 3
+    # relative to each element's own expectation, both parts together
+    assert np.sqrt((np.abs(e).astype(float) ** 2 / (2 * mean)).mean()) < 2.0
