@@ -41,6 +41,15 @@ __host__ __device__ __forceinline__ z zrcp(z a) {
 // |re| + |im|: the magnitude LAPACK's izamax ranks pivots by
 __host__ __device__ __forceinline__ double zabs1(z a) { return fabs(a.x) + fabs(a.y); }
 
+// the device's clock for bounded waits
+__device__ __forceinline__ unsigned long long global_ns() {
+    unsigned long long t = 0;
+#if defined(__CUDA_ARCH__)
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+#endif
+    return t;
+}
+
 // Programmatic dependent launch.  A kernel of a chain launched with it may begin while the kernel
 // before it in the stream still runs: pdl_wait() returns once that kernel has ended and its stores are
 // visible (at once in a kernel launched the usual way), and comes before every access to anything a

@@ -6,9 +6,10 @@
 // Robin-to-Robin matrix) and the scatter into the parent's face order happen inside the loads
 // and the epilogue instead of in copy kernels.
 //
-// FP64 has no tcgen05 kind: the large problems run on the FP64 tensor-core MMA
-// (mma.sync m8n8k4 .f64, rb_gemm_dmma.cuh), the small ones and the solve on DFMA register tiles
-// (rb_gemm_tile.cuh).
+// FP64 has no tcgen05 kind: problems above 16 x 16 and the solve run on the FP64 tensor-core MMA
+// (mma.sync m8n8k4 .f64, rb_gemm_dmma.cuh, rb_gemm_stream.cuh), smaller ones -- with RB_GEMM_ENGINE=dfma
+// all -- on DFMA register tiles (rb_gemm_tile.cuh).  The factor's largest maps run on the int8 tensor
+// cores instead (rb_gemm_crt.cu).
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>

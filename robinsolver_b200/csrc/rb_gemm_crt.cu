@@ -1,14 +1,19 @@
-// rb_gemm_crt.cu -- batched complex GEMM to FP64 accuracy on the int8 tensor cores: products modulo 16
-// coprime numbers, put together by the Chinese remainder theorem (the "Ozaki scheme II" of Ozaki,
+// rb_gemm_crt.cu -- batched complex GEMM on the int8 tensor cores, for the FP64 factor's large maps: products
+// modulo 16 coprime numbers, put together by the Chinese remainder theorem (the "Ozaki scheme II" of Ozaki,
 // Uchino and Imamura, arXiv:2504.08009, here for complex operands).
 //
 // FP64 tensor cores give 37 TFLOP/s of real products, the int8 ones about 45 times that.  Every row of
 // A and column of B is scaled by a power of two and rounded to integers of CRT_P = 57 bits (their largest
-// entry below 2^56): anything within 2^-4 of its row's largest entry exactly, every entry to 2^-57 of
-// it, where FP64 products and sums round at 2^-53.  The integers are reduced modulo 16 numbers up to
-// 256; the integer product, below 2^123, is known from its 16 residues, each an int8 product with
-// exact int32 accumulation.  So the whole sum over k is exact, and the result is rounded once.  Five
-// passes:
+// entry below 2^56).  The integers are reduced modulo 16 numbers up to 256; the integer product, below
+// 2^123, is known from its 16 residues, each an int8 product with exact int32 accumulation.
+// Errors: an entry within 2^-4 of its row's or column's largest is held exactly, a smaller one to 2^-57 of
+// that largest and so with fewer bits the smaller it is; the sum over k adds none; the weights that put
+// the residues together are cut at 2^44, which leaves the integer up to 2^53.4 off, about 2^-57 of the
+// product of the two largest entries; then one rounding of the result.  So an element is off by at most
+// about 2^-56 (amax_i sum_k |b_kj| + bmax_j sum_k |a_ik|), where a chain of FP64 products is off by some
+// 2^-53 sqrt(k) sum_k |a_ik| |b_kj|: less where the operands are even, more where both are graded along k.
+// Which products of the factor are the one and which the other was measured (crt_level, rb_tree.cpp).
+// Four passes:
 //  1. launch_operand_scales: the row and column exponents;
 //  2. crt_split_kernel: 16 residues of the real and imaginary parts, one byte each, laid out block by
 //     block as the product kernel's shared memory holds them (K-major, 128-byte swizzle);
@@ -20,7 +25,8 @@
 //     other half of tensor memory while eight warps read the accumulators, reduce them and write one
 //     byte per real output;
 //  4. crt_combine_kernel: the 16 residues of an output to its value, sum_s r_s w_s mod M with the
-//     weights in two parts of 41 bits (every sum exact in FP64), the scales, and the usual epilogue.
+//     cut weights in two parts of 41 bits (every sum of which is exact in FP64), the scales, and the usual
+//     epilogue.
 // Why N = 160: an MMA reads its operands from shared memory, and below N of about 128 that, not the
 // tensor pipe, is its time; two accumulator sets of 3 x 80 columns fill tensor memory.
 // A row or column that holds an infinity or a NaN gives NaN.

@@ -31,11 +31,6 @@
 
 namespace rb {
 
-int gj_panel_width(int m) {
-    if (m <= GJ_SMALL_MAX) return 0;
-    return 8;
-}
-
 // the resident path's two words per panel of 8 columns and its counter, in complex elements per matrix
 long long gj_workspace_elems(int m) { return m <= GJ_SMALL_MAX ? 0 : (m + 7) / 8 + 1; }
 
@@ -258,11 +253,6 @@ __global__ void __launch_bounds__(256) gj_apply_kernel(const GJDesc* __restrict_
 // that waits longer than GJ_WAIT_NS sets RB_STATUS_GJ_TIMEOUT in the status word and returns.
 constexpr unsigned long long GJ_WAIT_NS = 1000000000ull;
 
-__device__ __forceinline__ unsigned long long global_ns() {
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
 __device__ __forceinline__ int ld_acquire_gpu(const int* p) {
     int v;
     asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");

@@ -82,8 +82,8 @@ int tc5_tile_n(const GemmBatch& b);
 // Row exponents of every A (rows per problem, padded) and column exponents of every B: 2^-e brings the
 // largest real or imaginary part of the row or column below 1/2.
 cudaError_t launch_operand_scales(const GemmBatch& b, int rows, int cols, int* ea, int* fb, cudaStream_t s);
-// The same batch to FP64 accuracy on the int8 tensor cores (rb_gemm_crt.cu), for the FP64 factor's large
-// products, as many problems at a time as its workspace holds (b.crt_ws of b.crt_cap bytes, 256-byte
+// The same batch on the int8 tensor cores by residues (rb_gemm_crt.cu: operands rounded to 2^-57 of their
+// row's or column's largest entry), for the FP64 factor's large maps, as many problems at a time as its workspace holds (b.crt_ws of b.crt_cap bytes, 256-byte
 // aligned).  crt_bytes: the workspace it makes use of within cap, or the one problem's that is its least;
 // 0 for a batch it does not take (k above CRT_MAX_K).
 constexpr int CRT_MAX_K = 1024;
@@ -122,7 +122,6 @@ struct GJDesc {
     z* Zb;         // workspace: the resident path's flag words (gj_workspace_elems)
 };
 constexpr int GJ_SMALL_MAX = 64;       // largest matrix held whole in registers; above: resident (else blocked) path
-int gj_panel_width(int m);                         // nb of the blocked path (0 for the small path)
 long long gj_workspace_elems(int m);               // complex elements of Zb per matrix
 constexpr int GJ_MAX_PPC = 32;                     // panels of 8 columns a resident CTA can hold, and more
 int gj_resident_split(int count, const int* slots, int n, int* chunk);

@@ -640,7 +640,8 @@ cudaError_t leaf_block_factor(const LeafGeom& g, int nleaves, const double* h, c
                               int* status, cudaStream_t s) {
     const size_t sh = leaf_block_factor_smem(g);
     if (g.a <= 32) {
-        // leaf grids this library accepts: those of the one-CTA form below, and 16-cell blocks
+        // The leaf grids this library accepts stay those that fit the one-CTA form below, and all that are 16
+        // wide, although these kernels need less.
         if (g.a != 16 && sh > (size_t)227 * 1024) return cudaErrorInvalidValue;
         if (g.a <= 16) {
             const int wpc = nleaves >= 4 * 148 ? 4 : 1;

@@ -54,8 +54,8 @@ extern "C" int rb_leaf_rtr_noalloc(int a, int b, double kb, const double* d_h, c
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 128)
         return noalloc_fail(RB_ERR_CUDA, "rb_leaf_rtr_noalloc: no current CUDA device");
     if (a != 16) {
-        // leaves other than 16 wide run the one-CTA-per-leaf kernel, whose shared memory grows
-        // with a and nb: refuse a grid it cannot hold on this device
+        // the grids this library accepts are those whose one-CTA-per-leaf factor fits the device's
+        // shared memory, and all that are 16 wide; the kernels for widths up to 32 need less
         int optin = 0;
         if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess)
             return noalloc_fail(RB_ERR_CUDA, "rb_leaf_rtr_noalloc: cannot query the device's shared memory");
