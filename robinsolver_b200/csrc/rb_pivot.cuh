@@ -11,10 +11,10 @@
 // and after the last step inv(A)(k, p_q) = A(p_k, q).
 // The pivot is the row not yet used with the largest |re|+|im|; equal ones go to the smaller row.  The
 // leading 15 (m <= 32) or 14 bits of the value and the row travel in one 32-bit warp reduction, and only
-// where two rows share the largest such bits are their values compared whole (PivotPick; the step of
-// 64^2 461 us without that, 465 with).
+// where two rows share the largest such bits are their values compared whole (PivotPick; the factor
+// of 16 leaves of 16 x 16 120 us without that, 123 with).
 // Measured (launch included): m = 16: 6.8 us (21 with the matrix in shared memory and five block
-// barriers a step), m = 32: 17 (53), m = 64: 56 (74 over several CTAs).
+// barriers a step), m = 32: 17 (53), m = 64: 58 (74 over several CTAs).
 // With two rows per lane (m > 32) the columns rotate by one register with each step, so that the
 // step is one loop body: eight of them in a row, one per register, do not stay in the instruction
 // caches (m = 64: 87 us, 56 rotating; m = 32: 17, 21 rotating).

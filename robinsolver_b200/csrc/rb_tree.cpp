@@ -624,7 +624,9 @@ static cudaError_t launch_gemm_level(rb_tree* t, const GemmBatch& b, int l, cuda
 // 1024^2, 768^2, 512^2, 32^3 and boxes between, and ten times less in the mean; but K = nu^2 I - A2 A1,
 // whose operands peak at the diagonal, 2e-15 to 4e-15 and 5e-15 to 9e-13, B1 and Y1, Y2 up to 5e-13 and 2e-14.
 // Those stay on the tiles.
-// At 256 points: 32^3 18.5 to 18.1 ms, a 768^2 step 12.6 to 12.3 (at any n: 1024^2 21.87 to 21.98).
+// Steps on the tiles alone and with this rule: 512^2 5.66 to 5.46 ms, 768^2 (32 right-hand sides) 15.83 to 14.77,
+// 1024^2 26.59 to 23.59, 32^3 27.17 to 20.66; with interfaces of 512 points and more only, 768^2 15.10 and 32^3
+// 21.03.  Without the bound on m n the 256-point levels of 1024^2 lose what they gain (by 0.5%).
 // The rule is one per level, so that the row sets of the pipelined factor and the whole map of the
 // serial one take the same engine, whose result for an element depends on its row and column only: the
 // two agree bit for bit.
