@@ -599,16 +599,20 @@ static int mixed_stage_mask() {
     const char* v = std::getenv("RB_MIXED_STAGES");
     return v ? std::atoi(v) : 30;
 }
+constexpr int MIXED_K = 1, MIXED_B1 = 2, MIXED_Y1 = 4, MIXED_Y2 = 8, MIXED_MAP = 16;
+static bool mixed_stage(const rb_tree* t, int l, int bit) {
+    return mixed_level(t, l) && (l >= t->P.L || bit == 0 || (mixed_stage_mask() & bit) != 0);
+}
 static bool mixed_batch(const rb_tree* t, const GemmBatch& b, int l) {
     if (!mixed_level(t, l)) return false;
     if (l >= t->P.L) return true;
     int bit = 0;
-    if (&b == &t->fK[l]) bit = 1;
-    else if (&b == &t->fM1[l]) bit = 2;
-    else if (&b == &t->fM2[l]) bit = 4;
-    else if (&b == &t->fM3[l]) bit = 8;
-    else if (&b == &t->fM4[l] || &b == &t->fM4F[l] || &b == &t->fM4N[l]) bit = 16;
-    return bit == 0 || (mixed_stage_mask() & bit) != 0;
+    if (&b == &t->fK[l]) bit = MIXED_K;
+    else if (&b == &t->fM1[l]) bit = MIXED_B1;
+    else if (&b == &t->fM2[l]) bit = MIXED_Y1;
+    else if (&b == &t->fM3[l]) bit = MIXED_Y2;
+    else if (&b == &t->fM4[l] || &b == &t->fM4F[l] || &b == &t->fM4N[l]) bit = MIXED_MAP;
+    return mixed_stage(t, l, bit);
 }
 static cudaError_t launch_gemm_level(rb_tree* t, const GemmBatch& b, int l, cudaStream_t s) {
     if (mixed_batch(t, b, l)) return launch_gemm_tc5(b, t->d_status, s);
@@ -639,7 +643,7 @@ constexpr size_t CRT_WS = size_t(1) << 30;
 static bool crt_level(const rb_tree* t, int l) {
     const PlanLevel& p = t->P.lv[l];
     return p.m >= CRT_MIN_M && p.m <= CRT_MAX_K && (long long)p.m * std::min(p.n1, p.n2) >= CRT_MIN_MN &&
-           !mixed_batch(t, t->fM4[l], l) && !t->fp64_products && gemm_on_tensor_cores();
+           !mixed_stage(t, l, MIXED_MAP) && !t->fp64_products && gemm_on_tensor_cores();
 }
 // a level's map on the main stream (lane 0: whole, or without the face rows) and on the chain stream (lane 1:
 // the face rows); the serial factor runs the whole one
